@@ -29,6 +29,7 @@
 #include "xg_common.cuh"
 #include "xg_kernels.h"
 #include "xg_matern.cuh"
+#include "xg_potrf128.cuh"
 
 /* ========================================================================== */
 /* Matern tile generation                                                     */
@@ -1203,223 +1204,20 @@ static size_t xg_trsm_gemm_smem_bytes()
  *                            one 128 x 128 block per CTA, K = 128).
  * The inverted diagonal blocks of the whole L_kk land in T.dinv on the way, so
  * the panel TRSM that follows needs no separate inversion. */
-#define XG_SUB 128
-#define XG_P_NB 16                      /* panel width inside the sub-block */
-#define XG_P_LDS (XG_SUB + 4)           /* DMMA operand reads: g * 2 * 132 = 8 g (mod 32 banks), conflict-free */
-#define XG_P_LDW (XG_P_NB + 4)
-#define XG_P_ROWS (XG_SUB + XG_P_NB)    /* the sub-block and one more block row for the right-hand side */
-#define XG_POTRF_SUB_THREADS 256
-/* [144][132] sub-block + rhs row, [8][16][20] inverses, [4][16][20] scratch, two mbarriers */
-#define XG_POTRF_SUB_SMEM                                                                                              \
-    ((size_t)(XG_P_ROWS * XG_P_LDS + (XG_SUB / XG_P_NB + 4) * XG_P_NB * XG_P_LDW) * sizeof(double) + 16)
-
-/* Cholesky of a 16 x 16 block by one warp, with its inverse: lane r < 16 holds
- * row r of the block, lane 16 + r row r of the identity.  The right-looking
- * column operations that turn the block into L turn the identity rows into
- * L^-T in the same instructions.  The next pivot needs only its own lane's
- * entry of the column just scaled, so the chain per column is one broadcast,
- * one reciprocal square root and two dependent FMAs; the broadcasts of the
- * column's other entries hide behind it.  S (leading dimension XG_P_LDS)
- * receives L, zeros above the diagonal; W receives L^-T; returns the first
- * column (1-based) whose pivot is not positive, or 0, in every lane. */
-__device__ __forceinline__ int xg_chol16_warp(double *S, double *W, int lane)
-{
-    const int r = lane & 15;
-    const bool ident = lane >= 16;
-    double a[XG_P_NB];
-#pragma unroll
-    for (int c = 0; c < XG_P_NB; c += 2) {
-        const double2 v = *reinterpret_cast<const double2 *>(S + r * XG_P_LDS + c);
-        a[c] = ident ? (c == r ? 1.0 : 0.0) : (c <= r ? v.x : 0.0);
-        a[c + 1] = ident ? (c + 1 == r ? 1.0 : 0.0) : (c + 1 <= r ? v.y : 0.0);
-    }
-    int fail = 0;
-#pragma unroll
-    for (int j = 0; j < XG_P_NB; ++j) {
-        double d = __shfl_sync(0xffffffffu, a[j], j);
-        const bool bad = !(d > 0.0);
-        fail = bad && !fail ? j + 1 : fail;
-        d = bad ? 1.0 : d;
-        const double ri = rsqrt(d);
-        a[j] *= ri;
-#pragma unroll
-        for (int c = j + 1; c < XG_P_NB; ++c) {
-            const double lcj = __shfl_sync(0xffffffffu, a[j], c);
-            /* lane c updates its own diagonal entry from its own value */
-            a[c] = fma(-a[j], lcj, a[c]);
-        }
-        /* L_jj = d ri with one Newton correction of the square root */
-        if (lane == j) {
-            const double l = d * ri;
-            a[j] = fma(fma(-l, l, d), 0.5 * ri, l);
-        }
-    }
-    double *dst = ident ? W + r * XG_P_LDW : S + r * XG_P_LDS;
-#pragma unroll
-    for (int c = 0; c < XG_P_NB; c += 2) {
-        const bool k0 = ident ? c >= r : c <= r, k1 = ident ? c + 1 >= r : c + 1 <= r;
-        *reinterpret_cast<double2 *>(dst + c) = make_double2(k0 ? a[c] : 0.0, k1 ? a[c + 1] : 0.0);
-    }
-    return fail;
-}
-
-/* acc (16 x 16: two 16 x 8 DMMA tiles) += A B over K = 16 for one warp;
- * A(m, k) = a[m lda + k]; B(k, n) = b[k ldb + n] (BT false) or b[n ldb + k]
- * (BT true), all in shared memory. */
-template <bool BT>
-__device__ __forceinline__ void xg_mma16(double (&acc)[2][4], const double *a, int lda, const double *b, int ldb,
-                                         int g, int tq)
-{
-#pragma unroll
-    for (int k = 0; k < XG_P_NB; k += 4) {
-        const double a0 = a[g * lda + k + tq], a1 = a[(g + 8) * lda + k + tq];
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const double bv = BT ? b[(n * 8 + g) * ldb + k + tq] : b[(k + tq) * ldb + n * 8 + g];
-            xg_dmma_16x8x4(acc[n][0], acc[n][1], acc[n][2], acc[n][3], a0, a1, bv);
-        }
-    }
-}
-
-/* Block (i, j) of the sub-block: S_ij -= X_i X_j^T, X the panel starting at
- * column c0 (one warp) */
-__device__ __forceinline__ void xg_potrf_update16(double *S, int i, int j, int c0, int g, int tq)
-{
-    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-    xg_mma16<true>(acc, S + i * XG_P_NB * XG_P_LDS + c0, XG_P_LDS, S + j * XG_P_NB * XG_P_LDS + c0, XG_P_LDS, g, tq);
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            double2 *p = reinterpret_cast<double2 *>(S + (i * XG_P_NB + g + 8 * h) * XG_P_LDS + j * XG_P_NB + n * 8 +
-                                                     2 * tq);
-            double2 v = *p;
-            v.x -= acc[n][2 * h];
-            v.y -= acc[n][2 * h + 1];
-            *p = v;
-        }
-}
-
-/* Cholesky of the 128 x 128 block in S by one CTA of 256 threads, in eight
- * 16-wide panels; with rhs the block row below (row 128 of S, the other 15
- * rows zero) holds the right-hand side v^T and leaves as (L^-1 v)^T -- the
- * forward solve is the panel solve of one more row.  Per panel: warp 0
- * factors the diagonal block and inverts it (xg_chol16_warp); every warp
- * multiplies one block row by the inverse on DMMA; warp 0 then updates the
- * next diagonal block and factors it while the other warps update the rest,
- * so the serial chain is 8 x (16 pivots + two 16 x 16 products).  W[p] keeps
- * the inverses L_pp^-T.  Returns the first failing column (1-based) or 0 to
- * every thread; on return S and W are complete and visible to all.
- *
- * One SM, a latency chain of 128 pivots bounds it. */
-__device__ __forceinline__ int xg_potrf128(double *S, double *W, int rhs)
-{
-    __shared__ int s_fail;
-    constexpr int NP = XG_SUB / XG_P_NB;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, tq = lane & 3;
-    const int last = rhs ? NP : NP - 1; /* last block row */
-    if (tid == 0) s_fail = 0;
-#pragma unroll 1
-    for (int p = 0; p < NP; ++p) {
-        const int c0 = p * XG_P_NB;
-        double *Wp = W + p * XG_P_NB * XG_P_LDW;
-        if (warp == 0) {
-            const int f = xg_chol16_warp(S + c0 * XG_P_LDS + c0, Wp, lane);
-            if (f && lane == 0) s_fail = c0 + f;
-        }
-        __syncthreads();
-        if (s_fail) return s_fail;
-        for (int i = p + 1 + warp; i <= last; i += XG_POTRF_SUB_THREADS / 32) {
-            double *B = S + i * XG_P_NB * XG_P_LDS + c0;
-            double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-            xg_mma16<false>(acc, B, XG_P_LDS, Wp, XG_P_LDW, g, tq);
-            __syncwarp();
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    *reinterpret_cast<double2 *>(B + (g + 8 * h) * XG_P_LDS + n * 8 + 2 * tq) =
-                        make_double2(acc[n][2 * h], acc[n][2 * h + 1]);
-        }
-        __syncthreads();
-        if (p + 1 < NP) {
-            if (warp == 0) {
-                xg_potrf_update16(S, p + 1, p + 1, c0, g, tq);
-                __syncwarp();
-            } else if (warp != 4) { /* warp 4 shares warp 0's scheduler */
-                /* blocks (i, j), p < j <= i <= last (j < NP) but (p + 1, p + 1), round robin over six warps */
-                int q = warp < 4 ? warp - 1 : warp - 2;
-                for (int j = p + 1; j < NP; ++j)
-                    for (int i = j == p + 1 ? j + 1 : j; i <= last; ++i) {
-                        if (q == 0) xg_potrf_update16(S, i, j, c0, g, tq);
-                        q = q == 0 ? 5 : q - 1;
-                    }
-            }
-        }
-    }
-    return 0;
-}
-
-/* The inverses of the four 32 x 32 diagonal blocks of L from those of its
- * 16 x 16 ones (warps 0-3, one block each; scratch T: [4][16][20]):
- * [[D11, 0], [-D22 L21 D11, D22]], D = W^T, to dinv[(32 b + i) * 32 + c]. */
-__device__ __forceinline__ void xg_potrf128_inverse32(const double *S, const double *W, double *T, double *dinv)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp >= 4) return;
-    const int g = lane >> 2, tq = lane & 3;
-    const double *W1 = W + (2 * warp) * XG_P_NB * XG_P_LDW, *W2 = W1 + XG_P_NB * XG_P_LDW;
-    double *Tw = T + warp * XG_P_NB * XG_P_LDW;
-    double *D = dinv + (long long)warp * 32 * 32;
-    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-    /* L21 D11: B(k, n) = D11(k, n) = W1(n, k) */
-    xg_mma16<true>(acc, S + (32 * warp + 16) * XG_P_LDS + 32 * warp, XG_P_LDS, W1, XG_P_LDW, g, tq);
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<double2 *>(Tw + (g + 8 * h) * XG_P_LDW + n * 8 + 2 * tq) =
-                make_double2(acc[n][2 * h], acc[n][2 * h + 1]);
-    __syncwarp();
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[n][e] = 0.0;
-    /* D22 (L21 D11): A(m, k) = D22(m, k) = W2(k, m) */
-#pragma unroll
-    for (int k = 0; k < XG_P_NB; k += 4) {
-        const double a0 = W2[(k + tq) * XG_P_LDW + g], a1 = W2[(k + tq) * XG_P_LDW + g + 8];
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-            xg_dmma_16x8x4(acc[n][0], acc[n][1], acc[n][2], acc[n][3], a0, a1, Tw[(k + tq) * XG_P_LDW + n * 8 + g]);
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<double2 *>(D + (16 + g + 8 * h) * 32 + n * 8 + 2 * tq) =
-                make_double2(-acc[n][2 * h], -acc[n][2 * h + 1]);
-    for (int idx = lane; idx < 16 * 16; idx += 32) {
-        const int i = idx >> 4, c = idx & 15;
-        D[i * 32 + c] = W1[c * XG_P_LDW + i];
-        D[i * 32 + 16 + c] = 0.0;
-        D[(16 + i) * 32 + 16 + c] = W2[c * XG_P_LDW + i];
-    }
-}
+#define XG_POTRF_SUB_SMEM ((size_t)XG_P_DOUBLES * sizeof(double) + 16)
 
 __global__ void __launch_bounds__(XG_POTRF_SUB_THREADS, 1)
     xg_potrf_sub_kernel(XgTileArgs T, int k, int s, double *v, double *part_logdet, double *part_dot, int with_rhs,
                         int *status, int *info)
 {
     extern __shared__ __align__(16) double xg_smem_d[];
-    double *S = xg_smem_d;                                           /* [144][132] */
-    double *W = S + XG_P_ROWS * XG_P_LDS;                            /* [8][16][20] */
-    double *X = W + (XG_SUB / XG_P_NB) * XG_P_NB * XG_P_LDW;          /* [4][16][20] */
-    uint64_t *bar = (uint64_t *)(X + 4 * XG_P_NB * XG_P_LDW);        /* the sub-block has landed */
-    __shared__ double s_red[2][8];
-    __shared__ int s_to;
-    if (xg_cta_should_skip(status)) return;
+    double *S = xg_smem_d;                                   /* [128][132] */
+    double *W = S + XG_SUB * XG_P_LDS;                       /* [8][16][20] */
+    double *X = W + (XG_SUB / XG_P_NB) * XG_P_WSZ;           /* [2][16][20] */
+    double *vs = X + 2 * XG_P_WSZ;                           /* [128] */
+    uint64_t *bar = (uint64_t *)(vs + XG_SUB);               /* the sub-block has landed */
+    __shared__ double s_sums[2];
+    __shared__ int s_stop;
     const int ts = T.ts, r0 = s * XG_SUB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double *A = T.data + xg_slot64(T, k, k) * (long long)ts * ts + (long long)r0 * ts;
@@ -1427,33 +1225,42 @@ __global__ void __launch_bounds__(XG_POTRF_SUB_THREADS, 1)
     if (tid == 0) {
         xg_mbar_init(bar, 1);
         xg_fence_barrier_init();
-        s_to = 0;
+        s_stop = 0;
         xg_mbar_arrive_expect_tx(bar, XG_P_NB * 8 * (XG_SUB / 2 + XG_P_NB / 2) * (XG_SUB / XG_P_NB));
     }
     __syncthreads();
     /* row r of the lower block columns: one bulk copy of 128 (r / 16 + 1) bytes each */
     if (tid < XG_SUB)
         xg_bulk_load(S + tid * XG_P_LDS, A + (long long)tid * ts + r0, (uint32_t)(tid / XG_P_NB + 1) * XG_P_NB * 8, bar);
-    /* meanwhile: the right-hand side's block row, zeros to the right of L_ss in the tile */
-    if (with_rhs)
-        for (int idx = tid; idx < XG_P_NB * XG_SUB; idx += XG_POTRF_SUB_THREADS)
-            S[(XG_SUB + idx / XG_SUB) * XG_P_LDS + idx % XG_SUB] = idx < XG_SUB ? vk[r0 + idx] : 0.0;
-    {
-        const int right = (ts - r0 - XG_SUB) / 2;
-        for (int r = warp; r < XG_SUB; r += XG_POTRF_SUB_THREADS / 32)
-            for (int c = lane; c < right; c += 32)
-                *reinterpret_cast<double2 *>(A + (long long)r * ts + r0 + XG_SUB + 2 * c) = make_double2(0.0, 0.0);
+    else if (with_rhs)
+        vs[tid - XG_SUB] = vk[r0 + tid - XG_SUB];
+    double ld0 = 0.0, dot0 = 0.0; /* the tile's sums over the sub-blocks before this one */
+    if (tid == 0) {
+        if (*(volatile const int *)status != 0) s_stop = 1;
+        if (s > 0) {
+            ld0 = part_logdet[k];
+            if (with_rhs) dot0 = part_dot[k];
+        }
     }
-    if (!xg_mbar_wait(bar, 0)) s_to = 1;
-    __syncthreads();
-    if (s_to) {
+    const bool landed = xg_mbar_wait(bar, 0);
+    if (!landed) {
         if (tid == 0) {
             atomicOr(status, XG_ST_TIMEOUT);
             xg_mbar_wait(bar, 0); /* the copies land before the CTA may exit */
         }
-        return;
+        s_stop = 1;
     }
-    const int fail = xg_potrf128(S, W, with_rhs);
+    __syncthreads();
+    if (s_stop) return;
+    /* zeros to the right of L_ss in the tile */
+    if (warp > 4) {
+        const int right = (ts - r0 - XG_SUB) / 2;
+        for (int r = warp - 5; r < XG_SUB; r += 3)
+            for (int c = lane; c < right; c += 32)
+                *reinterpret_cast<double2 *>(A + (long long)r * ts + r0 + XG_SUB + 2 * c) = make_double2(0.0, 0.0);
+    }
+    const int fail = xg_potrf128(S, W, X, vs, with_rhs, A + r0, ts, T.dinv ? T.dinv + (long long)r0 * 32 : nullptr,
+                                 s_sums);
     if (fail) {
         if (tid == 0) {
             atomicCAS(info, 0, (int)((long long)k * ts + r0 + fail));
@@ -1461,39 +1268,10 @@ __global__ void __launch_bounds__(XG_POTRF_SUB_THREADS, 1)
         }
         return;
     }
-    /* L_ss (zeros above its diagonal) back to the tile, the inverses of its
-     * 32 x 32 diagonal blocks, the solved right-hand side, log-det */
-    for (int r = warp; r < XG_SUB; r += XG_POTRF_SUB_THREADS / 32) {
-        const double2 *src = reinterpret_cast<const double2 *>(S + r * XG_P_LDS);
-        double2 *dst = reinterpret_cast<double2 *>(A + (long long)r * ts + r0);
-        const int n = (r / XG_P_NB + 1) * (XG_P_NB / 2);
-#pragma unroll
-        for (int c = lane; c < XG_SUB / 2; c += 32) dst[c] = c < n ? src[c] : make_double2(0.0, 0.0);
-    }
-    if (T.dinv) xg_potrf128_inverse32(S, W, X, T.dinv + (long long)r0 * 32);
-    double ld = 0.0, dot = 0.0;
-    if (tid < XG_SUB) {
-        ld = log(S[tid * XG_P_LDS + tid]);
-        if (with_rhs) {
-            const double w = S[XG_SUB * XG_P_LDS + tid];
-            vk[r0 + tid] = w;
-            dot = w * w;
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        ld += __shfl_xor_sync(0xffffffffu, ld, off);
-        dot += __shfl_xor_sync(0xffffffffu, dot, off);
-    }
-    if (lane == 0) {
-        s_red[0][warp] = ld;
-        s_red[1][warp] = dot;
-    }
-    __syncthreads();
+    if (with_rhs && tid < XG_SUB) vk[r0 + tid] = vs[tid];
     if (tid == 0) {
-        const double l4 = s_red[0][0] + s_red[0][1] + s_red[0][2] + s_red[0][3];
-        const double d4 = s_red[1][0] + s_red[1][1] + s_red[1][2] + s_red[1][3];
-        part_logdet[k] = (s == 0 ? 0.0 : part_logdet[k]) + l4;
-        if (with_rhs) part_dot[k] = (s == 0 ? 0.0 : part_dot[k]) + d4;
+        part_logdet[k] = ld0 + s_sums[0];
+        if (with_rhs) part_dot[k] = dot0 + s_sums[1];
     }
 }
 
