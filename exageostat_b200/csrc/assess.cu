@@ -524,7 +524,7 @@ int xg_assess_create(XgAssess **out, int nmiss, int nobs, int ts)
     if (!rc) rc = xg_assess_alloc(&q->xm, nmiss);
     if (!rc) rc = xg_assess_alloc(&q->ym, nmiss);
     if (!rc) rc = xg_assess_alloc(&q->terms, 6 * (size_t)nmiss);
-    if (!rc) rc = xg_assess_alloc(&q->part, 2 * (size_t)q->nt);
+    if (!rc) rc = xg_assess_alloc(&q->part, 2 * (size_t)q->nt * q->ts / XG_DAG_BLOCK);
     if (!rc && cudaMalloc(&q->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status");
     for (int i = 0; i < 4 && !rc; ++i)
         if (cudaEventCreate(&q->ev[i]) != cudaSuccess) rc = xg_fail(XG_ERR_CUDA, "events");

@@ -94,6 +94,7 @@ int xg_context_start(int dts)
     cudaError_t e = xg_kernels_configure();
     if (e == cudaSuccess) e = xg_gradient_kernels_configure();
     if (e == cudaSuccess) e = xg_mixed_kernels_configure();
+    if (e == cudaSuccess) e = xg_dag_kernels_configure();
     if (e == cudaSuccess) e = xg_sliced_kernels_configure();
     if (e != cudaSuccess) return xg_cuda_fail(e, "kernel attribute setup");
     g_xg.device = dev;
@@ -149,10 +150,15 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
     if (e == cudaSuccess) e = cudaMemcpy(M.ij, hij, sizeof(int2) * M.ntiles, cudaMemcpyHostToDevice);
     free(hij);
     if (e != cudaSuccess) return xg_cuda_fail(e, "tile index table");
-    e = cudaMalloc(&M.dinv, sizeof(double) * (size_t)ts * 32);
+    e = cudaMalloc(&M.dinv, sizeof(double) * (size_t)M.nt * ts * 32);
     if (e != cudaSuccess) {
         M.dinv = nullptr;
         return xg_cuda_fail(e, "diagonal-block inverses");
+    }
+    e = cudaMalloc(&M.dag, sizeof(int) * (size_t)xg_dag_words((N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK));
+    if (e != cudaSuccess) {
+        M.dag = nullptr;
+        return xg_cuda_fail(e, "block flags");
     }
     return xg_encode_tiles(&M.map, M.d, M.ntiles, ts);
 }
@@ -177,6 +183,8 @@ void xg_tm_free(XgTileMatrix &M)
     if (M.d) cudaFree(M.d);
     if (M.ij) cudaFree(M.ij);
     if (M.dinv) cudaFree(M.dinv);
+    if (M.dag) cudaFree(M.dag);
+    M.dag = nullptr;
     M.d = nullptr;
     M.ij = nullptr;
     M.dinv = nullptr;
@@ -298,9 +306,41 @@ int xg_check_theta(const double *theta, int kernel)
     return XG_OK;
 }
 
-/* Cholesky of M in place; with v != nullptr also v <- L^-1 v and the per-tile
- * partial sums (log-det in part[0:nt], |v_k|^2 in part[nt:2nt]). */
-/* Right-looking tile Cholesky with the fused z solve.  Per step k:
+/* Largest dimension factored by the tile DAG.  Milliseconds per evaluation,
+ * per-step launches against the DAG: N = 1000 0.73 / 0.45, 3000 2.83 / 1.35,
+ * 6000 6.43 / 3.57, 10000 17.9 / 12.8, 14000 38.2 / 32.4, 20000 97.7 / 90.9,
+ * 26000 192.3 / 196.1, 32000 352 / 358: past about 22000 the trailing updates
+ * fill the chip by themselves and the operands of the DAG's tasks, spread over
+ * many columns, no longer stay in L2. */
+#define XG_DAG_MAX_N 22000
+
+/* The factorisation of M as one launch of the tile DAG (tile_dag.cu); returns
+ * the number of partial sums of either kind. */
+static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, cudaStream_t st)
+{
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    XgDag G = {};
+    G.data = M.d;
+    G.ts = M.ts;
+    G.one.nt = M.nt;
+    G.one.nb = nb;
+    G.ntasks = xg_num_lower_tiles(nb);
+    G.next = (unsigned *)M.dag;
+    G.abort = M.dag + 1;
+    G.flags = M.dag + 2;
+    G.dinv = M.dinv;
+    G.v = v;
+    G.part = part;
+    G.status = status;
+    xg_launch_dag(M.map, G, g_xg.sm_count, st);
+    return nb;
+}
+
+/* Cholesky of M in place; with v != nullptr also v <- L^-1 v.  Returns the
+ * number n of partial sums of either kind: log-det in part[0:n], |v|^2 in
+ * part[n:2n].  Up to XG_DAG_MAX_N one launch of the tile DAG, else a
+ * right-looking sequence of launches.  Per step k:
  *   panel   : POTRF(k,k) [+ log-det, + L_kk v_k = v_k]  ->  TRSM(i,k) [+ v_i -= L_ik v_k]
  *   trailing: A_ij -= L_ik L_jk^T, j >= k+1
  * With fs.st_hi the panel of step k+1 runs on the high-priority stream as soon
@@ -308,8 +348,10 @@ int xg_check_theta(const double *theta, int kernel)
  * into "column k+1" and "the rest"), so it overlaps the rest of step k.
  * Profiling events (5 per step): panel start, after POTRF, after TRSM,
  * trailing start, trailing end. */
-void xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs)
+int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs)
 {
+    /* profiled evaluations keep the per-step launches, whose kernels the profile tells apart */
+    if (M.dag && !fs.pev && M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, fs.st);
     XgTileArgs T{M.d, M.ts, M.nt};
     T.dinv = M.dinv;
     const bool la = fs.st_hi != nullptr;
@@ -345,14 +387,15 @@ void xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, 
         }
         if (pev) cudaEventRecord(pev[5 * k + 4], fs.st);
     }
+    return M.nt;
 }
 
-void xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st, cudaEvent_t *pev)
+int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st, cudaEvent_t *pev)
 {
     XgFactorStreams fs;
     fs.st = st;
     fs.pev = pev;
-    xg_factor_lookahead(M, v, part, status, info, fs);
+    return xg_factor_lookahead(M, v, part, status, info, fs);
 }
 
 /* Algorithmic flops of the trailing update after step k: a GEMM (2 ts^3) per
@@ -477,7 +520,7 @@ int xg_field_create(XgField **out, int N, int ts, const double *x, const double 
     if (!rc) rc = xg_dev_alloc(&f->z, Np);
     if (!rc) rc = xg_dev_alloc(&f->v, Np);
     if (!rc) rc = xg_dev_alloc(&f->e, Np);
-    if (!rc) rc = xg_dev_alloc(&f->part, 2 * (size_t)f->C.nt);
+    if (!rc) rc = xg_dev_alloc(&f->part, 2 * Np / XG_DAG_BLOCK);
     if (!rc) rc = xg_dev_alloc(&f->out, 8);
     if (!rc && cudaMalloc(&f->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status word");
     if (!rc && cudaMallocHost(&f->h_out, 8 * sizeof(double)) != cudaSuccess)
@@ -541,8 +584,8 @@ int xg_field_loglik(XgField *f, const double *theta, double *res, double *times)
     fs.ev_panel = f->ev_panel;
     fs.ev_upd = f->ev_upd;
     fs.pev = f->profiling ? f->pev : nullptr;
-    xg_factor_lookahead(f->C, f->v, f->part, f->status, f->info, fs);
-    xg_launch_finalize(f->part, f->part + f->C.nt, f->C.nt, f->N, f->out, f->status, f->info, st);
+    const int np = xg_factor_lookahead(f->C, f->v, f->part, f->status, f->info, fs);
+    xg_launch_finalize(f->part, f->part + np, np, f->N, f->out, f->status, f->info, st);
     XG_CU(cudaEventRecord(f->ev[2], st));
     XG_CU(cudaMemcpyAsync(f->h_out, f->out, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
     XG_CU(cudaGetLastError());
@@ -1575,7 +1618,7 @@ int xg_predict_create(XgPredict **out, int nmiss, int nobs, int ts)
     if (!rc) rc = xg_dev_alloc(&q->ym, nmiss);
     if (!rc) rc = xg_dev_alloc(&q->zact, nmiss);
     if (!rc) rc = xg_dev_alloc(&q->zmiss, nmiss);
-    if (!rc) rc = xg_dev_alloc(&q->part, 2 * (size_t)q->C22.nt);
+    if (!rc) rc = xg_dev_alloc(&q->part, 2 * Np / XG_DAG_BLOCK);
     if (!rc) rc = xg_dev_alloc(&q->out, 8);
     if (!rc && cudaMalloc(&q->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status");
     if (!rc && (cudaEventCreateWithFlags(&q->ev_panel, cudaEventDisableTiming) != cudaSuccess ||

@@ -1,0 +1,389 @@
+/*
+ * Tile Cholesky in one persistent launch: a dataflow of 128 x 128 blocks.
+ *
+ * The per-step launches (POTRF, panel TRSM, trailing update per tile column)
+ * leave a small or mid-size factorisation waiting on launch gaps, on kernels
+ * of a few CTAs, and on reading and writing every trailing block once per
+ * step.  Here block (I, J) of the factor is ONE task of one CTA:
+ *
+ *   C = A_IJ - sum_{K < J} L_IK L_JK^T     TMA-fed DMMA, C in registers throughout
+ *   I == J: L_JJ = chol(C) (xg_potrf128), log-det, forward solve of v_J
+ *   I >  J: L_IJ = C L_JJ^-T in the same registers, v_I -= L_IJ v_J
+ *
+ * so each block is read and written once (left-looking).  Tasks are taken in
+ * block-column order from one counter; a task waits, block by block, for the
+ * flags of the operands it is about to read, so a CTA runs ahead into later
+ * columns as far as its operands are ready, and the serial chain per column
+ * is POTRF -> TRSM of one block -> the last product of the next diagonal
+ * block.  A task waits only on tasks taken earlier by a running CTA: the
+ * launch cannot deadlock.  Every wait is bounded.
+ *
+ * The blocks are sub-blocks of the stored ts x ts tiles (ts a multiple of
+ * 128), so the layout of the factor is the one every other kernel reads;
+ * blocks that are padding only (rows past N) already hold the identity and
+ * are no tasks.  Replaces CHAMELEON_dpotrf_Tile with core_dmdet and the Z
+ * solve of MLE_dexact.c:372-391 (the StarPU task graph of psdportf.c:85-186
+ * with an infinite band).
+ */
+#include <math.h>
+#include <stdint.h>
+
+#include "xg_common.cuh"
+#include "xg_kernels.h"
+#include "xg_potrf128.cuh"
+
+#define XG_D_BK 16
+#define XG_D_STAGES 4
+#define XG_D_THREADS 256
+#define XG_D_BOX_BYTES (XG_SUB * XG_D_BK * 8)
+#define XG_D_STAGE_BYTES (2 * XG_D_BOX_BYTES)
+#define XG_D_RING_BYTES (XG_D_STAGES * XG_D_STAGE_BYTES)
+/* L_JJ as six 128 x 16 boxes (its last 32 columns are not needed), the inverted 32 x 32 blocks, v_J */
+#define XG_D_TRSM_BOXES 6
+#define XG_D_TRSM_BYTES (XG_D_TRSM_BOXES * XG_D_BOX_BYTES + (XG_SUB * 32 + XG_SUB) * 8)
+#define XG_D_POTRF_BYTES (XG_P_DOUBLES * 8)
+#define XG_D_MAX2(a, b) ((a) > (b) ? (a) : (b))
+#define XG_D_AREA_BYTES XG_D_MAX2(XG_D_RING_BYTES, XG_D_MAX2(XG_D_TRSM_BYTES, XG_D_POTRF_BYTES))
+#define XG_D_SMEM (1024 + XG_D_AREA_BYTES + 128)
+
+__device__ __forceinline__ int xg_dag_acquire(const int *p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void xg_dag_release(int *p)
+{
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(1) : "memory");
+}
+
+/* One thread: waits until *p is set; false after 2 s or when another CTA aborted the launch */
+__device__ __forceinline__ bool xg_dag_wait(const int *p, const int *abort)
+{
+    if (xg_dag_acquire(p)) return true;
+    const uint64_t t0 = xg_globaltimer_ns();
+    for (uint32_t it = 0;; ++it) {
+        if (xg_dag_acquire(p)) return true;
+        if ((it & 31u) == 31u) {
+            if (*(volatile const int *)abort) return false;
+            if (xg_globaltimer_ns() - t0 > 2000000000ull) return false;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(XG_D_THREADS, 1)
+    xg_tile_dag_kernel(const __grid_constant__ CUtensorMap map, XgDag G)
+{
+    extern __shared__ __align__(1024) unsigned char xg_smem_raw[];
+    unsigned char *smem = (unsigned char *)(((uintptr_t)xg_smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t *full = (uint64_t *)(smem + XG_D_AREA_BYTES);
+    uint64_t *empty = full + XG_D_STAGES;
+    uint64_t *lbar = empty + XG_D_STAGES; /* the triangle and inverses of L_JJ have landed */
+    __shared__ long long s_task;
+    __shared__ int s_skip, s_bad;
+    __shared__ double s_sums[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tq = lane & 3;
+    /* 16-row strip of the block owned by this warp: paired so that the two
+     * warps of a scheduler share a diagonal block's triangle evenly */
+    const int strip = warp < 4 ? warp : 11 - warp;
+    const int r0 = strip * 16 + g;
+    const int ts = G.ts, b = ts / XG_SUB;
+    if (tid == 0) {
+        for (int s = 0; s < XG_D_STAGES; ++s) {
+            xg_mbar_init(&full[s], 1);
+            xg_mbar_init(&empty[s], XG_D_THREADS / 32);
+        }
+        xg_mbar_init(lbar, 1);
+        xg_fence_barrier_init();
+        xg_prefetch_tensormap(&map);
+        s_bad = 0;
+    }
+    uint32_t it0 = 0, lphase = 0; /* slabs of all tasks so far; phase of lbar */
+    for (bool first = true;; first = false) {
+        __syncthreads(); /* the previous task is finished by every thread */
+        if (tid == 0) {
+            long long q = -1;
+            if (!*(volatile int *)G.abort) {
+                q = first ? (long long)blockIdx.x : (long long)gridDim.x + (long long)atomicAdd(G.next, 1u);
+                if (q >= G.ntasks) q = -1;
+            }
+            s_task = q;
+        }
+        __syncthreads();
+        const long long q = s_task;
+        if (q < 0) break;
+        int f = 0, I, J;
+        if (G.tasks) {
+            const int4 t = G.tasks[q];
+            f = t.x;
+            I = t.y;
+            J = t.z;
+        } else {
+            const int2 t = xg_tile_decode_fast(q, G.one.nb);
+            I = t.x;
+            J = t.y;
+        }
+        const XgDagField fd = G.tasks ? G.F[f] : G.one;
+        const int nt = fd.nt, nb = fd.nb;
+        const bool diag = I == J;
+        int *status = G.status + 2 * f;
+        int *flags = G.flags + fd.flag_off;
+        const int *flagI = flags, *flagJ = flags;
+        const int i = I / b, j = J / b;
+        double *C = G.data + (fd.tile_off + xg_tile_index(i, j, nt)) * (long long)ts * ts +
+                    (long long)(I % b * XG_SUB) * ts + J % b * XG_SUB;
+        double *dinv = G.dinv + fd.dinv_off * 32 + (long long)J * XG_SUB * 32;
+        double *v = G.v ? G.v + fd.vec_off : nullptr;
+        if (tid == 0) s_skip = *(volatile int *)status != 0;
+        __syncthreads();
+        if (!s_skip) {
+            /* ---- C = A_IJ - sum_K L_IK L_JK^T: accumulators hold -C ---- */
+            const int nlim = diag ? 2 * strip + 2 : 16; /* 8-column groups: a diagonal block's lower part */
+            double acc[16][4];
+#pragma unroll
+            for (int n = 0; n < 16; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    double2 c = make_double2(0.0, 0.0);
+                    if (n < nlim)
+                        c = __ldcg(reinterpret_cast<const double2 *>(C + (long long)(r0 + 8 * h) * ts + 8 * n + 2 * tq));
+                    acc[n][2 * h] = -c.x;
+                    acc[n][2 * h + 1] = -c.y;
+                }
+            const int KT = J * (XG_SUB / XG_D_BK);
+            int issued = 0, ready = 0; /* thread 0: slabs issued; operand blocks known to be finished */
+            bool ok = true;
+            /* the slabs reuse shared memory that generic accesses touched */
+            xg_fence_proxy_async();
+            __syncthreads();
+            for (int kb = 0; kb < KT; ++kb) {
+                if (tid == 0) {
+                    while (issued < KT && issued < kb + XG_D_STAGES) {
+                        const int kblk = issued / (XG_SUB / XG_D_BK);
+                        if (kblk >= ready) {
+                            const int *pi = flagI + xg_tile_index(I, kblk, nb), *pj = flagJ + xg_tile_index(J, kblk, nb);
+                            /* with slabs in flight an unfinished operand is looked at again after
+                             * the next one; with none it is waited for */
+                            if (issued > kb) {
+                                if (!xg_dag_acquire(pi) || !xg_dag_acquire(pj)) break;
+                            } else if (!xg_dag_wait(pi, G.abort) || !xg_dag_wait(pj, G.abort)) {
+                                ok = false;
+                                break;
+                            }
+                            ready = kblk + 1;
+                            asm volatile("fence.proxy.async.global;" ::: "memory");
+                        }
+                        const uint32_t s = (it0 + issued) % XG_D_STAGES, use = (it0 + issued) / XG_D_STAGES;
+                        if (use > 0 && !xg_mbar_wait(&empty[s], (use - 1) & 1)) {
+                            ok = false;
+                            break;
+                        }
+                        const int k = kblk / b, kx = kblk % b * XG_SUB + issued % (XG_SUB / XG_D_BK) * XG_D_BK;
+                        unsigned char *sa = smem + s * XG_D_STAGE_BYTES;
+                        xg_mbar_arrive_expect_tx(&full[s], diag ? XG_D_BOX_BYTES : XG_D_STAGE_BYTES);
+                        xg_tma_load_2d(sa, &map, kx,
+                                       (int)((fd.tile_off + xg_tile_index(i, k, nt)) * ts + I % b * XG_SUB), &full[s]);
+                        if (!diag)
+                            xg_tma_load_2d(sa + XG_D_BOX_BYTES, &map, kx,
+                                           (int)((fd.tile_off + xg_tile_index(j, k, nt)) * ts + J % b * XG_SUB),
+                                           &full[s]);
+                        ++issued;
+                    }
+                    if (!ok) *(volatile int *)&s_bad = 1;
+                }
+                __syncwarp();
+                if (*(volatile int *)&s_bad) ok = false;
+                const uint32_t s = (it0 + kb) % XG_D_STAGES;
+                if (ok && !xg_mbar_wait(&full[s], ((it0 + kb) / XG_D_STAGES) & 1)) ok = false;
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    *(volatile int *)&s_bad = 1;
+                    break;
+                }
+                const unsigned char *sa = smem + s * XG_D_STAGE_BYTES;
+                const unsigned char *sb = diag ? sa : sa + XG_D_BOX_BYTES;
+                /* k permutation inside the slab as in xg_gemm_core: lane slot tq holds k = 4 tq + {0..3} */
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int sw = ((2 * tq + half) ^ g) << 4; /* rows g + 8 m: row & 7 = g */
+                    const double2 a0 = *(const double2 *)(sa + (r0 << 7) + sw);
+                    const double2 a1 = *(const double2 *)(sa + ((r0 + 8) << 7) + sw);
+#pragma unroll
+                    for (int n0 = 0; n0 < 16; n0 += 4) {
+                        /* groups of 32 columns: the branch must skip enough work to stay a
+                         * branch (skipped by predicates, the DMMAs take their full time) */
+                        if (n0 >= nlim) break;
+                        double2 bv[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) bv[u] = *(const double2 *)(sb + ((8 * (n0 + u) + g) << 7) + sw);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.x, a1.x,
+                                           bv[u].x);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.y, a1.y,
+                                           bv[u].y);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) xg_mbar_arrive(&empty[s]);
+            }
+            __syncthreads();
+            if (s_bad) {
+                /* copies in flight land before the CTA may exit */
+                if (tid == 0) {
+                    atomicOr(status, XG_ST_TIMEOUT);
+                    atomicExch(G.abort, 1);
+                    for (int u = issued > XG_D_STAGES ? issued - XG_D_STAGES : 0; u < issued; ++u)
+                        xg_mbar_wait(&full[(it0 + u) % XG_D_STAGES], ((it0 + u) / XG_D_STAGES) & 1);
+                }
+                return;
+            }
+            it0 += KT;
+            if (diag) {
+                /* ---- L_JJ, v_J, log-det ---- */
+                double *S = (double *)smem;
+                double *W = S + XG_SUB * XG_P_LDS, *X = W + (XG_SUB / XG_P_NB) * XG_P_WSZ, *vs = X + 2 * XG_P_WSZ;
+#pragma unroll
+                for (int n = 0; n < 16; ++n)
+                    if (n < nlim)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            *reinterpret_cast<double2 *>(S + (r0 + 8 * h) * XG_P_LDS + 8 * n + 2 * tq) =
+                                make_double2(-acc[n][2 * h], -acc[n][2 * h + 1]);
+                if (v && tid < XG_SUB) vs[tid] = __ldcg(v + J * XG_SUB + tid);
+                /* zeros to the right of L_JJ in its tile */
+                const int right = (ts - (J % b + 1) * XG_SUB) / 2;
+                for (int r = warp; r < XG_SUB; r += XG_D_THREADS / 32)
+                    for (int c = lane; c < right; c += 32)
+                        *reinterpret_cast<double2 *>(C + (long long)r * ts + XG_SUB + 2 * c) = make_double2(0.0, 0.0);
+                const int fail = xg_potrf128(S, W, X, vs, v != nullptr, C, ts, dinv, s_sums);
+                if (fail) {
+                    if (tid == 0) {
+                        atomicCAS(status + 1, 0, J * XG_SUB + fail);
+                        atomicOr(status, XG_ST_NOT_SPD);
+                    }
+                } else {
+                    if (v && tid < XG_SUB) v[J * XG_SUB + tid] = vs[tid];
+                    if (tid == 0) {
+                        G.part[fd.part_off + J] = s_sums[0];
+                        if (v) G.part[fd.part_off + nb + J] = s_sums[1];
+                    }
+                }
+            } else {
+                /* ---- L_IJ = C L_JJ^-T: L_JJ (as operand boxes) and the inverses of its
+                 * 32 x 32 diagonal blocks into shared memory, then each warp solves its
+                 * 16 rows in registers ---- */
+                const unsigned char *LS = smem;                                    /* [6][128][16], swizzled */
+                double *DS = (double *)(smem + XG_D_TRSM_BOXES * XG_D_BOX_BYTES); /* [128][32] */
+                double *VS = DS + XG_SUB * 32;                                     /* [128] v_J */
+                if (tid == 0) {
+                    if (xg_dag_wait(flagJ + xg_tile_index(J, J, nb), G.abort)) {
+                        const int row = (int)((fd.tile_off + xg_tile_index(j, j, nt)) * ts + J % b * XG_SUB);
+                        asm volatile("fence.proxy.async;" ::: "memory");
+                        xg_mbar_arrive_expect_tx(lbar, XG_D_TRSM_BOXES * XG_D_BOX_BYTES + (XG_SUB * 32 + (v ? XG_SUB : 0)) * 8);
+                        xg_bulk_load(DS, dinv, XG_SUB * 32 * 8, lbar);
+                        for (int u = 0; u < XG_D_TRSM_BOXES; ++u)
+                            xg_tma_load_2d(smem + u * XG_D_BOX_BYTES, &map, J % b * XG_SUB + u * XG_D_BK, row, lbar);
+                        if (v) xg_bulk_load(VS, v + J * XG_SUB, XG_SUB * 8, lbar);
+                    } else {
+                        *(volatile int *)&s_bad = 1;
+                    }
+                }
+                __syncthreads();
+                if (!s_bad && !xg_mbar_wait(lbar, lphase)) *(volatile int *)&s_bad = 2;
+                lphase ^= 1;
+                __syncthreads();
+                if (s_bad) {
+                    if (tid == 0) {
+                        atomicOr(status, XG_ST_TIMEOUT);
+                        atomicExch(G.abort, 1);
+                        if (s_bad == 2) xg_mbar_wait(lbar, lphase ^ 1);
+                    }
+                    return;
+                }
+#pragma unroll
+                for (int cb = 0; cb < 4; ++cb) {
+                    /* X = -(acc D^T) over the 32 columns of block cb; the accumulators are the
+                     * A fragments as they stand (K runs over the columns in the lanes' order) */
+                    double x[4][4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[m][e] = 0.0;
+#pragma unroll
+                        for (int k = 0; k <= m; ++k) { /* D is lower triangular */
+                            const double2 d =
+                                *reinterpret_cast<const double2 *>(DS + (32 * cb + 8 * m + g) * 32 + 8 * k + 2 * tq);
+                            xg_dmma_16x8x4(x[m][0], x[m][1], x[m][2], x[m][3], acc[4 * cb + k][0], acc[4 * cb + k][2],
+                                           d.x);
+                            xg_dmma_16x8x4(x[m][0], x[m][1], x[m][2], x[m][3], acc[4 * cb + k][1], acc[4 * cb + k][3],
+                                           d.y);
+                        }
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[4 * cb + m][e] = -x[m][e];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            *reinterpret_cast<double2 *>(C + (long long)(r0 + 8 * h) * ts + 32 * cb + 8 * m + 2 * tq) =
+                                make_double2(acc[4 * cb + m][2 * h], acc[4 * cb + m][2 * h + 1]);
+                    }
+                    /* the columns to the right: acc += X L^T */
+#pragma unroll
+                    for (int m = 4 * cb + 4; m < 16; ++m)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const double2 l = *reinterpret_cast<const double2 *>(
+                                LS + (2 * cb + (k >> 1)) * XG_D_BOX_BYTES + ((8 * m + g) << 7) +
+                                ((((k & 1) * 4 + tq) ^ g) << 4));
+                            xg_dmma_16x8x4(acc[m][0], acc[m][1], acc[m][2], acc[m][3], acc[4 * cb + k][0],
+                                           acc[4 * cb + k][2], l.x);
+                            xg_dmma_16x8x4(acc[m][0], acc[m][1], acc[m][2], acc[m][3], acc[4 * cb + k][1],
+                                           acc[4 * cb + k][3], l.y);
+                        }
+                }
+                if (v) {
+                    double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+                    for (int n = 0; n < 16; ++n) {
+                        const double2 w = *reinterpret_cast<const double2 *>(VS + 8 * n + 2 * tq);
+                        t0 = fma(acc[n][0], w.x, fma(acc[n][1], w.y, t0));
+                        t1 = fma(acc[n][2], w.x, fma(acc[n][3], w.y, t1));
+                    }
+                    for (int o = 1; o < 4; o <<= 1) {
+                        t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+                        t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+                    }
+                    if (tq == 0) {
+                        double *vi = v + I * XG_SUB + r0;
+                        vi[0] = __ldcg(vi) - t0;
+                        vi[8] = __ldcg(vi + 8) - t1;
+                    }
+                }
+            }
+        }
+        /* publish: every thread's stores, then the flag (also for a field that
+         * has failed: its later tasks skip their bodies) */
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) xg_dag_release(flags + xg_tile_index(I, J, nb));
+    }
+}
+
+cudaError_t xg_dag_kernels_configure()
+{
+    return cudaFuncSetAttribute(xg_tile_dag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_D_SMEM);
+}
+
+void xg_launch_dag(const CUtensorMap &map, const XgDag &G, int max_ctas, cudaStream_t st)
+{
+    if (G.ntasks <= 0) return;
+    const unsigned grid = (unsigned)(G.ntasks < max_ctas ? G.ntasks : max_ctas);
+    xg_tile_dag_kernel<<<grid, XG_D_THREADS, XG_D_SMEM, st>>>(map, G);
+}

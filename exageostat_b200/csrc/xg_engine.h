@@ -38,7 +38,12 @@ struct XgTileMatrix {
     double *d = nullptr;
     int2 *ij = nullptr; /* (i, j) of every packed tile */
     CUtensorMap map;    /* TMA view for the trailing-update kernel */
-    double *dinv = nullptr; /* ts x 32: inverted 32 x 32 diagonal blocks of the current panel */
+    /* nt ts x 32: the inverted 32 x 32 diagonal blocks of L (the tile DAG keeps
+     * every column's; the per-step launches use the first ts rows for the current one) */
+    double *dinv = nullptr;
+    /* tile DAG: next task, abort flag, one flag per lower 128-block; null where
+     * the matrix is factored by the per-step launches only */
+    int *dag = nullptr;
 };
 
 /* Banded mixed-precision workspace (mixed.cu): compact FP64 band tiles,
@@ -76,7 +81,7 @@ struct XgField {
     double *z = nullptr;               /* observations (zero padded); never modified by evaluations */
     double *v = nullptr;               /* solve work vector */
     double *e = nullptr;               /* N(0,1) draws for MLE_zvg */
-    double *part = nullptr;            /* per-tile log-det / dot partials (2 nt) */
+    double *part = nullptr;            /* log-det / dot partials (2 per 128 rows) */
     double *out = nullptr;             /* device result record */
     int *status = nullptr, *info = nullptr;
     double *h_out = nullptr; /* pinned copy of out */
@@ -121,9 +126,9 @@ int xg_encode_tiles(CUtensorMap *map, double *base, long long ntiles, int ts);
 void xg_tm_free(XgTileMatrix &M);
 XgMaternParams xg_params(const double *theta, int kernel);
 int xg_check_theta(const double *theta, int kernel);
-void xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
-               cudaEvent_t *pev = nullptr);
-void xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
+int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
+              cudaEvent_t *pev = nullptr);
+int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
 double xg_trailing_flops(int nt, int ts, int k);
 int xg_field_set_data(XgField *f, const double *x, const double *y, const double *z);
 int xg_field_set_profiling(XgField *f, int on);

@@ -148,6 +148,47 @@ __host__ __device__ inline int2 xg_tile_decode(long long t, int nt)
     return make_int2(j + (int)t, j);
 }
 
+/* the same in a constant number of steps (for the long lists of the tile DAG) */
+__device__ inline int2 xg_tile_decode_fast(long long t, int nt)
+{
+    /* column j starts at j nt - j (j - 1) / 2 */
+    const double h = nt + 0.5;
+    int j = (int)(h - sqrt(h * h - 2.0 * (double)t));
+    if (j < 0) j = 0;
+    while (j > 0 && (long long)j * nt - (long long)j * (j - 1) / 2 > t) --j;
+    while ((long long)(j + 1) * nt - (long long)(j + 1) * j / 2 <= t) ++j;
+    return make_int2(j + (int)(t - ((long long)j * nt - (long long)j * (j - 1) / 2)), j);
+}
+
+/* tile_dag.cu: the whole Cholesky of one or more fields in one persistent
+ * launch, a dataflow of 128 x 128 blocks. */
+#define XG_DAG_BLOCK 128
+/* device words of a field's DAG state: next task, abort flag, block flags */
+static inline long long xg_dag_words(int nb) { return 2 + (long long)nb * (nb + 1) / 2; }
+struct XgDagField {
+    long long tile_off; /* first packed tile inside the tile store */
+    long long vec_off;  /* first entry of v */
+    long long part_off; /* partial sums: nb log-det, nb |v_J|^2 */
+    long long flag_off; /* nb (nb + 1) / 2 block flags */
+    long long dinv_off; /* first row of the inverted 32 x 32 diagonal blocks (32 doubles a row) */
+    int nt, nb;         /* tiles per side; 128-blocks per side that hold rows < N */
+};
+struct XgDag {
+    double *data; /* the tile store behind the TMA map */
+    int ts;
+    XgDagField one;       /* a single field (tasks == nullptr: every block, in block-column order) */
+    const XgDagField *F;  /* several fields */
+    const int4 *tasks;    /* (field, I, J, -) in an order that never puts a block before its operands */
+    long long ntasks;
+    unsigned *next;       /* zero on launch: tasks taken beyond each CTA's first */
+    int *abort;           /* zero on launch; set by a wait that timed out */
+    int *flags;           /* zero on launch */
+    double *dinv, *v, *part; /* v may be null */
+    int *status;          /* two words per field: status, info */
+};
+cudaError_t xg_dag_kernels_configure();
+void xg_launch_dag(const CUtensorMap &map, const XgDag &G, int max_ctas, cudaStream_t st);
+
 cudaError_t xg_kernels_configure();
 size_t xg_potrf_smem_bytes(int ts);
 size_t xg_trsm_smem_bytes(int ts);

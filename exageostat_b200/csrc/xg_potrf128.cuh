@@ -117,7 +117,7 @@ __device__ __forceinline__ int xg_chol16_pass(double *S, double *W, double *buf,
 
 /* the general form: kept out of line, it runs only for the odd block whose
  * pivots are out of range or not positive */
-__device__ __noinline__ int xg_chol16_general(double *S, double *W, double *buf, int lane)
+static __device__ __noinline__ int xg_chol16_general(double *S, double *W, double *buf, int lane)
 {
     return xg_chol16_pass<false>(S, W, buf, lane);
 }
