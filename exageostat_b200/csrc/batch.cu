@@ -6,14 +6,12 @@
  * store (fields packed one after the other, one TMA tensor over all of them).
  * Generation is one launch over every tile of every field; the whole
  * factorisation (with the fused log-det and z solve) of all fields is ONE
- * persistent launch driven by a device-resident tile scheduler
- * (xg_batch_sched_kernel): the task list -- every POTRF, TRSM and trailing
- * tile update of every field, in one topological order built here -- is
- * taken by persistent CTAs, each task waiting (bounded) on per-tile
- * dependency counters and publishing its completion, so the fields' steps
- * interleave freely instead of proceeding in lock-step.  The reduction to
- * log-likelihoods is a third launch.  The memsets and the three launches are
- * captured once into a CUDA graph; each evaluation uploads the fields'
+ * persistent launch of the tile DAG (tile_dag.cu): the task list -- every
+ * 128 x 128 block of every field, in one topological order built here -- is
+ * taken by persistent CTAs, each task waiting (bounded) for the blocks it
+ * reads, so the fields' columns interleave freely instead of proceeding in
+ * lock-step.  The reduction to log-likelihoods is a third launch.  The
+ * memsets and the three launches are captured once into a CUDA graph; each evaluation uploads the fields'
  * parameters (computed on the host exactly as for a single field) and replays
  * the graph.  Every field has its own status word, so a field whose
  * covariance is not positive definite reports -inf without stopping the
@@ -49,7 +47,7 @@ struct XgBTable {
 
 struct XgBatch {
     int nfields = 0, ts = 0, kernel = 0, metric = 0, maxnt = 0;
-    long long total_tiles = 0, total_vec = 0, total_part = 0, total_cnt = 0;
+    long long total_tiles = 0, total_vec = 0, total_part = 0, total_flags = 0, total_tflags = 0;
     std::vector<XgBField> F;
     XgBField *F_dev = nullptr, *F_pinned = nullptr;
     double *tiles = nullptr, *x = nullptr, *y = nullptr, *z = nullptr, *v = nullptr, *part = nullptr,
@@ -57,13 +55,14 @@ struct XgBatch {
     int *status = nullptr, *h_status = nullptr;
     void *table_buf = nullptr;
     XgBTable gen;
-    /* device tile scheduler: task list, counters, next-task index, abort flag */
+    /* tile DAG: fields, block tasks, state (next task, abort flag, block flags) and
+     * the kept inverses of the 32 x 32 diagonal blocks; the same of the backward solve */
+    XgDagField *D_dev = nullptr;
     int4 *tasks = nullptr;
-    long long ntasks = 0;
-    int *cnt = nullptr;
-    unsigned long long *next = nullptr;
-    int *abort_flag = nullptr;
-    double *dinv = nullptr; /* per scheduler CTA: ts x 32 inverted diagonal blocks */
+    int2 *ttasks = nullptr;
+    long long ntasks = 0, nttasks = 0;
+    int *words = nullptr, *twords = nullptr;
+    double *dinv = nullptr;
     CUtensorMap map;
     cudaGraphExec_t graph = nullptr;
     /* gradients (allocated on the first request): per stream an inverse-factor
@@ -71,6 +70,7 @@ struct XgBatch {
      * view of its tiles; one (i, j) table per tile count; 4 sums per field */
     static const int GS = 8;
     cudaStream_t gst[GS] = {};
+    cudaEvent_t ev = nullptr; /* the backward solves are done */
     XgTileMatrix gX[GS];
     double *gpart[GS] = {};
     double *gout = nullptr, *h_gout = nullptr;
@@ -87,12 +87,13 @@ static void xg_batch_free(XgBatch *b)
         if (b->gpart[s]) cudaFree(b->gpart[s]);
         if (b->gst[s]) cudaStreamDestroy(b->gst[s]);
     }
+    if (b->ev) cudaEventDestroy(b->ev);
     for (int2 *p : b->ij_by_nt)
         if (p) cudaFree(p);
     if (b->gout) cudaFree(b->gout);
     if (b->h_gout) cudaFreeHost(b->h_gout);
     void *dev[] = {b->F_dev, b->tiles, b->x, b->y, b->z, b->v, b->part, b->out, b->status, b->table_buf,
-                   b->tasks, b->cnt, b->next, b->abort_flag, b->dinv};
+                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (b->F_pinned) cudaFreeHost(b->F_pinned);
@@ -280,6 +281,30 @@ extern "C" long long exageostat_b200_batch_plan(int nfields, const int *nt, int 
     return (long long)tl.size();
 }
 
+/* Block tasks of every field for the tile DAG and block columns of the
+ * backward solves.  The fields advance together, each by the same share of
+ * its columns (J / nb): neighbouring columns of one field then lie far apart
+ * in the list, so a task rarely waits for the one before it, and the fields
+ * end together, so the last columns of the largest one do not run alone. */
+static void xg_batch_order(const std::vector<XgDagField> &D, std::vector<int4> &tl, std::vector<int2> &tt)
+{
+    struct Col {
+        double key;
+        int f, J;
+    };
+    std::vector<Col> cols;
+    for (int f = 0; f < (int)D.size(); ++f)
+        for (int J = 0; J < D[f].nb; ++J) cols.push_back(Col{(double)J / D[f].nb, f, J});
+    std::sort(cols.begin(), cols.end(), [](const Col &a, const Col &b) {
+        return a.key != b.key ? a.key < b.key : a.f != b.f ? a.f < b.f : a.J < b.J;
+    });
+    tl.clear();
+    tt.clear();
+    for (const Col &c : cols)
+        for (int I = c.J; I < D[c.f].nb; ++I) tl.push_back(make_int4(c.f, I, c.J, 0));
+    for (size_t q = cols.size(); q-- > 0;) tt.push_back(make_int2(cols[q].f, cols[q].J));
+}
+
 extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const double *x, const double *y,
                                             const double *z, int kernel, int metric, int ts, void **handle)
 {
@@ -294,6 +319,7 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
     b->kernel = kernel;
     b->metric = metric;
     b->F.resize(nfields);
+    std::vector<XgDagField> D(nfields);
     for (int f = 0; f < nfields; ++f) {
         if (n[f] <= 0) {
             xg_batch_free(b);
@@ -303,15 +329,24 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
         memset(&fd, 0, sizeof fd);
         fd.N = n[f];
         fd.nt = (n[f] + b->ts - 1) / b->ts;
+        fd.nb = (n[f] + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
         fd.kernel = kernel;
         fd.tile_off = b->total_tiles;
         fd.vec_off = b->total_vec;
         fd.part_off = b->total_part;
-        fd.sched_off = b->total_cnt;
+        XgDagField &dd = D[f];
+        dd.tile_off = fd.tile_off;
+        dd.vec_off = dd.dinv_off = fd.vec_off;
+        dd.part_off = fd.part_off;
+        dd.flag_off = b->total_flags;
+        dd.tflag_off = b->total_tflags;
+        dd.nt = fd.nt;
+        dd.nb = fd.nb;
+        b->total_flags += xg_num_lower_tiles(fd.nb);
+        b->total_tflags += fd.nb;
         b->total_tiles += xg_num_lower_tiles(fd.nt);
         b->total_vec += (long long)fd.nt * b->ts;
-        b->total_part += 2LL * fd.nt;
-        b->total_cnt += fd.nt + 2 * xg_num_lower_tiles(fd.nt);
+        b->total_part += 2LL * fd.nb;
         if (fd.nt > b->maxnt) b->maxnt = fd.nt;
     }
     const size_t tile = (size_t)b->ts * b->ts;
@@ -349,20 +384,22 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
     std::vector<long long> cnt(nfields);
     for (int f = 0; f < nfields; ++f) cnt[f] = xg_num_lower_tiles(b->F[f].nt) * (b->ts / 8);
     xg_table_fill(b->gen, cnt);
-    /* the scheduler's task list: a critical-path-first list schedule over
-     * every field's tasks for the launch's CTAs (xg_batch_plan) */
+    /* the DAG's tasks and the backward solve's */
     {
-        std::vector<int> nts(nfields);
-        for (int f = 0; f < nfields; ++f) nts[f] = b->F[f].nt;
         std::vector<int4> tl;
-        xg_batch_plan(nts, g_xg.sm_count, tl);
+        std::vector<int2> tt;
+        xg_batch_order(D, tl, tt);
         b->ntasks = (long long)tl.size();
+        b->nttasks = (long long)tt.size();
         e = cudaMalloc(&b->tasks, tl.size() * sizeof(int4));
         if (e == cudaSuccess) e = cudaMemcpy(b->tasks, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&b->cnt, (size_t)b->total_cnt * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&b->next, sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMalloc(&b->abort_flag, sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&b->dinv, (size_t)g_xg.sm_count * b->ts * 32 * sizeof(double));
+        if (e == cudaSuccess) e = cudaMalloc(&b->ttasks, tt.size() * sizeof(int2));
+        if (e == cudaSuccess) e = cudaMemcpy(b->ttasks, tt.data(), tt.size() * sizeof(int2), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMalloc(&b->D_dev, nfields * sizeof(XgDagField));
+        if (e == cudaSuccess) e = cudaMemcpy(b->D_dev, D.data(), nfields * sizeof(XgDagField), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMalloc(&b->words, (size_t)(2 + b->total_flags) * sizeof(int));
+        if (e == cudaSuccess) e = cudaMalloc(&b->twords, (size_t)(2 + b->total_tflags) * sizeof(int));
+        if (e == cudaSuccess) e = cudaMalloc(&b->dinv, (size_t)b->total_vec * 32 * sizeof(double));
         if (e != cudaSuccess) {
             xg_batch_free(b);
             return xg_fail(XG_ERR_NO_MEMORY, "batch task list (%lld tasks): %s", (long long)tl.size(),
@@ -405,20 +442,23 @@ static void xg_batch_record(XgBatch *b, cudaStream_t st)
 {
     XgTileArgs base{b->tiles, b->ts, 0};
     cudaMemsetAsync(b->status, 0, 2 * (size_t)b->nfields * sizeof(int), st);
-    cudaMemsetAsync(b->cnt, 0, (size_t)b->total_cnt * sizeof(int), st);
-    cudaMemsetAsync(b->next, 0, sizeof(unsigned long long), st);
-    cudaMemsetAsync(b->abort_flag, 0, sizeof(int), st);
+    cudaMemsetAsync(b->words, 0, (size_t)(2 + b->total_flags) * sizeof(int), st);
     cudaMemcpyAsync(b->v, b->z, b->total_vec * sizeof(double), cudaMemcpyDeviceToDevice, st);
     xg_launch_batch_gen(base, b->F_dev, b->gen.dev, b->gen.blocks, b->x, b->y, b->metric, st);
-    XgSched sch;
-    sch.tasks = b->tasks;
-    sch.ntasks = b->ntasks;
-    sch.next = b->next;
-    sch.abort = b->abort_flag;
-    sch.cnt = b->cnt;
-    sch.dinv = b->dinv;
-    const int ctas = (int)std::min<long long>(g_xg.sm_count, b->ntasks);
-    xg_launch_batch_sched(b->map, base, b->F_dev, sch, ctas, b->v, b->part, b->status, st);
+    XgDag G = {};
+    G.data = b->tiles;
+    G.ts = b->ts;
+    G.F = b->D_dev;
+    G.tasks = b->tasks;
+    G.ntasks = b->ntasks;
+    G.next = (unsigned *)b->words;
+    G.abort = b->words + 1;
+    G.flags = b->words + 2;
+    G.dinv = b->dinv;
+    G.v = b->v;
+    G.part = b->part;
+    G.status = b->status;
+    xg_launch_dag(b->map, G, g_xg.sm_count, st);
     xg_launch_batch_finalize(b->F_dev, b->nfields, b->part, b->out, st);
 }
 
@@ -502,6 +542,7 @@ static int xg_batch_grad_workspace(XgBatch *b)
                                  ts);
         if (rc) return rc;
     }
+    XG_CU(cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming));
     XG_CU(cudaMalloc(&b->gout, 4 * (size_t)b->nfields * sizeof(double)));
     XG_CU(cudaMallocHost(&b->h_gout, 4 * (size_t)b->nfields * sizeof(double)));
     return XG_OK;
@@ -510,7 +551,7 @@ static int xg_batch_grad_workspace(XgBatch *b)
 /* Log-likelihoods and their gradients of every field: the batched
  * factorisation (the graph of exageostat_b200_batch_loglik), then per field,
  * round-robin over eight streams, the adjoint of the single-field path on
- * that field's tiles -- alpha = L^-T v by backward tile solves, X = L^-T,
+ * that field's tiles (alpha = L^-T v of all fields in one launch before) -- X = L^-T,
  * Sigma^-1 = X X^T over the factor, and the fused contraction with the
  * on-the-fly dSigma/dtheta tiles.  A field that is not positive definite
  * gets loglik -inf and a NaN gradient. */
@@ -524,6 +565,27 @@ extern "C" int exageostat_b200_batch_loglik_grad(void *handle, const double *the
     if (rc) return rc;
     const int ts = b->ts;
     const int np = b->kernel == 1 ? 4 : 3;
+    /* alpha = L^-T v of every field in one launch, before the adjoints (the
+     * gradient streams start after it) */
+    {
+        cudaStream_t st = g_xg.stream;
+        XG_CU(cudaMemsetAsync(b->twords, 0, (size_t)(2 + b->total_tflags) * sizeof(int), st));
+        XgTrsv G = {};
+        G.data = b->tiles;
+        G.ts = ts;
+        G.F = b->D_dev;
+        G.tasks = b->ttasks;
+        G.ntasks = b->nttasks;
+        G.next = (unsigned *)b->twords;
+        G.abort = b->twords + 1;
+        G.flags = b->twords + 2;
+        G.dinv = b->dinv;
+        G.v = b->v;
+        G.status = b->status;
+        xg_launch_trsv_lower_t(G, g_xg.sm_count, st);
+        XG_CU(cudaEventRecord(b->ev, st));
+        for (int s = 0; s < XgBatch::GS; ++s) XG_CU(cudaStreamWaitEvent(b->gst[s], b->ev, 0));
+    }
     for (int f = 0; f < b->nfields; ++f) {
         if (!std::isfinite(loglik[f])) continue;
         const XgBField &fd = b->F[f];
@@ -532,7 +594,6 @@ extern "C" int exageostat_b200_batch_loglik_grad(void *handle, const double *the
         XgTileArgs T{b->tiles + fd.tile_off * (long long)ts * ts, ts, fd.nt};
         double *vf = b->v + fd.vec_off;
         int *stf = b->status + 2 * f;
-        for (int k = fd.nt - 1; k >= 0; --k) xg_launch_trsv_lower_t_step(T, k, vf, stf, st);
         xg_launch_inverse_factor(b->gX[s].map, b->fmap[f], b->gX[s].d, T.data, fd.nt, ts, stf, st);
         xg_launch_inverse_syrk(b->gX[s].map, T.data, fd.nt, ts, stf, st);
         const double dlogcon = -(log(2.0) + xg_digamma(fd.p.nu));

@@ -518,25 +518,6 @@ __global__ void __launch_bounds__(XG_POTRF_THREADS) xg_potrf_diag_kernel(XgTileA
     xg_potrf_body<NB>(T, k, v, part_logdet, part_dot, with_rhs, status, info);
 }
 
-/* batched: one CTA per field active at step k; info records the first
- * failing column of any field */
-template <int NB>
-__global__ void __launch_bounds__(XG_POTRF_THREADS) xg_potrf_diag_batch_kernel(XgTileArgs base,
-                                                                               const XgBField *__restrict__ F,
-                                                                               XgBStep S, int k, double *v,
-                                                                               double *part, int *status, int *info)
-{
-    long long local;
-    const int f = xg_batch_resolve(S, blockIdx.x, &local);
-    const XgBField &fd = F[f];
-    XgTileArgs T = base;
-    T.data = base.data + fd.tile_off * (long long)base.ts * base.ts;
-    T.nt = fd.nt;
-    /* per-field status words: status[2 f] (flags), status[2 f + 1] (info) */
-    xg_potrf_body<NB>(T, k, v + fd.vec_off, part + fd.part_off, part + fd.part_off + fd.nt, 1, status + 2 * f,
-                      status + 2 * f + 1);
-}
-
 /* ========================================================================== */
 /* Inverses of the 32 x 32 diagonal blocks of L_kk (for the panel TRSM)       */
 /* ========================================================================== */
@@ -730,20 +711,6 @@ __global__ void __launch_bounds__(XG_TRSM_THREADS, 1) xg_trsm_panel_kernel(XgTil
                                                                         int with_rhs, const int *status)
 {
     xg_trsm_body(T, k, v, with_rhs, status, blockIdx.x);
-}
-
-__global__ void __launch_bounds__(XG_TRSM_THREADS, 1) xg_trsm_panel_batch_kernel(XgTileArgs base,
-                                                                              const XgBField *__restrict__ F,
-                                                                              XgBStep S, int k, double *v,
-                                                                              const int *status)
-{
-    long long local;
-    const int f = xg_batch_resolve(S, blockIdx.x, &local);
-    const XgBField &fd = F[f];
-    XgTileArgs T = base;
-    T.data = base.data + fd.tile_off * (long long)base.ts * base.ts;
-    T.nt = fd.nt;
-    xg_trsm_body(T, k, v + fd.vec_off, 1, status + 2 * f, local);
 }
 
 /* ========================================================================== */
@@ -954,22 +921,6 @@ __global__ void __launch_bounds__(XG_G_THREADS, 1) xg_syrk_gemm_kernel(const __g
                                                                        int *status)
 {
     xg_gemm_body(map, T, k, j0, single_col, status, blockIdx.x);
-}
-
-/* batched: the trailing update of step k of every field with nt > k + 1 */
-__global__ void __launch_bounds__(XG_G_THREADS, 1) xg_syrk_gemm_batch_kernel(const __grid_constant__ CUtensorMap map,
-                                                                             XgTileArgs base,
-                                                                             const XgBField *__restrict__ F,
-                                                                             XgBStep S, int k, int *status)
-{
-    long long local;
-    const int f = xg_batch_resolve(S, blockIdx.x, &local);
-    const XgBField &fd = F[f];
-    XgTileArgs T = base;
-    T.data = base.data + fd.tile_off * (long long)base.ts * base.ts;
-    T.nt = fd.nt;
-    T.tile_off = fd.tile_off;
-    xg_gemm_body(map, T, k, k + 1, 0, status + 2 * f, local);
 }
 
 /* ========================================================================== */
@@ -1303,160 +1254,6 @@ __global__ void __launch_bounds__(XG_G_THREADS, 1) xg_potrf_sub_gemm_kernel(cons
 }
 
 /* ========================================================================== */
-/* Batched factorisation in one persistent launch (device tile scheduler)     */
-/* ========================================================================== */
-
-__device__ __forceinline__ int xg_ld_acquire(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void xg_add_release(int *p, int v)
-{
-    asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-/* thread 0: waits until *p >= target; false when the wall-time limit passes
- * or another CTA aborted the launch */
-__device__ __forceinline__ bool xg_sched_wait(const int *p, int target, const int *abort, uint64_t t0)
-{
-    while (xg_ld_acquire(p) < target) {
-        if (*(volatile const int *)abort) return false;
-        if (xg_globaltimer_ns() - t0 > 2000000000ull) return false;
-        __nanosleep(256);
-    }
-    return true;
-}
-
-/* Persistent CTAs (one per SM, 256 threads) run the task list of XgSched:
- * thread 0 takes the next task, waits for its dependency counters, the CTA
- * runs the task body (the POTRF, TRSM and DMMA update bodies of the per-step
- * kernels, with L2-coherent loads), and thread 0 publishes it (release).
- * Tasks are taken in a topological order, so every task waited on was taken
- * earlier by a CTA that is running: the launch cannot deadlock.  A wait that
- * times out sets the field's XG_ST_TIMEOUT bit and the abort flag; a field
- * whose pivot fails skips its remaining bodies (status word) but still
- * publishes them, so no other field waits on it. */
-template <int NB>
-__global__ void __launch_bounds__(XG_G_THREADS, 1)
-    xg_batch_sched_kernel(const __grid_constant__ CUtensorMap map, XgTileArgs base, const XgBField *__restrict__ F,
-                          XgSched sch, double *v, double *part, int *status)
-{
-    __shared__ int4 s_task;
-    __shared__ int s_go;
-    const int tid = threadIdx.x;
-    const int ts = base.ts;
-    for (;;) {
-        __syncthreads(); /* the previous task is finished by every thread */
-        if (tid == 0) {
-            int4 t = make_int4(-1, 0, 0, 0);
-            if (!*(volatile int *)sch.abort) {
-                const unsigned long long q = atomicAdd(sch.next, 1ULL);
-                if (q < (unsigned long long)sch.ntasks) t = sch.tasks[q];
-            }
-            s_task = t;
-        }
-        __syncthreads();
-        const int4 tk = s_task;
-        if (tk.x < 0) break;
-        const int type = tk.x & 3, f = tk.x >> 2, i = tk.y, j = tk.z, k = tk.w;
-        const XgBField &fd = F[f];
-        XgTileArgs T = base;
-        T.data = base.data + fd.tile_off * (long long)ts * ts;
-        T.nt = fd.nt;
-        T.tile_off = fd.tile_off;
-        int *stf = status + 2 * f;
-        int *pdone = sch.cnt + fd.sched_off;
-        int *tdone = pdone + fd.nt;
-        int *ucnt = tdone + xg_num_lower_tiles(fd.nt);
-        if (tid == 0) {
-            const uint64_t t0 = xg_globaltimer_ns();
-            bool ok;
-            if (type == XG_TASK_POTRF)
-                ok = xg_sched_wait(ucnt + xg_tile_index(k, k, fd.nt), k, sch.abort, t0);
-            else if (type == XG_TASK_TRSM)
-                ok = xg_sched_wait(pdone + k, 1, sch.abort, t0) &&
-                     xg_sched_wait(ucnt + xg_tile_index(i, k, fd.nt), k, sch.abort, t0);
-            else
-                ok = xg_sched_wait(tdone + xg_tile_index(i, k, fd.nt), 1, sch.abort, t0) &&
-                     xg_sched_wait(tdone + xg_tile_index(j, k, fd.nt), 1, sch.abort, t0) &&
-                     xg_sched_wait(ucnt + xg_tile_index(i, j, fd.nt), k, sch.abort, t0);
-            if (!ok) {
-                atomicOr(stf, XG_ST_TIMEOUT);
-                atomicExch(sch.abort, 1);
-            }
-            s_go = ok ? 1 : 0;
-        }
-        __syncthreads();
-        if (s_go) {
-            if (type == XG_TASK_POTRF) {
-                xg_potrf_body<NB, true, true>(T, k, v + fd.vec_off, part + fd.part_off, part + fd.part_off + fd.nt, 1, stf,
-                                        stf + 1);
-            } else if (type == XG_TASK_TRSM) {
-                /* the inverted diagonal blocks of L_kk into this CTA's scratch
-                 * (warp w: blocks w, w + 8, ...), then the tile's row strips;
-                 * done even for a field that has failed (its strips then skip),
-                 * so every thread takes the same path */
-                {
-                    extern __shared__ __align__(16) double xg_smem_d[];
-                    const int warp = tid >> 5, lane = tid & 31;
-                    double *LB = xg_smem_d + warp * (32 * 33);
-                    double *D = sch.dinv + (long long)blockIdx.x * ts * 32;
-                    const double *Lkk = T.data + xg_tile_index(k, k, fd.nt) * (long long)ts * ts;
-                    for (int bb = warp; bb < ts / 32; bb += XG_G_THREADS / 32) {
-                        const double *Lb = Lkk + (long long)(bb * 32) * ts + bb * 32;
-                        for (int r = 0; r < 32; ++r) LB[r * 33 + lane] = __ldcg(Lb + (long long)r * ts + lane);
-                        __syncwarp();
-                        xg_lower32_inverse(LB, lane, D + (long long)(bb * 32) * 32);
-                        __syncwarp();
-                    }
-                    T.dinv = D;
-                }
-                __syncthreads();
-                /* the tile's 128-row blocks one after the other (xg_trsm_gemm_body;
-                 * a field that has failed skips them uniformly) */
-                if (!xg_cta_should_skip(stf))
-                    for (int rb = 0; rb < ts / XG_TB; ++rb)
-                        if (!xg_trsm_gemm_body<true>(map, T, k, i, rb, v + fd.vec_off, 1, stf)) break;
-            } else {
-                const int bpt = ts / XG_G_BM;
-                for (int b = 0; b < bpt * bpt; ++b)
-                    xg_gemm_body<true>(map, T, k, j, 1, stf, (long long)(i - j) * bpt * bpt + b);
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            if (type == XG_TASK_POTRF)
-                xg_add_release(pdone + k, 1);
-            else if (type == XG_TASK_TRSM)
-                xg_add_release(tdone + xg_tile_index(i, k, fd.nt), 1);
-            else
-                xg_add_release(ucnt + xg_tile_index(i, j, fd.nt), 1);
-        }
-    }
-}
-
-static size_t xg_sched_smem_bytes(int ts)
-{
-    size_t b = xg_trsm_gemm_smem_bytes();
-    b = b > xg_gemm_smem_bytes() ? b : xg_gemm_smem_bytes();
-    b = b > xg_potrf_smem_bytes(ts) ? b : xg_potrf_smem_bytes(ts);
-    b = b > xg_trsm_smem_bytes(ts) ? b : xg_trsm_smem_bytes(ts);
-    return b;
-}
-
-void xg_launch_batch_sched(const CUtensorMap &map, const XgTileArgs &base, const XgBField *F, const XgSched &sch,
-                           int ctas, double *v, double *part, int *status, cudaStream_t st)
-{
-    if (sch.ntasks <= 0 || ctas <= 0) return;
-    xg_batch_sched_kernel<32><<<ctas, XG_G_THREADS, xg_sched_smem_bytes(base.ts), st>>>(map, base, F, sch, v, part,
-                                                                                          status);
-}
-
-/* ========================================================================== */
 /* Log-likelihood assembly                                                    */
 /* ========================================================================== */
 
@@ -1487,9 +1284,9 @@ __global__ void xg_finalize_batch_kernel(const XgBField *__restrict__ F, int nfi
     if (f >= nfields) return;
     const XgBField &fd = F[f];
     double det = 0.0, dot = 0.0;
-    for (int k = 0; k < fd.nt; ++k) {
+    for (int k = 0; k < fd.nb; ++k) {
         det += part[fd.part_off + k];
-        dot += part[fd.part_off + fd.nt + k];
+        dot += part[fd.part_off + fd.nb + k];
     }
     const double logdet = 2.0 * det;
     out[2 * f] = -0.5 * dot - 0.5 * logdet - (double)(fd.N / 2.0) * log(2.0 * 3.141592653589793);
@@ -1517,18 +1314,6 @@ cudaError_t xg_kernels_configure()
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(xg_syrk_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)xg_gemm_smem_bytes());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(xg_potrf_diag_batch_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)xg_potrf_smem_bytes(512));
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(xg_trsm_panel_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)xg_trsm_smem_bytes(XG_MAX_TS));
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(xg_syrk_gemm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)xg_gemm_smem_bytes());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(xg_batch_sched_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)xg_sched_smem_bytes(XG_MAX_TS));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(xg_potrf_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_POTRF_SUB_SMEM);
     if (e != cudaSuccess) return e;
@@ -1635,30 +1420,6 @@ void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, const XgBSte
                          const double *x, const double *y, int metric, cudaStream_t st)
 {
     if (blocks > 0) xg_gen_matern_batch_kernel<<<(unsigned)blocks, 256, 0, st>>>(base, F, S, x, y, metric);
-}
-
-void xg_launch_batch_potrf(const XgTileArgs &base, const XgBField *F, const XgBStep &S, int k, double *v, double *part,
-                           int *status, int *info, cudaStream_t st)
-{
-    if (S.nact <= 0) return;
-    xg_potrf_diag_batch_kernel<32><<<S.nact, XG_POTRF_THREADS, xg_potrf_smem_bytes(base.ts), st>>>(
-        base, F, S, k, v, part, status, info);
-}
-
-void xg_launch_batch_trsm(const XgTileArgs &base, const XgBField *F, const XgBStep &S, long long blocks, int k,
-                          double *v, const int *status, cudaStream_t st)
-{
-    if (blocks > 0)
-        xg_trsm_panel_batch_kernel<<<(unsigned)blocks, XG_TRSM_THREADS, xg_trsm_smem_bytes(base.ts), st>>>(
-            base, F, S, k, v, status);
-}
-
-void xg_launch_batch_gemm(const CUtensorMap &map, const XgTileArgs &base, const XgBField *F, const XgBStep &S,
-                          long long blocks, int k, int *status, cudaStream_t st)
-{
-    if (blocks > 0)
-        xg_syrk_gemm_batch_kernel<<<(unsigned)blocks, XG_G_THREADS, xg_gemm_smem_bytes(), st>>>(map, base, F, S, k,
-                                                                                               status);
 }
 
 void xg_launch_batch_finalize(const XgBField *F, int nfields, const double *part, double *out, cudaStream_t st)

@@ -95,6 +95,7 @@ int xg_context_start(int dts)
     if (e == cudaSuccess) e = xg_gradient_kernels_configure();
     if (e == cudaSuccess) e = xg_mixed_kernels_configure();
     if (e == cudaSuccess) e = xg_dag_kernels_configure();
+    if (e == cudaSuccess) e = xg_solve_kernels_configure();
     if (e == cudaSuccess) e = xg_sliced_kernels_configure();
     if (e != cudaSuccess) return xg_cuda_fail(e, "kernel attribute setup");
     g_xg.device = dev;
@@ -155,7 +156,8 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
         M.dinv = nullptr;
         return xg_cuda_fail(e, "diagonal-block inverses");
     }
-    e = cudaMalloc(&M.dag, sizeof(int) * (size_t)xg_dag_words((N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK));
+    const int nb = (N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    e = cudaMalloc(&M.dag, sizeof(int) * (size_t)(xg_dag_words(nb) + xg_trsv_words(nb)));
     if (e != cudaSuccess) {
         M.dag = nullptr;
         return xg_cuda_fail(e, "block flags");
@@ -337,6 +339,27 @@ static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, 
     return nb;
 }
 
+/* v <- L^-T v for a factored M */
+void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st)
+{
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    int *words = M.dag + xg_dag_words(nb);
+    cudaMemsetAsync(words, 0, sizeof(int) * (size_t)xg_trsv_words(nb), st);
+    XgTrsv G = {};
+    G.data = M.d;
+    G.ts = M.ts;
+    G.one.nt = M.nt;
+    G.one.nb = nb;
+    G.ntasks = nb;
+    G.next = (unsigned *)words;
+    G.abort = words + 1;
+    G.flags = words + 2;
+    G.dinv = M.dinv;
+    G.v = v;
+    G.status = status;
+    xg_launch_trsv_lower_t(G, g_xg.sm_count, st);
+}
+
 /* Cholesky of M in place; with v != nullptr also v <- L^-1 v.  Returns the
  * number n of partial sums of either kind: log-det in part[0:n], |v|^2 in
  * part[n:2n].  Up to XG_DAG_MAX_N one launch of the tile DAG, else a
@@ -353,7 +376,6 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
     /* profiled evaluations keep the per-step launches, whose kernels the profile tells apart */
     if (M.dag && !fs.pev && M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, fs.st);
     XgTileArgs T{M.d, M.ts, M.nt};
-    T.dinv = M.dinv;
     const bool la = fs.st_hi != nullptr;
     cudaStream_t sp = la ? fs.st_hi : fs.st; /* panel stream */
     cudaEvent_t *pev = fs.pev;
@@ -362,6 +384,7 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
         cudaEventRecord(fs.ev_upd, fs.st); /* the generated matrix */
     }
     for (int k = 0; k < M.nt; ++k) {
+        if (M.dinv) T.dinv = M.dinv + (size_t)k * M.ts * 32;
         if (la) cudaStreamWaitEvent(sp, fs.ev_upd, 0);
         if (pev) cudaEventRecord(pev[5 * k], sp);
         xg_launch_potrf_tiled(M.map, T, k, v, part, part + M.nt, rhs, status, info, sp);
@@ -707,7 +730,7 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
     const XgMaternParams p = xg_params(theta, f->kernel);
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
-    for (int k = f->C.nt - 1; k >= 0; --k) xg_launch_trsv_lower_t_step(T, k, f->v, f->status, st);
+    xg_solve_transposed(f->C, f->v, f->status, st);
     xg_launch_inverse_factor(f->X.map, f->C.map, f->X.d, f->C.d, f->C.nt, f->C.ts, f->status, st);
     xg_launch_inverse_syrk(f->X.map, f->C.d, f->C.nt, f->C.ts, f->status, st);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, f->C.nt, f->C.ts, f->x, f->y, f->v, f->N, p, f->kernel,
@@ -1204,7 +1227,6 @@ static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
     XgSliced *sl = f->sl;
     XgTileMatrix &M = f->C;
     XgTileArgs T{M.d, M.ts, M.nt};
-    T.dinv = M.dinv;
     const int nt = M.nt;
     const long long plane = sl->plane_rows * M.ts;
     const int pr = (int)sl->plane_rows;
@@ -1220,6 +1242,7 @@ static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
     const int all = 1 << 30; /* one CTA per job */
     if (la) cudaEventRecord(sl->ev_a, fs.st); /* the generated matrix */
     for (int j = 0; j < nt; ++j) {
+        T.dinv = M.dinv + (size_t)j * M.ts * 32;
         if (la) cudaStreamWaitEvent(sp, sl->ev_a, 0); /* chunks k < j-1 of column j */
         rec(j, 0, sp);
         const int band_ctas = xg_panel_share(j, sms), upd_ctas = sms - band_ctas;
@@ -1233,10 +1256,7 @@ static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
         rec(j, 1, sp);
         xg_launch_potrf_tiled(M.map, T, j, v, f->part, f->part + nt, rhs, f->status, f->info, sp);
         rec(j, 2, sp);
-        if (T.dinv)
-            xg_launch_trsm_gemm(M.map, T, j, v, rhs, f->status, sp);
-        else
-            xg_launch_trsm_panel(T, j, v, rhs, f->status, sp);
+        xg_launch_trsm_gemm(M.map, T, j, v, rhs, f->status, sp);
         if (j + 1 < nt) xg_launch_slice_panel(T, j, 0, sl->dig, sl->scale, plane, f->status, sp);
         rec(j, 3, sp);
         if (la) {
@@ -1413,7 +1433,7 @@ int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, do
     const XgMaternParams p = xg_params(theta, f->kernel);
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
-    for (int k = nt - 1; k >= 0; --k) xg_launch_trsv_lower_t_step(T, k, f->v, f->status, st);
+    xg_solve_transposed(f->C, f->v, f->status, st);
     xg_launch_identity_x(f->X.d, nt, ts, st);
     /* X = L^-T column by column: the update of column b from the finished
      * columns c < b (INT8-sliced), the FP64 solve with L_bb, the slicing of
@@ -1664,7 +1684,7 @@ int xg_predict_run(XgPredict *q, const double *theta, int kernel, int metric, co
     fs.ev_panel = q->ev_panel;
     fs.ev_upd = q->ev_upd;
     xg_factor_lookahead(q->C22, q->v, q->part, q->status, q->info(), fs);
-    for (int k = q->C22.nt - 1; k >= 0; --k) xg_launch_trsv_lower_t_step(T, k, q->v, q->status, st);
+    xg_solve_transposed(q->C22, q->v, q->status, st);
     /* zmiss = Sigma(miss, obs) alpha, C12 generated on the fly */
     xg_launch_predict_cross(q->xm, q->ym, nmiss, q->xo, q->yo, nobs, q->v, p, metric, q->zmiss, st);
     if (zactual) xg_launch_mse(q->zact, q->zmiss, nmiss, q->out, st);

@@ -51,67 +51,173 @@ void xg_launch_trmv_lower(const XgTileArgs &T, const double *e, double *z, const
     xg_trmv_lower_kernel<<<T.nt * (T.ts / 32), 256, 0, st>>>(T, e, z, status);
 }
 
-/* ---- alpha = L^-T v, right-looking over tile columns from the last ---- */
+/* ---- alpha = L^-T v ---- */
 
-/* Diagonal tile k: solve L_kk^T a = v_k in place, 32-row blocks from the
- * bottom; within a block one lane per row, then the rows above are updated
- * by all threads. */
-__global__ void __launch_bounds__(512) xg_trsv_lt_diag_kernel(XgTileArgs T, int k, double *__restrict__ v,
-                                                              const int *status)
+#define XG_TL_THREADS 256
+#define XG_TL_LDS 130 /* row stride of the staged L_JJ */
+#define XG_TL_SMEM ((128 * XG_TL_LDS + 128 * 33 + 8 * 128 + 128 + 128) * 8)
+
+__device__ __forceinline__ bool xg_trsv_wait(const int *p, const int *abort)
 {
-    if (xg_cta_should_skip(status)) return;
-    const int ts = T.ts;
-    extern __shared__ double vsh[];
-    const double *L = T.data + xg_tile_index(k, k, T.nt) * (long long)ts * ts;
-    double *vk = v + (long long)k * ts;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int r = tid; r < ts; r += blockDim.x) vsh[r] = vk[r];
-    __syncthreads();
-    for (int b0 = ts - 32; b0 >= 0; b0 -= 32) {
-        if (warp == 0) {
-            /* L_D^T a_D = w_D, L_D = L[b0:b0+32, b0:b0+32] lower: backward substitution */
-            double w = vsh[b0 + lane];
-            for (int j = 31; j >= 0; --j) {
-                if (lane == j) w = w / L[(long long)(b0 + j) * ts + b0 + j];
-                const double aj = __shfl_sync(0xffffffffu, w, j);
-                if (lane < j) w -= L[(long long)(b0 + j) * ts + b0 + lane] * aj;
-            }
-            vsh[b0 + lane] = w;
-        }
-        __syncthreads();
-        /* rows above: w[c] -= sum_{r in block} L[r][c] a[r], c < b0 */
-        for (int c = tid; c < b0; c += blockDim.x) {
-            double s = vsh[c];
-#pragma unroll 8
-            for (int r = 0; r < 32; ++r) s -= L[(long long)(b0 + r) * ts + c] * vsh[b0 + r];
-            vsh[c] = s;
-        }
-        __syncthreads();
+    int v;
+    const uint64_t t0 = xg_globaltimer_ns();
+    for (uint32_t it = 1;; ++it) {
+        asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        if (v) return true;
+        if ((it & 63u) == 0u &&
+            (*(volatile const int *)abort || xg_globaltimer_ns() - t0 > 2000000000ull))
+            return false;
     }
-    for (int r = tid; r < ts; r += blockDim.x) vk[r] = vsh[r];
 }
 
-/* Tiles i < k: v_i -= L_ki^T a_k; one CTA per (i, 256-column chunk). */
-__global__ void __launch_bounds__(256) xg_trsv_lt_update_kernel(XgTileArgs T, int k, double *__restrict__ v,
-                                                                const int *status)
+/* Block column J of the backward solve is one task of one CTA:
+ *   w = v_J - sum_{I > J} L_IJ^T a_I  (I from the last block up), a_J = L_JJ^-T w.
+ * Persistent CTAs take the columns from the last one down, so a task waits
+ * only on tasks taken earlier.  The entries of a block are in registers
+ * before its a_I is waited for, and L_JJ with the inverses of its 32 x 32
+ * diagonal blocks in shared memory before the first wait, so the serial chain
+ * per 128 rows is one flag, one 128-term product and four 32-row steps.
+ * Bound: the chain (about 5 us per 128 rows), and one read of L for large N;
+ * the launches per tile row that this replaces took 230 us (ts = 256) to
+ * 450 us (ts = 512) each for the serial substitution in the diagonal tile. */
+__global__ void __launch_bounds__(XG_TL_THREADS, 1) xg_trsv_lt_kernel(XgTrsv G)
 {
-    if (*status != 0) return;
-    const int ts = T.ts;
-    const int chunks = (ts + 255) / 256;
-    const int i = blockIdx.x / chunks;
-    const int c = (blockIdx.x % chunks) * 256 + threadIdx.x;
-    if (c >= ts) return;
-    const double *tile = T.data + xg_tile_index(k, i, T.nt) * (long long)ts * ts;
-    const double *ak = v + (long long)k * ts;
-    double s = 0.0;
-    for (int r = 0; r < ts; ++r) s += tile[(long long)r * ts + c] * ak[r];
-    v[(long long)i * ts + c] -= s;
+    extern __shared__ __align__(16) double xg_smem_d[];
+    double *LS = xg_smem_d;             /* [128][130] L_JJ */
+    double *DS = LS + 128 * XG_TL_LDS;  /* [128][33] its inverted 32 x 32 diagonal blocks */
+    double *red = DS + 128 * 33;        /* [8][128] */
+    double *w = red + 8 * 128;          /* [128] */
+    double *a = w + 128;                /* [128] */
+    __shared__ long long s_task;
+    __shared__ int s_skip, s_bad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ts = G.ts, b = ts / 128;
+    if (tid == 0) s_bad = 0;
+    for (bool first = true;; first = false) {
+        __syncthreads();
+        if (tid == 0) {
+            long long q = first ? (long long)blockIdx.x : (long long)gridDim.x + (long long)atomicAdd(G.next, 1u);
+            if (q >= G.ntasks || *(volatile int *)G.abort) q = -1;
+            s_task = q;
+        }
+        __syncthreads();
+        const long long q = s_task;
+        if (q < 0) break;
+        const int2 t = G.tasks ? G.tasks[q] : make_int2(0, G.one.nb - 1 - (int)q);
+        const int f = t.x, J = t.y;
+        const XgDagField fd = G.tasks ? G.F[f] : G.one;
+        const int nt = fd.nt, nb = fd.nb, j = J / b, cj = J % b * 128;
+        int *flags = G.flags + fd.tflag_off;
+        double *v = G.v + fd.vec_off;
+        if (tid == 0) s_skip = *(volatile int *)(G.status + 2 * f) != 0;
+        __syncthreads();
+        if (s_skip) continue; /* the whole field is skipped: nobody waits for the flag */
+        const double *Ljj = G.data + (fd.tile_off + xg_tile_index(j, j, nt)) * (long long)ts * ts + (long long)cj * ts + cj;
+        const double *D = G.dinv + (fd.dinv_off + (long long)J * 128) * 32;
+#pragma unroll 8
+        for (int u = 0; u < 32; ++u) {
+            const int idx = tid + u * XG_TL_THREADS, r = idx >> 6, c = idx & 63;
+            const double2 x = *(reinterpret_cast<const double2 *>(Ljj + (long long)r * ts) + c);
+            *reinterpret_cast<double2 *>(LS + r * XG_TL_LDS + 2 * c) = x;
+        }
+#pragma unroll 8
+        for (int u = 0; u < 16; ++u) {
+            const int idx = tid + u * XG_TL_THREADS;
+            DS[(idx >> 5) * 33 + (idx & 31)] = D[idx];
+        }
+        if (tid < 128) w[tid] = v[J * 128 + tid];
+        /* warp: rows 16 warp .. + 15 of each block; lane: columns 2 lane, + 1, 64 + 2 lane, + 1 */
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        bool ok = true;
+        for (int I = nb - 1; I > J && ok; --I) {
+            const int i = I / b;
+            const double *T = G.data + (fd.tile_off + xg_tile_index(i, j, nt)) * (long long)ts * ts +
+                              (long long)(I % b * 128 + 16 * warp) * ts + cj + 2 * lane;
+            double2 x[16][2];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                x[r][0] = *reinterpret_cast<const double2 *>(T + (long long)r * ts);
+                x[r][1] = *reinterpret_cast<const double2 *>(T + (long long)r * ts + 64);
+            }
+            if (lane == 0) ok = xg_trsv_wait(flags + I, G.abort);
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            __syncwarp(); /* lane 0's acquire orders the other lanes' loads */
+            double av = 0.0;
+            if (lane < 16)
+                asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];"
+                             : "=d"(av)
+                             : "l"(v + I * 128 + 16 * warp + lane)
+                             : "memory");
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const double ar = __shfl_sync(0xffffffffu, av, r);
+                acc[0] = fma(x[r][0].x, ar, acc[0]);
+                acc[1] = fma(x[r][0].y, ar, acc[1]);
+                acc[2] = fma(x[r][1].x, ar, acc[2]);
+                acc[3] = fma(x[r][1].y, ar, acc[3]);
+            }
+        }
+        if (!ok) s_bad = 1;
+        *reinterpret_cast<double2 *>(red + warp * 128 + 2 * lane) = make_double2(acc[0], acc[1]);
+        *reinterpret_cast<double2 *>(red + warp * 128 + 64 + 2 * lane) = make_double2(acc[2], acc[3]);
+        __syncthreads();
+        if (s_bad) {
+            if (tid == 0) {
+                atomicOr(G.status + 2 * f, XG_ST_TIMEOUT);
+                atomicExch(G.abort, 1);
+            }
+            return;
+        }
+        if (tid < 128) {
+            double sum = 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) sum += red[u * 128 + tid];
+            w[tid] -= sum;
+        }
+        __syncthreads();
+        /* a_JJ block by block from the bottom: a_q = D_q^T w_q, then w above -= L_q^T a_q */
+#pragma unroll 1
+        for (int qb = 3; qb >= 0; --qb) {
+            if (warp == 0) {
+                double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+                for (int r = 0; r < 32; r += 2) {
+                    s0 = fma(DS[(32 * qb + r) * 33 + lane], w[32 * qb + r], s0);
+                    s1 = fma(DS[(32 * qb + r + 1) * 33 + lane], w[32 * qb + r + 1], s1);
+                }
+                a[32 * qb + lane] = s0 + s1;
+            }
+            __syncthreads();
+            if (warp < qb) {
+                double s0 = w[32 * warp + lane], s1 = 0.0;
+#pragma unroll
+                for (int r = 0; r < 32; r += 2) {
+                    s0 = fma(-LS[(32 * qb + r) * XG_TL_LDS + 32 * warp + lane], a[32 * qb + r], s0);
+                    s1 = fma(-LS[(32 * qb + r + 1) * XG_TL_LDS + 32 * warp + lane], a[32 * qb + r + 1], s1);
+                }
+                w[32 * warp + lane] = s0 + s1;
+            }
+            __syncthreads();
+        }
+        if (tid < 128) {
+            v[J * 128 + tid] = a[tid];
+            __threadfence();
+        }
+        __syncthreads();
+        if (tid == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(flags + J), "r"(1) : "memory");
+    }
 }
 
-void xg_launch_trsv_lower_t_step(const XgTileArgs &T, int k, double *v, const int *status, cudaStream_t st)
+cudaError_t xg_solve_kernels_configure()
 {
-    xg_trsv_lt_diag_kernel<<<1, 512, T.ts * sizeof(double), st>>>(T, k, v, status);
-    if (k > 0) xg_trsv_lt_update_kernel<<<k * ((T.ts + 255) / 256), 256, 0, st>>>(T, k, v, status);
+    return cudaFuncSetAttribute(xg_trsv_lt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_TL_SMEM);
+}
+
+void xg_launch_trsv_lower_t(const XgTrsv &G, int max_ctas, cudaStream_t st)
+{
+    if (G.ntasks <= 0) return;
+    const unsigned grid = (unsigned)(G.ntasks < max_ctas ? G.ntasks : max_ctas);
+    xg_trsv_lt_kernel<<<grid, XG_TL_THREADS, XG_TL_SMEM, st>>>(G);
 }
 
 /* ---- kriging: zmiss[m] = sum_o Sigma(miss_m, obs_o) alpha_o ---- */

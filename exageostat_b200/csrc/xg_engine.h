@@ -38,11 +38,10 @@ struct XgTileMatrix {
     double *d = nullptr;
     int2 *ij = nullptr; /* (i, j) of every packed tile */
     CUtensorMap map;    /* TMA view for the trailing-update kernel */
-    /* nt ts x 32: the inverted 32 x 32 diagonal blocks of L (the tile DAG keeps
-     * every column's; the per-step launches use the first ts rows for the current one) */
+    /* nt ts x 32: the inverted 32 x 32 diagonal blocks of L */
     double *dinv = nullptr;
-    /* tile DAG: next task, abort flag, one flag per lower 128-block; null where
-     * the matrix is factored by the per-step launches only */
+    /* tile DAG and backward solve: next task, abort flag and block flags of each;
+     * null where the matrix is factored by the per-step launches only */
     int *dag = nullptr;
 };
 
@@ -129,6 +128,7 @@ int xg_check_theta(const double *theta, int kernel);
 int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
               cudaEvent_t *pev = nullptr);
 int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
+void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st);
 double xg_trailing_flops(int nt, int ts, int k);
 int xg_field_set_data(XgField *f, const double *x, const double *y, const double *z);
 int xg_field_set_profiling(XgField *f, int on);

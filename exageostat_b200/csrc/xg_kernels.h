@@ -85,35 +85,16 @@ struct XgMaternParams {
 struct XgBField {
     long long tile_off; /* first packed tile of the field in the batch store */
     long long vec_off;  /* first entry of its vectors (x, y, z, v); a multiple of ts */
-    long long part_off; /* first entry of its partial sums (2 nt) */
-    long long sched_off; /* first of its scheduler counters (nt + 2 lower tiles) */
-    int N, nt;
-    int kernel, pad_;
+    long long part_off; /* first entry of its partial sums (2 nb) */
+    int N, nt, nb;      /* nb: 128-blocks per side */
+    int kernel;
     XgMaternParams p;   /* this evaluation's parameters */
 };
 
-/* Device-resident tile scheduler of a batch (xg_batch_sched_kernel).  The
- * task list holds every POTRF(k), TRSM(i, k) and update (i, j) <- step k of
- * every field in one topological order; persistent CTAs take tasks in list
- * order (one atomic counter), wait (bounded) on the task's dependency
- * counters, run it and publish its completion.  Per field, at sched_off:
- *   pdone[k]            POTRF(k) done
- *   tdone[tile (i, k)]  TRSM(i, k) done
- *   ucount[tile (i, j)] updates applied to tile (i, j) (final at min(i, j))
- * Dependencies: POTRF(k) <- ucount(k, k) = k; TRSM(i, k) <- pdone(k),
- * ucount(i, k) = k; update (i, j, k) <- tdone(i, k), tdone(j, k),
- * ucount(i, j) = k (the updates of a tile are applied in k order). */
+/* task types of the right-looking plan (exageostat_b200_batch_plan) */
 #define XG_TASK_POTRF 0
 #define XG_TASK_TRSM 1
 #define XG_TASK_GEMM 2
-struct XgSched {
-    const int4 *tasks;         /* x = type | field << 2, y = i, z = j, w = k */
-    long long ntasks;
-    unsigned long long *next;  /* index of the next task to take */
-    int *abort;                /* set after a wait that timed out: no CTA takes another task */
-    int *cnt;                  /* the counters of every field */
-    double *dinv;              /* per CTA, ts x 32: the inverted diagonal blocks of its TRSM task's L_kk */
-};
 
 /* The fields taking part in one batched launch and the CTA ranges they own. */
 struct XgBStep {
@@ -165,11 +146,14 @@ __device__ inline int2 xg_tile_decode_fast(long long t, int nt)
 #define XG_DAG_BLOCK 128
 /* device words of a field's DAG state: next task, abort flag, block flags */
 static inline long long xg_dag_words(int nb) { return 2 + (long long)nb * (nb + 1) / 2; }
+/* the same of its backward solve: next task, abort flag, a flag per block */
+static inline long long xg_trsv_words(int nb) { return 2 + (long long)nb; }
 struct XgDagField {
     long long tile_off; /* first packed tile inside the tile store */
     long long vec_off;  /* first entry of v */
     long long part_off; /* partial sums: nb log-det, nb |v_J|^2 */
     long long flag_off; /* nb (nb + 1) / 2 block flags */
+    long long tflag_off; /* nb flags of the backward solve */
     long long dinv_off; /* first row of the inverted 32 x 32 diagonal blocks (32 doubles a row) */
     int nt, nb;         /* tiles per side; 128-blocks per side that hold rows < N */
 };
@@ -258,21 +242,26 @@ void xg_launch_finalize(const double *part_logdet, const double *part_dot, int n
 /* batched fields (one launch per tile step covering every active field) */
 void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, const XgBStep &S, long long blocks,
                          const double *x, const double *y, int metric, cudaStream_t st);
-void xg_launch_batch_potrf(const XgTileArgs &base, const XgBField *F, const XgBStep &S, int k, double *v, double *part,
-                           int *status, int *info, cudaStream_t st);
-void xg_launch_batch_trsm(const XgTileArgs &base, const XgBField *F, const XgBStep &S, long long blocks, int k,
-                          double *v, const int *status, cudaStream_t st);
-void xg_launch_batch_gemm(const CUtensorMap &map, const XgTileArgs &base, const XgBField *F, const XgBStep &S,
-                          long long blocks, int k, int *status, cudaStream_t st);
 void xg_launch_batch_finalize(const XgBField *F, int nfields, const double *part, double *out, cudaStream_t st);
-/* the whole batched factorisation (with the fused log-det and solve) in one
- * persistent launch of `ctas` CTAs driven by the task list of `sch` */
-void xg_launch_batch_sched(const CUtensorMap &map, const XgTileArgs &base, const XgBField *F, const XgSched &sch,
-                           int ctas, double *v, double *part, int *status, cudaStream_t st);
-
 /* solve.cu */
 void xg_launch_trmv_lower(const XgTileArgs &T, const double *e, double *z, const int *status, cudaStream_t st);
-void xg_launch_trsv_lower_t_step(const XgTileArgs &T, int k, double *v, const int *status, cudaStream_t st);
+/* v <- L^-T v in one launch, with the inverted 32 x 32 diagonal blocks that
+ * the factorisation kept */
+struct XgTrsv {
+    const double *data;
+    int ts;
+    XgDagField one;      /* a single field (tasks == nullptr) */
+    const XgDagField *F; /* several */
+    const int2 *tasks;   /* (field, J), every field's columns in descending order */
+    long long ntasks;
+    unsigned *next;      /* zero on launch */
+    int *abort, *flags;  /* zero on launch */
+    const double *dinv;
+    double *v;
+    int *status;
+};
+cudaError_t xg_solve_kernels_configure();
+void xg_launch_trsv_lower_t(const XgTrsv &G, int max_ctas, cudaStream_t st);
 void xg_launch_predict_cross(const double *xm, const double *ym, int nmiss, const double *xo, const double *yo,
                              int nobs, const double *alpha, const XgMaternParams &p, int metric, double *zmiss,
                              cudaStream_t st);
