@@ -247,8 +247,14 @@ __global__ void __launch_bounds__(256) xg_dsigma_full_kernel(double *__restrict_
 }
 
 void xg_launch_dsigma_full(double *D, int nt, int ts, const double *x, const double *y, int N,
-                           const XgMaternParams &p, double dlogcon, int metric, int which, cudaStream_t st)
+                           const XgMaternParams &p, double dlogcon, int metric, int which, double *tab,
+                           cudaStream_t st)
 {
+    if (tab && xg_tab_covers(p, N)) {
+        if (which == 0) xg_launch_grad_tables(p, dlogcon, tab, st); /* the calls for 1 and 2 follow on the stream */
+        xg_launch_dsigma_full_tab(D, nt, ts, x, y, N, p, dlogcon, metric, which, tab, st);
+        return;
+    }
     const long long blocks = (long long)nt * nt * (ts / XG_AS_ROWS);
     xg_dsigma_full_kernel<<<(unsigned)blocks, 256, 0, st>>>(D, nt, ts, x, y, N, p, dlogcon, metric, which);
 }
@@ -419,7 +425,7 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
         cudaEventRecord(f->ev[0], st);
         /* Sigma (MLE_dexact.c:1824-1825), its factor (:1830) and S = Sigma^-1 */
-        xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, N, N, p, f->metric, 1, st);
+        xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, N, N, p, f->metric, 1, f->C.tab, st);
         XgFactorStreams fs;
         fs.st = st;
         fs.st_hi = g_xg.stream_hi;
@@ -431,7 +437,7 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         xg_launch_sym_full(f->C.d, Sf, nt, ts, st);
         /* G_j = S dSigma_j (dSigma_j symmetric: S dSigma_j^T) */
         for (int j = 0; j < 3; ++j) {
-            xg_launch_dsigma_full(D, nt, ts, f->x, f->y, N, p, dlogcon, f->metric, j, st);
+            xg_launch_dsigma_full(D, nt, ts, f->x, f->y, N, p, dlogcon, f->metric, j, f->C.tab, st);
             xg_launch_dense_gemm_nt(mS, mD, G + j * full, nt, ts, f->status, st);
         }
         const double *g[4] = {G, G + full, G + 2 * full, Sf};
@@ -563,8 +569,8 @@ int xg_assess_run(XgAssess *q, const double *truth, const double *est, int kerne
     /* K_a = Sigma(obs, obs; estimated), K_t (truth) (MLE_dexact.c:1239-1245),
      * k_a and k_t for every missing point at once (:1283-1286) */
     XgTileArgs Ta{q->Ca.d, ts, nt}, Tt{q->Ct.d, ts, nt};
-    xg_launch_gen(Ta, q->Ca.ij, q->Ca.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, pa, metric, 1, st);
-    xg_launch_gen(Tt, q->Ct.ij, q->Ct.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, pt, metric, 1, st);
+    xg_launch_gen(Ta, q->Ca.ij, q->Ca.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, pa, metric, 1, q->Ca.tab, st);
+    xg_launch_gen(Tt, q->Ct.ij, q->Ct.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, pt, metric, 1, q->Ct.tab, st);
     xg_launch_cross_gen_r(RA, mt, nt, ts, q->xm, q->ym, nmiss, q->xo, q->yo, nobs, pa, metric, st);
     xg_launch_cross_gen_r(RU, mt, nt, ts, q->xm, q->ym, nmiss, q->xo, q->yo, nobs, pt, metric, st);
     XG_ACU(cudaMemcpyAsync(RT, RU, rbytes, cudaMemcpyDeviceToDevice, st));

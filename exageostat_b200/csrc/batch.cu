@@ -63,6 +63,7 @@ struct XgBatch {
     long long ntasks = 0, nttasks = 0;
     int *words = nullptr, *twords = nullptr;
     double *dinv = nullptr;
+    double *tab = nullptr; /* one element table per field */
     CUtensorMap map;
     cudaGraphExec_t graph = nullptr;
     /* gradients (allocated on the first request): per stream an inverse-factor
@@ -93,7 +94,7 @@ static void xg_batch_free(XgBatch *b)
     if (b->gout) cudaFree(b->gout);
     if (b->h_gout) cudaFreeHost(b->h_gout);
     void *dev[] = {b->F_dev, b->tiles, b->x, b->y, b->z, b->v, b->part, b->out, b->status, b->table_buf,
-                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv};
+                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv, b->tab};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (b->F_pinned) cudaFreeHost(b->F_pinned);
@@ -400,6 +401,7 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
         if (e == cudaSuccess) e = cudaMalloc(&b->words, (size_t)(2 + b->total_flags) * sizeof(int));
         if (e == cudaSuccess) e = cudaMalloc(&b->twords, (size_t)(2 + b->total_tflags) * sizeof(int));
         if (e == cudaSuccess) e = cudaMalloc(&b->dinv, (size_t)b->total_vec * 32 * sizeof(double));
+        if (e == cudaSuccess) e = cudaMalloc(&b->tab, (size_t)nfields * xg_tab_doubles() / 3 * sizeof(double));
         if (e != cudaSuccess) {
             xg_batch_free(b);
             return xg_fail(XG_ERR_NO_MEMORY, "batch task list (%lld tasks): %s", (long long)tl.size(),
@@ -444,7 +446,7 @@ static void xg_batch_record(XgBatch *b, cudaStream_t st)
     cudaMemsetAsync(b->status, 0, 2 * (size_t)b->nfields * sizeof(int), st);
     cudaMemsetAsync(b->words, 0, (size_t)(2 + b->total_flags) * sizeof(int), st);
     cudaMemcpyAsync(b->v, b->z, b->total_vec * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    xg_launch_batch_gen(base, b->F_dev, b->gen.dev, b->gen.blocks, b->x, b->y, b->metric, st);
+    xg_launch_batch_gen(base, b->F_dev, b->nfields, b->gen.dev, b->gen.blocks, b->x, b->y, b->metric, b->tab, st);
     XgDag G = {};
     G.data = b->tiles;
     G.ts = b->ts;
@@ -598,7 +600,7 @@ extern "C" int exageostat_b200_batch_loglik_grad(void *handle, const double *the
         xg_launch_inverse_syrk(b->gX[s].map, T.data, fd.nt, ts, stf, st);
         const double dlogcon = -(log(2.0) + xg_digamma(fd.p.nu));
         xg_launch_grad_contract(T.data, b->ij_by_nt[fd.nt], xg_num_lower_tiles(fd.nt), fd.nt, ts, b->x + fd.vec_off,
-                                b->y + fd.vec_off, vf, fd.N, fd.p, b->kernel, b->metric, dlogcon, b->gpart[s],
+                                b->y + fd.vec_off, vf, fd.N, fd.p, b->kernel, b->metric, dlogcon, b->gX[s].tab, b->gpart[s],
                                 b->gout + 4 * (size_t)f, st);
     }
     XG_CU(cudaGetLastError());

@@ -169,23 +169,6 @@ __global__ void __launch_bounds__(256) xg_gen_matern_kernel(XgTileArgs T, const 
                 identity_pad);
 }
 
-/* batched: every field's lower tiles, CTAs resolved through the step table */
-__global__ void __launch_bounds__(256) xg_gen_matern_batch_kernel(XgTileArgs base, const XgBField *__restrict__ F,
-                                                                  XgBStep S, const double *__restrict__ x,
-                                                                  const double *__restrict__ y, int metric)
-{
-    long long local;
-    const int f = xg_batch_resolve(S, blockIdx.x, &local);
-    const XgBField &fd = F[f];
-    XgTileArgs T = base;
-    T.data = base.data + fd.tile_off * (long long)base.ts * base.ts;
-    T.nt = fd.nt;
-    const int strips = T.ts / XG_GEN_ROWS;
-    const long long t = local / strips;
-    const double *xf = x + fd.vec_off, *yf = y + fd.vec_off;
-    xg_gen_body(T, t, xg_tile_decode(t, fd.nt), (int)(local % strips), xf, yf, xf, yf, fd.N, fd.N, fd.p, metric, 1);
-}
-
 /* ========================================================================== */
 /* Loads of tile data.  COH = false: ordinary loads (the data was written by   */
 /* an earlier launch).  COH = true: the bodies run inside the persistent       */
@@ -1330,8 +1313,12 @@ cudaError_t xg_kernels_configure()
 
 void xg_launch_gen(const XgTileArgs &T, const int2 *tile_ij, long long ntiles, const double *xr, const double *yr,
                    const double *xc, const double *yc, int n_rows, int n_cols, const XgMaternParams &p, int metric,
-                   int identity_pad, cudaStream_t st)
+                   int identity_pad, double *tab, cudaStream_t st)
 {
+    if (tab && p.half_integer < 0 && xg_tab_covers(p, n_cols)) {
+        xg_launch_gen_tab(T, tile_ij, ntiles, xr, yr, xc, yc, n_rows, n_cols, p, metric, identity_pad, tab, st);
+        return;
+    }
     const long long blocks = ntiles * (T.ts / XG_GEN_ROWS);
     xg_gen_matern_kernel<<<(unsigned)blocks, 256, 0, st>>>(T, tile_ij, xr, yr, xc, yc, n_rows, n_cols, p, metric,
                                                             identity_pad);
@@ -1414,12 +1401,6 @@ void xg_launch_band_gemm(const CUtensorMap &p64map, const XgTileArgs &T, int k, 
     const long long blocks = ncol * (T.band ? T.band : T.band_targets) * bpt * bpt;
     xg_syrk_gemm_kernel<<<(unsigned)blocks, XG_G_THREADS, xg_gemm_smem_bytes(), st>>>(p64map, T, k, j0, part == 1,
                                                                                        status);
-}
-
-void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, const XgBStep &S, long long blocks,
-                         const double *x, const double *y, int metric, cudaStream_t st)
-{
-    if (blocks > 0) xg_gen_matern_batch_kernel<<<(unsigned)blocks, 256, 0, st>>>(base, F, S, x, y, metric);
 }
 
 void xg_launch_batch_finalize(const XgBField *F, int nfields, const double *part, double *out, cudaStream_t st)

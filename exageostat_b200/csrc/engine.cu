@@ -96,6 +96,7 @@ int xg_context_start(int dts)
     if (e == cudaSuccess) e = xg_mixed_kernels_configure();
     if (e == cudaSuccess) e = xg_dag_kernels_configure();
     if (e == cudaSuccess) e = xg_solve_kernels_configure();
+    if (e == cudaSuccess) e = xg_tab_kernels_configure(prop.multiProcessorCount);
     if (e == cudaSuccess) e = xg_sliced_kernels_configure();
     if (e != cudaSuccess) return xg_cuda_fail(e, "kernel attribute setup");
     g_xg.device = dev;
@@ -162,6 +163,11 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
         M.dag = nullptr;
         return xg_cuda_fail(e, "block flags");
     }
+    e = cudaMalloc(&M.tab, sizeof(double) * xg_tab_doubles());
+    if (e != cudaSuccess) {
+        M.tab = nullptr;
+        return xg_cuda_fail(e, "element tables");
+    }
     return xg_encode_tiles(&M.map, M.d, M.ntiles, ts);
 }
 
@@ -186,6 +192,8 @@ void xg_tm_free(XgTileMatrix &M)
     if (M.ij) cudaFree(M.ij);
     if (M.dinv) cudaFree(M.dinv);
     if (M.dag) cudaFree(M.dag);
+    if (M.tab) cudaFree(M.tab);
+    M.tab = nullptr;
     M.dag = nullptr;
     M.d = nullptr;
     M.ij = nullptr;
@@ -599,7 +607,7 @@ int xg_field_loglik(XgField *f, const double *theta, double *res, double *times)
     XG_CU(cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemcpyAsync(f->v, f->z, Np * sizeof(double), cudaMemcpyDeviceToDevice, st));
     XG_CU(cudaEventRecord(f->ev[0], st));
-    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, st);
+    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, f->C.tab, st);
     XG_CU(cudaEventRecord(f->ev[1], st));
     XgFactorStreams fs;
     fs.st = st;
@@ -640,7 +648,7 @@ int xg_field_zvg(XgField *f, const double *theta, const double *nrand, double *t
     XG_CU(cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemcpyAsync(f->e, nrand, f->N * sizeof(double), cudaMemcpyHostToDevice, st));
     XG_CU(cudaEventRecord(f->ev[0], st));
-    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, st);
+    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, f->C.tab, st);
     XG_CU(cudaEventRecord(f->ev[1], st));
     XgFactorStreams fs;
     fs.st = st;
@@ -734,7 +742,7 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
     xg_launch_inverse_factor(f->X.map, f->C.map, f->X.d, f->C.d, f->C.nt, f->C.ts, f->status, st);
     xg_launch_inverse_syrk(f->X.map, f->C.d, f->C.nt, f->C.ts, f->status, st);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, f->C.nt, f->C.ts, f->x, f->y, f->v, f->N, p, f->kernel,
-                            f->metric, dlogcon, f->gpart, f->gout, st);
+                            f->metric, dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));
     double g4[4];
     int sv[2];
@@ -1343,7 +1351,7 @@ int xg_field_loglik_sliced(XgField *f, const double *theta, double *res, double 
     XG_CU(cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemcpyAsync(f->v, f->z, Np * sizeof(double), cudaMemcpyDeviceToDevice, st));
     XG_CU(cudaEventRecord(f->ev[0], st));
-    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, st);
+    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, f->N, f->N, p, f->metric, 1, f->C.tab, st);
     XG_CU(cudaEventRecord(f->ev[1], st));
     XgFactorStreams fs;
     fs.st = st;
@@ -1390,7 +1398,7 @@ int xg_sliced_factor_dense(int n, const double *x, const double *y, const double
     cudaStream_t st = g_xg.stream;
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
-    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, xg_params(theta, kernel), metric, 1, st);
+    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, xg_params(theta, kernel), metric, 1, f->C.tab, st);
     XgFactorStreams fs;
     fs.st = st;
     fs.st_hi = g_xg.stream_hi;
@@ -1464,7 +1472,7 @@ int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, do
     S.overwrite = 1;
     xg_launch_sliced(sl->xmap, sl->xmap, sl->xscale, sl->xscale, T, S, pr, g_xg.sm_count, f->status, st);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, nt, ts, f->x, f->y, f->v, f->N, p, f->kernel, f->metric,
-                            dlogcon, f->gpart, f->gout, st);
+                            dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));
     double g4[4];
     int sv[2];
@@ -1677,7 +1685,7 @@ int xg_predict_run(XgPredict *q, const double *theta, int kernel, int metric, co
     XG_CU(cudaMemcpyAsync(q->ym, ym, lmiss * sizeof(double), cudaMemcpyHostToDevice, st));
     if (zactual) XG_CU(cudaMemcpyAsync(q->zact, zactual, nmiss * sizeof(double), cudaMemcpyHostToDevice, st));
     /* C22 = Sigma(obs, obs); POSV: L L^T alpha = zobs */
-    xg_launch_gen(T, q->C22.ij, q->C22.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, p, metric, 1, st);
+    xg_launch_gen(T, q->C22.ij, q->C22.ntiles, q->xo, q->yo, q->xo, q->yo, nobs, nobs, p, metric, 1, q->C22.tab, st);
     XgFactorStreams fs;
     fs.st = st;
     fs.st_hi = g_xg.stream_hi;
@@ -1721,7 +1729,7 @@ int xg_covariance_dense(int n, const double *x, const double *y, const double *t
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, kernel);
     cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
-    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, p, metric, 1, st);
+    xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, p, metric, 1, f->C.tab, st);
     if (factor) xg_factor(f->C, nullptr, f->part, f->status, f->info, st);
     rc = xg_tiles_to_dense(f, n, out);
     xg_field_destroy(f);

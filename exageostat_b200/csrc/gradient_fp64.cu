@@ -515,8 +515,14 @@ long long xg_grad_contract_blocks(long long ntiles, int ts) { return ntiles * (t
 
 void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long ntiles, int nt, int ts, const double *x,
                              const double *y, const double *alpha, int N, const XgMaternParams &mp, int kernel,
-                             int metric, double dlogcon, double *part, double *out, cudaStream_t st)
+                             int metric, double dlogcon, double *tab, double *part, double *out, cudaStream_t st)
 {
+    if (tab && xg_tab_covers(mp, N)) {
+        xg_launch_grad_tables(mp, dlogcon, tab, st);
+        xg_launch_grad_contract_tab(S, ntiles, nt, ts, x, y, alpha, N, mp, kernel, metric, dlogcon, tab, part, st);
+        xg_grad_reduce_kernel<<<1, dim3(32, 4), 0, st>>>(part, xg_grad_contract_tab_blocks(ntiles, ts), out);
+        return;
+    }
     XgGradParams p;
     p.sigma2 = mp.sigma2;
     p.beta = mp.beta;

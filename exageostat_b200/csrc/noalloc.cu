@@ -166,7 +166,7 @@ extern "C" int exageostat_b200_dmle_device_noalloc(int n, const double *d_x, con
     xg_noalloc_table_kernel<<<1, 32, 0, st>>>(M.ij, M.nt);
     const XgMaternParams p = xg_params(theta, kernel);
     XgTileArgs T{M.d, M.ts, M.nt};
-    xg_launch_gen(T, M.ij, M.ntiles, d_x, d_y, d_x, d_y, n, n, p, metric, 1, st);
+    xg_launch_gen(T, M.ij, M.ntiles, d_x, d_y, d_x, d_y, n, n, p, metric, 1, nullptr, st);
     xg_factor(M, v, part, status, status + 1, st);
     xg_launch_finalize(part, part + M.nt, M.nt, n, out, status, status + 1, st);
     e = cudaGetLastError();

@@ -43,6 +43,7 @@ struct XgTileMatrix {
     /* tile DAG and backward solve: next task, abort flag and block flags of each;
      * null where the matrix is factored by the per-step launches only */
     int *dag = nullptr;
+    double *tab = nullptr; /* element tables of the current parameters (xg_matern_tab.cuh) */
 };
 
 /* Banded mixed-precision workspace (mixed.cu): compact FP64 band tiles,

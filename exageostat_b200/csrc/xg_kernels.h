@@ -178,9 +178,11 @@ size_t xg_potrf_smem_bytes(int ts);
 size_t xg_trsm_smem_bytes(int ts);
 size_t xg_gemm_smem_bytes();
 
+/* covariance tiles; tab: xg_tab_doubles() doubles of workspace for the
+ * piecewise polynomial form, or null for the direct evaluation */
 void xg_launch_gen(const XgTileArgs &T, const int2 *tile_ij, long long ntiles, const double *xr, const double *yr,
                    const double *xc, const double *yc, int n_rows, int n_cols, const XgMaternParams &p, int metric,
-                   int identity_pad, cudaStream_t st);
+                   int identity_pad, double *tab, cudaStream_t st);
 void xg_launch_potrf_diag(const XgTileArgs &T, int k, double *v, double *part_logdet, double *part_dot, int with_rhs,
                           int *status, int *info, cudaStream_t st);
 void xg_launch_trsm_panel(const XgTileArgs &T, int k, double *v, int with_rhs, const int *status, cudaStream_t st,
@@ -192,6 +194,27 @@ void xg_launch_potrf_tiled(const CUtensorMap &map, const XgTileArgs &T, int k, d
 int xg_potrf_tiled_launches(int ts);
 void xg_launch_syrk_gemm(const CUtensorMap &map, const XgTileArgs &T, int k, int *status, cudaStream_t st,
                          int part = 0);
+
+/* matern_tab.cu: tiles of general order from piecewise polynomial tables.
+ * Smallest field that builds them: the table's own evaluations take as long as
+ * the direct elements of about 1000 locations. */
+#define XG_TAB_MIN_N 1024
+cudaError_t xg_tab_kernels_configure(int sm_count);
+size_t xg_tab_doubles();
+/* whether the tables cover the orders of p and pay for n locations */
+bool xg_tab_covers(const XgMaternParams &p, int n);
+void xg_launch_gen_tab(const XgTileArgs &T, const int2 *tile_ij, long long ntiles, const double *xr, const double *yr,
+                       const double *xc, const double *yc, int n_rows, int n_cols, const XgMaternParams &p, int metric,
+                       int identity_pad, double *tab, cudaStream_t st);
+/* the three derivative tables of p into tab, then what reads them */
+void xg_launch_grad_tables(const XgMaternParams &p, double dlogcon, double *tab, cudaStream_t st);
+long long xg_grad_contract_tab_blocks(long long ntiles, int ts);
+void xg_launch_grad_contract_tab(const double *S, long long ntiles, int nt, int ts, const double *x, const double *y,
+                                 const double *alpha, int N, const XgMaternParams &p, int kernel, int metric,
+                                 double dlogcon, const double *tab, double *part, cudaStream_t st);
+void xg_launch_dsigma_full_tab(double *D, int nt, int ts, const double *x, const double *y, int N,
+                               const XgMaternParams &p, double dlogcon, int metric, int which, const double *tab,
+                               cudaStream_t st);
 
 /* mixed.cu: banded mixed precision */
 struct XgMixedMaps {
@@ -240,8 +263,8 @@ void xg_launch_finalize(const double *part_logdet, const double *part_dot, int n
                         const int *status, const int *info, cudaStream_t st);
 
 /* batched fields (one launch per tile step covering every active field) */
-void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, const XgBStep &S, long long blocks,
-                         const double *x, const double *y, int metric, cudaStream_t st);
+void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, int nfields, const XgBStep &S, long long blocks,
+                         const double *x, const double *y, int metric, double *tab, cudaStream_t st);
 void xg_launch_batch_finalize(const XgBField *F, int nfields, const double *part, double *out, cudaStream_t st);
 /* solve.cu */
 void xg_launch_trmv_lower(const XgTileArgs &T, const double *e, double *z, const int *status, cudaStream_t st);
@@ -290,7 +313,7 @@ void xg_launch_dense_gemm_nt(const CUtensorMap &mapA, const CUtensorMap &mapB, d
 long long xg_grad_contract_blocks(long long ntiles, int ts);
 void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long ntiles, int nt, int ts, const double *x,
                              const double *y, const double *alpha, int N, const XgMaternParams &mp, int kernel,
-                             int metric, double dlogcon, double *part, double *out, cudaStream_t st);
+                             int metric, double dlogcon, double *tab, double *part, double *out, cudaStream_t st);
 
 /* assess.cu (Fisher information, MLOE / MMOM) */
 void xg_launch_cross_gen_r(double *D, int mt, int nt, int ts, const double *xm, const double *ym, int nmiss,
@@ -301,7 +324,8 @@ void xg_launch_mloe_terms(const double *A, const double *U, const double *T, con
                           int nmiss, double sigma2_t, double sigma2_a, double *terms, cudaStream_t st);
 void xg_launch_sym_full(const double *S, double *F, int nt, int ts, cudaStream_t st);
 void xg_launch_dsigma_full(double *D, int nt, int ts, const double *x, const double *y, int N,
-                           const XgMaternParams &p, double dlogcon, int metric, int which, cudaStream_t st);
+                           const XgMaternParams &p, double dlogcon, int metric, int which, double *tab,
+                           cudaStream_t st);
 void xg_launch_fisher_trace(const double *const g[4], int np, int nt, int ts, int N, double *part, int nctas,
                             cudaStream_t st);
 
