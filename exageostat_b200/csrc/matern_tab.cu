@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(XG_GT_THREADS)
 }
 
 /* closed forms of half-integer order and orders beyond the table, for a batch */
-__device__ __forceinline__ void xg_gen_direct_strip(double *tile, int ts, int2 ij, int strip,
+__device__ __noinline__ void xg_gen_direct_strip(double *tile, int ts, int2 ij, int strip,
                                                     const double *__restrict__ x, const double *__restrict__ y, int n,
                                                     const XgMaternParams &p, int metric)
 {
@@ -203,12 +203,13 @@ __device__ __forceinline__ void xg_gen_direct_strip(double *tile, int ts, int2 i
 
 /* every field of a batch: the strips of all fields in one list (S.blk_start),
  * a CTA's range restaging the table where a new field begins */
-__global__ void __launch_bounds__(XG_GT_THREADS)
+__global__ void __launch_bounds__(XG_GT_THREADS, 3)
     xg_gen_tab_batch_kernel(XgTileArgs base, const XgBField *__restrict__ F, XgBStep S, long long units,
                             const double *__restrict__ x, const double *__restrict__ y, int metric,
                             const double *__restrict__ gtab)
 {
     extern __shared__ __align__(16) double xg_smem_d[];
+    __shared__ XgMaternParams p; /* the field's, restaged with its table */
     const int strips = base.ts / XG_GT_ROWS;
     const long long u1 = units * (blockIdx.x + 1LL) / gridDim.x;
     int field = -1;
@@ -220,10 +221,10 @@ __global__ void __launch_bounds__(XG_GT_THREADS)
         if (f != field) {
             __syncthreads();
             if (tabbed) xg_tab_stage(xg_smem_d, gtab + (long long)f * XG_TAB_SIZE, XG_TAB_SIZE);
+            if (threadIdx.x == 0) p = fd.p;
             __syncthreads();
             field = f;
         }
-        const XgMaternParams p = fd.p;
         const double *xf = x + fd.vec_off, *yf = y + fd.vec_off;
         const long long n = xg_num_lower_tiles(fd.nt) * strips;
         for (; u < u1 && local < n; ++u, ++local) {

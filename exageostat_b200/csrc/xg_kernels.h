@@ -196,9 +196,10 @@ void xg_launch_syrk_gemm(const CUtensorMap &map, const XgTileArgs &T, int k, int
                          int part = 0);
 
 /* matern_tab.cu: tiles of general order from piecewise polynomial tables.
- * Smallest field that builds them: the table's own evaluations take as long as
- * the direct elements of about 1000 locations. */
-#define XG_TAB_MIN_N 1024
+ * Smallest field that builds them: the build takes 9 us, one direct element's
+ * own latency as much; an evaluation of 256 locations takes 135 us with the
+ * table and 172 us without, one of 1024 455 and 514 us. */
+#define XG_TAB_MIN_N 64
 cudaError_t xg_tab_kernels_configure(int sm_count);
 size_t xg_tab_doubles();
 /* whether the tables cover the orders of p and pay for n locations */

@@ -1,4 +1,4 @@
-"""Covariance elements from the piecewise polynomial tables (fields of 1024
+"""Covariance elements from the piecewise polynomial tables (fields of 64
 locations and more, general order) against the direct evaluation of the same
 elements, over the whole table and both of its ends.
 
