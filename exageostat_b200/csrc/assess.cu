@@ -432,8 +432,7 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         fs.ev_panel = f->ev_panel;
         fs.ev_upd = f->ev_upd;
         xg_factor_lookahead(f->C, nullptr, f->part, f->status, f->info, fs);
-        xg_launch_inverse_factor(f->X.map, f->C.map, f->X.d, f->C.d, nt, ts, f->status, st);
-        xg_launch_inverse_syrk(f->X.map, f->C.d, nt, ts, f->status, st);
+        xg_inverse_product(f->C, f->X, f->status, st);
         xg_launch_sym_full(f->C.d, Sf, nt, ts, st);
         /* G_j = S dSigma_j (dSigma_j symmetric: S dSigma_j^T) */
         for (int j = 0; j < 3; ++j) {
@@ -487,6 +486,7 @@ void xg_assess_destroy(XgAssess *q)
     cudaFree(q->ym);
     cudaFree(q->terms);
     cudaFree(q->part);
+    cudaFree(q->words);
     cudaFree(q->status);
     for (int i = 0; i < 4; ++i)
         if (q->ev[i]) cudaEventDestroy(q->ev[i]);
@@ -532,6 +532,9 @@ int xg_assess_create(XgAssess **out, int nmiss, int nobs, int ts)
     if (!rc) rc = xg_assess_alloc(&q->terms, 6 * (size_t)nmiss);
     if (!rc) rc = xg_assess_alloc(&q->part, 2 * (size_t)q->nt * q->ts / XG_DAG_BLOCK);
     if (!rc && cudaMalloc(&q->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status");
+    const long long flags = 3LL * ((nobs + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK) * ((nmiss + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK);
+    if (!rc && cudaMalloc(&q->words, (size_t)(2 + flags) * sizeof(int)) != cudaSuccess)
+        rc = xg_fail(XG_ERR_NO_MEMORY, "block flags");
     for (int i = 0; i < 4 && !rc; ++i)
         if (cudaEventCreate(&q->ev[i]) != cudaSuccess) rc = xg_fail(XG_ERR_CUDA, "events");
     if (!rc && (cudaEventCreateWithFlags(&q->ev_panel, cudaEventDisableTiming) != cudaSuccess ||
@@ -585,9 +588,32 @@ int xg_assess_run(XgAssess *q, const double *truth, const double *est, int kerne
     xg_factor_lookahead(q->Ct, nullptr, q->part, q->status, q->status + 1, fs);
     XG_ACU(cudaEventRecord(q->ev[2], st));
     /* the per-point solves (:1300-1364) for all points */
-    xg_launch_rhs_forward_solve(q->mR[0], RA, mt, q->Ca.map, q->Ca.d, nt, ts, q->status, st); /* A = L_a^-1 k_a */
-    xg_launch_rhs_forward_solve(q->mR[1], RU, mt, q->Ca.map, q->Ca.d, nt, ts, q->status, st); /* U = L_a^-1 k_t */
-    xg_launch_rhs_forward_solve(q->mR[2], RT, mt, q->Ct.map, q->Ct.d, nt, ts, q->status, st); /* T = L_t^-1 k_t */
+    {
+        /* A = L_a^-1 k_a, U = L_a^-1 k_t, T = L_t^-1 k_t */
+        const XgTileMatrix *L[3] = {&q->Ca, &q->Ca, &q->Ct};
+        XgRowsMaps maps;
+        XgRows G = {};
+        for (int i = 0; i < 3; ++i) {
+            maps.y[i] = q->mR[i];
+            maps.l[i] = L[i]->map;
+            G.y[i] = q->R[i];
+            G.dinv[i] = L[i]->dinv;
+        }
+        G.ts = ts;
+        G.nsys = 3;
+        G.one.nt = nt;
+        G.one.nb = (nobs + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+        G.one.mt = mt;
+        G.one.mr = (nmiss + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+        G.sys_flags = (long long)G.one.nb * G.one.mr;
+        G.ntasks = 3 * G.sys_flags;
+        G.next = (unsigned *)q->words;
+        G.abort = q->words + 1;
+        G.flags = q->words + 2;
+        G.status = q->status;
+        XG_ACU(cudaMemsetAsync(q->words, 0, sizeof(int) * (size_t)(2 + 3 * G.sys_flags), st));
+        xg_launch_rows(XG_ROWS_RHS, maps, G, g_xg.sm_count, st);
+    }
     /* W = L_a^-T A: the factor's tiles transposed in place, then the backward solve */
     XG_ACU(cudaMemcpyAsync(RW, RA, rbytes, cudaMemcpyDeviceToDevice, st));
     xg_launch_tile_transpose(q->Ca.d, q->Ca.ntiles, ts, st);

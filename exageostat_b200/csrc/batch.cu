@@ -66,16 +66,25 @@ struct XgBatch {
     double *tab = nullptr; /* one element table per field */
     CUtensorMap map;
     cudaGraphExec_t graph = nullptr;
-    /* gradients (allocated on the first request): per stream an inverse-factor
-     * store for the largest field and contraction partials; per field a TMA
-     * view of its tiles; one (i, j) table per tile count; 4 sums per field */
+    /* gradients (allocated on the first request): the inverse factors of one
+     * group of fields at a time (xstore; the groups' tasks one after the other in
+     * rtasks), per stream contraction partials and element tables, one (i, j)
+     * table per tile count, 4 sums per field */
     static const int GS = 8;
     cudaStream_t gst[GS] = {};
     cudaEvent_t ev = nullptr; /* the backward solves are done */
-    XgTileMatrix gX[GS];
-    double *gpart[GS] = {};
+    struct Group {
+        int f0, f1; /* fields f0 .. f1 - 1 */
+        long long task0, ntasks, flags;
+    };
+    std::vector<Group> groups;
+    double *xstore = nullptr;
+    CUtensorMap xmap;
+    XgRowsField *R_dev = nullptr;
+    int4 *rtasks = nullptr;
+    int *rwords = nullptr;
+    double *gpart[GS] = {}, *gtab[GS] = {};
     double *gout = nullptr, *h_gout = nullptr;
-    std::vector<CUtensorMap> fmap;
     std::vector<int2 *> ij_by_nt;
 };
 
@@ -84,8 +93,8 @@ static void xg_batch_free(XgBatch *b)
     if (!b) return;
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (int s = 0; s < XgBatch::GS; ++s) {
-        xg_tm_free(b->gX[s]);
         if (b->gpart[s]) cudaFree(b->gpart[s]);
+        if (b->gtab[s]) cudaFree(b->gtab[s]);
         if (b->gst[s]) cudaStreamDestroy(b->gst[s]);
     }
     if (b->ev) cudaEventDestroy(b->ev);
@@ -94,7 +103,7 @@ static void xg_batch_free(XgBatch *b)
     if (b->gout) cudaFree(b->gout);
     if (b->h_gout) cudaFreeHost(b->h_gout);
     void *dev[] = {b->F_dev, b->tiles, b->x, b->y, b->z, b->v, b->part, b->out, b->status, b->table_buf,
-                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv, b->tab};
+                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv, b->tab, b->xstore, b->R_dev, b->rtasks, b->rwords};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (b->F_pinned) cudaFreeHost(b->F_pinned);
@@ -515,6 +524,34 @@ extern "C" int exageostat_b200_batch_loglik(void *handle, const double *theta, d
     return XG_OK;
 }
 
+/* device memory for the inverse factors of one group of fields */
+#define XG_BATCH_X_BYTES (8ull << 30)
+
+/* The inverse tasks of fields f0 .. f1 - 1: the solves, the fields advancing
+ * together by the same share of their columns as in xg_batch_order, then the
+ * products, the longest sums first. */
+static void xg_group_order(const std::vector<XgRowsField> &R, int f0, int f1, std::vector<int4> &tl)
+{
+    struct Col {
+        double key;
+        int f, J;
+    };
+    std::vector<Col> cols;
+    for (int f = f0; f < f1; ++f)
+        for (int J = 0; J < R[f].nb; ++J) cols.push_back(Col{(double)J / R[f].nb, f, J});
+    std::sort(cols.begin(), cols.end(), [](const Col &a, const Col &b) {
+        return a.key != b.key ? a.key < b.key : a.f != b.f ? a.f < b.f : a.J < b.J;
+    });
+    for (const Col &c : cols)
+        for (int I = 0; I <= c.J; ++I) tl.push_back(make_int4(c.f, I, c.J, 0));
+    std::sort(cols.begin(), cols.end(), [&](const Col &a, const Col &b) {
+        const int la = R[a.f].nb - a.J, lb = R[b.f].nb - b.J;
+        return la != lb ? la > lb : a.f < b.f;
+    });
+    for (const Col &c : cols)
+        for (int J = 0; J <= c.J; ++J) tl.push_back(make_int4(c.f, c.J, J, 1));
+}
+
 /* gradient workspace of a batch (first gradient request) */
 static int xg_batch_grad_workspace(XgBatch *b)
 {
@@ -532,18 +569,58 @@ static int xg_batch_grad_workspace(XgBatch *b)
         maxblocks = std::max(maxblocks, xg_grad_contract_blocks(ntl, ts));
     }
     for (int s = 0; s < XgBatch::GS; ++s) {
-        int rc = xg_tm_alloc(b->gX[s], b->maxnt * ts, ts);
-        if (rc) return rc;
         XG_CU(cudaMalloc(&b->gpart[s], 4 * (size_t)maxblocks * sizeof(double)));
+        XG_CU(cudaMalloc(&b->gtab[s], xg_tab_doubles() * sizeof(double)));
         XG_CU(cudaStreamCreateWithFlags(&b->gst[s], cudaStreamNonBlocking));
     }
-    b->fmap.resize(b->nfields);
-    for (int f = 0; f < b->nfields; ++f) {
-        const XgBField &fd = b->F[f];
-        int rc = xg_encode_tiles(&b->fmap[f], b->tiles + fd.tile_off * (long long)ts * ts, xg_num_lower_tiles(fd.nt),
-                                 ts);
-        if (rc) return rc;
+    /* Groups of consecutive fields whose inverse factors fit XG_BATCH_X_BYTES
+     * together (or a single larger field); half of that again, down to the
+     * largest field, while the device cannot provide it. */
+    const size_t tile_bytes = (size_t)ts * ts * sizeof(double);
+    const long long largest = xg_num_lower_tiles(b->maxnt);
+    long long cap = std::min(b->total_tiles, std::max(largest, (long long)(XG_BATCH_X_BYTES / tile_bytes)));
+    while (cudaMalloc(&b->xstore, (size_t)cap * tile_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b->xstore = nullptr;
+        if (cap <= largest)
+            return xg_fail(XG_ERR_NO_MEMORY, "batch inverse factors (%.2f GB)", cap * tile_bytes / 1e9);
+        cap = std::max(largest, cap / 2);
     }
+    int rc = xg_encode_tiles(&b->xmap, b->xstore, cap, ts);
+    if (rc) return rc;
+    std::vector<XgRowsField> R(b->nfields);
+    std::vector<int4> tl;
+    long long maxflags = 0;
+    b->groups.clear();
+    for (int f = 0; f < b->nfields;) {
+        XgBatch::Group g = {f, f, (long long)tl.size(), 0, 0};
+        long long tiles = 0;
+        for (; g.f1 < b->nfields; ++g.f1) {
+            const XgBField &fd = b->F[g.f1];
+            const long long n = xg_num_lower_tiles(fd.nt);
+            if (tiles + n > cap) break;
+            XgRowsField &r = R[g.f1];
+            r.l_off = fd.tile_off;
+            r.y_off = tiles;
+            r.flag_off = g.flags;
+            r.dinv_off = fd.vec_off;
+            r.nt = fd.nt;
+            r.nb = fd.nb;
+            r.mt = r.mr = 0;
+            tiles += n;
+            g.flags += xg_num_lower_tiles(fd.nb);
+        }
+        xg_group_order(R, g.f0, g.f1, tl);
+        g.ntasks = (long long)tl.size() - g.task0;
+        maxflags = std::max(maxflags, g.flags);
+        b->groups.push_back(g);
+        f = g.f1;
+    }
+    XG_CU(cudaMalloc(&b->R_dev, b->nfields * sizeof(XgRowsField)));
+    XG_CU(cudaMemcpy(b->R_dev, R.data(), b->nfields * sizeof(XgRowsField), cudaMemcpyHostToDevice));
+    XG_CU(cudaMalloc(&b->rtasks, tl.size() * sizeof(int4)));
+    XG_CU(cudaMemcpy(b->rtasks, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    XG_CU(cudaMalloc(&b->rwords, (size_t)(2 + maxflags) * sizeof(int)));
     XG_CU(cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming));
     XG_CU(cudaMalloc(&b->gout, 4 * (size_t)b->nfields * sizeof(double)));
     XG_CU(cudaMallocHost(&b->h_gout, 4 * (size_t)b->nfields * sizeof(double)));
@@ -551,11 +628,10 @@ static int xg_batch_grad_workspace(XgBatch *b)
 }
 
 /* Log-likelihoods and their gradients of every field: the batched
- * factorisation (the graph of exageostat_b200_batch_loglik), then per field,
- * round-robin over eight streams, the adjoint of the single-field path on
- * that field's tiles (alpha = L^-T v of all fields in one launch before) -- X = L^-T,
- * Sigma^-1 = X X^T over the factor, and the fused contraction with the
- * on-the-fly dSigma/dtheta tiles.  A field that is not positive definite
+ * factorisation (the graph of exageostat_b200_batch_loglik), alpha = L^-T v of
+ * all fields in one launch, X = L^-T and Sigma^-1 = X X^T over the factor in
+ * one launch per group of fields, and per field, round-robin over eight
+ * streams, the fused contraction with the on-the-fly dSigma/dtheta tiles.  A field that is not positive definite
  * gets loglik -inf and a NaN gradient. */
 extern "C" int exageostat_b200_batch_loglik_grad(void *handle, const double *theta, double *loglik, double *grad)
 {
@@ -585,23 +661,41 @@ extern "C" int exageostat_b200_batch_loglik_grad(void *handle, const double *the
         G.v = b->v;
         G.status = b->status;
         xg_launch_trsv_lower_t(G, g_xg.sm_count, st);
+    }
+    for (const XgBatch::Group &g : b->groups) {
+        cudaStream_t st = g_xg.stream;
+        XG_CU(cudaMemsetAsync(b->rwords, 0, (size_t)(2 + g.flags) * sizeof(int), st));
+        XgRowsMaps maps = {};
+        maps.y[0] = b->xmap;
+        maps.l[0] = b->map;
+        XgRows G = {};
+        G.y[0] = b->xstore;
+        G.dinv[0] = b->dinv;
+        G.s = b->tiles;
+        G.ts = ts;
+        G.nsys = 1;
+        G.F = b->R_dev;
+        G.tasks = b->rtasks + g.task0;
+        G.ntasks = g.ntasks;
+        G.next = (unsigned *)b->rwords;
+        G.abort = b->rwords + 1;
+        G.flags = b->rwords + 2;
+        G.status = b->status;
+        xg_launch_rows(XG_ROWS_INVERSE, maps, G, g_xg.sm_count, st);
         XG_CU(cudaEventRecord(b->ev, st));
         for (int s = 0; s < XgBatch::GS; ++s) XG_CU(cudaStreamWaitEvent(b->gst[s], b->ev, 0));
-    }
-    for (int f = 0; f < b->nfields; ++f) {
-        if (!std::isfinite(loglik[f])) continue;
-        const XgBField &fd = b->F[f];
-        const int s = f % XgBatch::GS;
-        cudaStream_t st = b->gst[s];
-        XgTileArgs T{b->tiles + fd.tile_off * (long long)ts * ts, ts, fd.nt};
-        double *vf = b->v + fd.vec_off;
-        int *stf = b->status + 2 * f;
-        xg_launch_inverse_factor(b->gX[s].map, b->fmap[f], b->gX[s].d, T.data, fd.nt, ts, stf, st);
-        xg_launch_inverse_syrk(b->gX[s].map, T.data, fd.nt, ts, stf, st);
-        const double dlogcon = -(log(2.0) + xg_digamma(fd.p.nu));
-        xg_launch_grad_contract(T.data, b->ij_by_nt[fd.nt], xg_num_lower_tiles(fd.nt), fd.nt, ts, b->x + fd.vec_off,
-                                b->y + fd.vec_off, vf, fd.N, fd.p, b->kernel, b->metric, dlogcon, b->gX[s].tab, b->gpart[s],
-                                b->gout + 4 * (size_t)f, st);
+        /* the next group's inverse factors overwrite these, not S: the
+         * contractions overlap it */
+        for (int f = g.f0; f < g.f1; ++f) {
+            if (!std::isfinite(loglik[f])) continue;
+            const XgBField &fd = b->F[f];
+            const int s = f % XgBatch::GS;
+            const double dlogcon = -(log(2.0) + xg_digamma(fd.p.nu));
+            xg_launch_grad_contract(b->tiles + fd.tile_off * (long long)ts * ts, b->ij_by_nt[fd.nt],
+                                    xg_num_lower_tiles(fd.nt), fd.nt, ts, b->x + fd.vec_off, b->y + fd.vec_off,
+                                    b->v + fd.vec_off, fd.N, fd.p, b->kernel, b->metric, dlogcon, b->gtab[s],
+                                    b->gpart[s], b->gout + 4 * (size_t)f, b->gst[s]);
+        }
     }
     XG_CU(cudaGetLastError());
     for (int s = 0; s < XgBatch::GS; ++s) XG_CU(cudaStreamSynchronize(b->gst[s]));

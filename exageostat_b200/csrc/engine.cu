@@ -95,6 +95,7 @@ int xg_context_start(int dts)
     if (e == cudaSuccess) e = xg_gradient_kernels_configure();
     if (e == cudaSuccess) e = xg_mixed_kernels_configure();
     if (e == cudaSuccess) e = xg_dag_kernels_configure();
+    if (e == cudaSuccess) e = xg_rows_kernels_configure();
     if (e == cudaSuccess) e = xg_solve_kernels_configure();
     if (e == cudaSuccess) e = xg_tab_kernels_configure(prop.multiProcessorCount);
     if (e == cudaSuccess) e = xg_sliced_kernels_configure();
@@ -345,6 +346,30 @@ static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, 
     G.status = status;
     xg_launch_dag(M.map, G, g_xg.sm_count, st);
     return nb;
+}
+
+/* X = L^-T, then Sigma^-1 = X X^T over the factor M (lower tiles) */
+void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st)
+{
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    cudaMemsetAsync(X.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    XgRowsMaps maps = {};
+    maps.y[0] = X.map;
+    maps.l[0] = M.map;
+    XgRows G = {};
+    G.y[0] = X.d;
+    G.dinv[0] = M.dinv;
+    G.s = M.d;
+    G.ts = M.ts;
+    G.nsys = 1;
+    G.one.nt = M.nt;
+    G.one.nb = nb;
+    G.ntasks = 2 * xg_num_lower_tiles(nb);
+    G.next = (unsigned *)X.dag;
+    G.abort = X.dag + 1;
+    G.flags = X.dag + 2;
+    G.status = status;
+    xg_launch_rows(XG_ROWS_INVERSE, maps, G, g_xg.sm_count, st);
 }
 
 /* v <- L^-T v for a factored M */
@@ -739,8 +764,7 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
     xg_solve_transposed(f->C, f->v, f->status, st);
-    xg_launch_inverse_factor(f->X.map, f->C.map, f->X.d, f->C.d, f->C.nt, f->C.ts, f->status, st);
-    xg_launch_inverse_syrk(f->X.map, f->C.d, f->C.nt, f->C.ts, f->status, st);
+    xg_inverse_product(f->C, f->X, f->status, st);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, f->C.nt, f->C.ts, f->x, f->y, f->v, f->N, p, f->kernel,
                             f->metric, dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));

@@ -9,14 +9,13 @@
  * exageostat_exact/cpu_core/compute/core_zcmg.c:315-488) are the math spec.
  *
  * After the forward factorisation (Sigma = L L^T in the lower tiles):
- *   1. alpha = L^-T (L^-1 z) with the backward tile solve (solve.cu).
- *   2. X = L^-T, upper triangular, by the right-looking blocked solve
- *      X L^T = I: per tile column K, X_IK = B_IK L_KK^-T (I <= K, panel TRSM
- *      on row strips), then B_IK' -= X_IK L_K'K^T (K' > K) on the FP64 tensor
- *      cores.  X_IK is stored row-major at packed slot (K, I) of a second
- *      lower-tile buffer, so both GEMM operands stay K-major for TMA.
- *   3. Sigma^-1 lower = X X^T: S_IJ = sum_{K >= I} X_IK X_JK^T, a K-looped
- *      DMMA SYRK written over the factor.
+ *   1. alpha = L^-T (L^-1 z) with the backward solve (solve.cu).
+ *   2. X = L^-T, upper triangular (rows_dag.cu; on the INT8-sliced path column
+ *      by column with the kernels below), X_IK stored row-major at packed slot
+ *      (K, I) of a second lower-tile buffer, so both GEMM operands stay
+ *      K-major for TMA.
+ *   3. Sigma^-1 lower = X X^T: S_IJ = sum_{K >= I} X_IK X_JK^T, written over
+ *      the factor (rows_dag.cu, or the sliced kernel).
  *   4. One fused pass over the lower tiles of S generates dSigma/dtheta_p on
  *      the fly (never stored) and contracts it with W.
  * Steps 2 and 3 are N^3/3 flops each (TRTRI- and LAUUM-class), so a gradient
@@ -43,9 +42,6 @@
 /* modes.  "R layout": an mt x nt grid of tiles whose tile (R, K) sits at
  * slot K * mt + R (right-hand sides stored transposed, one row per
  * right-hand side). */
-#define XG_TG_XUPDATE 1 /* step K of X L^T = I: slot(K', I) of X -= X_slot(K, I) L_slot(K', K)^T */
-#define XG_TG_SYRKX 2   /* S_IJ = sum_{K >= I} X_slot(K, I) X_slot(K, J)^T, written to C storage */
-#define XG_TG_RFWD 3    /* step K of Y L^T = B (R layout): B(R, K') -= Y(R, K) L_slot(K', K)^T, K' > K */
 #define XG_TG_RTRI 4    /* C(R, I) = sum_{K >= I} A(R, K) B_slot(K, I)^T (R layout, B lower-tile packed) */
 #define XG_TG_DENSE 5   /* full nt x nt tiles (slot A nt + B): C(A, B) = sum_K A(A, K) B(B, K)^T */
 #define XG_TG_RBWD 6    /* step K of Z L = B (R layout), B holding L's tiles transposed in place:
@@ -65,14 +61,7 @@ __device__ inline XgTileGemmJob xg_tg_decode(int mode, long long job, int nt, in
 {
     XgTileGemmJob j;
     j.skip = false;
-    if (mode == XG_TG_RFWD) {
-        const int R = (int)(job % mt), Kp = K + 1 + (int)(job / mt);
-        j.c_slot = Kp * mt + R;
-        j.a_slot0 = K * mt + R;
-        j.b_slot0 = (int)xg_tile_index(Kp, K, nt);
-        j.ntiles_k = 1;
-        j.k_step_a = j.k_step_b = 0;
-    } else if (mode == XG_TG_RTRI) {
+    if (mode == XG_TG_RTRI) {
         const int R = (int)(job % mt), I = (int)(job / mt);
         j.c_slot = I * mt + R;
         j.a_slot0 = I * mt + R;
@@ -88,31 +77,13 @@ __device__ inline XgTileGemmJob xg_tg_decode(int mode, long long job, int nt, in
         j.b_slot0 = (int)xg_tile_index(K, Kp, nt);
         j.ntiles_k = 1;
         j.k_step_a = j.k_step_b = 0;
-    } else if (mode == XG_TG_DENSE) {
+    } else { /* XG_TG_DENSE */
         const int A = (int)(job / nt), B = (int)(job % nt);
         j.c_slot = A * nt + B;
         j.a_slot0 = A * nt;
         j.b_slot0 = B * nt;
         j.k_step_a = j.k_step_b = 1;
         j.ntiles_k = nt;
-    } else if (mode == XG_TG_XUPDATE) {
-        const int width = K + 1; /* I in [0, K] */
-        const int I = (int)(job % width), Kp = K + 1 + (int)(job / width);
-        j.c_slot = (int)xg_tile_index(Kp, I, nt);
-        j.a_slot0 = (int)xg_tile_index(K, I, nt);
-        j.b_slot0 = (int)xg_tile_index(Kp, K, nt);
-        j.ntiles_k = 1;
-        j.k_step_a = j.k_step_b = 0;
-    } else {
-        int I, J;
-        xg_pair_decode(job, &I, &J); /* I >= J */
-        j.c_slot = (int)xg_tile_index(I, J, nt);
-        /* slot(K, I) for K = I.. nt-1 are consecutive in the packed column I */
-        j.a_slot0 = (int)xg_tile_index(I, I, nt);
-        j.b_slot0 = (int)xg_tile_index(I, J, nt);
-        j.ntiles_k = nt - I;
-        j.k_step_a = 1;
-        j.k_step_b = 1;
     }
     return j;
 }
@@ -130,14 +101,7 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     const int blk = blockIdx.x % (bpt * bpt);
     const int bi = blk / bpt, bj = blk % bpt;
     const XgTileGemmJob J = xg_tg_decode(mode, job, nt, K, mt);
-    /* S output is symmetric: skip the strictly upper 128-blocks of diagonal tiles */
-    bool diag_upper = false;
-    if (mode == XG_TG_SYRKX) {
-        int I, Jc;
-        xg_pair_decode(job, &I, &Jc);
-        diag_upper = (I == Jc && bj > bi);
-    }
-    if (xg_cta_should_skip(status, diag_upper)) return;
+    if (xg_cta_should_skip(status)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int s = 0; s < XG_TG_STAGES; ++s) {
@@ -168,7 +132,7 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     const int g = lane >> 2, tq = lane & 3;
     double *C = Cbase + (long long)J.c_slot * ts * ts + (long long)(bi * XG_TG_BM) * ts + bj * XG_TG_BM;
     double acc[4][4][4];
-    const bool subtract = (mode == XG_TG_XUPDATE || mode == XG_TG_RFWD || mode == XG_TG_RBWD);
+    const bool subtract = mode == XG_TG_RBWD;
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
@@ -472,25 +436,6 @@ cudaError_t xg_gradient_kernels_configure()
                                 (int)xg_xtrsm_smem_bytes(XG_MAX_TS));
 }
 
-/* X = L^-T into Xbuf (lower-tile layout, X_IK at slot (K, I)) */
-void xg_launch_inverse_factor(const CUtensorMap &mapX, const CUtensorMap &mapL, double *X, const double *L, int nt,
-                              int ts, int *status, cudaStream_t st)
-{
-    const size_t bytes = (size_t)xg_num_lower_tiles(nt) * ts * ts * sizeof(double);
-    cudaMemsetAsync(X, 0, bytes, st);
-    xg_identity_diag_kernel<<<dim3(1, nt), 256, 0, st>>>(X, nt, ts);
-    const int bpt = ts / XG_TG_BM;
-    for (int K = 0; K < nt; ++K) {
-        xg_xtrsm_kernel<false><<<(K + 1) * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(X, L, nt, ts, K, 0,
-                                                                                                 status);
-        const long long jobs = (long long)(K + 1) * (nt - K - 1);
-        if (jobs > 0)
-            xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-                mapX, mapL, X, nt, ts, XG_TG_XUPDATE, K, 0, status);
-    }
-}
-
-/* S = X X^T (lower tiles) into Sbuf */
 void xg_launch_identity_x(double *X, int nt, int ts, cudaStream_t st)
 {
     cudaMemsetAsync(X, 0, (size_t)xg_num_lower_tiles(nt) * ts * ts * sizeof(double), st);
@@ -501,14 +446,6 @@ void xg_launch_xtrsm(double *X, const double *L, int nt, int ts, int K, int *sta
 {
     xg_xtrsm_kernel<false><<<(K + 1) * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(X, L, nt, ts, K, 0,
                                                                                              status);
-}
-
-void xg_launch_inverse_syrk(const CUtensorMap &mapX, double *S, int nt, int ts, int *status, cudaStream_t st)
-{
-    const int bpt = ts / XG_TG_BM;
-    const long long jobs = xg_num_lower_tiles(nt);
-    xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-        mapX, mapX, S, nt, ts, XG_TG_SYRKX, 0, 0, status);
 }
 
 long long xg_grad_contract_blocks(long long ntiles, int ts) { return ntiles * (ts / XG_GC_ROWS); }
@@ -535,23 +472,6 @@ void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long nti
     const long long blocks = xg_grad_contract_blocks(ntiles, ts);
     xg_grad_contract_kernel<<<(unsigned)blocks, 256, 0, st>>>(S, tile_ij, nt, ts, x, y, alpha, N, p, part);
     xg_grad_reduce_kernel<<<1, dim3(32, 4), 0, st>>>(part, blocks, out);
-}
-
-/* Y L^T = B for an R-layout right-hand side B (mt tile rows) and the lower
- * tile factor L, right-looking like the inverse factor: B is overwritten with
- * Y, the transpose of L^-1 B^T. */
-void xg_launch_rhs_forward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapL, const double *L,
-                                 int nt, int ts, int *status, cudaStream_t st)
-{
-    const int bpt = ts / XG_TG_BM;
-    for (int K = 0; K < nt; ++K) {
-        xg_xtrsm_kernel<false><<<mt * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(R, L, nt, ts, K, mt,
-                                                                                            status);
-        const long long jobs = (long long)mt * (nt - K - 1);
-        if (jobs > 0)
-            xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-                mapR, mapL, R, nt, ts, XG_TG_RFWD, K, mt, status);
-    }
 }
 
 /* Z L = B for an R-layout right-hand side B and a factor whose tiles were

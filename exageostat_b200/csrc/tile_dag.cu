@@ -29,48 +29,18 @@
 #include <stdint.h>
 
 #include "xg_common.cuh"
+#include "xg_dag.cuh"
 #include "xg_kernels.h"
 #include "xg_potrf128.cuh"
 
-#define XG_D_BK 16
 #define XG_D_STAGES 4
-#define XG_D_THREADS 256
-#define XG_D_BOX_BYTES (XG_SUB * XG_D_BK * 8)
-#define XG_D_STAGE_BYTES (2 * XG_D_BOX_BYTES)
 #define XG_D_RING_BYTES (XG_D_STAGES * XG_D_STAGE_BYTES)
-/* L_JJ as six 128 x 16 boxes (its last 32 columns are not needed), the inverted 32 x 32 blocks, v_J */
-#define XG_D_TRSM_BOXES 6
-#define XG_D_TRSM_BYTES (XG_D_TRSM_BOXES * XG_D_BOX_BYTES + (XG_SUB * 32 + XG_SUB) * 8)
+/* the triangle and the inverses (xg_dag.cuh), v_J */
+#define XG_D_TRSM_BYTES (XG_D_TRI_BYTES + XG_SUB * 8)
 #define XG_D_POTRF_BYTES (XG_P_DOUBLES * 8)
 #define XG_D_MAX2(a, b) ((a) > (b) ? (a) : (b))
 #define XG_D_AREA_BYTES XG_D_MAX2(XG_D_RING_BYTES, XG_D_MAX2(XG_D_TRSM_BYTES, XG_D_POTRF_BYTES))
 #define XG_D_SMEM (1024 + XG_D_AREA_BYTES + 128)
-
-__device__ __forceinline__ int xg_dag_acquire(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void xg_dag_release(int *p)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(1) : "memory");
-}
-
-/* One thread: waits until *p is set; false after 2 s or when another CTA aborted the launch */
-__device__ __forceinline__ bool xg_dag_wait(const int *p, const int *abort)
-{
-    if (xg_dag_acquire(p)) return true;
-    const uint64_t t0 = xg_globaltimer_ns();
-    for (uint32_t it = 0;; ++it) {
-        if (xg_dag_acquire(p)) return true;
-        if ((it & 31u) == 31u) {
-            if (*(volatile const int *)abort) return false;
-            if (xg_globaltimer_ns() - t0 > 2000000000ull) return false;
-        }
-    }
-}
 
 __global__ void __launch_bounds__(XG_D_THREADS, 1)
     xg_tile_dag_kernel(const __grid_constant__ CUtensorMap map, XgDag G)
@@ -204,30 +174,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
                 }
                 const unsigned char *sa = smem + s * XG_D_STAGE_BYTES;
                 const unsigned char *sb = diag ? sa : sa + XG_D_BOX_BYTES;
-                /* k permutation inside the slab as in xg_gemm_core: lane slot tq holds k = 4 tq + {0..3} */
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int sw = ((2 * tq + half) ^ g) << 4; /* rows g + 8 m: row & 7 = g */
-                    const double2 a0 = *(const double2 *)(sa + (r0 << 7) + sw);
-                    const double2 a1 = *(const double2 *)(sa + ((r0 + 8) << 7) + sw);
-#pragma unroll
-                    for (int n0 = 0; n0 < 16; n0 += 4) {
-                        /* groups of 32 columns: the branch must skip enough work to stay a
-                         * branch (skipped by predicates, the DMMAs take their full time) */
-                        if (n0 >= nlim) break;
-                        double2 bv[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) bv[u] = *(const double2 *)(sb + ((8 * (n0 + u) + g) << 7) + sw);
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.x, a1.x,
-                                           bv[u].x);
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.y, a1.y,
-                                           bv[u].y);
-                    }
-                }
+                xg_dag_slab(acc, sa, sb, r0, g, tq, nlim);
                 __syncwarp();
                 if (lane == 0) xg_mbar_arrive(&empty[s]);
             }
@@ -277,17 +224,14 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
                 /* ---- L_IJ = C L_JJ^-T: L_JJ (as operand boxes) and the inverses of its
                  * 32 x 32 diagonal blocks into shared memory, then each warp solves its
                  * 16 rows in registers ---- */
-                const unsigned char *LS = smem;                                    /* [6][128][16], swizzled */
-                double *DS = (double *)(smem + XG_D_TRSM_BOXES * XG_D_BOX_BYTES); /* [128][32] */
-                double *VS = DS + XG_SUB * 32;                                     /* [128] v_J */
+                const double *DS = (const double *)(smem + XG_D_TRI_BOXES * XG_D_BOX_BYTES);
+                double *VS = (double *)(smem + XG_D_TRI_BYTES); /* [128] v_J */
                 if (tid == 0) {
                     if (xg_dag_wait(flagJ + xg_tile_index(J, J, nb), G.abort)) {
                         const int row = (int)((fd.tile_off + xg_tile_index(j, j, nt)) * ts + J % b * XG_SUB);
                         asm volatile("fence.proxy.async;" ::: "memory");
-                        xg_mbar_arrive_expect_tx(lbar, XG_D_TRSM_BOXES * XG_D_BOX_BYTES + (XG_SUB * 32 + (v ? XG_SUB : 0)) * 8);
-                        xg_bulk_load(DS, dinv, XG_SUB * 32 * 8, lbar);
-                        for (int u = 0; u < XG_D_TRSM_BOXES; ++u)
-                            xg_tma_load_2d(smem + u * XG_D_BOX_BYTES, &map, J % b * XG_SUB + u * XG_D_BK, row, lbar);
+                        xg_mbar_arrive_expect_tx(lbar, XG_D_TRI_BYTES + (v ? XG_SUB : 0) * 8);
+                        xg_dag_load_tri(smem, &map, J % b * XG_SUB, row, dinv, lbar);
                         if (v) xg_bulk_load(VS, v + J * XG_SUB, XG_SUB * 8, lbar);
                     } else {
                         *(volatile int *)&s_bad = 1;
@@ -305,48 +249,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
                     }
                     return;
                 }
-#pragma unroll
-                for (int cb = 0; cb < 4; ++cb) {
-                    /* X = -(acc D^T) over the 32 columns of block cb; the accumulators are the
-                     * A fragments as they stand (K runs over the columns in the lanes' order) */
-                    double x[4][4];
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) x[m][e] = 0.0;
-#pragma unroll
-                        for (int k = 0; k <= m; ++k) { /* D is lower triangular */
-                            const double2 d =
-                                *reinterpret_cast<const double2 *>(DS + (32 * cb + 8 * m + g) * 32 + 8 * k + 2 * tq);
-                            xg_dmma_16x8x4(x[m][0], x[m][1], x[m][2], x[m][3], acc[4 * cb + k][0], acc[4 * cb + k][2],
-                                           d.x);
-                            xg_dmma_16x8x4(x[m][0], x[m][1], x[m][2], x[m][3], acc[4 * cb + k][1], acc[4 * cb + k][3],
-                                           d.y);
-                        }
-                    }
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) acc[4 * cb + m][e] = -x[m][e];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            *reinterpret_cast<double2 *>(C + (long long)(r0 + 8 * h) * ts + 32 * cb + 8 * m + 2 * tq) =
-                                make_double2(acc[4 * cb + m][2 * h], acc[4 * cb + m][2 * h + 1]);
-                    }
-                    /* the columns to the right: acc += X L^T */
-#pragma unroll
-                    for (int m = 4 * cb + 4; m < 16; ++m)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const double2 l = *reinterpret_cast<const double2 *>(
-                                LS + (2 * cb + (k >> 1)) * XG_D_BOX_BYTES + ((8 * m + g) << 7) +
-                                ((((k & 1) * 4 + tq) ^ g) << 4));
-                            xg_dmma_16x8x4(acc[m][0], acc[m][1], acc[m][2], acc[m][3], acc[4 * cb + k][0],
-                                           acc[4 * cb + k][2], l.x);
-                            xg_dmma_16x8x4(acc[m][0], acc[m][1], acc[m][2], acc[m][3], acc[4 * cb + k][1],
-                                           acc[4 * cb + k][3], l.y);
-                        }
-                }
+                xg_dag_solve(acc, smem, DS, C, ts, r0, g, tq);
                 if (v) {
                     double t0 = 0.0, t1 = 0.0;
 #pragma unroll

@@ -129,6 +129,7 @@ int xg_check_theta(const double *theta, int kernel);
 int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
               cudaEvent_t *pev = nullptr);
 int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
+void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st);
 void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st);
 double xg_trailing_flops(int nt, int ts, int k);
 int xg_field_set_data(XgField *f, const double *x, const double *y, const double *z);
@@ -174,6 +175,7 @@ struct XgAssess {
     double *xo = nullptr, *yo = nullptr, *xm = nullptr, *ym = nullptr;
     double *terms = nullptr, *part = nullptr;
     int *status = nullptr;
+    int *words = nullptr; /* the forward solves: next task, abort flag, block flags of three systems */
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t ev_panel = nullptr, ev_upd = nullptr;
 };

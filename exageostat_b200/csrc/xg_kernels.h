@@ -171,6 +171,38 @@ struct XgDag {
     int *status;          /* two words per field: status, info */
 };
 cudaError_t xg_dag_kernels_configure();
+
+/* rows_dag.cu: row blocks solved against the factor, one persistent launch */
+#define XG_ROWS_INVERSE 0
+#define XG_ROWS_RHS 1
+#define XG_ROWS_MAX_SYS 3
+struct XgRowsField {
+    long long l_off, y_off; /* first packed tile of the factor and of the rows */
+    long long flag_off;     /* INVERSE: nb (nb + 1) / 2 flags; RHS: nb mr */
+    long long dinv_off;     /* first row of the inverted 32 x 32 diagonal blocks */
+    int nt, nb;             /* tiles and 128-blocks per side of the factor */
+    int mt, mr;             /* RHS: tile rows, 128-row blocks that are not padding */
+};
+struct XgRowsMaps {
+    CUtensorMap y[XG_ROWS_MAX_SYS], l[XG_ROWS_MAX_SYS];
+};
+struct XgRows {
+    double *y[XG_ROWS_MAX_SYS];          /* rows (solved in place, INVERSE: written) */
+    const double *dinv[XG_ROWS_MAX_SYS];
+    double *s;                           /* INVERSE: the factor's store, receives S */
+    int ts, nsys;
+    XgRowsField one;
+    const XgRowsField *F;
+    const int4 *tasks;                   /* (field, I, J, product?); null: a single field, every task */
+    long long ntasks;
+    unsigned *next;                      /* zero on launch, as abort and flags */
+    int *abort, *flags;
+    long long sys_flags;                 /* flags per system */
+    int *status;
+};
+cudaError_t xg_rows_kernels_configure();
+void xg_launch_rows(int mode, const XgRowsMaps &M, const XgRows &G, int max_ctas, cudaStream_t st);
+
 void xg_launch_dag(const CUtensorMap &map, const XgDag &G, int max_ctas, cudaStream_t st);
 
 cudaError_t xg_kernels_configure();
@@ -297,14 +329,9 @@ void xg_launch_bessel(const double *nu, const double *x, int n, double *out, cud
 
 /* gradient_fp64.cu */
 cudaError_t xg_gradient_kernels_configure();
-void xg_launch_inverse_factor(const CUtensorMap &mapX, const CUtensorMap &mapL, double *X, const double *L, int nt,
-                              int ts, int *status, cudaStream_t st);
-void xg_launch_inverse_syrk(const CUtensorMap &mapX, double *S, int nt, int ts, int *status, cudaStream_t st);
 /* X = 0 with identity diagonal tiles; step K of X L^T = I: X(I, K) <- X(I, K) L_KK^-T for I <= K */
 void xg_launch_identity_x(double *X, int nt, int ts, cudaStream_t st);
 void xg_launch_xtrsm(double *X, const double *L, int nt, int ts, int K, int *status, cudaStream_t st);
-void xg_launch_rhs_forward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapL, const double *L,
-                                 int nt, int ts, int *status, cudaStream_t st);
 void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapLT,
                                   const double *LT, int nt, int ts, int *status, cudaStream_t st);
 void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int mt, int nt, int ts,

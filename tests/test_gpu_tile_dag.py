@@ -56,3 +56,28 @@ def test_wide_pivot_range(gpu, ora):
         theta = [s2, 0.1, 0.5]
         z = ora.dzvg(x, y, theta, ora.dlarnv(7, n))
         assert gpu.dmle_host(x, y, z, theta, ts=128)[1] == pytest.approx(ora.dmle(x, y, z, theta)[1], rel=1e-10)
+
+
+@pytest.mark.parametrize("n", [2, 127, 129, 257, 513])
+@pytest.mark.parametrize("ts", [128, 384])
+def test_gradient_at_block_edges(gpu, ora, n, ts):
+    """The inverse and product launch and the backward solve through the
+    gradient, against the dense adjoint on the oracle's derivative tiles (1e-9
+    of its largest entry, the bar of the batched gradients); batched likewise."""
+    x, y = ora.generate_xy_loc(n, 8)
+    z = ora.dzvg(x, y, THETA, ora.dlarnv(9, n))
+    S = ora.covariance_full(x, y, THETA)
+    inv = np.linalg.inv(S)
+    a = inv @ z
+    ref = []
+    for p in range(3):
+        D = ora.dcmg_deriv(n, n, 0, 0, x, y, x, y, THETA, p, 0)
+        ref.append(0.5 * a @ D @ a - 0.5 * np.sum(inv * D))
+    with gpu.Session(x, y, dts=ts) as s:
+        s.set_data(z=z)
+        _, g = s.loglik(THETA, grad=True)
+    assert np.abs(g - ref).max() <= 1e-9 * max(1.0, np.abs(ref).max())
+    with gpu.Batch([x, x[:1], x], [y, y[:1], y], [z, z[:1], z], ts=ts) as b:
+        _, gb = b.loglik([THETA] * 3, grad=True)
+    for f in (0, 2):
+        assert np.abs(gb[f] - ref).max() <= 1e-9 * max(1.0, np.abs(ref).max())
