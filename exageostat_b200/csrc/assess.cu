@@ -397,19 +397,25 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
     const int np = kernel == 1 ? 4 : 3;
     if (!f->X.d) {
         rc = xg_tm_alloc(f->X, N, ts);
+        if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) {
+            xg_tm_free(f->X);
+            rc = xg_tm_alloc(f->X, N, ts);
+        }
         if (rc) return rc;
     }
     const size_t full = (size_t)nt * nt * ts * ts;
     const int nctas = g_xg.sm_count * 8;
     double *Sf = nullptr, *D = nullptr, *G = nullptr, *part = nullptr;
-    if (cudaMalloc(&Sf, full * sizeof(double)) != cudaSuccess || cudaMalloc(&D, full * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&G, 3 * full * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&part, 10 * (size_t)nctas * sizeof(double)) != cudaSuccess) {
+    while (cudaMalloc(&Sf, full * sizeof(double)) != cudaSuccess || cudaMalloc(&D, full * sizeof(double)) != cudaSuccess ||
+           cudaMalloc(&G, 3 * full * sizeof(double)) != cudaSuccess ||
+           cudaMalloc(&part, 10 * (size_t)nctas * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(Sf);
         cudaFree(D);
         cudaFree(G);
         cudaFree(part);
+        Sf = D = G = part = nullptr;
+        if (xg_i8_release(f->C)) continue;
         return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", 5.0 * full * sizeof(double) / 1e9);
     }
     std::vector<double> hp(10 * (size_t)nctas);

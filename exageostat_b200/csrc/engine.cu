@@ -167,6 +167,7 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
     e = cudaMalloc(&M.tab, sizeof(double) * xg_tab_doubles());
     if (e != cudaSuccess) {
         M.tab = nullptr;
+    xg_i8_release(M);
         return xg_cuda_fail(e, "element tables");
     }
     return xg_encode_tiles(&M.map, M.d, M.ntiles, ts);
@@ -317,7 +318,7 @@ int xg_check_theta(const double *theta, int kernel)
     return XG_OK;
 }
 
-/* Largest dimension factored by the tile DAG.  Milliseconds per evaluation,
+/* Largest dimension factored by the tile DAG where the INT8 path does not apply.  Milliseconds per evaluation,
  * per-step launches against the DAG: N = 1000 0.73 / 0.45, 3000 2.83 / 1.35,
  * 6000 6.43 / 3.57, 10000 17.9 / 12.8, 14000 38.2 / 32.4, 20000 97.7 / 90.9,
  * 26000 192.3 / 196.1, 32000 352 / 358: past about 22000 the trailing updates
@@ -325,19 +326,27 @@ int xg_check_theta(const double *theta, int kernel)
  * many columns, no longer stay in L2. */
 #define XG_DAG_MAX_N 22000
 
-/* The factorisation of M as one launch of the tile DAG (tile_dag.cu); returns
- * the number of partial sums of either kind. */
-static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, cudaStream_t st)
+static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *part, int *status,
+                            const XgFactorStreams &fs);
+static bool xg_i8_prepare(XgTileMatrix &M);
+static bool xg_i8_prepare_inverse(XgTileMatrix &M);
+
+/* Block columns J0 .. J1 - 1 of M by the tile DAG: the whole factorisation
+ * (0, nb), or one window of it (words: its next-task word; the flags of the
+ * whole matrix were cleared when the factorisation began). */
+static void xg_launch_dag_columns(XgTileMatrix &M, int J0, int J1, int *next, double *v, double *part, int *status,
+                                  cudaStream_t st)
 {
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
-    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    if (J1 > nb) J1 = nb;
     XgDag G = {};
     G.data = M.d;
     G.ts = M.ts;
     G.one.nt = M.nt;
     G.one.nb = nb;
-    G.ntasks = xg_num_lower_tiles(nb);
-    G.next = (unsigned *)M.dag;
+    G.J0 = J0;
+    G.ntasks = xg_num_lower_tiles(nb - J0) - xg_num_lower_tiles(nb - J1);
+    G.next = (unsigned *)next;
     G.abort = M.dag + 1;
     G.flags = M.dag + 2;
     G.dinv = M.dinv;
@@ -345,12 +354,94 @@ static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, 
     G.part = part;
     G.status = status;
     xg_launch_dag(M.map, G, g_xg.sm_count, st);
+}
+
+/* Smallest dimension whose FP64 factorisation runs its updates on the INT8
+ * tensor cores (seven digits, sliced.cu) instead of DMMA, by tile size: a
+ * panel is one chunk of the product, and each chunk's sums are brought back
+ * and scaled once, so small tiles pay that more often.  Milliseconds per
+ * evaluation, INT8 against DMMA: ts = 512 N = 5000 2.88 / 2.55, 7000 4.44 /
+ * 5.03, 20000 46.5 / 90.3, 40000 313 / 681; ts = 384 N = 9000 7.60 / 9.60; ts =
+ * 256 N = 9000 10.0 / 9.6, 14000 25.2 / 32.5; ts = 128 N = 20000 106 / 91.7. */
+static int xg_i8_min(int ts) { return ts >= 512 ? 6500 : ts >= 384 ? 8000 : ts >= 256 ? 11000 : 1 << 30; }
+
+/* The factorisation of M as one launch of the tile DAG (tile_dag.cu); returns
+ * the number of partial sums of either kind. */
+static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, cudaStream_t st)
+{
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    xg_launch_dag_columns(M, 0, nb, M.dag, v, part, status, st);
     return nb;
+}
+
+static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits);
+static void xg_digits_free(XgDigits &D);
+
+/* X = L^-T tile column by tile column -- the update from the finished columns
+ * (INT8, from the digit planes of X and L), the FP64 block solves with L_bb
+ * (one dataflow launch), the slicing of column b -- then S = X X^T over the
+ * factor in one launch.  (Overlapping the solve and slicing of column b with
+ * the update of column b + 1 on two streams, as the factorisation does,
+ * measured the same at N = 100 000: the update dominates each column.) */
+static void xg_inverse_product_sliced(XgTileMatrix &M, XgTileMatrix &X, XgSliced *sl, int *status, cudaStream_t st)
+{
+    const int ts = M.ts, nt = M.nt, bpt = ts / XG_DAG_BLOCK;
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    XgTileArgs T{M.d, ts, nt}, TX{X.d, ts, nt};
+    const long long plane = (long long)sl->X.plane_rows * ts;
+    int *windows = X.dag + xg_dag_words(nb) - nb;
+    cudaMemsetAsync(X.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    xg_launch_zero_diag(X.d, nt, ts, st);
+    XgRowsMaps maps = {};
+    maps.y[0] = X.map;
+    maps.l[0] = M.map;
+    for (int b = 0; b < nt; ++b) {
+        if (b >= 1) {
+            XgSlTask S;
+            S.mode = XG_SL_INVERSE;
+            S.col = b;
+            S.k0 = 0;
+            S.k1 = b;
+            S.sign = -1.0;
+            S.overwrite = 1;
+            xg_launch_sliced(sl->X, sl->L, TX, S, g_xg.sm_count, status, st);
+        }
+        const int J0 = b * bpt, J1 = J0 + bpt < nb ? J0 + bpt : nb;
+        XgRows G = {};
+        G.y[0] = X.d;
+        G.dinv[0] = M.dinv;
+        G.s = M.d;
+        G.ts = ts;
+        G.nsys = 1;
+        G.J0 = J0;
+        G.one.nt = nt;
+        G.one.nb = nb;
+        G.ntasks = xg_num_lower_tiles(J1) - xg_num_lower_tiles(J0);
+        G.next = (unsigned *)(windows + b);
+        G.abort = X.dag + 1;
+        G.flags = X.dag + 2;
+        G.status = status;
+        xg_launch_rows(XG_ROWS_INVERSE, maps, G, g_xg.sm_count, st);
+        xg_launch_slice_panel(TX, b, 1, sl->X.digits, sl->X.dig, sl->X.scale, plane, status, st);
+    }
+    XgSlTask S;
+    S.mode = XG_SL_SYRK;
+    S.col = 0;
+    S.k0 = 0;
+    S.k1 = nt;
+    S.sign = 1.0;
+    S.overwrite = 1;
+    xg_launch_sliced(sl->X, sl->X, T, S, g_xg.sm_count, status, st);
 }
 
 /* X = L^-T, then Sigma^-1 = X X^T over the factor M (lower tiles) */
 void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st)
 {
+    if (M.i8_factor && M.i8 && (M.i8->X.dig || xg_i8_prepare_inverse(M))) {
+        xg_inverse_product_sliced(M, X, M.i8, status, st);
+        return;
+    }
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     cudaMemsetAsync(X.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
     XgRowsMaps maps = {};
@@ -407,7 +498,14 @@ void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t s
 int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs)
 {
     /* profiled evaluations keep the per-step launches, whose kernels the profile tells apart */
-    if (M.dag && !fs.pev && M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, fs.st);
+    M.i8_factor = false;
+    if (M.dag && !fs.pev) {
+        if (M.N >= xg_i8_min(M.ts) && xg_i8_prepare(M)) {
+            M.i8_factor = true;
+            return xg_factor_sliced(M, M.i8, v, part, status, fs);
+        }
+        if (M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, fs.st);
+    }
     XgTileArgs T{M.d, M.ts, M.nt};
     const bool la = fs.st_hi != nullptr;
     cudaStream_t sp = la ? fs.st_hi : fs.st; /* panel stream */
@@ -736,6 +834,10 @@ static int xg_grad_workspace(XgField *f)
 {
     if (!f->X.d) {
         int rc = xg_tm_alloc(f->X, f->N, f->C.ts);
+        if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) {
+            xg_tm_free(f->X);
+            rc = xg_tm_alloc(f->X, f->N, f->C.ts);
+        }
         if (rc) return rc;
     }
     const long long blocks = xg_grad_contract_blocks(f->C.ntiles, f->C.ts);
@@ -759,7 +861,6 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
     rc = xg_field_loglik(f, theta, res, times);
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
-    XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, f->kernel);
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
@@ -996,7 +1097,9 @@ int xg_field_set_mixed(XgField *f, int band, int passes)
         xg_mixed_destroy(f->mx);
         f->mx = nullptr;
     }
-    return xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
+    int rc = xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
+    if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) rc = xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
+    return rc;
 }
 
 int xg_field_loglik_mixed(XgField *f, const double *theta, double *res, double *times)
@@ -1140,38 +1243,54 @@ static int xg_tiles_to_dense(XgField *f, int n, double *out)
 /* FP64 tiles, INT8-sliced off-band updates                                  */
 /* ------------------------------------------------------------------------- */
 
+static void xg_digits_free(XgDigits &D)
+{
+    if (D.dig) cudaFree(D.dig);
+    if (D.scale) cudaFree(D.scale);
+    D.dig = nullptr;
+    D.scale = nullptr;
+}
+
+/* digit planes for every tile of M's packed store */
+static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits)
+{
+    const long long rows = M.ntiles * M.ts;
+    const size_t plane = (size_t)rows * M.ts;
+    if (digits * rows > 0x7fffffffLL)
+        return xg_fail(XG_ERR_BAD_ARGUMENT, "N = %d is beyond the sliced path's 2^31-row digit store", M.N);
+    D.digits = digits;
+    D.plane_rows = (int)rows;
+    if (cudaMalloc(&D.dig, digits * plane) != cudaSuccess ||
+        cudaMalloc(&D.scale, (size_t)rows * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        xg_digits_free(D);
+        return xg_fail(XG_ERR_NO_MEMORY, "digit planes (%.2f GB)", digits * (double)plane / 1e9);
+    }
+    /* both operands are staged in boxes of 128 rows x 64 bytes (and 32 bytes for seven digits) */
+    int rc = xg_encode(&D.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 64, 128,
+                       CU_TENSOR_MAP_SWIZZLE_64B);
+    if (!rc && digits == 7)
+        rc = xg_encode(&D.map32, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 32, 128,
+                       CU_TENSOR_MAP_SWIZZLE_32B);
+    if (rc) xg_digits_free(D);
+    return rc;
+}
+
 void xg_sliced_destroy(XgSliced *s)
 {
     if (!s) return;
-    if (s->dig) cudaFree(s->dig);
-    if (s->scale) cudaFree(s->scale);
-    if (s->xdig) cudaFree(s->xdig);
-    if (s->xscale) cudaFree(s->xscale);
+    xg_digits_free(s->L);
+    xg_digits_free(s->X);
     if (s->ev_a) cudaEventDestroy(s->ev_a);
     for (int b = 0; b < 2; ++b)
         if (s->ev_p[b]) cudaEventDestroy(s->ev_p[b]);
     delete s;
 }
 
-int xg_field_set_sliced(XgField *f)
+int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits)
 {
-    if (f->sl) return XG_OK;
-    const int ts = f->C.ts;
-    if (ts % 128 != 0) return xg_fail(XG_ERR_BAD_ARGUMENT, "the sliced path needs a tile size multiple of 128");
     XgSliced *s = new XgSliced();
-    s->plane_rows = f->C.ntiles * ts;
-    const size_t plane = (size_t)s->plane_rows * ts;
-    int rc = XG_OK;
-    if (4 * s->plane_rows > 0x7fffffffLL)
-        rc = xg_fail(XG_ERR_BAD_ARGUMENT, "N = %d is beyond the sliced path's 2^31-row digit store", f->N);
-    if (!rc && (cudaMalloc(&s->dig, 4 * plane) != cudaSuccess ||
-                cudaMalloc(&s->scale, (size_t)s->plane_rows * sizeof(double)) != cudaSuccess))
-        rc = xg_fail(XG_ERR_NO_MEMORY, "digit planes (%.2f GB)", 4.0 * plane / 1e9);
-    /* both operands are staged in boxes of 128 rows x 64 bytes */
-    if (!rc)
-        rc = xg_encode(&s->map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s->dig, ts, 4 * s->plane_rows, 64, 128,
-                       CU_TENSOR_MAP_SWIZZLE_64B);
-    if (!rc) s->map_b = s->map_a;
+    int rc = xg_digits_alloc(s->L, M, digits);
     if (!rc && (cudaEventCreateWithFlags(&s->ev_a, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&s->ev_p[0], cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&s->ev_p[1], cudaEventDisableTiming) != cudaSuccess))
@@ -1180,8 +1299,50 @@ int xg_field_set_sliced(XgField *f)
         xg_sliced_destroy(s);
         return rc;
     }
-    f->sl = s;
+    *out = s;
     return XG_OK;
+}
+
+/* Gives the seven-digit planes of M back (other allocations come first) */
+bool xg_i8_release(XgTileMatrix &M)
+{
+    M.no_i8 = true;
+    if (!M.i8) return false;
+    xg_sliced_destroy(M.i8);
+    M.i8 = nullptr;
+    M.i8_factor = false;
+    return true;
+}
+
+/* whether the device has `bytes` and three times as much for others */
+static bool xg_i8_memory(size_t bytes)
+{
+    size_t fr = 0, total = 0;
+    return cudaMemGetInfo(&fr, &total) == cudaSuccess && bytes <= fr / 4;
+}
+
+static bool xg_i8_prepare(XgTileMatrix &M)
+{
+    if (M.i8) return true;
+    if (M.no_i8) return false;
+    const size_t bytes = 7 * (size_t)M.ntiles * M.ts * M.ts;
+    if (!xg_i8_memory(bytes) || xg_sliced_create(&M.i8, M, 7) != XG_OK) M.no_i8 = true;
+    return M.i8 != nullptr;
+}
+
+static bool xg_i8_prepare_inverse(XgTileMatrix &M)
+{
+    const size_t bytes = 7 * (size_t)M.ntiles * M.ts * M.ts;
+    return xg_i8_memory(bytes) && xg_digits_alloc(M.i8->X, M, 7) == XG_OK;
+}
+
+int xg_field_set_sliced(XgField *f)
+{
+    if (f->sl) return XG_OK;
+    if (f->C.ts % 128 != 0) return xg_fail(XG_ERR_BAD_ARGUMENT, "the sliced path needs a tile size multiple of 128");
+    int rc = xg_sliced_create(&f->sl, f->C, 4);
+    if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) rc = xg_sliced_create(&f->sl, f->C, 4);
+    return rc;
 }
 
 /* Left-looking factorisation with FP64 tiles and INT8-sliced updates.  For
@@ -1254,42 +1415,40 @@ static bool xg_sl_dynamic_share()
     return v == 1;
 }
 
-static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
+static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *part, int *status,
+                            const XgFactorStreams &fs)
 {
-    XgSliced *sl = f->sl;
-    XgTileMatrix &M = f->C;
     XgTileArgs T{M.d, M.ts, M.nt};
-    const int nt = M.nt;
-    const long long plane = sl->plane_rows * M.ts;
-    const int pr = (int)sl->plane_rows;
+    const int nt = M.nt, bpt = M.ts / XG_DAG_BLOCK;
+    const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    const long long plane = (long long)sl->L.plane_rows * M.ts;
+    int *windows = M.dag + xg_dag_words(nb) - nb;
     const bool la = fs.st_hi != nullptr;
     cudaStream_t sp = la ? fs.st_hi : fs.st;
     cudaEvent_t *pev = fs.pev;
     auto rec = [&](int k, int e, cudaStream_t s) {
         if (pev) cudaEventRecord(pev[8 * k + e], s);
     };
-    const int rhs = v != nullptr;
     const int sms = g_xg.sm_count;
     const bool dyn = xg_sl_dynamic_share();
     const int all = 1 << 30; /* one CTA per job */
+    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), fs.st);
     if (la) cudaEventRecord(sl->ev_a, fs.st); /* the generated matrix */
     for (int j = 0; j < nt; ++j) {
-        T.dinv = M.dinv + (size_t)j * M.ts * 32;
         if (la) cudaStreamWaitEvent(sp, sl->ev_a, 0); /* chunks k < j-1 of column j */
         rec(j, 0, sp);
         const int band_ctas = xg_panel_share(j, sms), upd_ctas = sms - band_ctas;
         if (la) {
-            if (j >= 1) xg_launch_sliced(sl->map_a, sl->map_b, sl->scale, sl->scale, T, factor_task(j, j - 1, j), pr,
-                                         dyn ? all : band_ctas, f->status, sp);
+            if (j >= 1)
+                xg_launch_sliced(sl->L, sl->L, T, factor_task(j, j - 1, j), dyn ? all : band_ctas, status, sp);
         } else {
-            xg_launch_sliced(sl->map_a, sl->map_b, sl->scale, sl->scale, T, factor_task(j, 0, j), pr, sms, f->status,
-                             sp);
+            xg_launch_sliced(sl->L, sl->L, T, factor_task(j, 0, j), sms, status, sp);
         }
         rec(j, 1, sp);
-        xg_launch_potrf_tiled(M.map, T, j, v, f->part, f->part + nt, rhs, f->status, f->info, sp);
+        /* POTRF and TRSM of the tile column: a window of the tile DAG */
+        xg_launch_dag_columns(M, j * bpt, (j + 1) * bpt, windows + j, v, part, status, sp);
         rec(j, 2, sp);
-        xg_launch_trsm_gemm(M.map, T, j, v, rhs, f->status, sp);
-        if (j + 1 < nt) xg_launch_slice_panel(T, j, 0, sl->dig, sl->scale, plane, f->status, sp);
+        if (j + 1 < nt) xg_launch_slice_panel(T, j, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, sp);
         rec(j, 3, sp);
         if (la) {
             cudaEventRecord(sl->ev_p[j & 1], sp);
@@ -1297,8 +1456,7 @@ static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
             if (j >= 1 && j + 1 < nt) cudaStreamWaitEvent(fs.st, sl->ev_p[(j - 1) & 1], 0);
             rec(j, 4, fs.st);
             if (j >= 1 && j + 1 < nt)
-                xg_launch_sliced(sl->map_a, sl->map_b, sl->scale, sl->scale, T, factor_task(j + 1, 0, j), pr,
-                                 dyn ? all : upd_ctas, f->status, fs.st);
+                xg_launch_sliced(sl->L, sl->L, T, factor_task(j + 1, 0, j), dyn ? all : upd_ctas, status, fs.st);
             rec(j, 5, fs.st);
             cudaEventRecord(sl->ev_a, fs.st);
         } else {
@@ -1312,6 +1470,7 @@ static void xg_factor_sliced(XgField *f, double *v, const XgFactorStreams &fs)
         cudaEventRecord(fs.ev_panel, sp);
         cudaStreamWaitEvent(fs.st, fs.ev_panel, 0);
     }
+    return nb;
 }
 
 /* Per-kernel-class times of the sliced factorisation from its events:
@@ -1353,9 +1512,8 @@ static void xg_field_collect_profile_sliced(XgField *f, bool lookahead)
     }
     cudaEventElapsedTime(&ms, f->ev[0], f->ev[2]);
     f->prof[7] += ms * 1e-3;
-    /* generation, finalize; per column two update launches, the sub-block POTRF
-     * sequence, TRSM, slicing */
-    f->prof[5] += 2 + (4.0 + xg_potrf_tiled_launches(f->C.ts)) * nt;
+    /* generation, finalize; per column two update launches, the panel, slicing */
+    f->prof[5] += 2 + 4.0 * nt;
     f->prof[6] += 1;
 }
 
@@ -1383,8 +1541,8 @@ int xg_field_loglik_sliced(XgField *f, const double *theta, double *res, double 
     fs.ev_panel = f->ev_panel;
     fs.ev_upd = f->ev_upd;
     fs.pev = f->profiling ? f->pev : nullptr;
-    xg_factor_sliced(f, f->v, fs);
-    xg_launch_finalize(f->part, f->part + f->C.nt, f->C.nt, f->N, f->out, f->status, f->info, st);
+    const int np = xg_factor_sliced(f->C, f->sl, f->v, f->part, f->status, fs);
+    xg_launch_finalize(f->part, f->part + np, np, f->N, f->out, f->status, f->info, st);
     XG_CU(cudaEventRecord(f->ev[2], st));
     XG_CU(cudaMemcpyAsync(f->h_out, f->out, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
     XG_CU(cudaGetLastError());
@@ -1428,7 +1586,7 @@ int xg_sliced_factor_dense(int n, const double *x, const double *y, const double
     fs.st_hi = g_xg.stream_hi;
     fs.ev_panel = f->ev_panel;
     fs.ev_upd = f->ev_upd;
-    xg_factor_sliced(f, nullptr, fs);
+    xg_factor_sliced(f->C, f->sl, nullptr, f->part, f->status, fs);
     rc = xg_tiles_to_dense(f, n, out);
     xg_field_destroy(f);
     return rc;
@@ -1447,54 +1605,17 @@ int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, do
     XgSliced *sl = f->sl;
     if ((rc = xg_grad_workspace(f))) return rc;
     const int ts = f->C.ts, nt = f->C.nt;
-    const size_t plane = (size_t)sl->plane_rows * ts;
-    if (!sl->xdig) {
-        if (cudaMalloc(&sl->xdig, 4 * plane) != cudaSuccess ||
-            cudaMalloc(&sl->xscale, (size_t)sl->plane_rows * sizeof(double)) != cudaSuccess)
-            return xg_fail(XG_ERR_NO_MEMORY, "digit planes of the inverse factor (%.2f GB)", 4.0 * plane / 1e9);
-        rc = xg_encode(&sl->xmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, sl->xdig, ts, 4 * sl->plane_rows, 64, 128,
-                       CU_TENSOR_MAP_SWIZZLE_64B);
-        if (rc) return rc;
+    if (!sl->X.dig && (rc = xg_digits_alloc(sl->X, f->C, 4))) {
+        if (rc != XG_ERR_NO_MEMORY || !xg_i8_release(f->C) || (rc = xg_digits_alloc(sl->X, f->C, 4))) return rc;
     }
     rc = xg_field_loglik_sliced(f, theta, res, times);
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
-    XgTileArgs T{f->C.d, ts, nt};
-    XgTileArgs TX{f->X.d, ts, nt};
-    const int pr = (int)sl->plane_rows;
     const XgMaternParams p = xg_params(theta, f->kernel);
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
     xg_solve_transposed(f->C, f->v, f->status, st);
-    xg_launch_identity_x(f->X.d, nt, ts, st);
-    /* X = L^-T column by column: the update of column b from the finished
-     * columns c < b (INT8-sliced), the FP64 solve with L_bb, the slicing of
-     * column b.  (Overlapping the solve and slicing of column b with the
-     * update of column b + 1 on two streams, as the factorisation does, was
-     * measured at the same 5.87 s per gradient at N = 100 000: the update
-     * dominates each column.) */
-    for (int b = 0; b < nt; ++b) {
-        if (b >= 1) {
-            XgSlTask S;
-            S.mode = XG_SL_INVERSE;
-            S.col = b;
-            S.k0 = 0;
-            S.k1 = b;
-            S.sign = -1.0;
-            S.overwrite = 0;
-            xg_launch_sliced(sl->xmap, sl->map_b, sl->xscale, sl->scale, TX, S, pr, g_xg.sm_count, f->status, st);
-        }
-        xg_launch_xtrsm(f->X.d, f->C.d, nt, ts, b, f->status, st);
-        xg_launch_slice_panel(TX, b, 1, sl->xdig, sl->xscale, (long long)plane, f->status, st);
-    }
-    XgSlTask S;
-    S.mode = XG_SL_SYRK;
-    S.col = 0;
-    S.k0 = 0;
-    S.k1 = nt;
-    S.sign = 1.0;
-    S.overwrite = 1;
-    xg_launch_sliced(sl->xmap, sl->xmap, sl->xscale, sl->xscale, T, S, pr, g_xg.sm_count, f->status, st);
+    xg_inverse_product_sliced(f->C, f->X, sl, f->status, st);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, nt, ts, f->x, f->y, f->v, f->N, p, f->kernel, f->metric,
                             dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));

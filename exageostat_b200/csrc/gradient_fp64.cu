@@ -217,18 +217,15 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
 }
 
 /* ========================================================================== */
-/* Right-side TRSM on the row of X tiles of step K: X_IK <- X_IK L_KK^-T      */
+/* Right-side backward solve of step K: Z_RK <- Z_RK L_KK^-1                 */
 /* ========================================================================== */
 
 #define XG_XT_THREADS 512
 #define XG_XT_SR 32
 
-/* mt == 0: the tiles X_IK, I <= K, at slot (K, I) (inverse factor);
- * mt  > 0: the tiles (R, K), R < mt, of an R-layout matrix (right-hand sides).
- * UPPER: the diagonal tile holds U = L_KK^T (a factor transposed in place)
- * and the solve is B <- B U^-T = B L_KK^-1, by 32-column blocks from the
- * right (backward substitution). */
-template <bool UPPER>
+/* The tiles (R, K), R < mt, of an R-layout matrix; the diagonal tile holds U =
+ * L_KK^T (a factor transposed in place) and the solve is B <- B U^-T = B
+ * L_KK^-1, by 32-column blocks from the right (backward substitution). */
 __global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restrict__ X, const double *__restrict__ Lt,
                                                                  int nt, int ts, int K, int mt, const int *status)
 {
@@ -238,10 +235,10 @@ __global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restr
     double *LD = S + XG_XT_SR * LDS;   /* [32][33] */
     if (xg_cta_should_skip(status)) return;
     const int strips = ts / XG_XT_SR;
-    const int I = blockIdx.x / strips, strip = blockIdx.x % strips; /* I in [0, K] */
+    const int I = blockIdx.x / strips, strip = blockIdx.x % strips;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    const long long bslot = mt > 0 ? (long long)K * mt + I : xg_tile_index(K, I, nt);
+    const long long bslot = (long long)K * mt + I;
     double *B = X + bslot * (long long)ts * ts + (long long)strip * XG_XT_SR * ts;
     const double *L = Lt + xg_tile_index(K, K, nt) * (long long)ts * ts;
     for (int idx = tid; idx < XG_XT_SR * ts; idx += blockDim.x) {
@@ -249,7 +246,7 @@ __global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restr
         S[r * LDS + c] = B[(long long)r * ts + c];
     }
     for (int blk = 0; blk < ts / 32; ++blk) {
-        const int cb = UPPER ? ts - 32 * (blk + 1) : 32 * blk;
+        const int cb = ts - 32 * (blk + 1);
         for (int idx = tid; idx < 32 * 32; idx += blockDim.x) {
             const int r = idx >> 5, c = idx & 31;
             LD[r * 33 + c] = L[(long long)(cb + r) * ts + cb + c];
@@ -259,32 +256,21 @@ __global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restr
             double row[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) row[j] = S[lane * LDS + cb + j];
-            if (UPPER) {
 #pragma unroll
-                for (int j = 31; j >= 0; --j) {
-                    double s = row[j];
+            for (int j = 31; j >= 0; --j) {
+                double s = row[j];
 #pragma unroll
-                    for (int q = j + 1; q < 32; ++q) s -= row[q] * LD[j * 33 + q];
-                    row[j] = s / LD[j * 33 + j];
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    double s = row[j];
-#pragma unroll
-                    for (int q = 0; q < j; ++q) s -= row[q] * LD[j * 33 + q];
-                    row[j] = s / LD[j * 33 + j];
-                }
+                for (int q = j + 1; q < 32; ++q) s -= row[q] * LD[j * 33 + q];
+                row[j] = s / LD[j * 33 + j];
             }
 #pragma unroll
             for (int j = 0; j < 32; ++j) S[lane * LDS + cb + j] = row[j];
         }
         __syncthreads();
-        /* the solved block's contribution to the columns still to solve:
-         * right of it (lower) or left of it (upper) */
-        const int ngrp = UPPER ? cb / 32 : (ts - cb - 32) / 32;
+        /* the solved block's contribution to the columns still to solve */
+        const int ngrp = cb / 32;
         for (int grp = warp; grp < ngrp; grp += XG_XT_THREADS / 32) {
-            const int c0 = UPPER ? grp * 32 : cb + 32 + grp * 32;
+            const int c0 = grp * 32;
             double acc[2][4][4];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
@@ -328,12 +314,13 @@ __global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restr
     }
 }
 
-/* X starts as the identity on its diagonal tiles and zero elsewhere. */
-__global__ void xg_identity_diag_kernel(double *X, int nt, int ts)
+/* zeros the diagonal tiles: the block solves of X = L^-T write only its upper
+ * 128-blocks, the digit slicing reads whole tiles */
+__global__ void xg_zero_diag_kernel(double *X, int nt, int ts)
 {
-    const int K = blockIdx.y;
-    double *T = X + xg_tile_index(K, K, nt) * (long long)ts * ts;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < ts; r += gridDim.x * blockDim.x) T[(long long)r * ts + r] = 1.0;
+    double2 *T = reinterpret_cast<double2 *>(X + xg_tile_index((int)blockIdx.y, (int)blockIdx.y, nt) * (long long)ts * ts);
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ts * ts / 2; e += gridDim.x * blockDim.x)
+        T[e] = make_double2(0.0, 0.0);
 }
 
 /* ========================================================================== */
@@ -429,23 +416,13 @@ cudaError_t xg_gradient_kernels_configure()
     cudaError_t e = cudaFuncSetAttribute(xg_tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)xg_tile_gemm_smem_bytes());
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(xg_xtrsm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)xg_xtrsm_smem_bytes(XG_MAX_TS));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(xg_xtrsm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(xg_xtrsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)xg_xtrsm_smem_bytes(XG_MAX_TS));
 }
 
-void xg_launch_identity_x(double *X, int nt, int ts, cudaStream_t st)
+void xg_launch_zero_diag(double *X, int nt, int ts, cudaStream_t st)
 {
-    cudaMemsetAsync(X, 0, (size_t)xg_num_lower_tiles(nt) * ts * ts * sizeof(double), st);
-    xg_identity_diag_kernel<<<dim3(1, nt), 256, 0, st>>>(X, nt, ts);
-}
-
-void xg_launch_xtrsm(double *X, const double *L, int nt, int ts, int K, int *status, cudaStream_t st)
-{
-    xg_xtrsm_kernel<false><<<(K + 1) * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(X, L, nt, ts, K, 0,
-                                                                                             status);
+    xg_zero_diag_kernel<<<dim3(16, nt), 256, 0, st>>>(X, nt, ts);
 }
 
 long long xg_grad_contract_blocks(long long ntiles, int ts) { return ntiles * (ts / XG_GC_ROWS); }
@@ -482,7 +459,7 @@ void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, co
 {
     const int bpt = ts / XG_TG_BM;
     for (int K = nt - 1; K >= 0; --K) {
-        xg_xtrsm_kernel<true><<<mt * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(R, LT, nt, ts, K,
+        xg_xtrsm_kernel<<<mt * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(R, LT, nt, ts, K,
                                                                                                  mt, status);
         const long long jobs = (long long)mt * K;
         if (jobs > 0)

@@ -5,7 +5,9 @@
  *
  *   XG_ROWS_INVERSE  X L^T = I (X = L^-T, upper triangular, X_IK at packed tile slot (K, I)), then
  *                    S = X X^T written over the factor: the inverse and product of the adjoint
- *                    gradient and of the Fisher matrix (steps 2 and 3 of gradient_fp64.cu)
+ *                    gradient and of the Fisher matrix (steps 2 and 3 of gradient_fp64.cu);
+ *                    a window of columns J0 .. : the sums over K < J0 are in place already
+ *                    and there are no products (the INT8 path)
  *   XG_ROWS_RHS      Y L^T = B for row blocks in R layout (tile (R, K) at slot K mt + R), up to
  *                    three systems at once: the forward solves of MLOE / MMOM (MLE_dexact.c:1300-1364)
  *
@@ -58,12 +60,12 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1) xg_rows_dag_kernel(const __gr
         s_bad = 0;
     }
     uint32_t it0 = 0, lphase = 0;
-    for (bool first = true;; first = false) {
+    for (;;) {
         __syncthreads(); /* the previous task is finished by every thread */
         if (tid == 0) {
             long long q = -1;
             if (!*(volatile int *)G.abort) {
-                q = first ? (long long)blockIdx.x : (long long)gridDim.x + (long long)atomicAdd(G.next, 1u);
+                q = (long long)atomicAdd(G.next, 1u);
                 if (q >= G.ntasks) q = -1;
             }
             s_task = q;
@@ -90,7 +92,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1) xg_rows_dag_kernel(const __gr
             if (product)
                 xg_pair_decode(q - nx, &I, &J); /* I ascending: the longest sums first */
             else
-                xg_pair_decode(q, &J, &I);
+                xg_pair_decode(q + xg_num_lower_tiles(G.J0), &J, &I);
         }
         const XgRowsField fd = G.tasks ? G.F[f] : G.one;
         const int nt = fd.nt, nb = fd.nb, i = I / b, j = J / b;
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1) xg_rows_dag_kernel(const __gr
             double *C = product ? G.s + (fd.l_off + xg_tile_index(i, j, nt)) * (long long)ts * ts
                                 : G.y[sys] + slotY(I, J) * (long long)ts * ts;
             C += (long long)(I % b * XG_DAG_BLOCK) * ts + J % b * XG_DAG_BLOCK;
-            const int k0 = MODE == XG_ROWS_RHS ? 0 : I, k1 = product ? nb : J;
+            const int k0 = MODE == XG_ROWS_RHS ? 0 : product || I > G.J0 ? I : G.J0, k1 = product ? nb : J;
             const int KT = (k1 - k0) * SPB;
             const bool same = product && I == J; /* both operands are the same rows */
             double acc[16][4];
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1) xg_rows_dag_kernel(const __gr
                 for (int h = 0; h < 2; ++h) {
                     double2 c = make_double2(0.0, 0.0);
                     const int r = r0 + 8 * h, cc = 8 * n + 2 * tq;
-                    if (MODE == XG_ROWS_RHS)
+                    if (MODE == XG_ROWS_RHS || I < G.J0)
                         c = __ldcg(reinterpret_cast<const double2 *>(C + (long long)r * ts + cc));
                     else if (!product && I == J) /* the identity */
                         c = make_double2(r == cc ? 1.0 : 0.0, r == cc + 1 ? 1.0 : 0.0);

@@ -68,6 +68,7 @@
 #define XG_SL_STAGES 3
 #define XG_SL_ABOX_BYTES (XG_SL_BM * XG_SL_BK)                                  /* one digit plane, 128 rows */
 #define XG_SL_BBOX_BYTES (XG_SL_BN * XG_SL_BK)                                  /* one digit plane, 128 rows */
+#define XG_SL_BOX32_BYTES (128 * 32) /* second pass: one digit plane, 128 rows, 32 bytes */
 #define XG_SL_STAGE_BYTES (XG_SL_SLICES * (XG_SL_ABOX_BYTES + XG_SL_BBOX_BYTES)) /* 64 KB */
 /* per panel chunk, the 128 A-row and 128 B-row scales, double-buffered */
 #define XG_SL_SCALE_BYTES (2 * 2 * 128 * 8)
@@ -92,7 +93,12 @@ __device__ __forceinline__ double xg_i64_to_f64(long long x)
 
 /* One warp per panel row: rows of tiles k+1 .. nt-1 of column k.  Lane l owns
  * elements c * 128 + 4 l .. + 3 for every 128-column chunk c, so each load
- * instruction reads 1 KB of the row and each digit store writes 128 bytes. */
+ * instruction reads 1 KB of the row and each digit store writes 128 bytes.
+ * ND = 4: the scale is max / 127.  ND = 7: the power of two that brings the
+ * maximum into (63.5, 127], so that the scaling, every digit's remainder and
+ * the product of two scales are exact; the digits then hold the element to
+ * 2^-54.9 of the row's maximum or better. */
+template <int ND>
 __global__ void __launch_bounds__(256) xg_slice_panel_kernel(XgTileArgs T, int k, int row_mode,
                                                              int8_t *__restrict__ dig, double *__restrict__ scale,
                                                              long long plane, const int *status)
@@ -110,6 +116,7 @@ __global__ void __launch_bounds__(256) xg_slice_panel_kernel(XgTileArgs T, int k
     const int nch = ts / 128; /* <= 4 */
     double v[16];
     double m = 0.0;
+    bool nan = false; /* ND = 7: a row with a NaN or infinity keeps it in its scale */
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         if (c < nch) {
@@ -120,22 +127,37 @@ __global__ void __launch_bounds__(256) xg_slice_panel_kernel(XgTileArgs T, int k
             v[4 * c + 2] = b.x;
             v[4 * c + 3] = b.y;
             m = fmax(m, fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y))));
+            if (ND == 7) nan = nan || isnan(a.x + a.y + b.x + b.y);
         }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (ND == 7) nan = __any_sync(0xffffffffu, nan) || isinf(m);
     const long long grow = slot * ts + r; /* tile-packed row index */
-    const double c0 = m > 0.0 ? XG_SL_TOP / m : 0.0;
-    if (lane == 0) scale[grow] = m / XG_SL_TOP;
+    double c0, sc;
+    if (ND == 4) {
+        c0 = m > 0.0 ? XG_SL_TOP / m : 0.0;
+        sc = m / XG_SL_TOP;
+    } else {
+        /* m = f 2^e, 1/2 <= f < 1: times 2^(7 - e) it is in [64, 128); one less where that passes 127 */
+        int e = 0;
+        const double fr = m > 0.0 ? frexp(m, &e) : 0.0;
+        e = 7 - e - (fr > XG_SL_TOP / 128.0 ? 1 : 0);
+        c0 = m > 0.0 ? ldexp(1.0, e) : 0.0;
+        sc = nan ? m + __longlong_as_double(0x7FF8000000000000LL) : m > 0.0 ? ldexp(1.0, -e) : 0.0;
+    }
+    if (lane == 0) scale[grow] = sc;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         if (c < nch) {
-            uint32_t w[XG_SL_SLICES] = {0u, 0u, 0u, 0u};
+            uint32_t w[ND];
+#pragma unroll
+            for (int t = 0; t < ND; ++t) w[t] = 0u;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 double x = v[4 * c + e] * c0; /* |x| <= 127 */
 #pragma unroll
-                for (int t = 0; t < XG_SL_SLICES; ++t) {
+                for (int t = 0; t < ND; ++t) {
                     double d = rint(x);
                     d = fmin(fmax(d, -XG_SL_TOP), XG_SL_TOP);
                     x = (x - d) * XG_SL_RADIX; /* remainder in [-1/2, 1/2] digit units, scaled to the next digit */
@@ -143,7 +165,7 @@ __global__ void __launch_bounds__(256) xg_slice_panel_kernel(XgTileArgs T, int k
                 }
             }
 #pragma unroll
-            for (int t = 0; t < XG_SL_SLICES; ++t)
+            for (int t = 0; t < ND; ++t)
                 *reinterpret_cast<uint32_t *>(dig + t * plane + grow * ts + c * 128 + 4 * lane) = w[t];
         }
     }
@@ -222,8 +244,15 @@ __device__ __forceinline__ long long xg_sl_slot_b(const XgSlTask &S, const XgSlJ
     return S.mode == XG_SL_SYRK ? xg_tile_index(k, J.tb, nt) : xg_tile_index(J.tb, k, nt); /* X(b,k) | L(j,k) */
 }
 
+/* ND = 4: one pass per chunk, levels 0-3 of digits 0-3.  ND = 7: a second
+ * pass for levels 4-6 (18 pairs of digits 0-6, K in 32-byte slabs so that the
+ * fourteen digit boxes fit a stage), whose sums are below the first pass's by
+ * 254^-3: together 28 pairs, an FP64-grade product (the digits to 2^-55 of the
+ * row maxima, products below 254^-6 dropped, sums exact). */
+template <int ND>
 __global__ void __launch_bounds__(XG_SL_THREADS, 1)
     xg_sliced_left_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                          const __grid_constant__ CUtensorMap map_a32, const __grid_constant__ CUtensorMap map_b32,
                           const double *__restrict__ scale_a, const double *__restrict__ scale_b, XgTileArgs T,
                           XgSlTask S, long long njobs, int plane_rows, int *status)
 {
@@ -261,6 +290,7 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
     xg_tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const int KT = ts / XG_SL_BK;
+    constexpr int PASSES = ND == 4 ? 1 : 2;
     bool ok = true;
 
     if (warp < 4) {
@@ -292,7 +322,7 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                         xg_bulk_load(sscale + sb * 256 + 128, scale_b + slot_b * ts + J.bn * XG_SL_BN, XG_SL_BN * 8,
                                      &sfull[sb]);
                     }
-                    for (int kb = 0; kb < KT; ++kb, ++it) {
+                    for (int kb = 0; kb < (PASSES == 1 ? KT : 3 * KT); ++kb, ++it) {
                         const int s = (int)(it % XG_SL_STAGES);
                         if (it >= XG_SL_STAGES &&
                             !xg_mbar_wait(&empty[s], (uint32_t)((it / XG_SL_STAGES) - 1) & 1)) {
@@ -300,6 +330,17 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                             break;
                         }
                         unsigned char *st = smem + s * XG_SL_STAGE_BYTES;
+                        if (kb >= KT) { /* second pass: 32-byte slabs of all seven digits */
+                            const int x = (kb - KT) * 32;
+                            xg_mbar_arrive_expect_tx(&full[s], 2 * ND * XG_SL_BOX32_BYTES);
+#pragma unroll
+                            for (int t = 0; t < ND; ++t) {
+                                xg_tma_load_2d(st + t * XG_SL_BOX32_BYTES, &map_a32, x, t * plane_rows + rowA, &full[s]);
+                                xg_tma_load_2d(st + (ND + t) * XG_SL_BOX32_BYTES, &map_b32, x, t * plane_rows + rowB,
+                                               &full[s]);
+                            }
+                            continue;
+                        }
                         xg_mbar_arrive_expect_tx(&full[s], XG_SL_STAGE_BYTES);
 #pragma unroll
                         for (int t = 0; t < XG_SL_SLICES; ++t) {
@@ -327,14 +368,15 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
             for (long long job = blockIdx.x; job < njobs && ok; job += gridDim.x) {
                 XgSlJob J;
                 if (!xg_sl_job(S, job, nt, ts, J)) continue;
-                for (int k = J.k0; k < J.k1 && ok; ++k, ++cc) {
+                for (int k = J.k0; k < J.k1 && ok; ++k)
+                for (int pass = 0; pass < PASSES && ok; ++pass, ++cc) {
                     if (cc >= 1 && !xg_mbar_wait(acc_empty, (uint32_t)(cc - 1) & 1)) {
                         ok = false;
                         break;
                     }
                     xg_tc_fence_after();
                     const uint32_t dt = tmem;
-                    for (int kb = 0; kb < KT; ++kb, ++it) {
+                    for (int kb = 0; kb < (pass ? 2 * KT : KT); ++kb, ++it) {
                         const int s = (int)(it % XG_SL_STAGES);
                         if (!xg_mbar_wait(&full[s], (uint32_t)(it / XG_SL_STAGES) & 1)) {
                             ok = false;
@@ -342,22 +384,33 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                         }
                         xg_tc_fence_after();
                         const uint32_t sa = sbase + s * XG_SL_STAGE_BYTES;
-                        const uint32_t sb = sa + XG_SL_SLICES * XG_SL_ABOX_BYTES;
+                        if (pass == 0) {
+                            const uint32_t sb = sa + XG_SL_SLICES * XG_SL_ABOX_BYTES;
 #pragma unroll
-                        for (int kk = 0; kk < XG_SL_BK / 32; ++kk) {
-                            /* K = 32 int8 = 32 bytes per MMA inside the 64-byte swizzled row */
+                            for (int kk = 0; kk < XG_SL_BK / 32; ++kk) {
+                                /* K = 32 int8 = 32 bytes per MMA inside the 64-byte swizzled row */
 #pragma unroll
-                            for (int p = 0; p < 10; ++p) {
-                                int a, b;
-                                xg_sl_pair(p, a, b);
-                                const uint64_t ad = xg_umma_desc_sw64(sa + a * XG_SL_ABOX_BYTES + kk * 32);
-                                const uint64_t bd = xg_umma_desc_sw64(sb + b * XG_SL_BBOX_BYTES + kk * 32);
-                                const bool starts = (p == 0 || p == 1 || p == 3 || p == 6);
-                                /* the transposed block E_b D_a^T: TMEM lane = column of
-                                 * C, TMEM column = row of C */
-                                xg_umma_i8(dt + (uint32_t)((a + b) * XG_SL_BM), bd, ad, idesc,
-                                           (kb | kk) != 0 || !starts);
+                                for (int p = 0; p < 10; ++p) {
+                                    int a, b;
+                                    xg_sl_pair(p, a, b);
+                                    const uint64_t ad = xg_umma_desc_sw64(sa + a * XG_SL_ABOX_BYTES + kk * 32);
+                                    const uint64_t bd = xg_umma_desc_sw64(sb + b * XG_SL_BBOX_BYTES + kk * 32);
+                                    const bool starts = (p == 0 || p == 1 || p == 3 || p == 6);
+                                    /* the transposed block E_b D_a^T: TMEM lane = column of
+                                     * C, TMEM column = row of C */
+                                    xg_umma_i8(dt + (uint32_t)((a + b) * XG_SL_BM), bd, ad, idesc,
+                                               (kb | kk) != 0 || !starts);
+                                }
                             }
+                        } else {
+                            const uint32_t sb = sa + ND * XG_SL_BOX32_BYTES;
+#pragma unroll
+                            for (int lv = 4; lv < 7; ++lv)
+#pragma unroll
+                                for (int a = 0; a <= lv; ++a)
+                                    xg_umma_i8(dt + (uint32_t)((lv - 4) * XG_SL_BM),
+                                               xg_umma_desc_sw32(sb + (lv - a) * XG_SL_BOX32_BYTES),
+                                               xg_umma_desc_sw32(sa + a * XG_SL_BOX32_BYTES), idesc, kb != 0 || a != 0);
                         }
                         xg_umma_commit(&empty[s]);
                     }
@@ -378,7 +431,7 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
          * Per chunk k it adds s_A(row) s_B(col) sum_t 254^-t level_t to 64 FP64
          * sums; after the last chunk C -= sums. ---- */
         const int q = warp & 3, h = (warp - 4) >> 2;
-        long long cc = 0;
+        long long cc = 0, ck = 0; /* accumulations, chunks */
         for (long long job = blockIdx.x; job < njobs && ok; job += gridDim.x) {
             XgSlJob J;
             if (!xg_sl_job(S, job, nt, ts, J)) continue;
@@ -398,9 +451,9 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
             double res[64];
 #pragma unroll
             for (int u = 0; u < 64; ++u) res[u] = 0.0;
-            for (int k = J.k0; k < J.k1; ++k, ++cc) {
-                const int sb = (int)(cc & 1);
-                if (!xg_mbar_wait(&sfull[sb], (uint32_t)(cc >> 1) & 1) || !xg_mbar_wait(acc_full, (uint32_t)cc & 1)) {
+            for (int k = J.k0; k < J.k1; ++k, ++cc, ++ck) {
+                const int sb = (int)(ck & 1);
+                if (!xg_mbar_wait(&sfull[sb], (uint32_t)(ck >> 1) & 1) || !xg_mbar_wait(acc_full, (uint32_t)cc & 1)) {
                     if (lane == 0) atomicOr(status, XG_ST_TIMEOUT);
                     ok = false;
                     break;
@@ -463,6 +516,47 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                         if (lane == 0) xg_mbar_arrive(acc_empty);
                     }
                 }
+                if (PASSES == 2) {
+                    /* levels 4-6: v = (L4 254 + L5) 254 + L6 (|v| < 2^42), weighted 254^-6;
+                     * eight batches of 8 columns, pipelined like the first pass */
+                    ++cc;
+                    if (!xg_mbar_wait(acc_full, (uint32_t)cc & 1)) {
+                        if (lane == 0) atomicOr(status, XG_ST_TIMEOUT);
+                        ok = false;
+                        break;
+                    }
+                    xg_tc_fence_after();
+                    const double sc6 = sc * XG_SL_INV_RADIX3;
+                    uint32_t P[2][3][8];
+#pragma unroll
+                    for (int l = 0; l < 3; ++l) xg_tmem_ld_32x32b_x8(base + (uint32_t)(l * XG_SL_BM), P[0][l]);
+                    xg_tmem_ld_wait();
+#pragma unroll
+                    for (int b = 0; b < 8; ++b) {
+                        if (b < 7)
+#pragma unroll
+                            for (int l = 0; l < 3; ++l)
+                                xg_tmem_ld_32x32b_x8(base + (uint32_t)(l * XG_SL_BM + (b + 1) * 8), P[(b + 1) & 1][l]);
+#pragma unroll
+                        for (int u = 0; u < 8; u += 2) {
+                            const double2 s2 = sr2[(b * 8 + u) >> 1];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const long long v = (long long)(int)P[b & 1][0][u + e] * 64516 +
+                                                    ((long long)(int)P[b & 1][1][u + e] * 254 +
+                                                     (int)P[b & 1][2][u + e]);
+                                res[b * 8 + u + e] =
+                                    fma((e ? s2.y : s2.x) * sc6, xg_i64_to_f64(v), res[b * 8 + u + e]);
+                            }
+                        }
+                        if (b < 7) xg_tmem_ld_wait();
+                        if (b == 6) {
+                            xg_tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) xg_mbar_arrive(acc_empty);
+                        }
+                    }
+                }
                 /* this chunk's scale buffer may be refilled */
                 __syncwarp();
                 if (lane == 0) xg_mbar_arrive(&sempty[sb]);
@@ -498,19 +592,25 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
 
 cudaError_t xg_sliced_kernels_configure()
 {
-    return cudaFuncSetAttribute(xg_sliced_left_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM);
+    cudaError_t e =
+        cudaFuncSetAttribute(xg_sliced_left_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(xg_sliced_left_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM);
 }
 
-void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int8_t *dig, double *scale, long long plane,
-                           const int *status, cudaStream_t st)
+void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int digits, int8_t *dig, double *scale,
+                           long long plane, const int *status, cudaStream_t st)
 {
     const long long rows = (long long)(row_mode ? k + 1 : T.nt - k - 1) * T.ts;
     if (rows <= 0) return;
-    xg_slice_panel_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(T, k, row_mode, dig, scale, plane, status);
+    const unsigned grid = (unsigned)((rows + 7) / 8);
+    if (digits == 4)
+        xg_slice_panel_kernel<4><<<grid, 256, 0, st>>>(T, k, row_mode, dig, scale, plane, status);
+    else
+        xg_slice_panel_kernel<7><<<grid, 256, 0, st>>>(T, k, row_mode, dig, scale, plane, status);
 }
 
-void xg_launch_sliced(const CUtensorMap &map_a, const CUtensorMap &map_b, const double *scale_a,
-                      const double *scale_b, const XgTileArgs &T, const XgSlTask &S, int plane_rows, int max_ctas,
+void xg_launch_sliced(const XgDigits &A, const XgDigits &B, const XgTileArgs &T, const XgSlTask &S, int max_ctas,
                       int *status, cudaStream_t st)
 {
     if (S.k1 <= S.k0 || S.col >= T.nt) return;
@@ -522,6 +622,10 @@ void xg_launch_sliced(const CUtensorMap &map_a, const CUtensorMap &map_b, const 
     const long long njobs = units * per;
     if (njobs <= 0) return;
     const unsigned grid = (unsigned)(njobs < max_ctas ? njobs : max_ctas);
-    xg_sliced_left_kernel<<<grid, XG_SL_THREADS, XG_SL_SMEM, st>>>(map_a, map_b, scale_a, scale_b, T, S, njobs,
-                                                                   plane_rows, status);
+    if (A.digits == 4)
+        xg_sliced_left_kernel<4><<<grid, XG_SL_THREADS, XG_SL_SMEM, st>>>(A.map, B.map, A.map, B.map, A.scale, B.scale,
+                                                                          T, S, njobs, A.plane_rows, status);
+    else
+        xg_sliced_left_kernel<7><<<grid, XG_SL_THREADS, XG_SL_SMEM, st>>>(A.map, B.map, A.map32, B.map32, A.scale,
+                                                                          B.scale, T, S, njobs, A.plane_rows, status);
 }

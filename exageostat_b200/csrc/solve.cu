@@ -93,10 +93,10 @@ __global__ void __launch_bounds__(XG_TL_THREADS, 1) xg_trsv_lt_kernel(XgTrsv G)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ts = G.ts, b = ts / 128;
     if (tid == 0) s_bad = 0;
-    for (bool first = true;; first = false) {
+    for (;;) {
         __syncthreads();
         if (tid == 0) {
-            long long q = first ? (long long)blockIdx.x : (long long)gridDim.x + (long long)atomicAdd(G.next, 1u);
+            long long q = (long long)atomicAdd(G.next, 1u);
             if (q >= G.ntasks || *(volatile int *)G.abort) q = -1;
             s_task = q;
         }

@@ -7,6 +7,9 @@
  * step.  Here block (I, J) of the factor is ONE task of one CTA:
  *
  *   C = A_IJ - sum_{K < J} L_IK L_JK^T     TMA-fed DMMA, C in registers throughout
+ *                                          (K >= J0 in a window of columns J0 .. : the
+ *                                          panels of the INT8 path, whose earlier columns
+ *                                          are already applied)
  *   I == J: L_JJ = chol(C) (xg_potrf128), log-det, forward solve of v_J
  *   I >  J: L_IJ = C L_JJ^-T in the same registers, v_I -= L_IJ v_J
  *
@@ -71,12 +74,12 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
         s_bad = 0;
     }
     uint32_t it0 = 0, lphase = 0; /* slabs of all tasks so far; phase of lbar */
-    for (bool first = true;; first = false) {
+    for (;;) {
         __syncthreads(); /* the previous task is finished by every thread */
         if (tid == 0) {
             long long q = -1;
             if (!*(volatile int *)G.abort) {
-                q = first ? (long long)blockIdx.x : (long long)gridDim.x + (long long)atomicAdd(G.next, 1u);
+                q = (long long)atomicAdd(G.next, 1u);
                 if (q >= G.ntasks) q = -1;
             }
             s_task = q;
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
             I = t.y;
             J = t.z;
         } else {
-            const int2 t = xg_tile_decode_fast(q, G.one.nb);
+            const int2 t = xg_tile_decode_fast(q + xg_tile_index(G.J0, G.J0, G.one.nb), G.one.nb);
             I = t.x;
             J = t.y;
         }
@@ -122,8 +125,8 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
                     acc[n][2 * h] = -c.x;
                     acc[n][2 * h + 1] = -c.y;
                 }
-            const int KT = J * (XG_SUB / XG_D_BK);
-            int issued = 0, ready = 0; /* thread 0: slabs issued; operand blocks known to be finished */
+            const int KT = (J - G.J0) * (XG_SUB / XG_D_BK);
+            int issued = 0, ready = G.J0; /* thread 0: slabs issued; operand blocks known to be finished */
             bool ok = true;
             /* the slabs reuse shared memory that generic accesses touched */
             xg_fence_proxy_async();
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1)
             for (int kb = 0; kb < KT; ++kb) {
                 if (tid == 0) {
                     while (issued < KT && issued < kb + XG_D_STAGES) {
-                        const int kblk = issued / (XG_SUB / XG_D_BK);
+                        const int kblk = G.J0 + issued / (XG_SUB / XG_D_BK);
                         if (kblk >= ready) {
                             const int *pi = flagI + xg_tile_index(I, kblk, nb), *pj = flagJ + xg_tile_index(J, kblk, nb);
                             /* with slabs in flight an unfinished operand is looked at again after

@@ -32,6 +32,15 @@ struct XgFactorStreams {
 };
 extern XgContext g_xg;
 
+/* INT8-sliced updates (sliced.cu), left-looking: the digit planes and row
+ * scales of every factored panel tile (tile-packed, `digits` bytes + 8 / ts
+ * bytes per element) and the lookahead events; for gradients also those of the
+ * inverse factor X = L^-T (slot layout of X). */
+struct XgSliced {
+    XgDigits L, X;
+    cudaEvent_t ev_a = nullptr, ev_p[2] = {nullptr, nullptr};
+};
+
 struct XgTileMatrix {
     int N = 0, ts = 0, nt = 0;
     long long ntiles = 0;
@@ -43,6 +52,9 @@ struct XgTileMatrix {
     /* tile DAG and backward solve: next task, abort flag and block flags of each;
      * null where the matrix is factored by the per-step launches only */
     int *dag = nullptr;
+    XgSliced *i8 = nullptr; /* seven-digit planes: large FP64 factorisations on the INT8 tensor cores */
+    bool no_i8 = false;     /* their memory was refused or given back */
+    bool i8_factor = false; /* the last factorisation went through them (they hold L) */
     double *tab = nullptr; /* element tables of the current parameters (xg_matern_tab.cuh) */
 };
 
@@ -54,21 +66,6 @@ struct XgMixed {
     double *p64[2] = {nullptr, nullptr};
     float *phi[2] = {nullptr, nullptr}, *plo[2] = {nullptr, nullptr};
     XgMixedMaps maps[2];
-};
-
-/* FP64 tiles with INT8-sliced trailing updates (sliced.cu), left-looking:
- * the digit planes and row scales of every factored panel tile
- * (tile-packed, 4 bytes + 8 / ts bytes per element) and the lookahead events. */
-struct XgSliced {
-    long long plane_rows = 0; /* rows per digit plane (ntiles * ts) */
-    int8_t *dig = nullptr;
-    double *scale = nullptr;
-    CUtensorMap map_a, map_b; /* A and B operand views (boxes of 128 rows x 64 bytes) */
-    cudaEvent_t ev_a = nullptr, ev_p[2] = {nullptr, nullptr};
-    /* gradient: digit planes of the inverse factor X = L^-T (slot layout of X) */
-    int8_t *xdig = nullptr;
-    double *xscale = nullptr;
-    CUtensorMap xmap;
 };
 
 /* One dataset: locations, observations and the covariance / factor. */
@@ -129,6 +126,8 @@ int xg_check_theta(const double *theta, int kernel);
 int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
               cudaEvent_t *pev = nullptr);
 int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
+int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits);
+bool xg_i8_release(XgTileMatrix &M);
 void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st);
 void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st);
 double xg_trailing_flops(int nt, int ts, int k);

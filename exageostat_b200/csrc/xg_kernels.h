@@ -144,8 +144,9 @@ __device__ inline int2 xg_tile_decode_fast(long long t, int nt)
 /* tile_dag.cu: the whole Cholesky of one or more fields in one persistent
  * launch, a dataflow of 128 x 128 blocks. */
 #define XG_DAG_BLOCK 128
-/* device words of a field's DAG state: next task, abort flag, block flags */
-static inline long long xg_dag_words(int nb) { return 2 + (long long)nb * (nb + 1) / 2; }
+/* device words of a field's DAG state: next task, abort flag, block flags, then
+ * a next-task word per window of columns */
+static inline long long xg_dag_words(int nb) { return 2 + (long long)nb * (nb + 1) / 2 + nb; }
 /* the same of its backward solve: next task, abort flag, a flag per block */
 static inline long long xg_trsv_words(int nb) { return 2 + (long long)nb; }
 struct XgDagField {
@@ -160,7 +161,8 @@ struct XgDagField {
 struct XgDag {
     double *data; /* the tile store behind the TMA map */
     int ts;
-    XgDagField one;       /* a single field (tasks == nullptr: every block, in block-column order) */
+    XgDagField one;       /* a single field (tasks == nullptr: ntasks blocks in block-column order) */
+    int J0;               /* first block column; the columns before it are applied already */
     const XgDagField *F;  /* several fields */
     const int4 *tasks;    /* (field, I, J, -) in an order that never puts a block before its operands */
     long long ntasks;
@@ -190,7 +192,7 @@ struct XgRows {
     double *y[XG_ROWS_MAX_SYS];          /* rows (solved in place, INVERSE: written) */
     const double *dinv[XG_ROWS_MAX_SYS];
     double *s;                           /* INVERSE: the factor's store, receives S */
-    int ts, nsys;
+    int ts, nsys, J0;                    /* J0: first block column of a window (INVERSE, no products) */
     XgRowsField one;
     const XgRowsField *F;
     const int4 *tasks;                   /* (field, I, J, product?); null: a single field, every task */
@@ -286,10 +288,17 @@ struct XgSlTask {
     int overwrite; /* C = sign sum (C is not read) */
 };
 cudaError_t xg_sliced_kernels_configure();
-void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int8_t *dig, double *scale, long long plane,
-                           const int *status, cudaStream_t st);
-void xg_launch_sliced(const CUtensorMap &map_a, const CUtensorMap &map_b, const double *scale_a,
-                      const double *scale_b, const XgTileArgs &T, const XgSlTask &S, int plane_rows, int max_ctas,
+/* a digit store: `digits` planes of plane_rows rows (ts bytes each), one scale per row */
+struct XgDigits {
+    int digits = 4, plane_rows = 0;
+    int8_t *dig = nullptr;
+    double *scale = nullptr;
+    CUtensorMap map;   /* boxes of 128 rows x 64 bytes, 64-byte swizzle */
+    CUtensorMap map32; /* digits == 7: boxes of 128 rows x 32 bytes, 32-byte swizzle */
+};
+void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int digits, int8_t *dig, double *scale,
+                           long long plane, const int *status, cudaStream_t st);
+void xg_launch_sliced(const XgDigits &A, const XgDigits &B, const XgTileArgs &T, const XgSlTask &S, int max_ctas,
                       int *status, cudaStream_t st);
 
 void xg_launch_finalize(const double *part_logdet, const double *part_dot, int nt, int N, double *out,
@@ -329,9 +338,8 @@ void xg_launch_bessel(const double *nu, const double *x, int n, double *out, cud
 
 /* gradient_fp64.cu */
 cudaError_t xg_gradient_kernels_configure();
-/* X = 0 with identity diagonal tiles; step K of X L^T = I: X(I, K) <- X(I, K) L_KK^-T for I <= K */
-void xg_launch_identity_x(double *X, int nt, int ts, cudaStream_t st);
-void xg_launch_xtrsm(double *X, const double *L, int nt, int ts, int K, int *status, cudaStream_t st);
+/* zeros the diagonal tiles of a lower-tile store */
+void xg_launch_zero_diag(double *X, int nt, int ts, cudaStream_t st);
 void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapLT,
                                   const double *LT, int nt, int ts, int *status, cudaStream_t st);
 void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int mt, int nt, int ts,

@@ -1,0 +1,61 @@
+"""Large FP64 evaluations, whose updates run as seven-digit integer products,
+against the DMMA path (tile 128, which keeps it) on the same data: tiles
+filled exactly, one row past, a nearly empty last tile.
+
+Bars: l 1e-10 relative; the gradient 1e-9 of its largest entry; kriging 1e-9."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,ts,theta,kernel", [
+    (6656, 512, [1.0, 0.1, 0.5], 0),
+    (6657, 512, [1.3, 0.07, 0.73], 0),
+    (7041, 512, [1.0, 0.1, 1.0, 0.01], 1),
+    (8065, 384, [0.8, 0.06, 1.5], 0),
+    (11265, 256, [1.0, 0.1, 0.5], 0),
+])
+def test_matches_the_dmma_path(gpu, ora, n, ts, theta, kernel):
+    x, y = ora.generate_xy_loc(n, 3)
+    z = np.random.default_rng(1).standard_normal(n)
+    got = {}
+    for t in (ts, 128):
+        with gpu.Session(x, y, kernel=kernel, dts=t) as s:
+            s.set_data(z=z)
+            ll = s.loglik(theta)
+            ll2, g = s.loglik(theta, grad=True)
+            assert ll2 == ll
+            got[t] = (ll, g)
+    assert got[ts][0] == pytest.approx(got[128][0], rel=1e-10)
+    assert np.abs(got[ts][1] - got[128][1]).max() <= 1e-9 * np.abs(got[128][1]).max()
+
+
+def test_kriging_and_synthetic_data(gpu, ora):
+    n, m, theta = 6700, 50, [1.0, 0.1, 0.5]
+    x, y = ora.generate_xy_loc(n + m, 5)
+    e = ora.dlarnv(6, n + m)
+    out = {}
+    for t in (512, 128):
+        with gpu.Session(x, y, dts=t) as s:
+            s.zvg(theta, e)
+            z = s.z()
+            out[t] = (z, s.predict(theta, x[:m], y[:m], x[m:], y[m:], out[512][0][m:] if t == 128 else z[m:])[1])
+    assert np.linalg.norm(out[512][0] - out[128][0]) <= 1e-10 * np.linalg.norm(out[128][0])
+    assert np.linalg.norm(out[512][1] - out[128][1]) <= 1e-9 * np.linalg.norm(out[128][1])
+
+
+def test_a_failing_pivot_is_reported(gpu, ora):
+    n = 6657
+    x, y = ora.generate_xy_loc(n, 3)
+    bad = x.copy()
+    bad[5000] = np.nan
+    with gpu.Session(x, y, dts=512) as s:
+        s.set_data(z=np.ones(n))
+        ll = s.loglik([1.0, 0.1, 0.5])
+        s.set_data(x=bad)
+        with pytest.raises(gpu.XgError) as err:
+            s.loglik([1.0, 0.1, 0.5])
+        assert err.value.code == gpu.XG_ERR_NOT_SPD and "pivot 5001)" in str(err.value)
+        s.set_data(x=x)
+        assert s.loglik([1.0, 0.1, 0.5]) == ll
