@@ -57,25 +57,37 @@ __device__ __forceinline__ bool xg_dag_wait(const int *p, const int *abort)
 __device__ __forceinline__ void xg_dag_slab(double (&acc)[16][4], const unsigned char *sa, const unsigned char *sb,
                                             int r0, int g, int tq, int nlim)
 {
+    /* rows g + 8 m: row & 7 = g */
+    const int sw[2] = {((2 * tq) ^ g) << 4, ((2 * tq + 1) ^ g) << 4};
+    double2 a0[2], a1[2], bv[2][4];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int sw = ((2 * tq + half) ^ g) << 4; /* rows g + 8 m: row & 7 = g */
-        const double2 a0 = *(const double2 *)(sa + (r0 << 7) + sw);
-        const double2 a1 = *(const double2 *)(sa + ((r0 + 8) << 7) + sw);
+    for (int h = 0; h < 2; ++h) {
+        a0[h] = *(const double2 *)(sa + (r0 << 7) + sw[h]);
+        a1[h] = *(const double2 *)(sa + ((r0 + 8) << 7) + sw[h]);
+    }
 #pragma unroll
-        for (int n0 = 0; n0 < 16; n0 += 4) {
-            /* groups of 32 columns: the branch must skip enough work to stay a
-             * branch (skipped by predicates, the DMMAs take their full time) */
-            if (n0 >= nlim) break;
-            double2 bv[4];
+    for (int u = 0; u < 4; ++u) bv[0][u] = *(const double2 *)(sb + ((8 * u + g) << 7) + sw[0]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) bv[u] = *(const double2 *)(sb + ((8 * (n0 + u) + g) << 7) + sw);
+    for (int n0 = 0; n0 < 16; n0 += 4) {
+        /* groups of 32 columns: the branch must skip enough work to stay a
+         * branch (skipped by predicates, the DMMAs take their full time) */
+        if (n0 >= nlim) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            /* the next step's B fragments, in flight under this one's DMMAs */
+            const int nn = h ? n0 + 4 : n0;
+            if (nn < 16)
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    bv[h ^ 1][u] = *(const double2 *)(sb + ((8 * (nn + u) + g) << 7) + sw[h ^ 1]);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.x, a1.x, bv[u].x);
+                xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0[h].x, a1[h].x,
+                               bv[h][u].x);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0.y, a1.y, bv[u].y);
+                xg_dmma_16x8x4(acc[n0 + u][0], acc[n0 + u][1], acc[n0 + u][2], acc[n0 + u][3], a0[h].y, a1[h].y,
+                               bv[h][u].y);
         }
     }
 }

@@ -160,29 +160,65 @@ __device__ __forceinline__ void xg_mma16(double (&acc)[2][4], const double *a, i
             xg_dmma_16x8x4(acc[n][0], acc[n][1], acc[n][2], acc[n][3], av[k][0], av[k][1], bv[k][n]);
 }
 
-/* One 16 x 8 half (columns 8 n ..) of block (i, j): S_ij -= sum over the
- * panels k0 <= k < k1 of X_ik X_jk^T (one warp) */
-__device__ __forceinline__ void xg_potrf_update(double *S, int i, int j, int n, int k0, int k1, int g, int tq)
+/* NH 16 x 8 halves (columns 8 n0 ..) of block row i, one warp: column q = p + 1
+ * by panel p, column q + 1 by the panels 0 .. p,
+ *   S_iq -= X_ip X_qp^T,   S_i,q+1 -= sum_{k <= p} X_ik X_{q+1,k}^T,
+ * in one call, so that the chains of dependent DMMAs overlap and panel p's
+ * rows of X are read once. */
+template <int NH>
+__device__ __forceinline__ void xg_potrf_update(double *S, int i, int p, int n0, int g, int tq)
 {
-    double *p = S + (i * XG_P_NB + g) * XG_P_LDS + j * XG_P_NB + n * 8;
+    const int q = p + 1, pg = xg_p_perm(g);
+    double *c0 = S + (i * XG_P_NB + g) * XG_P_LDS + q * XG_P_NB + n0 * 8;
     const double *a = S + (i * XG_P_NB + g) * XG_P_LDS + tq;
-    const double *b = S + (j * XG_P_NB + n * 8 + xg_p_perm(g)) * XG_P_LDS + tq;
-    double acc[4]; /* starts at -S, stored negated */
+    const double *b = S + (q * XG_P_NB + n0 * 8 + pg) * XG_P_LDS + tq;
+    double cq[NH][4], cn[NH][4]; /* start at -S, stored negated */
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[e] = -p[8 * (e >> 1) * XG_P_LDS + xg_p_col(e & 1, tq)];
-    for (int k = k0; k < k1; ++k) {
-        double a0[4], a1[4], bv[4];
+    for (int n = 0; n < NH; ++n)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            a0[q] = a[k * XG_P_NB + 4 * q];
-            a1[q] = a[8 * XG_P_LDS + k * XG_P_NB + 4 * q];
-            bv[q] = b[k * XG_P_NB + 4 * q];
+        for (int e = 0; e < 4; ++e) {
+            const double *c = c0 + 8 * (e >> 1) * XG_P_LDS + n * 8 + xg_p_col(e & 1, tq);
+            cq[n][e] = -c[0];
+            cn[n][e] = -c[XG_P_NB];
         }
+    for (int k = p; k >= 0; --k) {
+        double a0[4], a1[4], bn[NH][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) xg_dmma_16x8x4(acc[0], acc[1], acc[2], acc[3], a0[q], a1[q], bv[q]);
+        for (int s = 0; s < 4; ++s) {
+            a0[s] = a[k * XG_P_NB + 4 * s];
+            a1[s] = a[8 * XG_P_LDS + k * XG_P_NB + 4 * s];
+#pragma unroll
+            for (int n = 0; n < NH; ++n) bn[n][s] = b[(XG_P_NB + 8 * n) * XG_P_LDS + k * XG_P_NB + 4 * s];
+        }
+        if (k == p) {
+            double bq[NH][4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int n = 0; n < NH; ++n) bq[n][s] = b[8 * n * XG_P_LDS + k * XG_P_NB + 4 * s];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int n = 0; n < NH; ++n) {
+                    xg_dmma_16x8x4(cq[n][0], cq[n][1], cq[n][2], cq[n][3], a0[s], a1[s], bq[n][s]);
+                    xg_dmma_16x8x4(cn[n][0], cn[n][1], cn[n][2], cn[n][3], a0[s], a1[s], bn[n][s]);
+                }
+        } else {
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int n = 0; n < NH; ++n)
+                    xg_dmma_16x8x4(cn[n][0], cn[n][1], cn[n][2], cn[n][3], a0[s], a1[s], bn[n][s]);
+        }
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) p[8 * (e >> 1) * XG_P_LDS + xg_p_col(e & 1, tq)] = -acc[e];
+    for (int n = 0; n < NH; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            double *c = c0 + 8 * (e >> 1) * XG_P_LDS + n * 8 + xg_p_col(e & 1, tq);
+            c[0] = -cq[n][e];
+            c[XG_P_NB] = -cn[n][e];
+        }
 }
 
 /* Block row p + 1 of panel p and the next diagonal block, by one warp: X = B W
@@ -360,12 +396,12 @@ __device__ __forceinline__ int xg_potrf128(double *S, double *W, double *T, doub
                     xg_potrf_product16<false>(B, XG_P_LDS, 1.0, B, XG_P_LDS, Wp, XG_P_LDW, g, tq);
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                /* halves n of the block rows i > q = p + 1: column q by panel p, column q + 1 by panels <= p */
-                const int q = p + 1;
-                for (int t = w6; t < 2 * (NP - 1 - q); t += 6) {
-                    const int i = q + 1 + (t >> 1), n = t & 1;
-                    xg_potrf_update(S, i, q, n, p, q, g, tq);
-                    xg_potrf_update(S, i, q + 1, n, 0, q, g, tq);
+                /* block rows i > q = p + 1, a warp each; of three rows or fewer, half a row each */
+                const int rows = NP - 2 - p;
+                if (rows > 3) {
+                    if (w6 < rows) xg_potrf_update<2>(S, p + 2 + w6, p, 0, g, tq);
+                } else if (w6 < 2 * rows) {
+                    xg_potrf_update<1>(S, p + 2 + (w6 >> 1), p, w6 & 1, g, tq);
                 }
             }
             if (dinv && warp == 7 && (p & 1)) xg_potrf_inverse32(S, W, T, p >> 1, dinv + (p >> 1) * 32 * 32, lane);
