@@ -1266,12 +1266,9 @@ static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits)
         xg_digits_free(D);
         return xg_fail(XG_ERR_NO_MEMORY, "digit planes (%.2f GB)", digits * (double)plane / 1e9);
     }
-    /* both operands are staged in boxes of 128 rows x 64 bytes (and 32 bytes for seven digits) */
+    /* both operands are staged in boxes of 128 rows x 64 bytes */
     int rc = xg_encode(&D.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 64, 128,
                        CU_TENSOR_MAP_SWIZZLE_64B);
-    if (!rc && digits == 7)
-        rc = xg_encode(&D.map32, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 32, 128,
-                       CU_TENSOR_MAP_SWIZZLE_32B);
     if (rc) xg_digits_free(D);
     return rc;
 }
@@ -1345,22 +1342,46 @@ int xg_field_set_sliced(XgField *f)
     return rc;
 }
 
-/* Left-looking factorisation with FP64 tiles and INT8-sliced updates.  For
- * each column j:
- *   update  : A_ij -= sum_{k<j} L_ik L_jk^T for i >= j (xg_sliced_left_kernel)
- *   panel   : POTRF(j, j) [+ log-det, + z block solve] -> TRSM(i, j) [+ z update]
- *             -> slicing of the tiles (i, j), i > j, into digit planes
- * With fs.st_hi the update of column j+1 is split: chunks k < j (needing
- * panels already sliced) run on the main stream on all but xg_panel_share(j)
- * SMs while the panel chain of column j runs on the high-priority stream, and
- * chunk k = j joins the panel chain of column j+1.  Profiling events (8 per
- * column): panel stream before / after the last-chunk update, after POTRF,
- * after TRSM + slicing; main stream before / after the split update. */
-static XgSlTask factor_task(int col, int k0, int k1)
+/* Left-looking factorisation with FP64 tiles and INT8-sliced updates, by
+ * groups of G = xg_sl_group tile columns [a, b):
+ *   U1     chunks k < a0 (the group before begins at a0) to every target of the group (main stream,
+ *          on all but xg_panel_share SMs, beside the panels of the group before)
+ *   U2     chunks a0 <= k < a, when those panels are sliced: column a on the panel stream, the
+ *          others on the main stream
+ *   panel  per column c: chunks a <= k < c (for c > a), POTRF and TRSM of the tile column (a window
+ *          of the tile DAG, with log-det and z solve), slicing into digit planes
+ * Profiling events (8 per column c, those of the main stream on a group's
+ * first column): panel stream before / after the column's updates, after its
+ * panel, after slicing; main stream before / after U1. */
+
+/* Tile columns per group.  One column gives an update 16 (nt - j) jobs of 128
+ * x 128, whose last round leaves most of the persistent CTAs idle: counted
+ * over the columns 1.7 x the even distribution at 38 tile columns, 1.36 x at
+ * 79, 1.24 x at 137; groups of four bring that to 1.21, 1.09 and 1.05, but put
+ * three columns' panels between two updates, which the short matrices have
+ * nothing to run beside.  Log-likelihood in ms, tiles of 512, K = 4 below:
+ *   7 digits   N = 8200  10000  14000  20000  28000  40000
+ *     G = 1        6.00   8.80     -    46.6     -    316
+ *     G = 2        5.71   7.98   17.9   44.7   109    308
+ *     G = 3        6.13   8.17   16.6   42.2   107    305
+ *     G = 4        6.52   8.81   17.3   41.1   105    298
+ *   4 digits   N = 9000  20000  40000  70000
+ *     G = 1        5.00   20.2    117   560
+ *     G = 2        5.02   20.1    119   574
+ *     G = 3        5.20   21.4    118   573
+ * (28 pairs cost an update 2.8 times what ten do, the panels the same: the
+ * four-digit form has the panels to hide, not the last rounds.) */
+static int xg_sl_group(int nt, int digits)
+{
+    return digits == 4 ? 1 : nt < 24 ? 2 : nt < 36 ? 3 : 4;
+}
+
+static XgSlTask factor_task(int col, int ncol, int k0, int k1)
 {
     XgSlTask S;
     S.mode = XG_SL_FACTOR;
     S.col = col;
+    S.ncol = ncol;
     S.k0 = k0;
     S.k1 = k1;
     S.sign = -1.0;
@@ -1368,16 +1389,15 @@ static XgSlTask factor_task(int col, int k0, int k1)
     return S;
 }
 
-/* SMs given to the panel chain of column j (last-chunk update, POTRF, TRSM,
- * slicing) while the split update of column j+1 runs on the others.  The
- * chain's work grows like nt - j and the split update's like j (nt - j), so
- * the chain gets sms K / (K + j), clamped to [XG_PANEL_SMS, sms -
- * XG_PANEL_SMS].  K = 4 (EXAGEOSTAT_B200_PANEL_K overrides it) measured best
- * at N = 100 000 with the 128-column-block TRSM: 1.589-1.644 s per
- * evaluation against 1.614-1.665 s for K = 2, 3, 6, 8, 1.624 s for a cost
- * model balancing the chain against the update, and 1.639 s for that model
- * with the update's round count in it (each compared within one GPU
- * session; the sessions differ by up to 3 %). */
+/* SMs left to the panels of the group that begins at tile column a while U1 of
+ * the next group runs on the others.  Per target tile the panels cost the DMMA
+ * flops of the TRSM and the group's own chunks, U1 a chunks: sms K / (K + a),
+ * clamped to [XG_PANEL_SMS, sms - XG_PANEL_SMS].  K = 4
+ * (EXAGEOSTAT_B200_PANEL_K overrides it): seven digits in groups of four at
+ * N = 10000 / 20000 / 40000 took 11.0 / 51.4 / 325 ms with K = 1, 9.9 / 46.5 /
+ * 317 with 2, 9.2 / 43.8 / 309 with 3, 8.9 / 41.6 / 308 with 4 and 8.6 / 43.6 /
+ * 311 with 6; four digits at 20000 / 70000 20.4 / 570 with 4 and 20.9 / 572
+ * with 7. */
 static int xg_panel_k()
 {
     static int v = -1;
@@ -1389,10 +1409,10 @@ static int xg_panel_k()
     return v;
 }
 
-static int xg_panel_share(int j, int sms)
+static int xg_panel_share(int a, int sms)
 {
     const int K = xg_panel_k();
-    int r = (int)((long long)sms * K / (K + j));
+    int r = (int)((long long)sms * K / (K + a));
     if (r < XG_PANEL_SMS) r = XG_PANEL_SMS;
     if (r > sms - XG_PANEL_SMS) r = sms - XG_PANEL_SMS;
     return r;
@@ -1400,7 +1420,7 @@ static int xg_panel_share(int j, int sms)
 
 /* How the SMs are divided between the panel chain and the split update.
  * "static" (default): the split update runs as a persistent launch on
- * sms - xg_panel_share(j) CTAs, leaving the rest to the panel chain.
+ * sms - xg_panel_share(a) CTAs, leaving the rest to the panel chain.
  * "dynamic" (EXAGEOSTAT_B200_SL_SHARE=dynamic): both updates launch one CTA
  * per job, so CTAs retire throughout the update and the hardware hands each
  * freed SM to the pending panel kernels first (higher stream priority), the
@@ -1424,51 +1444,66 @@ static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *pa
     const long long plane = (long long)sl->L.plane_rows * M.ts;
     int *windows = M.dag + xg_dag_words(nb) - nb;
     const bool la = fs.st_hi != nullptr;
-    cudaStream_t sp = la ? fs.st_hi : fs.st;
+    cudaStream_t st = fs.st, sp = la ? fs.st_hi : fs.st;
     cudaEvent_t *pev = fs.pev;
     auto rec = [&](int k, int e, cudaStream_t s) {
         if (pev) cudaEventRecord(pev[8 * k + e], s);
     };
     const int sms = g_xg.sm_count;
+    const int G = xg_sl_group(nt, sl->L.digits);
     const bool dyn = xg_sl_dynamic_share();
     const int all = 1 << 30; /* one CTA per job */
-    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), fs.st);
-    if (la) cudaEventRecord(sl->ev_a, fs.st); /* the generated matrix */
-    for (int j = 0; j < nt; ++j) {
-        if (la) cudaStreamWaitEvent(sp, sl->ev_a, 0); /* chunks k < j-1 of column j */
-        rec(j, 0, sp);
-        const int band_ctas = xg_panel_share(j, sms), upd_ctas = sms - band_ctas;
-        if (la) {
-            if (j >= 1)
-                xg_launch_sliced(sl->L, sl->L, T, factor_task(j, j - 1, j), dyn ? all : band_ctas, status, sp);
-        } else {
-            xg_launch_sliced(sl->L, sl->L, T, factor_task(j, 0, j), sms, status, sp);
+    auto update = [&](int col, int ncol, int k0, int k1, int ctas, cudaStream_t s) {
+        if (ncol > 0 && k1 > k0) xg_launch_sliced(sl->L, sl->L, T, factor_task(col, ncol, k0, k1), ctas, status, s);
+    };
+    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
+    if (la) {
+        cudaEventRecord(sl->ev_a, st); /* the generated matrix */
+        cudaStreamWaitEvent(sp, sl->ev_a, 0);
+    }
+    for (int a = 0; a < nt; a += G) {
+        const int b = a + G < nt ? a + G : nt, a0 = a - G;
+        /* main stream: U1 of this group was issued with the group before; U2 of
+         * the columns after the first */
+        if (la && a > 0) {
+            cudaEventRecord(sl->ev_p[0], sp); /* the group before is sliced */
+            cudaEventRecord(sl->ev_a, st);    /* U1 of this group is done */
+            cudaStreamWaitEvent(st, sl->ev_p[0], 0);
+            cudaStreamWaitEvent(sp, sl->ev_a, 0);
+            update(a + 1, b - a - 1, a0, a, sms, st);
+            cudaEventRecord(sl->ev_p[1], st);
+        } else if (a > 0) {
+            update(a + 1, b - a - 1, a0, a, sms, st);
         }
-        rec(j, 1, sp);
-        /* POTRF and TRSM of the tile column: a window of the tile DAG */
-        xg_launch_dag_columns(M, j * bpt, (j + 1) * bpt, windows + j, v, part, status, sp);
-        rec(j, 2, sp);
-        if (j + 1 < nt) xg_launch_slice_panel(T, j, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, sp);
-        rec(j, 3, sp);
-        if (la) {
-            cudaEventRecord(sl->ev_p[j & 1], sp);
-            /* chunks k < j of column j+1, behind the slicing of panel j-1 */
-            if (j >= 1 && j + 1 < nt) cudaStreamWaitEvent(fs.st, sl->ev_p[(j - 1) & 1], 0);
-            rec(j, 4, fs.st);
-            if (j >= 1 && j + 1 < nt)
-                xg_launch_sliced(sl->L, sl->L, T, factor_task(j + 1, 0, j), dyn ? all : upd_ctas, status, fs.st);
-            rec(j, 5, fs.st);
-            cudaEventRecord(sl->ev_a, fs.st);
-        } else {
-            rec(j, 4, fs.st);
-            rec(j, 5, fs.st);
+        rec(a, 4, st);
+        const int b1 = b + G < nt ? b + G : nt; /* the next group: chunks k < a */
+        update(b, b1 - b, 0, a, !la ? sms : dyn ? all : sms - xg_panel_share(a, sms), st);
+        rec(a, 5, st);
+        for (int c = a; c < b; ++c) {
+            rec(c, 0, sp);
+            if (c == a) {
+                /* alone in its group it runs beside U1 of the next column */
+                if (a > 0) update(a, 1, a0, a, !la || G > 1 ? sms : dyn ? all : xg_panel_share(a, sms), sp);
+            } else {
+                if (la && a > 0 && c == a + 1) cudaStreamWaitEvent(sp, sl->ev_p[1], 0);
+                update(c, 1, a, c, la && b < nt ? (dyn ? all : xg_panel_share(a, sms)) : sms, sp);
+            }
+            rec(c, 1, sp);
+            xg_launch_dag_columns(M, c * bpt, (c + 1) * bpt, windows + c, v, part, status, sp);
+            rec(c, 2, sp);
+            if (c + 1 < nt) xg_launch_slice_panel(T, c, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, sp);
+            rec(c, 3, sp);
+            if (c > a) {
+                rec(c, 4, st);
+                rec(c, 5, st);
+            }
+            rec(c, 6, st);
+            rec(c, 7, st);
         }
-        rec(j, 6, fs.st);
-        rec(j, 7, fs.st);
     }
     if (la) {
         cudaEventRecord(fs.ev_panel, sp);
-        cudaStreamWaitEvent(fs.st, fs.ev_panel, 0);
+        cudaStreamWaitEvent(st, fs.ev_panel, 0);
     }
     return nb;
 }
@@ -1501,10 +1536,14 @@ static void xg_field_collect_profile_sliced(XgField *f, bool lookahead)
         f->prof[3] += ta + tb;
         f->prof[4] += col_flops(j, j);
         if (lookahead) {
+            /* on the panel stream: a group's first column by the group before,
+             * the others by their own group; U1 of the next group on the main stream */
+            const int G = xg_sl_group(nt, f->sl->L.digits), a = j / G * G, b1 = a + 2 * G < nt ? a + 2 * G : nt;
             f->prof[10] += tb;
-            f->prof[11] += j >= 1 ? col_flops(j, 1) : 0.0;
+            f->prof[11] += j > a ? col_flops(j, j - a) : j > 0 ? col_flops(j, G) : 0.0;
             f->prof[8] += ta;
-            f->prof[9] += (j >= 1 && j + 1 < nt) ? col_flops(j + 1, j) : 0.0;
+            if (j == a)
+                for (int c = a + G; c < b1; ++c) f->prof[9] += col_flops(c, a);
         } else {
             f->prof[8] += tb;
             f->prof[9] += col_flops(j, j);

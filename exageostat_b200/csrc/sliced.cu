@@ -68,11 +68,13 @@
 #define XG_SL_STAGES 3
 #define XG_SL_ABOX_BYTES (XG_SL_BM * XG_SL_BK)                                  /* one digit plane, 128 rows */
 #define XG_SL_BBOX_BYTES (XG_SL_BN * XG_SL_BK)                                  /* one digit plane, 128 rows */
-#define XG_SL_BOX32_BYTES (128 * 32) /* second pass: one digit plane, 128 rows, 32 bytes */
 #define XG_SL_STAGE_BYTES (XG_SL_SLICES * (XG_SL_ABOX_BYTES + XG_SL_BBOX_BYTES)) /* 64 KB */
 /* per panel chunk, the 128 A-row and 128 B-row scales, double-buffered */
 #define XG_SL_SCALE_BYTES (2 * 2 * 128 * 8)
-#define XG_SL_SMEM (XG_SL_STAGES * XG_SL_STAGE_BYTES + XG_SL_SCALE_BYTES + 1024 + 256)
+/* stage of the seven-digit form: nine planes */
+#define XG_SL_STAGE7_BYTES (9 * XG_SL_ABOX_BYTES)
+#define XG_SL_SMEM(ND)                                                                                                 \
+    (XG_SL_STAGES * ((ND) == 4 ? XG_SL_STAGE_BYTES : XG_SL_STAGE7_BYTES) + XG_SL_SCALE_BYTES + 1024 + 256)
 #define XG_SL_RADIX 254.0
 #define XG_SL_TOP 127.0
 #define XG_SL_INV_RADIX3 (1.0 / (254.0 * 254.0 * 254.0))
@@ -207,9 +209,12 @@ __device__ __forceinline__ bool xg_sl_job(const XgSlTask &S, long long job, int 
     J.bm = blk / bpt;
     J.bn = blk % bpt;
     bool diag = false;
-    if (S.mode == XG_SL_FACTOR) { /* targets (i, j), i >= j, of column j */
-        J.ta = S.col + (int)unit;
-        J.tb = S.col;
+    if (S.mode == XG_SL_FACTOR) { /* targets (i, j), i >= j, of columns col .. col + ncol - 1 */
+        int c = S.col;
+        long long u = unit;
+        for (; u >= nt - c; ++c) u -= nt - c;
+        J.ta = c + (int)u;
+        J.tb = c;
         J.k0 = S.k0;
         J.k1 = S.k1;
         J.c_slot = xg_tile_index(J.ta, J.tb, nt);
@@ -245,21 +250,25 @@ __device__ __forceinline__ long long xg_sl_slot_b(const XgSlTask &S, const XgSlJ
 }
 
 /* ND = 4: one pass per chunk, levels 0-3 of digits 0-3.  ND = 7: a second
- * pass for levels 4-6 (18 pairs of digits 0-6, K in 32-byte slabs so that the
- * fourteen digit boxes fit a stage), whose sums are below the first pass's by
- * 254^-3: together 28 pairs, an FP64-grade product (the digits to 2^-55 of the
- * row maxima, products below 254^-6 dropped, sums exact). */
+ * pass for levels 4-6 (18 pairs of digits 0-6), whose sums are below the first
+ * pass's by 254^-3: together 28 pairs, an FP64-grade product (the digits to
+ * 2^-55 of the row maxima, products below 254^-6 dropped, sums exact).  The
+ * second pass takes each 64-byte slab in two stages, A digits 0-3 with B
+ * digits 2-6 (11 pairs) and A digits 3-6 with B digits 0-2 (the 7 others):
+ * all fourteen planes at once fit a stage only as 32-byte slabs, which need
+ * their own tensor maps and swizzle and took 316 ms for a log-likelihood at
+ * N = 40000 where this takes 313. */
 template <int ND>
 __global__ void __launch_bounds__(XG_SL_THREADS, 1)
     xg_sliced_left_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                          const __grid_constant__ CUtensorMap map_a32, const __grid_constant__ CUtensorMap map_b32,
                           const double *__restrict__ scale_a, const double *__restrict__ scale_b, XgTileArgs T,
                           XgSlTask S, long long njobs, int plane_rows, int *status)
 {
+    constexpr int STAGE = ND == 4 ? XG_SL_STAGE_BYTES : XG_SL_STAGE7_BYTES;
     extern __shared__ __align__(1024) unsigned char xg_smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)xg_smem_raw + 1023) & ~(uintptr_t)1023);
-    double *sscale = (double *)(smem + XG_SL_STAGES * XG_SL_STAGE_BYTES); /* [2][A 128 | B 128] */
-    uint64_t *full = (uint64_t *)(smem + XG_SL_STAGES * XG_SL_STAGE_BYTES + XG_SL_SCALE_BYTES);
+    double *sscale = (double *)(smem + XG_SL_STAGES * STAGE); /* [2][A 128 | B 128] */
+    uint64_t *full = (uint64_t *)(smem + XG_SL_STAGES * STAGE + XG_SL_SCALE_BYTES);
     uint64_t *empty = full + XG_SL_STAGES;
     uint64_t *acc_full = empty + XG_SL_STAGES;
     uint64_t *acc_empty = acc_full + 1;
@@ -329,16 +338,17 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                             ok = false;
                             break;
                         }
-                        unsigned char *st = smem + s * XG_SL_STAGE_BYTES;
-                        if (kb >= KT) { /* second pass: 32-byte slabs of all seven digits */
-                            const int x = (kb - KT) * 32;
-                            xg_mbar_arrive_expect_tx(&full[s], 2 * ND * XG_SL_BOX32_BYTES);
-#pragma unroll
-                            for (int t = 0; t < ND; ++t) {
-                                xg_tma_load_2d(st + t * XG_SL_BOX32_BYTES, &map_a32, x, t * plane_rows + rowA, &full[s]);
-                                xg_tma_load_2d(st + (ND + t) * XG_SL_BOX32_BYTES, &map_b32, x, t * plane_rows + rowB,
+                        unsigned char *st = smem + s * STAGE;
+                        if (kb >= KT) { /* second pass */
+                            const int x = ((kb - KT) >> 1) * XG_SL_BK, part = (kb - KT) & 1;
+                            const int a0 = part ? 3 : 0, b0 = part ? 0 : 2, nb = part ? 3 : 5;
+                            xg_mbar_arrive_expect_tx(&full[s], (4 + nb) * XG_SL_ABOX_BYTES);
+                            for (int t = 0; t < 4; ++t)
+                                xg_tma_load_2d(st + t * XG_SL_ABOX_BYTES, &map_a, x, (a0 + t) * plane_rows + rowA,
                                                &full[s]);
-                            }
+                            for (int t = 0; t < nb; ++t)
+                                xg_tma_load_2d(st + (4 + t) * XG_SL_ABOX_BYTES, &map_b, x, (b0 + t) * plane_rows + rowB,
+                                               &full[s]);
                             continue;
                         }
                         xg_mbar_arrive_expect_tx(&full[s], XG_SL_STAGE_BYTES);
@@ -383,7 +393,7 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                             break;
                         }
                         xg_tc_fence_after();
-                        const uint32_t sa = sbase + s * XG_SL_STAGE_BYTES;
+                        const uint32_t sa = sbase + s * STAGE;
                         if (pass == 0) {
                             const uint32_t sb = sa + XG_SL_SLICES * XG_SL_ABOX_BYTES;
 #pragma unroll
@@ -403,14 +413,31 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
                                 }
                             }
                         } else {
-                            const uint32_t sb = sa + ND * XG_SL_BOX32_BYTES;
+                            const uint32_t sb = sa + 4 * XG_SL_ABOX_BYTES;
+                            const bool start = kb < 2; /* part 0 of the first slab starts every level */
 #pragma unroll
-                            for (int lv = 4; lv < 7; ++lv)
+                            for (int kk = 0; kk < XG_SL_BK / 32; ++kk)
+                                if (!(kb & 1)) {
 #pragma unroll
-                                for (int a = 0; a <= lv; ++a)
-                                    xg_umma_i8(dt + (uint32_t)((lv - 4) * XG_SL_BM),
-                                               xg_umma_desc_sw32(sb + (lv - a) * XG_SL_BOX32_BYTES),
-                                               xg_umma_desc_sw32(sa + a * XG_SL_BOX32_BYTES), idesc, kb != 0 || a != 0);
+                                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                                        for (int b = 2; b < 7; ++b)
+                                            if (a + b >= 4 && a + b <= 6)
+                                                xg_umma_i8(dt + (uint32_t)((a + b - 4) * XG_SL_BM),
+                                                           xg_umma_desc_sw64(sb + (b - 2) * XG_SL_BBOX_BYTES + kk * 32),
+                                                           xg_umma_desc_sw64(sa + a * XG_SL_ABOX_BYTES + kk * 32), idesc,
+                                                           !(start && kk == 0 && a == 0));
+                                } else {
+#pragma unroll
+                                    for (int a = 3; a < 7; ++a)
+#pragma unroll
+                                        for (int b = 0; b < 3; ++b)
+                                            if (a + b >= 4 && a + b <= 6 && !(a == 3 && b == 2)) /* in part 0 */
+                                                xg_umma_i8(dt + (uint32_t)((a + b - 4) * XG_SL_BM),
+                                                           xg_umma_desc_sw64(sb + b * XG_SL_BBOX_BYTES + kk * 32),
+                                                           xg_umma_desc_sw64(sa + (a - 3) * XG_SL_ABOX_BYTES + kk * 32),
+                                                           idesc, 1);
+                                }
                         }
                         xg_umma_commit(&empty[s]);
                     }
@@ -593,9 +620,9 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
 cudaError_t xg_sliced_kernels_configure()
 {
     cudaError_t e =
-        cudaFuncSetAttribute(xg_sliced_left_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM);
+        cudaFuncSetAttribute(xg_sliced_left_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM(4));
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(xg_sliced_left_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM);
+    return cudaFuncSetAttribute(xg_sliced_left_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SL_SMEM(7));
 }
 
 void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int digits, int8_t *dig, double *scale,
@@ -616,16 +643,19 @@ void xg_launch_sliced(const XgDigits &A, const XgDigits &B, const XgTileArgs &T,
     if (S.k1 <= S.k0 || S.col >= T.nt) return;
     const long long per = (long long)(T.ts / XG_SL_BM) * (T.ts / XG_SL_BN);
     long long units;
-    if (S.mode == XG_SL_FACTOR) units = T.nt - S.col;
+    if (S.mode == XG_SL_FACTOR) {
+        const int end = S.col + S.ncol < T.nt ? S.col + S.ncol : T.nt;
+        units = xg_num_lower_tiles(T.nt - S.col) - xg_num_lower_tiles(T.nt - end);
+    }
     else if (S.mode == XG_SL_INVERSE) units = S.col;
     else units = (long long)T.nt * (T.nt + 1) / 2;
     const long long njobs = units * per;
     if (njobs <= 0) return;
     const unsigned grid = (unsigned)(njobs < max_ctas ? njobs : max_ctas);
     if (A.digits == 4)
-        xg_sliced_left_kernel<4><<<grid, XG_SL_THREADS, XG_SL_SMEM, st>>>(A.map, B.map, A.map, B.map, A.scale, B.scale,
-                                                                          T, S, njobs, A.plane_rows, status);
+        xg_sliced_left_kernel<4><<<grid, XG_SL_THREADS, XG_SL_SMEM(4), st>>>(A.map, B.map, A.scale, B.scale, T, S, njobs,
+                                                                             A.plane_rows, status);
     else
-        xg_sliced_left_kernel<7><<<grid, XG_SL_THREADS, XG_SL_SMEM, st>>>(A.map, B.map, A.map32, B.map32, A.scale,
-                                                                          B.scale, T, S, njobs, A.plane_rows, status);
+        xg_sliced_left_kernel<7><<<grid, XG_SL_THREADS, XG_SL_SMEM(7), st>>>(A.map, B.map, A.scale, B.scale, T, S, njobs,
+                                                                             A.plane_rows, status);
 }

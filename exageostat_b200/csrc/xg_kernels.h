@@ -274,7 +274,8 @@ void xg_launch_offband_gemm(const XgMixedMaps &maps, const XgTileArgs &T, int k,
 /* sliced.cu: FP64 tiles, trailing updates on INT8 tensor cores (four digit slices), left-looking.
  * One launch of xg_sliced_left_kernel computes, for each output tile, C (+)= sign sum_k A_k B_k^T
  * over panel chunks k, with A_k, B_k read from digit stores:
- *   XG_SL_FACTOR : column col of the Cholesky factor, chunks k0 <= k < k1: L(i,col) -= sum L(i,k) L(col,k)^T
+ *   XG_SL_FACTOR : ncol columns of the Cholesky factor from col on, chunks k0 <= k < k1:
+ *                  L(i,j) -= sum L(i,k) L(j,k)^T
  *   XG_SL_INVERSE: column col of X = L^-T (X(a,b) at slot (b,a)): X(a,col) -= sum_{a<=c<col} X(a,c) L(col,c)^T
  *   XG_SL_SYRK   : S = X X^T into the lower tiles: S(a,b) = sum_{c>=a} X(a,c) X(b,c)^T */
 #define XG_SL_FACTOR 0
@@ -283,6 +284,7 @@ void xg_launch_offband_gemm(const XgMixedMaps &maps, const XgTileArgs &T, int k,
 struct XgSlTask {
     int mode;
     int col;       /* target column (factor, inverse) */
+    int ncol;      /* factor: that many target columns from col on */
     int k0, k1;    /* chunk window */
     double sign;   /* -1: C -= sum; +1: C += sum */
     int overwrite; /* C = sign sum (C is not read) */
@@ -293,8 +295,7 @@ struct XgDigits {
     int digits = 4, plane_rows = 0;
     int8_t *dig = nullptr;
     double *scale = nullptr;
-    CUtensorMap map;   /* boxes of 128 rows x 64 bytes, 64-byte swizzle */
-    CUtensorMap map32; /* digits == 7: boxes of 128 rows x 32 bytes, 32-byte swizzle */
+    CUtensorMap map; /* boxes of 128 rows x 64 bytes, 64-byte swizzle */
 };
 void xg_launch_slice_panel(const XgTileArgs &T, int k, int row_mode, int digits, int8_t *dig, double *scale,
                            long long plane, const int *status, cudaStream_t st);

@@ -41,19 +41,6 @@ __device__ inline uint64_t xg_umma_desc_sw64(uint32_t smem_addr)
     return d;
 }
 
-/* The same with the 32-byte swizzle: rows of 32 B, 8-row (256 B) atoms, stride
- * byte offset 256 B, layout [61,64) = 6. */
-__device__ inline uint64_t xg_umma_desc_sw32(uint32_t smem_addr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1u << 16;
-    d |= (uint64_t)((256u >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= (uint64_t)6u << 61;
-    return d;
-}
-
 /* Instruction descriptor, kind::i8: D = S32 (2 at [4,6)), A = B = signed
  * 8-bit (1 at [7,10) and [10,13)), both K-major, no saturation, dense;
  * N >> 3 at [17,23), M >> 4 at [24,29). */

@@ -2,7 +2,12 @@
 against the DMMA path (tile 128, which keeps it) on the same data: tiles
 filled exactly, one row past, a nearly empty last tile.
 
-Bars: l 1e-10 relative; the gradient 1e-9 of its largest entry; kriging 1e-9."""
+Bars: l 2e-12 relative, ten times what a CPU model of the tiled factorisation
+gives for the product as it should be (n = 2048, order 1.5, condition 2e6:
+2e-13 from FP64).  One digit pair of level 5 counted twice or lost moves l by
+9e-10 there, but by 6e-13 only at order 0.5 and condition 2e3: it is the
+smoother orders that hold the pairs.  The gradient 1e-9 of its largest entry;
+kriging 1e-11."""
 import numpy as np
 import pytest
 
@@ -27,7 +32,7 @@ def test_matches_the_dmma_path(gpu, ora, n, ts, theta, kernel):
             ll2, g = s.loglik(theta, grad=True)
             assert ll2 == ll
             got[t] = (ll, g)
-    assert got[ts][0] == pytest.approx(got[128][0], rel=1e-10)
+    assert got[ts][0] == pytest.approx(got[128][0], rel=2e-12)
     assert np.abs(got[ts][1] - got[128][1]).max() <= 1e-9 * np.abs(got[128][1]).max()
 
 
@@ -41,8 +46,8 @@ def test_kriging_and_synthetic_data(gpu, ora):
             s.zvg(theta, e)
             z = s.z()
             out[t] = (z, s.predict(theta, x[:m], y[:m], x[m:], y[m:], out[512][0][m:] if t == 128 else z[m:])[1])
-    assert np.linalg.norm(out[512][0] - out[128][0]) <= 1e-10 * np.linalg.norm(out[128][0])
-    assert np.linalg.norm(out[512][1] - out[128][1]) <= 1e-9 * np.linalg.norm(out[128][1])
+    assert np.linalg.norm(out[512][0] - out[128][0]) <= 1e-11 * np.linalg.norm(out[128][0])
+    assert np.linalg.norm(out[512][1] - out[128][1]) <= 1e-11 * np.linalg.norm(out[128][1])
 
 
 def test_a_failing_pivot_is_reported(gpu, ora):
