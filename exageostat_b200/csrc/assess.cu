@@ -6,15 +6,23 @@
  *   F_jk = 1/2 tr(Sigma^-1 dSigma_j Sigma^-1 dSigma_k), then F^-1.
  *   The reference forms Sigma^-1 dSigma_j by two N x N triangular solves per
  *   (j, k) pair and multiplies the pairs (30 N^3 flops for three parameters).
- *   Here S = Sigma^-1 comes from the gradient's inverse factor and SYRK
- *   (2/3 N^3), each G_j = S dSigma_j is one DMMA GEMM on full tiles (2 N^3),
- *   and all traces tr(G_j G_k) come from one pass over the G_j
- *   (xg_fisher_trace_kernel).  dSigma_j is generated on the fly into full
- *   tiles from the element derivatives (core_dcmg_matern_dsigma_square /
- *   _dbeta / _dnu, exageostat_exact/cpu_core/compute/core_zcmg.c:315-488;
- *   the nu derivative of K_nu is exact instead of the reference's 1e-9
- *   forward difference, core_zcmg.c:228-235).  The nugget parameter has
- *   dSigma = I, so its G is S itself.
+ *   Here tr(Sigma^-1 D_j Sigma^-1 D_k) = <W_j, W_k> with the symmetric
+ *   W_j = L^-1 D_j L^-T: Y_j = D_j L^-T are the rows Y_j L^T = D_j (N^3 flops),
+ *   and the lower half of W_j the rows W_j L^T = Y_j^T (N^3 / 3), all j in one
+ *   dataflow launch each (rows_dag.cu), then one pass over the W_j
+ *   (xg_fisher_trace_kernel).  dSigma_sigma^2 = (Sigma - tau^2 I) / sigma^2
+ *   gives W = (I - tau^2 M) / sigma^2 without a product, dSigma_tau^2 = I
+ *   gives M = L^-1 L^-T.  (A location met twice makes two rows of Sigma equal:
+ *   no factor, so zero distances are on the diagonal only.)  2.67 N^3 flops,
+ *   4 N^3 with the nugget, where S = Sigma^-1 and full products G_j = S D_j
+ *   took 6.67 N^3, and 16 or 24 bytes per element of workspace for 44: device
+ *   time with / without the nugget at N = 4000 11.1 / 8.3 ms (15.6 / 15.5),
+ *   8000 72 / 51 (113), 16000 511 / 349 (823); DMMA bound.  Error of F at
+ *   N = 4000 against 64-bit dense algebra 3.4e-12 (6.4e-11).  The derivatives
+ *   come from core_dcmg_matern_dsigma_square / _dbeta / _dnu
+ *   (exageostat_exact/cpu_core/compute/core_zcmg.c:315-488; the nu derivative
+ *   of K_nu is exact instead of the reference's 1e-9 forward difference,
+ *   core_zcmg.c:228-235).
  *
  * MLOE / MMOM (EXAGEOSTAT_dmle_mloe_mmom_Tile, MLE_dexact.c:1109-1434, with
  * the per-point accumulation of CORE_dmloe_mmom_starpu,
@@ -178,41 +186,32 @@ void xg_launch_mloe_terms(const double *A, const double *U, const double *T, con
 /* Fisher kernels                                                            */
 /* ------------------------------------------------------------------------- */
 
-/* Full tiles (slot A nt + B) of the symmetric S from its lower-tile store, by
- * 32 x 32 blocks: a block on or below the diagonal is copied, one above it is
- * the transpose of its mirror.  Only the diagonal 128-blocks of S's diagonal
- * tiles and the blocks below them are read (what the inverse SYRK writes). */
-__global__ void __launch_bounds__(256) xg_sym_full_kernel(const double *__restrict__ S, double *__restrict__ F,
-                                                          int nt, int ts)
+/* Y^T into the lower half of the square R-layout matrices Y, Y + full, ..:
+ * the 32 x 32 block (a, b), a >= b, becomes the transpose of (b, a). */
+__global__ void __launch_bounds__(256) xg_lower_transpose_kernel(double *__restrict__ Y, int nt, int ts)
 {
     __shared__ double s[32][33];
     const int nb = ts / 32;
-    const long long nbg = (long long)nt * nb;
-    const int gb = (int)(blockIdx.x % nbg), ga = (int)(blockIdx.x / nbg);
-    const int A = ga / nb, a = ga % nb, B = gb / nb, b = gb % nb;
+    int a, b;
+    xg_pair_decode(blockIdx.x, &a, &b);
+    double *F = Y + blockIdx.y * (long long)nt * nt * ts * ts;
+    const double *src = F + (((long long)(a / nb) * nt + b / nb) * ts + b % nb * 32) * ts + a % nb * 32;
+    double *dst = F + (((long long)(b / nb) * nt + a / nb) * ts + a % nb * 32) * ts + b % nb * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    double *dst = F + ((long long)A * nt + B) * ts * ts;
-    if (ga >= gb) {
-        const double *src = S + xg_tile_index(A, B, nt) * ts * ts;
-        for (int i = ty; i < 32; i += 8)
-            dst[(long long)(a * 32 + i) * ts + b * 32 + tx] = src[(long long)(a * 32 + i) * ts + b * 32 + tx];
-    } else {
-        const double *src = S + xg_tile_index(B, A, nt) * ts * ts;
-        for (int i = ty; i < 32; i += 8) s[i][tx] = src[(long long)(b * 32 + i) * ts + a * 32 + tx];
-        __syncthreads();
-        for (int i = ty; i < 32; i += 8) dst[(long long)(a * 32 + i) * ts + b * 32 + tx] = s[tx][i];
-    }
+    for (int i = ty; i < 32; i += 8) s[i][tx] = src[(long long)i * ts + tx];
+    __syncthreads();
+    for (int i = ty; i < 32; i += 8) dst[(long long)i * ts + tx] = s[tx][i];
 }
 
-void xg_launch_sym_full(const double *S, double *F, int nt, int ts, cudaStream_t st)
+void xg_launch_lower_transpose(double *Y, int nsys, int nt, int ts, cudaStream_t st)
 {
-    const long long nbg = (long long)nt * (ts / 32);
-    xg_sym_full_kernel<<<(unsigned)(nbg * nbg), 256, 0, st>>>(S, F, nt, ts);
+    const long long nb = (long long)nt * (ts / 32);
+    xg_lower_transpose_kernel<<<dim3((unsigned)(nb * (nb + 1) / 2), nsys), 256, 0, st>>>(Y, nt, ts);
 }
 
-/* dSigma/dtheta_which (0 sigma^2, 1 beta, 2 nu) into full tiles, zero outside
- * N x N; at zero distance 1 for sigma^2 and 0 for beta and nu
- * (core_zcmg.c:331-332, 394-395, 471-472). */
+/* dSigma/dtheta_which (1 beta, 2 nu, 3 tau^2) into a square R-layout matrix,
+ * zero outside N x N and, for beta and nu, at zero distance
+ * (core_zcmg.c:394-395, 471-472). */
 __global__ void __launch_bounds__(256) xg_dsigma_full_kernel(double *__restrict__ D, int nt, int ts,
                                                              const double *__restrict__ x,
                                                              const double *__restrict__ y, int N, XgMaternParams p,
@@ -221,7 +220,7 @@ __global__ void __launch_bounds__(256) xg_dsigma_full_kernel(double *__restrict_
     const int strips = ts / XG_AS_ROWS;
     const long long slot = blockIdx.x / strips;
     const int strip = blockIdx.x % strips;
-    const int A = (int)(slot / nt), B = (int)(slot % nt);
+    const int B = (int)(slot / nt), A = (int)(slot % nt);
     double *tile = D + slot * (long long)ts * ts;
     for (int rr = 0; rr < XG_AS_ROWS; ++rr) {
         const int r = strip * XG_AS_ROWS + rr;
@@ -232,13 +231,15 @@ __global__ void __launch_bounds__(256) xg_dsigma_full_kernel(double *__restrict_
             const int gb = B * ts + c;
             double v = 0.0;
             if (rok && gb < N) {
-                const double rd = xg_distance(x1, y1, x[gb], y[gb], metric) / p.beta;
-                if (rd == 0.0) {
-                    v = which == 0 ? 1.0 : 0.0;
+                if (which == 3) {
+                    v = ga == gb ? 1.0 : 0.0;
                 } else {
-                    double m, ds, db, dn;
-                    xg_matern_grad(rd, p.nu, p.con, p.sigma2, p.beta, dlogcon, &m, &ds, &db, &dn);
-                    v = which == 0 ? ds : (which == 1 ? db : dn);
+                    const double rd = xg_distance(x1, y1, x[gb], y[gb], metric) / p.beta;
+                    if (rd != 0.0) {
+                        double m, ds, db, dn;
+                        xg_matern_grad(rd, p.nu, p.con, p.sigma2, p.beta, dlogcon, &m, &ds, &db, &dn);
+                        v = which == 1 ? db : dn;
+                    }
                 }
             }
             tile[(long long)r * ts + c] = v;
@@ -250,8 +251,8 @@ void xg_launch_dsigma_full(double *D, int nt, int ts, const double *x, const dou
                            const XgMaternParams &p, double dlogcon, int metric, int which, double *tab,
                            cudaStream_t st)
 {
-    if (tab && xg_tab_covers(p, N)) {
-        if (which == 0) xg_launch_grad_tables(p, dlogcon, tab, st); /* the calls for 1 and 2 follow on the stream */
+    if (which < 3 && tab && xg_tab_covers(p, N)) {
+        if (which == 1) xg_launch_grad_tables(p, dlogcon, tab, st); /* the call for 2 follows on the stream */
         xg_launch_dsigma_full_tab(D, nt, ts, x, y, N, p, dlogcon, metric, which, tab, st);
         return;
     }
@@ -259,54 +260,46 @@ void xg_launch_dsigma_full(double *D, int nt, int ts, const double *x, const dou
     xg_dsigma_full_kernel<<<(unsigned)blocks, 256, 0, st>>>(D, nt, ts, x, y, N, p, dlogcon, metric, which);
 }
 
-struct XgFisherG {
-    const double *g[4];
-};
-
 /* part[10 blockIdx.x + q] for the pairs q = (j, k), j <= k < 4, in row order
- * (pairs with k >= np stay zero):
- * sum over a, b < N of G_j[a, b] G_k[b, a].  A CTA walks pairs of 32-blocks
- * (ga <= gb): the (gb, ga) blocks of every G are staged transposed in shared
- * memory, the (ga, gb) blocks are read in rows. */
-__global__ void __launch_bounds__(256) xg_fisher_trace_kernel(XgFisherG G, int np, int nt, int ts, int N,
-                                                              long long npairs, double *__restrict__ part)
+ * (pairs with k >= np stay zero): sum over a, b < N of W_j[a, b] W_k[a, b],
+ * from the lower halves of W_1, W_2 (, M) at W, W + full (, W + 2 full). */
+__global__ void __launch_bounds__(256) xg_fisher_trace_kernel(const double *__restrict__ W, int np, int nt, int ts,
+                                                              int N, long long units, double inv_sigma2, double nugget,
+                                                              double *__restrict__ part)
 {
-    __shared__ double Q[4][32][33];
     __shared__ double red[10][8];
-    const int nb = ts / 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int nb = ts / XG_DAG_BLOCK;
+    const long long full = (long long)nt * nt * ts * ts;
     double acc[10];
 #pragma unroll
     for (int q = 0; q < 10; ++q) acc[q] = 0.0;
-    for (long long pid = blockIdx.x; pid < npairs; pid += gridDim.x) {
-        int gi, gj;
-        xg_pair_decode(pid, &gi, &gj);
-        const int ga = gj, gb = gi; /* ga <= gb */
-        const long long offQ =
-            (((long long)(gb / nb) * nt + ga / nb) * ts + (gb % nb) * 32) * ts + (ga % nb) * 32;
-        const long long offP =
-            (((long long)(ga / nb) * nt + gb / nb) * ts + (ga % nb) * 32) * ts + (gb % nb) * 32;
-        __syncthreads();
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) { /* 32 rows of a lower 128-block */
+        int I, J;
+        xg_pair_decode(u / 4, &I, &J);
+        const int c = 2 * (threadIdx.x & 63), gb = J * XG_DAG_BLOCK + c;
+        for (int i = 0; i < 8; ++i) {
+            const int r = (int)(u % 4) * 32 + 4 * i + (int)(threadIdx.x >> 6), ga = I * XG_DAG_BLOCK + r;
+            if (ga >= N || gb > ga) continue;
+            const double *at = W + (((long long)(J / nb) * nt + I / nb) * ts + I % nb * XG_DAG_BLOCK + r) * ts +
+                               J % nb * XG_DAG_BLOCK + c;
+            double2 w[3];
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
-            if (m < np)
-                for (int i = ty; i < 32; i += 8) Q[m][i][tx] = G.g[m][offQ + (long long)i * ts + tx];
-        __syncthreads();
-        for (int i = ty; i < 32; i += 8) {
-            if (ga * 32 + i >= N || gb * 32 + tx >= N) continue;
-            double P[4];
+            for (int m = 0; m < 3; ++m)
+                w[m] = m < np - 1 ? *(const double2 *)(at + m * full) : make_double2(0.0, 0.0);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) P[m] = m < np ? G.g[m][offP + (long long)i * ts + tx] : 0.0;
-            int q = 0;
+            for (int h = 0; h < 2; ++h) {
+                if (gb + h > ga) continue;
+                const double d = ga == gb + h ? 1.0 : 0.0, f = 2.0 - d; /* the mirror counts too */
+                double P[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+                for (int m = 0; m < 3; ++m) P[m + 1] = h ? w[m].y : w[m].x;
+                P[0] = (d - nugget * P[3]) * inv_sigma2;
+                int q = 0;
 #pragma unroll
-                for (int k = j; k < 4; ++k, ++q)
-                    if (k < np) {
-                        double t = P[j] * Q[k][tx][i];
-                        if (ga != gb) t += P[k] * Q[j][tx][i];
-                        acc[q] += t;
-                    }
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int k = j; k < 4; ++k, ++q) acc[q] += f * P[j] * P[k];
+            }
         }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -324,14 +317,11 @@ __global__ void __launch_bounds__(256) xg_fisher_trace_kernel(XgFisherG G, int n
     }
 }
 
-void xg_launch_fisher_trace(const double *const g[4], int np, int nt, int ts, int N, double *part, int nctas,
-                            cudaStream_t st)
+void xg_launch_fisher_trace(const double *W, int np, int nt, int ts, int N, double sigma2, double nugget, double *part,
+                            int nctas, cudaStream_t st)
 {
-    XgFisherG G;
-    for (int m = 0; m < 4; ++m) G.g[m] = m < np ? g[m] : nullptr;
-    const long long nbg = (long long)nt * (ts / 32);
-    const long long npairs = nbg * (nbg + 1) / 2;
-    xg_fisher_trace_kernel<<<nctas, 256, 0, st>>>(G, np, nt, ts, N, npairs, part);
+    const long long units = 4 * xg_num_lower_tiles((N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK);
+    xg_fisher_trace_kernel<<<nctas, 256, 0, st>>>(W, np, nt, ts, N, units, 1.0 / sigma2, nugget, part);
 }
 
 /* ------------------------------------------------------------------------- */
@@ -394,35 +384,43 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
     int rc = xg_check_theta(theta, kernel);
     if (rc) return rc;
     const int nt = f->C.nt, ts = f->C.ts, N = f->N;
-    const int np = kernel == 1 ? 4 : 3;
-    if (!f->X.d) {
-        rc = xg_tm_alloc(f->X, N, ts);
-        if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) {
-            xg_tm_free(f->X);
-            rc = xg_tm_alloc(f->X, N, ts);
-        }
-        if (rc) return rc;
-    }
+    const int np = kernel == 1 ? 4 : 3, nsys = np - 1;
+    const int nb = (N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     const size_t full = (size_t)nt * nt * ts * ts;
+    const size_t words = 2 + (size_t)nsys * nb * nb; /* next task, abort, block flags */
     const int nctas = g_xg.sm_count * 8;
-    double *Sf = nullptr, *D = nullptr, *G = nullptr, *part = nullptr;
-    while (cudaMalloc(&Sf, full * sizeof(double)) != cudaSuccess || cudaMalloc(&D, full * sizeof(double)) != cudaSuccess ||
-           cudaMalloc(&G, 3 * full * sizeof(double)) != cudaSuccess ||
-           cudaMalloc(&part, 10 * (size_t)nctas * sizeof(double)) != cudaSuccess) {
+    double *Y = nullptr, *part = nullptr;
+    int *w = nullptr;
+    while (cudaMalloc(&Y, nsys * full * sizeof(double)) != cudaSuccess ||
+           cudaMalloc(&part, 10 * (size_t)nctas * sizeof(double)) != cudaSuccess ||
+           cudaMalloc(&w, words * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(Sf);
-        cudaFree(D);
-        cudaFree(G);
+        cudaFree(Y);
         cudaFree(part);
-        Sf = D = G = part = nullptr;
+        Y = part = nullptr;
+        w = nullptr;
         if (xg_i8_release(f->C)) continue;
-        return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", 5.0 * full * sizeof(double) / 1e9);
+        return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", nsys * full * sizeof(double) / 1e9);
     }
     std::vector<double> hp(10 * (size_t)nctas);
     int sv[2] = {0, 0};
-    CUtensorMap mS, mD;
-    rc = xg_encode_tiles(&mS, Sf, (long long)nt * nt, ts);
-    if (!rc) rc = xg_encode_tiles(&mD, D, (long long)nt * nt, ts);
+    XgRowsMaps maps = {};
+    XgRows R = {};
+    for (int k = 0; k < nsys && !rc; ++k) {
+        rc = xg_encode_tiles(&maps.y[k], Y + k * full, (long long)nt * nt, ts);
+        maps.l[k] = f->C.map;
+        R.y[k] = Y + k * full;
+        R.dinv[k] = f->C.dinv;
+    }
+    R.ts = ts;
+    R.nsys = nsys;
+    R.one.nt = R.one.mt = nt;
+    R.one.nb = R.one.mr = nb;
+    R.sys_flags = (long long)nb * nb;
+    R.next = (unsigned *)w;
+    R.abort = w + 1;
+    R.flags = w + 2;
+    R.status = f->status;
     if (!rc) {
         cudaStream_t st = g_xg.stream;
         XgTileArgs T{f->C.d, ts, nt};
@@ -430,7 +428,7 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
         cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
         cudaEventRecord(f->ev[0], st);
-        /* Sigma (MLE_dexact.c:1824-1825), its factor (:1830) and S = Sigma^-1 */
+        /* Sigma (MLE_dexact.c:1824-1825) and its factor (:1830) */
         xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, N, N, p, f->metric, 1, f->C.tab, st);
         XgFactorStreams fs;
         fs.st = st;
@@ -438,15 +436,18 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         fs.ev_panel = f->ev_panel;
         fs.ev_upd = f->ev_upd;
         xg_factor_lookahead(f->C, nullptr, f->part, f->status, f->info, fs);
-        xg_inverse_product(f->C, f->X, f->status, st);
-        xg_launch_sym_full(f->C.d, Sf, nt, ts, st);
-        /* G_j = S dSigma_j (dSigma_j symmetric: S dSigma_j^T) */
-        for (int j = 0; j < 3; ++j) {
-            xg_launch_dsigma_full(D, nt, ts, f->x, f->y, N, p, dlogcon, f->metric, j, f->C.tab, st);
-            xg_launch_dense_gemm_nt(mS, mD, G + j * full, nt, ts, f->status, st);
-        }
-        const double *g[4] = {G, G + full, G + 2 * full, Sf};
-        xg_launch_fisher_trace(g, np, nt, ts, N, part, nctas, st);
+        /* Y_j = dSigma_j L^-T, then the lower half of W_j = L^-1 Y_j */
+        for (int k = 0; k < nsys; ++k)
+            xg_launch_dsigma_full(Y + k * full, nt, ts, f->x, f->y, N, p, dlogcon, f->metric, k + 1, f->C.tab, st);
+        cudaMemsetAsync(w, 0, words * sizeof(int), st);
+        R.ntasks = (long long)nsys * nb * nb;
+        xg_launch_rows(XG_ROWS_RHS, maps, R, g_xg.sm_count, st);
+        xg_launch_lower_transpose(Y, nsys, nt, ts, st);
+        cudaMemsetAsync(w, 0, words * sizeof(int), st);
+        R.lower = 1;
+        R.ntasks = nsys * xg_num_lower_tiles(nb);
+        xg_launch_rows(XG_ROWS_RHS, maps, R, g_xg.sm_count, st);
+        xg_launch_fisher_trace(Y, np, nt, ts, N, p.sigma2, p.nugget, part, nctas, st);
         cudaEventRecord(f->ev[3], st);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -459,10 +460,9 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
             *seconds = ms * 1e-3;
         }
     }
-    cudaFree(Sf);
-    cudaFree(D);
-    cudaFree(G);
+    cudaFree(Y);
     cudaFree(part);
+    cudaFree(w);
     if (rc) return rc;
     if (sv[0]) return xg_status_error(sv, "the covariance");
     int q = 0;

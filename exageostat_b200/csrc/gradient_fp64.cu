@@ -43,7 +43,6 @@
  * slot K * mt + R (right-hand sides stored transposed, one row per
  * right-hand side). */
 #define XG_TG_RTRI 4    /* C(R, I) = sum_{K >= I} A(R, K) B_slot(K, I)^T (R layout, B lower-tile packed) */
-#define XG_TG_DENSE 5   /* full nt x nt tiles (slot A nt + B): C(A, B) = sum_K A(A, K) B(B, K)^T */
 #define XG_TG_RBWD 6    /* step K of Z L = B (R layout), B holding L's tiles transposed in place:
                            B(R, K') -= Z(R, K) B_slot(K, K')^T, K' < K */
 
@@ -70,20 +69,13 @@ __device__ inline XgTileGemmJob xg_tg_decode(int mode, long long job, int nt, in
         j.b_slot0 = (int)xg_tile_index(I, I, nt);
         j.k_step_b = 1;
         j.ntiles_k = nt - I;
-    } else if (mode == XG_TG_RBWD) {
+    } else { /* XG_TG_RBWD */
         const int R = (int)(job % mt), Kp = (int)(job / mt);
         j.c_slot = Kp * mt + R;
         j.a_slot0 = K * mt + R;
         j.b_slot0 = (int)xg_tile_index(K, Kp, nt);
         j.ntiles_k = 1;
         j.k_step_a = j.k_step_b = 0;
-    } else { /* XG_TG_DENSE */
-        const int A = (int)(job / nt), B = (int)(job % nt);
-        j.c_slot = A * nt + B;
-        j.a_slot0 = A * nt;
-        j.b_slot0 = B * nt;
-        j.k_step_a = j.k_step_b = 1;
-        j.ntiles_k = nt;
     }
     return j;
 }
@@ -478,14 +470,4 @@ void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB,
     const long long jobs = (long long)mt * nt;
     xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
         mapA, mapB, C, nt, ts, XG_TG_RTRI, 0, mt, status);
-}
-
-/* C = A B^T on full nt x nt tile grids (tile (A, B) at slot A nt + B) */
-void xg_launch_dense_gemm_nt(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int nt, int ts, int *status,
-                             cudaStream_t st)
-{
-    const int bpt = ts / XG_TG_BM;
-    const long long jobs = (long long)nt * nt;
-    xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-        mapA, mapB, C, nt, ts, XG_TG_DENSE, 0, 0, status);
 }

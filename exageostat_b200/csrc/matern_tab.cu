@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(XG_GT_THREADS)
     const long long u1 = units * (blockIdx.x + 1LL) / gridDim.x;
     for (long long u = units * blockIdx.x / gridDim.x; u < u1; ++u) {
         const long long slot = u / strips;
-        const int A = (int)(slot / nt), B = (int)(slot - (long long)A * nt);
+        const int B = (int)(slot / nt), A = (int)(slot - (long long)B * nt);
         double *tile = D + slot * (long long)ts * ts;
         const int row0 = (int)(u - slot * strips) * XG_GT_ROWS;
         for (int e = (int)threadIdx.x; e < XG_GT_ROWS * half; e += XG_GT_THREADS) {
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(XG_GT_THREADS)
                 const double q = xg_distance(x[ga], y[ga], x[gb + m], y[gb + m], metric) / P.beta;
                 const unsigned i = xg_tab_index(q);
                 if (q == 0.0) {
-                    v[m] = which == 0 ? 1.0 : 0.0;
+                    v[m] = 0.0;
                 } else if (i < XG_TAB_NINT) {
                     v[m] = xg_tab_poly(xg_smem_d, i, q - xg_tab_centre(q)) * exp(-q);
                 } else {

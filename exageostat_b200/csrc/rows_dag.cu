@@ -5,11 +5,13 @@
  *
  *   XG_ROWS_INVERSE  X L^T = I (X = L^-T, upper triangular, X_IK at packed tile slot (K, I)), then
  *                    S = X X^T written over the factor: the inverse and product of the adjoint
- *                    gradient and of the Fisher matrix (steps 2 and 3 of gradient_fp64.cu);
+ *                    gradient (steps 2 and 3 of gradient_fp64.cu);
  *                    a window of columns J0 .. : the sums over K < J0 are in place already
  *                    and there are no products (the INT8 path)
  *   XG_ROWS_RHS      Y L^T = B for row blocks in R layout (tile (R, K) at slot K mt + R), up to
  *                    three systems at once: the forward solves of MLOE / MMOM (MLE_dexact.c:1300-1364)
+ *                    and the two-sided solves of the Fisher matrix (the second with the lower
+ *                    blocks only)
  *
  * Solve task (I, J): Y_IJ = (B_IJ - sum_{K < J} Y_IK L_JK^T) L_JJ^-T with the
  * accumulators in registers from the first product to the store, so a block
@@ -84,8 +86,14 @@ __global__ void __launch_bounds__(XG_D_THREADS, 1) xg_rows_dag_kernel(const __gr
         } else if (MODE == XG_ROWS_RHS) {
             sys = (int)(q % G.nsys);
             q /= G.nsys;
-            I = (int)(q % G.one.mr);
-            J = (int)(q / G.one.mr);
+            if (G.lower) {
+                xg_pair_decode(G.ntasks / G.nsys - 1 - q, &J, &I);
+                I = G.one.nb - 1 - I;
+                J = G.one.nb - 1 - J;
+            } else {
+                I = (int)(q % G.one.mr);
+                J = (int)(q / G.one.mr);
+            }
         } else {
             const long long nx = xg_num_lower_tiles(G.one.nb);
             product = q >= nx;

@@ -193,6 +193,7 @@ struct XgRows {
     const double *dinv[XG_ROWS_MAX_SYS];
     double *s;                           /* INVERSE: the factor's store, receives S */
     int ts, nsys, J0;                    /* J0: first block column of a window (INVERSE, no products) */
+    int lower;                           /* RHS: as many rows as columns, only the blocks I >= J */
     XgRowsField one;
     const XgRowsField *F;
     const int4 *tasks;                   /* (field, I, J, product?); null: a single field, every task */
@@ -345,8 +346,6 @@ void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, co
                                   const double *LT, int nt, int ts, int *status, cudaStream_t st);
 void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int mt, int nt, int ts,
                                int *status, cudaStream_t st);
-void xg_launch_dense_gemm_nt(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int nt, int ts, int *status,
-                             cudaStream_t st);
 long long xg_grad_contract_blocks(long long ntiles, int ts);
 void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long ntiles, int nt, int ts, const double *x,
                              const double *y, const double *alpha, int N, const XgMaternParams &mp, int kernel,
@@ -359,11 +358,11 @@ void xg_launch_cross_gen_r(double *D, int mt, int nt, int ts, const double *xm, 
 void xg_launch_tile_transpose(double *D, long long ntiles, int ts, cudaStream_t st);
 void xg_launch_mloe_terms(const double *A, const double *U, const double *T, const double *V, int mt, int nt, int ts,
                           int nmiss, double sigma2_t, double sigma2_a, double *terms, cudaStream_t st);
-void xg_launch_sym_full(const double *S, double *F, int nt, int ts, cudaStream_t st);
+void xg_launch_lower_transpose(double *Y, int nsys, int nt, int ts, cudaStream_t st);
 void xg_launch_dsigma_full(double *D, int nt, int ts, const double *x, const double *y, int N,
                            const XgMaternParams &p, double dlogcon, int metric, int which, double *tab,
                            cudaStream_t st);
-void xg_launch_fisher_trace(const double *const g[4], int np, int nt, int ts, int N, double *part, int nctas,
-                            cudaStream_t st);
+void xg_launch_fisher_trace(const double *W, int np, int nt, int ts, int N, double sigma2, double nugget, double *part,
+                            int nctas, cudaStream_t st);
 
 #endif

@@ -29,6 +29,20 @@ def test_fisher_matches_oracle(gpu, ora, n, ts, theta, kernel, tol):
         assert F[0, 0] == pytest.approx(n / (2 * theta[0] ** 2), rel=1e-9)
 
 
+@pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("n,ts", [(5, 128), (127, 128), (128, 128), (129, 128), (257, 256), (385, 384), (1025, 512)])
+def test_fisher_block_edges(gpu, ora, n, ts, kernel):
+    """Exactly filled blocks of 128, one row past, one short: the bar of the
+    file.  F is checked with the nugget (a system more) and without."""
+    theta = [1.3, 0.1, 0.6] + [0.05] * kernel
+    x, y = ora.generate_xy_loc(n, 2)
+    F = gpu.fisher_host(x, y, theta, kernel=kernel, ts=ts)
+    Fo, _ = ora.fisher(x, y, theta, kernel)
+    scale = np.sqrt(np.outer(np.diag(Fo), np.diag(Fo)))
+    assert (np.abs(F - Fo) / scale).max() < 1e-8, (F, Fo)
+    assert np.array_equal(F, F.T)
+
+
 def test_fisher_reference_entry_points(gpu, ora):
     """EXAGEOSTAT_Fisher_Tile returns the inverse (10 doubles, column-major)
     and fills results.fisher_*; a log-likelihood and a gradient afterwards are
