@@ -167,7 +167,6 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
     e = cudaMalloc(&M.tab, sizeof(double) * xg_tab_doubles());
     if (e != cudaSuccess) {
         M.tab = nullptr;
-    xg_i8_release(M);
         return xg_cuda_fail(e, "element tables");
     }
     return xg_encode_tiles(&M.map, M.d, M.ntiles, ts);
@@ -195,6 +194,8 @@ void xg_tm_free(XgTileMatrix &M)
     if (M.dinv) cudaFree(M.dinv);
     if (M.dag) cudaFree(M.dag);
     if (M.tab) cudaFree(M.tab);
+    xg_i8_release(M);
+    M.no_i8 = M.i8_factor = false; /* of the matrix that was freed */
     M.tab = nullptr;
     M.dag = nullptr;
     M.d = nullptr;

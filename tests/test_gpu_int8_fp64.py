@@ -64,3 +64,22 @@ def test_a_failing_pivot_is_reported(gpu, ora):
         assert err.value.code == gpu.XG_ERR_NOT_SPD and "pivot 5001)" in str(err.value)
         s.set_data(x=x)
         assert s.loglik([1.0, 0.1, 0.5]) == ll
+
+
+def test_the_digit_planes_are_given_back(gpu, ora):
+    """Closed sessions and finished kriging calls leave the device's free
+    memory where it was; the planes of one N = 7000 factor are 0.2 GB."""
+    import torch
+
+    n, m, theta = 7000, 50, [1.0, 0.1, 0.5]
+    x, y = ora.generate_xy_loc(n + m, 3)
+    z = np.random.default_rng(1).standard_normal(n + m)
+    free = []
+    for _ in range(3):
+        with gpu.Session(x[m:], y[m:], dts=512) as s:
+            s.set_data(z=z[m:])
+            s.loglik(theta, grad=True)
+            s.predict(theta, x[:m], y[:m], x[m:], y[m:], z[m:])
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[2] < 64 << 20, free
