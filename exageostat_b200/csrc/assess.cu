@@ -391,14 +391,8 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
     const int nctas = g_xg.sm_count * 8;
     double *Y = nullptr, *part = nullptr;
     int *w = nullptr;
-    while (cudaMalloc(&Y, nsys * full * sizeof(double)) != cudaSuccess ||
-           cudaMalloc(&part, 10 * (size_t)nctas * sizeof(double)) != cudaSuccess ||
-           cudaMalloc(&w, words * sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(Y);
-        cudaFree(part);
-        Y = part = nullptr;
-        w = nullptr;
+    const XgPart parts[] = {{&Y, nsys * full}, {&part, 10 * (size_t)nctas}, {&w, words}};
+    while (xg_alloc_parts(parts, 3) != cudaSuccess) {
         if (xg_i8_release(f->C)) continue;
         return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", nsys * full * sizeof(double) / 1e9);
     }
@@ -461,8 +455,6 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
         }
     }
     cudaFree(Y);
-    cudaFree(part);
-    cudaFree(w);
     if (rc) return rc;
     if (sv[0]) return xg_status_error(sv, "the covariance");
     int q = 0;
@@ -485,30 +477,12 @@ void xg_assess_destroy(XgAssess *q)
     if (!q) return;
     xg_tm_free(q->Ca);
     xg_tm_free(q->Ct);
-    for (int i = 0; i < 5; ++i) cudaFree(q->R[i]);
-    cudaFree(q->xo);
-    cudaFree(q->yo);
-    cudaFree(q->xm);
-    cudaFree(q->ym);
-    cudaFree(q->terms);
-    cudaFree(q->part);
-    cudaFree(q->words);
-    cudaFree(q->status);
+    cudaFree(q->R[0]);
     for (int i = 0; i < 4; ++i)
         if (q->ev[i]) cudaEventDestroy(q->ev[i]);
     if (q->ev_panel) cudaEventDestroy(q->ev_panel);
     if (q->ev_upd) cudaEventDestroy(q->ev_upd);
     delete q;
-}
-
-static int xg_assess_alloc(double **p, size_t n)
-{
-    cudaError_t e = cudaMalloc(p, n * sizeof(double));
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        return xg_fail(XG_ERR_NO_MEMORY, "cudaMalloc(%zu doubles): %s", n, cudaGetErrorString(e));
-    }
-    return cudaMemset(*p, 0, n * sizeof(double)) == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }
 
 int xg_assess_create(XgAssess **out, int nmiss, int nobs, int ts)
@@ -526,21 +500,22 @@ int xg_assess_create(XgAssess **out, int nmiss, int nobs, int ts)
     q->nt = q->Ca.nt;
     q->mt = (nmiss + q->ts - 1) / q->ts;
     const long long rtiles = (long long)q->mt * q->nt;
-    for (int i = 0; i < 5 && !rc; ++i) {
-        rc = xg_assess_alloc(&q->R[i], (size_t)rtiles * q->ts * q->ts);
-        if (!rc) rc = xg_encode_tiles(&q->mR[i], q->R[i], rtiles, q->ts);
-    }
-    const size_t Np = (size_t)q->nt * q->ts;
-    if (!rc) rc = xg_assess_alloc(&q->xo, Np);
-    if (!rc) rc = xg_assess_alloc(&q->yo, Np);
-    if (!rc) rc = xg_assess_alloc(&q->xm, nmiss);
-    if (!rc) rc = xg_assess_alloc(&q->ym, nmiss);
-    if (!rc) rc = xg_assess_alloc(&q->terms, 6 * (size_t)nmiss);
-    if (!rc) rc = xg_assess_alloc(&q->part, 2 * (size_t)q->nt * q->ts / XG_DAG_BLOCK);
-    if (!rc && cudaMalloc(&q->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status");
+    const size_t Np = (size_t)q->nt * q->ts, rsize = (size_t)rtiles * q->ts * q->ts;
     const long long flags = 3LL * ((nobs + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK) * ((nmiss + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK);
-    if (!rc && cudaMalloc(&q->words, (size_t)(2 + flags) * sizeof(int)) != cudaSuccess)
-        rc = xg_fail(XG_ERR_NO_MEMORY, "block flags");
+    if (!rc) {
+        const XgPart parts[] = {{&q->R[0], rsize}, {&q->R[1], rsize}, {&q->R[2], rsize}, {&q->R[3], rsize},
+                                {&q->R[4], rsize}, {&q->xo, Np}, {&q->yo, Np}, {&q->xm, (size_t)nmiss},
+                                {&q->ym, (size_t)nmiss}, {&q->terms, 6 * (size_t)nmiss},
+                                {&q->part, 2 * Np / XG_DAG_BLOCK}, {&q->status, 2}, {&q->words, (size_t)(2 + flags)}};
+        cudaError_t e = xg_alloc_parts(parts, 13);
+        /* on the stream that fills them: the default stream does not wait for it, nor it for that */
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(q->R[0], 0, (char *)(q->words + 2 + flags) - (char *)q->R[0], g_xg.stream);
+        if (e != cudaSuccess)
+            rc = xg_fail(XG_ERR_NO_MEMORY, "MLOE / MMOM workspace (%.2f GB): %s", 5.0 * rsize * sizeof(double) / 1e9,
+                         cudaGetErrorString(e));
+    }
+    for (int i = 0; i < 5 && !rc; ++i) rc = xg_encode_tiles(&q->mR[i], q->R[i], rtiles, q->ts);
     for (int i = 0; i < 4 && !rc; ++i)
         if (cudaEventCreate(&q->ev[i]) != cudaSuccess) rc = xg_fail(XG_ERR_CUDA, "events");
     if (!rc && (cudaEventCreateWithFlags(&q->ev_panel, cudaEventDisableTiming) != cudaSuccess ||

@@ -129,6 +129,20 @@ int xg_choose_ts(int N, int dts)
     return ts;
 }
 
+cudaError_t xg_alloc_parts(const XgPart *parts, int n)
+{
+    size_t total = 0;
+    for (int i = 0; i < n; ++i) total += (parts[i].bytes + 255) / 256 * 256;
+    char *base = nullptr;
+    const cudaError_t e = cudaMalloc(&base, total);
+    if (e != cudaSuccess) cudaGetLastError();
+    for (int i = 0; i < n; ++i) {
+        *parts[i].p = base;
+        if (base) base += (parts[i].bytes + 255) / 256 * 256;
+    }
+    return e;
+}
+
 /* ------------------------------------------------------------------------- */
 /* lower-tile matrices                                                       */
 /* ------------------------------------------------------------------------- */
@@ -139,36 +153,23 @@ int xg_tm_alloc(XgTileMatrix &M, int N, int ts)
     M.ts = ts;
     M.nt = (N + ts - 1) / ts;
     M.ntiles = xg_num_lower_tiles(M.nt);
-    const size_t bytes = (size_t)M.ntiles * ts * ts * sizeof(double);
-    cudaError_t e = cudaMalloc(&M.d, bytes);
-    if (e != cudaSuccess) {
-        M.d = nullptr;
-        return xg_fail(XG_ERR_NO_MEMORY, "cannot allocate %.2f GB for %lld covariance tiles: %s", bytes / 1e9,
-                       M.ntiles, cudaGetErrorString(e));
-    }
+    const size_t elements = (size_t)M.ntiles * ts * ts;
+    const int nb = (N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
+    const XgPart parts[] = {{&M.d, elements},
+                            {&M.dinv, (size_t)M.nt * ts * 32},
+                            {&M.tab, xg_tab_doubles()},
+                            {&M.ij, (size_t)M.ntiles},
+                            {&M.dag, (size_t)(xg_dag_words(nb) + xg_trsv_words(nb))}};
+    cudaError_t e = xg_alloc_parts(parts, 5);
+    if (e != cudaSuccess)
+        return xg_fail(XG_ERR_NO_MEMORY, "cannot allocate %.2f GB for %lld covariance tiles: %s",
+                       elements * sizeof(double) / 1e9, M.ntiles, cudaGetErrorString(e));
     int2 *hij = (int2 *)malloc(sizeof(int2) * M.ntiles);
     for (int j = 0; j < M.nt; ++j)
         for (int i = j; i < M.nt; ++i) hij[xg_tile_index(i, j, M.nt)] = make_int2(i, j);
-    e = cudaMalloc(&M.ij, sizeof(int2) * M.ntiles);
-    if (e == cudaSuccess) e = cudaMemcpy(M.ij, hij, sizeof(int2) * M.ntiles, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(M.ij, hij, sizeof(int2) * M.ntiles, cudaMemcpyHostToDevice);
     free(hij);
     if (e != cudaSuccess) return xg_cuda_fail(e, "tile index table");
-    e = cudaMalloc(&M.dinv, sizeof(double) * (size_t)M.nt * ts * 32);
-    if (e != cudaSuccess) {
-        M.dinv = nullptr;
-        return xg_cuda_fail(e, "diagonal-block inverses");
-    }
-    const int nb = (N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
-    e = cudaMalloc(&M.dag, sizeof(int) * (size_t)(xg_dag_words(nb) + xg_trsv_words(nb)));
-    if (e != cudaSuccess) {
-        M.dag = nullptr;
-        return xg_cuda_fail(e, "block flags");
-    }
-    e = cudaMalloc(&M.tab, sizeof(double) * xg_tab_doubles());
-    if (e != cudaSuccess) {
-        M.tab = nullptr;
-        return xg_cuda_fail(e, "element tables");
-    }
     return xg_encode_tiles(&M.map, M.d, M.ntiles, ts);
 }
 
@@ -190,10 +191,6 @@ int xg_encode_tiles(CUtensorMap *map, double *base, long long ntiles, int ts)
 void xg_tm_free(XgTileMatrix &M)
 {
     if (M.d) cudaFree(M.d);
-    if (M.ij) cudaFree(M.ij);
-    if (M.dinv) cudaFree(M.dinv);
-    if (M.dag) cudaFree(M.dag);
-    if (M.tab) cudaFree(M.tab);
     xg_i8_release(M);
     M.no_i8 = M.i8_factor = false; /* of the matrix that was freed */
     M.tab = nullptr;
@@ -1246,8 +1243,7 @@ static int xg_tiles_to_dense(XgField *f, int n, double *out)
 
 static void xg_digits_free(XgDigits &D)
 {
-    if (D.dig) cudaFree(D.dig);
-    if (D.scale) cudaFree(D.scale);
+    if (D.dig) cudaFree(D.dig); /* and scale, behind it */
     D.dig = nullptr;
     D.scale = nullptr;
 }
@@ -1261,12 +1257,9 @@ static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits)
         return xg_fail(XG_ERR_BAD_ARGUMENT, "N = %d is beyond the sliced path's 2^31-row digit store", M.N);
     D.digits = digits;
     D.plane_rows = (int)rows;
-    if (cudaMalloc(&D.dig, digits * plane) != cudaSuccess ||
-        cudaMalloc(&D.scale, (size_t)rows * sizeof(double)) != cudaSuccess) {
-        cudaGetLastError();
-        xg_digits_free(D);
+    const XgPart parts[] = {{&D.dig, digits * plane}, {&D.scale, (size_t)rows}};
+    if (xg_alloc_parts(parts, 2) != cudaSuccess)
         return xg_fail(XG_ERR_NO_MEMORY, "digit planes (%.2f GB)", digits * (double)plane / 1e9);
-    }
     /* both operands are staged in boxes of 128 rows x 64 bytes */
     int rc = xg_encode(&D.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 64, 128,
                        CU_TENSOR_MAP_SWIZZLE_64B);
@@ -1804,10 +1797,7 @@ void xg_predict_destroy(XgPredict *q)
 {
     if (!q) return;
     xg_tm_free(q->C22);
-    double *bufs[] = {q->xm, q->ym, q->xo, q->yo, q->v, q->zact, q->zmiss, q->part, q->out};
-    for (double *b : bufs)
-        if (b) cudaFree(b);
-    if (q->status) cudaFree(q->status);
+    if (q->xo) cudaFree(q->xo);
     if (q->ev_panel) cudaEventDestroy(q->ev_panel);
     if (q->ev_upd) cudaEventDestroy(q->ev_upd);
     delete q;
@@ -1824,16 +1814,18 @@ int xg_predict_create(XgPredict **out, int nmiss, int nobs, int ts)
     q->nobs = nobs;
     rc = xg_tm_alloc(q->C22, nobs, xg_choose_ts(nobs, ts));
     const size_t Np = (size_t)q->C22.nt * q->C22.ts;
-    if (!rc) rc = xg_dev_alloc(&q->xo, Np);
-    if (!rc) rc = xg_dev_alloc(&q->yo, Np);
-    if (!rc) rc = xg_dev_alloc(&q->v, Np);
-    if (!rc) rc = xg_dev_alloc(&q->xm, nmiss);
-    if (!rc) rc = xg_dev_alloc(&q->ym, nmiss);
-    if (!rc) rc = xg_dev_alloc(&q->zact, nmiss);
-    if (!rc) rc = xg_dev_alloc(&q->zmiss, nmiss);
-    if (!rc) rc = xg_dev_alloc(&q->part, 2 * Np / XG_DAG_BLOCK);
-    if (!rc) rc = xg_dev_alloc(&q->out, 8);
-    if (!rc && cudaMalloc(&q->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status");
+    if (!rc) {
+        const size_t nm = (size_t)nmiss;
+        const XgPart parts[] = {{&q->xo, Np},   {&q->yo, Np},    {&q->v, Np},
+                                {&q->xm, nm},   {&q->ym, nm},    {&q->zact, nm},
+                                {&q->zmiss, nm}, {&q->part, 2 * Np / XG_DAG_BLOCK}, {&q->out, 8},
+                                {&q->status, 2}};
+        cudaError_t e = xg_alloc_parts(parts, 10);
+        /* on the stream that fills them: the default stream does not wait for it, nor it for that */
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(q->xo, 0, (char *)(q->status + 2) - (char *)q->xo, g_xg.stream);
+        if (e != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "kriging buffers: %s", cudaGetErrorString(e));
+    }
     if (!rc && (cudaEventCreateWithFlags(&q->ev_panel, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&q->ev_upd, cudaEventDisableTiming) != cudaSuccess))
         rc = xg_fail(XG_ERR_CUDA, "lookahead events");

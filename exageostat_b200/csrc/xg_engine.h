@@ -41,11 +41,22 @@ struct XgSliced {
     cudaEvent_t ev_a = nullptr, ev_p[2] = {nullptr, nullptr};
 };
 
+/* Device buffers in one allocation: *p of each part is set, 256-byte aligned;
+ * the first part's pointer is the one to free.  A cudaMalloc or cudaFree costs
+ * 0.3 to 3 ms whatever its size (0.001 to 128 MB alike), and MLOE / MMOM with
+ * one buffer each made 23 pairs of them per call. */
+struct XgPart {
+    void **p;
+    size_t bytes;
+    template <class T> XgPart(T **q, size_t n) : p((void **)q), bytes(n * sizeof(T)) {}
+};
+cudaError_t xg_alloc_parts(const XgPart *parts, int n);
+
 struct XgTileMatrix {
     int N = 0, ts = 0, nt = 0;
     long long ntiles = 0;
-    double *d = nullptr;
-    int2 *ij = nullptr; /* (i, j) of every packed tile */
+    double *d = nullptr; /* with ij, dinv, dag and tab in one allocation */
+    int2 *ij = nullptr;  /* (i, j) of every packed tile */
     CUtensorMap map;    /* TMA view for the trailing-update kernel */
     /* nt ts x 32: the inverted 32 x 32 diagonal blocks of L */
     double *dinv = nullptr;
