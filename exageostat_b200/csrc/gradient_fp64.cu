@@ -10,8 +10,8 @@
  *
  * After the forward factorisation (Sigma = L L^T in the lower tiles):
  *   1. alpha = L^-T (L^-1 z) with the backward solve (solve.cu).
- *   2. X = L^-T, upper triangular (rows_dag.cu; on the INT8-sliced path column
- *      by column with the kernels below), X_IK stored row-major at packed slot
+ *   2. X = L^-T, upper triangular (rows_dag.cu; on the INT8 path tile column by
+ *      tile column, with the updates of sliced.cu), X_IK stored row-major at packed slot
  *      (K, I) of a second lower-tile buffer, so both GEMM operands stay
  *      K-major for TMA.
  *   3. Sigma^-1 lower = X X^T: S_IJ = sum_{K >= I} X_IK X_JK^T, written over
@@ -30,7 +30,7 @@
 #include "xg_matern.cuh"
 
 /* ========================================================================== */
-/* Generalised tile GEMM: C (+)= -/+ sum_q A_q B_q^T over 128 x 128 blocks    */
+/* Triangular product of right-hand sides over 128 x 128 blocks               */
 /* ========================================================================== */
 
 #define XG_TG_BM 128
@@ -39,50 +39,12 @@
 #define XG_TG_THREADS 256
 #define XG_TG_STAGE_BYTES (2 * XG_TG_BM * XG_TG_BK * 8)
 
-/* modes.  "R layout": an mt x nt grid of tiles whose tile (R, K) sits at
- * slot K * mt + R (right-hand sides stored transposed, one row per
- * right-hand side). */
-#define XG_TG_RTRI 4    /* C(R, I) = sum_{K >= I} A(R, K) B_slot(K, I)^T (R layout, B lower-tile packed) */
-#define XG_TG_RBWD 6    /* step K of Z L = B (R layout), B holding L's tiles transposed in place:
-                           B(R, K') -= Z(R, K) B_slot(K, K')^T, K' < K */
-
-struct XgTileGemmJob {
-    int c_slot;  /* packed slot of the output tile */
-    int a_slot0; /* slot of the first A operand tile */
-    int b_slot0;
-    int ntiles_k; /* number of K tiles summed */
-    int k_step_a; /* slot stride between successive A tiles */
-    int k_step_b;
-    bool skip;
-};
-
-__device__ inline XgTileGemmJob xg_tg_decode(int mode, long long job, int nt, int K, int mt)
-{
-    XgTileGemmJob j;
-    j.skip = false;
-    if (mode == XG_TG_RTRI) {
-        const int R = (int)(job % mt), I = (int)(job / mt);
-        j.c_slot = I * mt + R;
-        j.a_slot0 = I * mt + R;
-        j.k_step_a = mt;
-        /* slot(K, I) for K = I.. nt-1 are consecutive in the packed column I */
-        j.b_slot0 = (int)xg_tile_index(I, I, nt);
-        j.k_step_b = 1;
-        j.ntiles_k = nt - I;
-    } else { /* XG_TG_RBWD */
-        const int R = (int)(job % mt), Kp = (int)(job / mt);
-        j.c_slot = Kp * mt + R;
-        j.a_slot0 = K * mt + R;
-        j.b_slot0 = (int)xg_tile_index(K, Kp, nt);
-        j.ntiles_k = 1;
-        j.k_step_a = j.k_step_b = 0;
-    }
-    return j;
-}
-
+/* C(R, I) = sum_{K >= I} A(R, K) B_slot(K, I)^T for "R layout" A and C, an mt x
+ * nt grid of tiles whose tile (R, K) sits at slot K * mt + R (right-hand sides
+ * stored transposed, one row per right-hand side), and lower-tile packed B. */
 __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     xg_tile_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                        double *__restrict__ Cbase, int nt, int ts, int mode, int K, int mt, int *status)
+                        double *__restrict__ Cbase, int nt, int ts, int mt, int *status)
 {
     extern __shared__ __align__(1024) unsigned char xg_smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)xg_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -92,7 +54,9 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     const long long job = blockIdx.x / (bpt * bpt);
     const int blk = blockIdx.x % (bpt * bpt);
     const int bi = blk / bpt, bj = blk % bpt;
-    const XgTileGemmJob J = xg_tg_decode(mode, job, nt, K, mt);
+    const int R = (int)(job % mt), I = (int)(job / mt);
+    /* the tiles (K, I), K = I .. nt - 1, are consecutive in the packed column I */
+    const int c_slot = I * mt + R, b_slot0 = (int)xg_tile_index(I, I, nt);
     if (xg_cta_should_skip(status)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
@@ -104,11 +68,11 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     }
     __syncthreads();
     const int kper = ts / XG_TG_BK;
-    const int KT = J.ntiles_k * kper;
+    const int KT = (nt - I) * kper;
     auto issue = [&](int q, int s) {
         const int kt = q / kper, kk = (q % kper) * XG_TG_BK;
-        const int ya = (J.a_slot0 + kt * J.k_step_a) * ts + bi * XG_TG_BM;
-        const int yb = (J.b_slot0 + kt * J.k_step_b) * ts + bj * XG_TG_BM;
+        const int ya = (c_slot + kt * mt) * ts + bi * XG_TG_BM;
+        const int yb = (b_slot0 + kt) * ts + bj * XG_TG_BM;
         unsigned char *sa = smem + s * XG_TG_STAGE_BYTES;
         xg_mbar_arrive_expect_tx(&full[s], XG_TG_STAGE_BYTES);
         xg_tma_load_2d(sa, &mapA, kk, ya, &full[s]);
@@ -122,26 +86,14 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
     }
     const int wm = warp >> 2, wn = warp & 3;
     const int g = lane >> 2, tq = lane & 3;
-    double *C = Cbase + (long long)J.c_slot * ts * ts + (long long)(bi * XG_TG_BM) * ts + bj * XG_TG_BM;
+    double *C = Cbase + (long long)c_slot * ts * ts + (long long)(bi * XG_TG_BM) * ts + bj * XG_TG_BM;
     double acc[4][4][4];
-    const bool subtract = mode == XG_TG_RBWD;
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                double cx = 0.0, cy = 0.0;
-                if (subtract) {
-                    const int r = wm * 64 + mi * 16 + g + 8 * h;
-                    const int c = wn * 32 + ni * 8 + 2 * tq;
-                    const double2 cv = *reinterpret_cast<const double2 *>(C + (long long)r * ts + c);
-                    cx = -cv.x;
-                    cy = -cv.y;
-                }
-                acc[mi][ni][2 * h] = cx;
-                acc[mi][ni][2 * h + 1] = cy;
-            }
+            for (int e = 0; e < 4; ++e) acc[mi][ni][e] = 0.0;
     bool ok = true;
     for (int kb = 0; kb < KT; ++kb) {
         const int s = kb % XG_TG_STAGES;
@@ -194,7 +146,6 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
                 xg_mbar_wait(&full[q % XG_TG_STAGES], (q / XG_TG_STAGES) & 1);
         return;
     }
-    const double sgn = subtract ? -1.0 : 1.0;
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
@@ -204,106 +155,8 @@ __global__ void __launch_bounds__(XG_TG_THREADS, 1)
                 const int r = wm * 64 + mi * 16 + g + 8 * h;
                 const int c = wn * 32 + ni * 8 + 2 * tq;
                 *reinterpret_cast<double2 *>(C + (long long)r * ts + c) =
-                    make_double2(sgn * acc[mi][ni][2 * h], sgn * acc[mi][ni][2 * h + 1]);
+                    make_double2(acc[mi][ni][2 * h], acc[mi][ni][2 * h + 1]);
             }
-}
-
-/* ========================================================================== */
-/* Right-side backward solve of step K: Z_RK <- Z_RK L_KK^-1                 */
-/* ========================================================================== */
-
-#define XG_XT_THREADS 512
-#define XG_XT_SR 32
-
-/* The tiles (R, K), R < mt, of an R-layout matrix; the diagonal tile holds U =
- * L_KK^T (a factor transposed in place) and the solve is B <- B U^-T = B
- * L_KK^-1, by 32-column blocks from the right (backward substitution). */
-__global__ void __launch_bounds__(XG_XT_THREADS) xg_xtrsm_kernel(double *__restrict__ X, const double *__restrict__ Lt,
-                                                                 int nt, int ts, int K, int mt, const int *status)
-{
-    const int LDS = ts + 4;
-    extern __shared__ __align__(16) double xg_smem_d[];
-    double *S = xg_smem_d;             /* [SR][LDS] */
-    double *LD = S + XG_XT_SR * LDS;   /* [32][33] */
-    if (xg_cta_should_skip(status)) return;
-    const int strips = ts / XG_XT_SR;
-    const int I = blockIdx.x / strips, strip = blockIdx.x % strips;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, tq = lane & 3;
-    const long long bslot = (long long)K * mt + I;
-    double *B = X + bslot * (long long)ts * ts + (long long)strip * XG_XT_SR * ts;
-    const double *L = Lt + xg_tile_index(K, K, nt) * (long long)ts * ts;
-    for (int idx = tid; idx < XG_XT_SR * ts; idx += blockDim.x) {
-        const int r = idx / ts, c = idx - r * ts;
-        S[r * LDS + c] = B[(long long)r * ts + c];
-    }
-    for (int blk = 0; blk < ts / 32; ++blk) {
-        const int cb = ts - 32 * (blk + 1);
-        for (int idx = tid; idx < 32 * 32; idx += blockDim.x) {
-            const int r = idx >> 5, c = idx & 31;
-            LD[r * 33 + c] = L[(long long)(cb + r) * ts + cb + c];
-        }
-        __syncthreads();
-        if (warp == 0) {
-            double row[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) row[j] = S[lane * LDS + cb + j];
-#pragma unroll
-            for (int j = 31; j >= 0; --j) {
-                double s = row[j];
-#pragma unroll
-                for (int q = j + 1; q < 32; ++q) s -= row[q] * LD[j * 33 + q];
-                row[j] = s / LD[j * 33 + j];
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) S[lane * LDS + cb + j] = row[j];
-        }
-        __syncthreads();
-        /* the solved block's contribution to the columns still to solve */
-        const int ngrp = cb / 32;
-        for (int grp = warp; grp < ngrp; grp += XG_XT_THREADS / 32) {
-            const int c0 = grp * 32;
-            double acc[2][4][4];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[mi][ni][e] = 0.0;
-#pragma unroll
-            for (int p0 = 0; p0 < 32; p0 += 4) {
-                double a[2][2], b[4];
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
-                    a[mi][0] = S[(mi * 16 + g) * LDS + cb + p0 + tq];
-                    a[mi][1] = S[(mi * 16 + g + 8) * LDS + cb + p0 + tq];
-                }
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) b[ni] = __ldg(L + (long long)(c0 + ni * 8 + g) * ts + cb + p0 + tq);
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni)
-                        xg_dmma_16x8x4(acc[mi][ni][0], acc[mi][ni][1], acc[mi][ni][2], acc[mi][ni][3], a[mi][0],
-                                       a[mi][1], b[ni]);
-            }
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        double *ps = S + (mi * 16 + g + 8 * h) * LDS + c0 + ni * 8 + 2 * tq;
-                        ps[0] -= acc[mi][ni][2 * h];
-                        ps[1] -= acc[mi][ni][2 * h + 1];
-                    }
-        }
-        __syncthreads();
-    }
-    for (int idx = tid; idx < XG_XT_SR * ts; idx += blockDim.x) {
-        const int r = idx / ts, c = idx - r * ts;
-        B[(long long)r * ts + c] = S[r * LDS + c];
-    }
 }
 
 /* zeros the diagonal tiles: the block solves of X = L^-T write only its upper
@@ -401,15 +254,11 @@ __global__ void xg_grad_reduce_kernel(const double *part, long long nblocks, dou
 /* ========================================================================== */
 
 size_t xg_tile_gemm_smem_bytes() { return (size_t)XG_TG_STAGES * XG_TG_STAGE_BYTES + 2 * XG_TG_STAGES * 8 + 1024; }
-size_t xg_xtrsm_smem_bytes(int ts) { return ((size_t)XG_XT_SR * (ts + 4) + 32 * 33) * sizeof(double); }
 
 cudaError_t xg_gradient_kernels_configure()
 {
-    cudaError_t e = cudaFuncSetAttribute(xg_tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)xg_tile_gemm_smem_bytes());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(xg_xtrsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)xg_xtrsm_smem_bytes(XG_MAX_TS));
+    return cudaFuncSetAttribute(xg_tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)xg_tile_gemm_smem_bytes());
 }
 
 void xg_launch_zero_diag(double *X, int nt, int ts, cudaStream_t st)
@@ -443,23 +292,6 @@ void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long nti
     xg_grad_reduce_kernel<<<1, dim3(32, 4), 0, st>>>(part, blocks, out);
 }
 
-/* Z L = B for an R-layout right-hand side B and a factor whose tiles were
- * transposed in place (LT: slot (i, j) holds L_ij^T), left-looking from the
- * last tile column: B is overwritten with Z, the transpose of L^-T B^T. */
-void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapLT,
-                                  const double *LT, int nt, int ts, int *status, cudaStream_t st)
-{
-    const int bpt = ts / XG_TG_BM;
-    for (int K = nt - 1; K >= 0; --K) {
-        xg_xtrsm_kernel<<<mt * (ts / XG_XT_SR), XG_XT_THREADS, xg_xtrsm_smem_bytes(ts), st>>>(R, LT, nt, ts, K,
-                                                                                                 mt, status);
-        const long long jobs = (long long)mt * K;
-        if (jobs > 0)
-            xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-                mapR, mapLT, R, nt, ts, XG_TG_RBWD, K, mt, status);
-    }
-}
-
 /* C(R, I) = sum_{K >= I} A(R, K) B_slot(K, I)^T: A and C R-layout (C != A),
  * B lower-tile packed.  With B = X (X_IK at slot (K, I)) this is C = A X^T;
  * with B holding the transposed tiles of a factor L, C = A L. */
@@ -469,5 +301,5 @@ void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB,
     const int bpt = ts / XG_TG_BM;
     const long long jobs = (long long)mt * nt;
     xg_tile_gemm_kernel<<<(unsigned)(jobs * bpt * bpt), XG_TG_THREADS, xg_tile_gemm_smem_bytes(), st>>>(
-        mapA, mapB, C, nt, ts, XG_TG_RTRI, 0, mt, status);
+        mapA, mapB, C, nt, ts, mt, status);
 }

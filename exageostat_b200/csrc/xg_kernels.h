@@ -342,8 +342,6 @@ void xg_launch_bessel(const double *nu, const double *x, int n, double *out, cud
 cudaError_t xg_gradient_kernels_configure();
 /* zeros the diagonal tiles of a lower-tile store */
 void xg_launch_zero_diag(double *X, int nt, int ts, cudaStream_t st);
-void xg_launch_rhs_backward_solve(const CUtensorMap &mapR, double *R, int mt, const CUtensorMap &mapLT,
-                                  const double *LT, int nt, int ts, int *status, cudaStream_t st);
 void xg_launch_rhs_tri_product(const CUtensorMap &mapA, const CUtensorMap &mapB, double *C, int mt, int nt, int ts,
                                int *status, cudaStream_t st);
 long long xg_grad_contract_blocks(long long ntiles, int ts);
@@ -355,6 +353,8 @@ void xg_launch_grad_contract(const double *S, const int2 *tile_ij, long long nti
 void xg_launch_cross_gen_r(double *D, int mt, int nt, int ts, const double *xm, const double *ym, int nmiss,
                            const double *xo, const double *yo, int nobs, const XgMaternParams &p, int metric,
                            cudaStream_t st);
+void xg_launch_reverse_factor(double *L, const int2 *ij, double *dinv, int nt, int ts, int used, cudaStream_t st);
+void xg_launch_reverse_columns(double *dst, const double *src, int mt, int nt, int ts, cudaStream_t st);
 void xg_launch_tile_transpose(double *D, long long ntiles, int ts, cudaStream_t st);
 void xg_launch_mloe_terms(const double *A, const double *U, const double *T, const double *V, int mt, int nt, int ts,
                           int nmiss, double sigma2_t, double sigma2_a, double *terms, cudaStream_t st);

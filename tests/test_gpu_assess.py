@@ -92,6 +92,20 @@ def test_mloe_mmom_matches_oracle(gpu, ora, nobs, nmiss, ts, truth, est, kernel)
     assert np.all(times > 0)
 
 
+@pytest.mark.parametrize("nobs,nmiss,ts", [(100, 5, 512), (128, 128, 128), (129, 130, 128), (383, 40, 384),
+                                           (513, 200, 512), (1024, 129, 256), (1153, 64, 384)])
+def test_mloe_mmom_block_edges(gpu, ora, nobs, nmiss, ts):
+    """The backward solve runs on the reversed factor, whose padding comes
+    first: filled blocks, one row past, a tile of padding blocks.  The bar of
+    the file."""
+    truth, est = [1.2, 0.1, 0.6], [1.0, 0.12, 0.7]
+    xm, ym, xo, yo = _split(ora, nobs + nmiss, nmiss, 6)
+    mloe, mmom, terms, _ = gpu.mloe_mmom_host(xm, ym, xo, yo, truth, est, ts=ts)
+    mo, mmo, to = ora.mloe_mmom(xm, ym, xo, yo, truth, est, 0)
+    assert np.abs(terms[:, :4] - to[:, :4]).max() < 1e-9 * truth[0]
+    assert abs(mloe - mo) < 1e-8 and abs(mmom - mmo) < 1e-8
+
+
 def test_mloe_mmom_identities_on_gpu(gpu, ora):
     xm, ym, xo, yo = _split(ora, 1200, 150, 7)
     theta = [1.3, 0.1, 0.7]
