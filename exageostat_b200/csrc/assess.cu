@@ -578,7 +578,7 @@ int xg_assess_create(XgAssess **out, int nmiss, int nobs, int ts)
         const XgPart parts[] = {{&q->R[0], rsize}, {&q->R[1], rsize}, {&q->R[2], rsize}, {&q->R[3], rsize},
                                 {&q->R[4], rsize}, {&q->xo, Np}, {&q->yo, Np}, {&q->xm, (size_t)nmiss},
                                 {&q->ym, (size_t)nmiss}, {&q->terms, 6 * (size_t)nmiss},
-                                {&q->part, 2 * Np / XG_DAG_BLOCK}, {&q->status, 2}, {&q->words, (size_t)(2 + flags)}};
+                                {&q->part, 4 * Np / XG_DAG_BLOCK}, {&q->status, 2}, {&q->words, (size_t)(2 + flags)}};
         cudaError_t e = xg_alloc_parts(parts, 13);
         /* on the stream that fills them: the default stream does not wait for it, nor it for that */
         if (e == cudaSuccess)
@@ -637,8 +637,7 @@ int xg_assess_run(XgAssess *q, const double *truth, const double *est, int kerne
     fs.st_hi = g_xg.stream_hi;
     fs.ev_panel = q->ev_panel;
     fs.ev_upd = q->ev_upd;
-    xg_factor_lookahead(q->Ca, nullptr, q->part, q->status, q->status + 1, fs);
-    xg_factor_lookahead(q->Ct, nullptr, q->part, q->status, q->status + 1, fs);
+    xg_factor_two(q->Ca, q->Ct, q->part, q->part + 2 * (size_t)nt * ts / XG_DAG_BLOCK, q->status, q->status + 1, fs);
     XG_ACU(cudaEventRecord(q->ev[2], st));
     /* the per-point solves (:1300-1364) for all points */
     {

@@ -333,7 +333,7 @@ static bool xg_i8_prepare_inverse(XgTileMatrix &M);
  * (0, nb), or one window of it (words: its next-task word; the flags of the
  * whole matrix were cleared when the factorisation began). */
 static void xg_launch_dag_columns(XgTileMatrix &M, int J0, int J1, int *next, double *v, double *part, int *status,
-                                  cudaStream_t st)
+                                  int ctas, cudaStream_t st)
 {
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     if (J1 > nb) J1 = nb;
@@ -351,7 +351,7 @@ static void xg_launch_dag_columns(XgTileMatrix &M, int J0, int J1, int *next, do
     G.v = v;
     G.part = part;
     G.status = status;
-    xg_launch_dag(M.map, G, g_xg.sm_count, st);
+    xg_launch_dag(M.map, G, ctas, st);
 }
 
 /* Smallest dimension whose FP64 factorisation runs its updates on the INT8
@@ -365,11 +365,11 @@ static int xg_i8_min(int ts) { return ts >= 512 ? 6500 : ts >= 384 ? 8000 : ts >
 
 /* The factorisation of M as one launch of the tile DAG (tile_dag.cu); returns
  * the number of partial sums of either kind. */
-static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, cudaStream_t st)
+static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, int ctas, cudaStream_t st)
 {
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
-    xg_launch_dag_columns(M, 0, nb, M.dag, v, part, status, st);
+    xg_launch_dag_columns(M, 0, nb, M.dag, v, part, status, ctas, st);
     return nb;
 }
 
@@ -502,7 +502,7 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
             M.i8_factor = true;
             return xg_factor_sliced(M, M.i8, v, part, status, fs);
         }
-        if (M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, fs.st);
+        if (M.N <= XG_DAG_MAX_N) return xg_factor_dag(M, v, part, status, g_xg.sm_count, fs.st);
     }
     XgTileArgs T{M.d, M.ts, M.nt};
     const bool la = fs.st_hi != nullptr;
@@ -540,6 +540,30 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
         if (pev) cudaEventRecord(pev[5 * k + 4], fs.st);
     }
     return M.nt;
+}
+
+/* The factorisations of two matrices of one size, without right-hand sides.
+ * Up to the INT8 path's sizes they run side by side on half the SMs each: a
+ * matrix of 4000 is bound by its chain of diagonal blocks (1.50 ms; its
+ * products would take 0.6).  Both, one after the other / side by side in ms: N =
+ * 300 0.24 / 0.12, 1000 0.70 / 0.35, 4000 3.00 / 2.04, 9000 13.0 / 12.3.  The
+ * launches do not wait on one another. */
+void xg_factor_two(XgTileMatrix &A, XgTileMatrix &B, double *part_a, double *part_b, int *status, int *info,
+                   const XgFactorStreams &fs)
+{
+    if (!A.dag || !B.dag || !fs.st_hi || A.N > XG_DAG_MAX_N || A.N >= xg_i8_min(A.ts)) {
+        xg_factor_lookahead(A, nullptr, part_a, status, info, fs);
+        xg_factor_lookahead(B, nullptr, part_b, status, info, fs);
+        return;
+    }
+    const int half = g_xg.sm_count / 2;
+    A.i8_factor = B.i8_factor = false;
+    cudaEventRecord(fs.ev_upd, fs.st); /* the generated matrices */
+    cudaStreamWaitEvent(fs.st_hi, fs.ev_upd, 0);
+    xg_factor_dag(B, nullptr, part_b, status, g_xg.sm_count - half, fs.st_hi);
+    xg_factor_dag(A, nullptr, part_a, status, half, fs.st);
+    cudaEventRecord(fs.ev_panel, fs.st_hi);
+    cudaStreamWaitEvent(fs.st, fs.ev_panel, 0);
 }
 
 int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st, cudaEvent_t *pev)
@@ -1483,7 +1507,7 @@ static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *pa
                 update(c, 1, a, c, la && b < nt ? (dyn ? all : xg_panel_share(a, sms)) : sms, sp);
             }
             rec(c, 1, sp);
-            xg_launch_dag_columns(M, c * bpt, (c + 1) * bpt, windows + c, v, part, status, sp);
+            xg_launch_dag_columns(M, c * bpt, (c + 1) * bpt, windows + c, v, part, status, sms, sp);
             rec(c, 2, sp);
             if (c + 1 < nt) xg_launch_slice_panel(T, c, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, sp);
             rec(c, 3, sp);

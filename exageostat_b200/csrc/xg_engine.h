@@ -137,6 +137,8 @@ int xg_check_theta(const double *theta, int kernel);
 int xg_factor(XgTileMatrix &M, double *v, double *part, int *status, int *info, cudaStream_t st,
               cudaEvent_t *pev = nullptr);
 int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, int *info, const XgFactorStreams &fs);
+void xg_factor_two(XgTileMatrix &A, XgTileMatrix &B, double *part_a, double *part_b, int *status, int *info,
+                   const XgFactorStreams &fs);
 int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits);
 bool xg_i8_release(XgTileMatrix &M);
 void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st);
