@@ -170,18 +170,6 @@ __global__ void __launch_bounds__(256) xg_gen_matern_kernel(XgTileArgs T, const 
 }
 
 /* ========================================================================== */
-/* Loads of tile data.  COH = false: ordinary loads (the data was written by   */
-/* an earlier launch).  COH = true: the bodies run inside the persistent       */
-/* scheduler, where other CTAs of the same launch wrote the data: the loads go */
-/* to L2 (ld.global.cg), never to a line this SM's L1 kept from an earlier     */
-/* task.                                                                      */
-/* ========================================================================== */
-
-template <bool COH> __device__ __forceinline__ double xg_ldt(const double *p) { return COH ? __ldcg(p) : *p; }
-template <bool COH> __device__ __forceinline__ double2 xg_ldt2(const double2 *p) { return COH ? __ldcg(p) : *p; }
-template <bool COH> __device__ __forceinline__ double xg_ldro(const double *p) { return COH ? __ldcg(p) : __ldg(p); }
-
-/* ========================================================================== */
 /* POTRF of a diagonal tile, fused with log-det and the z block solve         */
 /* ========================================================================== */
 
@@ -194,7 +182,7 @@ template <bool COH> __device__ __forceinline__ double xg_ldro(const double *p) {
  * lds), by all threads of the CTA with U loads in flight per thread before
  * any store (the loads of a plain loop would wait one by one where the
  * compiler cannot tell dst and src apart). */
-template <bool COH, int U = 8>
+template <int U = 8>
 __device__ __forceinline__ void xg_stage_rows(double *dst, int ldd, const double *src, long long lds, int rows,
                                               int cols)
 {
@@ -206,7 +194,7 @@ __device__ __forceinline__ void xg_stage_rows(double *dst, int ldd, const double
             const int idx = base + u * step;
             if (idx < total) {
                 const int r = idx / cols, c = idx - r * cols;
-                t[u] = xg_ldt<COH>(src + (long long)r * lds + c);
+                t[u] = src[(long long)r * lds + c];
             }
         }
 #pragma unroll
@@ -220,59 +208,15 @@ __device__ __forceinline__ void xg_stage_rows(double *dst, int ldd, const double
     }
 }
 
-/* Cholesky of the NB x NB block at P (leading dimension LDP, NB <= 32) by one
- * warp, lane r holding the part of row r still to be factored in registers:
- * at step j, w[t] is element (r, j + t), so the pivot column is always w[0]
- * and the loop over j stays rolled (one copy of the square root and the
- * division).  Per step the pivot is broadcast from lane j, the column is
- * scaled by the reciprocal of its square root (as LAPACK's dpotf2 scales by
- * ONE / AJJ) and stored, the lower trailing elements are updated with the
- * column's entries broadcast lane by lane, and the window shifts by one.
- * Writes L (zeros above the diagonal) back to P and 1 / L_jj to rdiag[j],
- * adds log L_rr to lane r's logdet; returns the first column (1-based) whose
- * pivot is not positive, or 0, the same value in every lane. */
+/* Cholesky of the NB x NB block at P (leading dimension LDP, NB <= 32; shared
+ * memory) by one warp: lane r updates row r in place (512 threads leave 128
+ * registers each, too few for a 32-double row).  Per step the column is scaled
+ * by the reciprocal of the pivot's square root (as LAPACK's dpotf2 scales by
+ * ONE / AJJ).  Writes L (zeros above the diagonal) back to P and 1 / L_jj to
+ * rdiag[j], adds log L_jj to lane j's logdet; returns the first column
+ * (1-based) whose pivot is not positive, or 0, the same value in every lane. */
 template <int NB, int LDP>
 __device__ __forceinline__ int xg_chol_warp(double *P, int lane, double &logdet_lane, double *rdiag)
-{
-    double w[NB];
-    const bool act = lane < NB;
-#pragma unroll
-    for (int c = 0; c < NB; ++c) w[c] = act ? P[lane * LDP + c] : 0.0;
-    int fail = 0;
-#pragma unroll 1
-    for (int j = 0; j < NB; ++j) {
-        double d = __shfl_sync(0xffffffffu, w[0], j);
-        if (!(d > 0.0)) {
-            if (!fail) fail = j + 1;
-            d = 1.0;
-        }
-        const double ljj = sqrt(d);
-        const double rj = 1.0 / ljj;
-        const double l = lane == j ? ljj : w[0] * rj; /* L(lane, j) for lane >= j */
-        if (lane == j) rdiag[j] = rj;
-        if (act && lane >= j) P[lane * LDP + j] = l;
-#pragma unroll
-        for (int t = 1; t < NB; ++t) {
-            const double lcj = __shfl_sync(0xffffffffu, l, (j + t) & 31);
-            if (t < NB - j && lane >= j + t) w[t] = fma(-l, lcj, w[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < NB - 1; ++t) w[t] = w[t + 1];
-        w[NB - 1] = 0.0;
-    }
-    if (act) {
-        for (int c = lane + 1; c < NB; ++c) P[lane * LDP + c] = 0.0;
-        logdet_lane += log(P[lane * LDP + lane]);
-    }
-    return fail;
-}
-
-/* The same factorisation with the block left in shared memory (lane r
- * updates row r in place), for kernels launched with 512 threads whose
- * 128-register budget cannot hold a 32-double row: same results, same
- * return value. */
-template <int NB, int LDP>
-__device__ __forceinline__ int xg_chol_warp_smem(double *P, int lane, double &logdet_lane, double *rdiag)
 {
     int fail = 0;
     for (int j = 0; j < NB; ++j) {
@@ -310,7 +254,7 @@ __device__ __forceinline__ int xg_chol_warp_smem(double *P, int lane, double &lo
  * pivot sets XG_ST_NOT_SPD and info = col0 + its 1-based column, and the call
  * returns false (CTA-uniformly).  *logdet_out = sum log L_ii, *dot_out = |vk|^2
  * after the solve (thread 0 / warp 0 write them). */
-template <int NB, bool COH, bool REGCHOL = false>
+template <int NB>
 __device__ __forceinline__ bool xg_potrf_block(double *A, int n, int lda, double *vk, int with_rhs, long long col0,
                                                int *status, int *info, double *logdet_out, double *dot_out,
                                                double *P, double *vs)
@@ -326,17 +270,16 @@ __device__ __forceinline__ bool xg_potrf_block(double *A, int n, int lda, double
         s_logdet = 0.0;
     }
     if (with_rhs)
-        for (int r = tid; r < ts; r += blockDim.x) vs[r] = xg_ldt<COH>(vk + r);
+        for (int r = tid; r < ts; r += blockDim.x) vs[r] = vk[r];
     double logdet_lane = 0.0;
     for (int c0 = 0; c0 < ts; c0 += NB) {
         const int rows = ts - c0;
         __syncthreads();
-        xg_stage_rows<COH>(P, LDP, A + (long long)c0 * lda + c0, lda, rows, NB);
+        xg_stage_rows(P, LDP, A + (long long)c0 * lda + c0, lda, rows, NB);
         __syncthreads();
-        /* unblocked Cholesky of the NB x NB diagonal block (warp 0, in registers) */
+        /* unblocked Cholesky of the NB x NB diagonal block (warp 0) */
         if (warp == 0) {
-            const int f = REGCHOL ? xg_chol_warp<NB, LDP>(P, lane, logdet_lane, s_rdiag)
-                                  : xg_chol_warp_smem<NB, LDP>(P, lane, logdet_lane, s_rdiag);
+            const int f = xg_chol_warp<NB, LDP>(P, lane, logdet_lane, s_rdiag);
             if (f && lane == 0) s_fail = c0 + f;
         }
         __syncthreads();
@@ -440,7 +383,7 @@ __device__ __forceinline__ bool xg_potrf_block(double *A, int n, int lda, double
                             const int rr = r0 + mi * 16 + g + 8 * h;
                             if (rr < R && cc < R) {
                                 double2 *pc = reinterpret_cast<double2 *>(At + (long long)rr * lda + cc);
-                                double2 cv = xg_ldt2<COH>(pc);
+                                double2 cv = *pc;
                                 cv.x -= acc[mi][ni][2 * h];
                                 cv.y -= acc[mi][ni][2 * h + 1];
                                 *pc = cv;
@@ -477,7 +420,7 @@ __device__ __forceinline__ bool xg_potrf_block(double *A, int n, int lda, double
     return true;
 }
 
-template <int NB, bool COH = false, bool REGCHOL = false>
+template <int NB>
 __device__ __forceinline__ void xg_potrf_body(const XgTileArgs &T, int k, double *__restrict__ v,
                                               double *__restrict__ part_logdet, double *__restrict__ part_dot,
                                               int with_rhs, int *status, int *info)
@@ -488,8 +431,8 @@ __device__ __forceinline__ void xg_potrf_body(const XgTileArgs &T, int k, double
     double *A = T.data + xg_slot64(T, k, k) * (long long)ts * ts;
     double *P = xg_smem_d;                     /* [ts][NB + 4] */
     double *vs = P + (size_t)ts * (NB + 4);    /* [ts] */
-    xg_potrf_block<NB, COH, REGCHOL>(A, ts, ts, v + (long long)k * ts, with_rhs, (long long)k * ts, status, info,
-                            part_logdet + k, part_dot + k, P, vs);
+    xg_potrf_block<NB>(A, ts, ts, v + (long long)k * ts, with_rhs, (long long)k * ts, status, info, part_logdet + k,
+                       part_dot + k, P, vs);
 }
 
 template <int NB>
@@ -500,29 +443,6 @@ __global__ void __launch_bounds__(XG_POTRF_THREADS) xg_potrf_diag_kernel(XgTileA
 {
     xg_potrf_body<NB>(T, k, v, part_logdet, part_dot, with_rhs, status, info);
 }
-
-/* ========================================================================== */
-/* Inverses of the 32 x 32 diagonal blocks of L_kk (for the panel TRSM)       */
-/* ========================================================================== */
-
-/* One warp inverts the 32 x 32 lower-triangular block LB (shared memory,
- * row stride 33): lane c forms column c by forward substitution,
- * z_i = (delta_ic - sum_{q<i} L_iq z_q) / L_ii, and stores D[i * 32 + c] = z_i.
- * The per-field and the batched paths share this arithmetic exactly. */
-__device__ __forceinline__ void xg_lower32_inverse(const double *LB, int lane, double *D)
-{
-    double z[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        double s = (i == lane) ? 1.0 : 0.0;
-#pragma unroll
-        for (int q = 0; q < i; ++q) s -= LB[i * 33 + q] * z[q];
-        z[i] = s / LB[i * 33 + i];
-    }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) D[i * 32 + lane] = z[i];
-}
-
 
 /* ========================================================================== */
 /* Panel TRSM: L_ik = A_ik L_kk^-T, fused with v_i -= L_ik v_k                */
@@ -541,7 +461,6 @@ __device__ __forceinline__ void xg_lower32_inverse(const double *LB, int lane, d
  * (32 fragments a thread) before its 64 DMMAs, so the L2 latency is paid
  * once per group.  With vk != nullptr also vi[0:32] -= B_new vk[0:w].
  * Called by every CTA thread after the status check. */
-template <bool COH>
 __device__ __forceinline__ void xg_trsm_core(double *B, const double *L, int ld, int w, const double *dinv,
                                              const double *vk, double *vi)
 {
@@ -552,14 +471,14 @@ __device__ __forceinline__ void xg_trsm_core(double *B, const double *L, int ld,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nwarps = (int)(blockDim.x >> 5);
     const int g = lane >> 2, tq = lane & 3;
-    xg_stage_rows<COH>(S, LDS, B, ld, XG_TRSM_SR, w);
-    if (dinv) xg_stage_rows<COH, 4>(LDb, 33, dinv, 32, 32, 32);
+    xg_stage_rows(S, LDS, B, ld, XG_TRSM_SR, w);
+    if (dinv) xg_stage_rows<4>(LDb, 33, dinv, 32, 32, 32);
     for (int cb = 0, b = 0; cb < w; cb += 32, ++b) {
         double *LD = LDb + (b & 1) * (32 * 33);
         if (!dinv) {
             for (int idx = tid; idx < 32 * 32; idx += blockDim.x) {
                 const int r = idx >> 5, c = idx & 31;
-                LD[r * 33 + c] = xg_ldt<COH>(L + (long long)(cb + r) * ld + cb + c);
+                LD[r * 33 + c] = L[(long long)(cb + r) * ld + cb + c];
             }
         }
         __syncthreads();
@@ -587,7 +506,7 @@ __device__ __forceinline__ void xg_trsm_core(double *B, const double *L, int ld,
                 double *LN = LDb + ((b + 1) & 1) * (32 * 33);
                 for (int idx = tid - 128; idx < 32 * 32; idx += (int)blockDim.x - 128) {
                     const int r = idx >> 5, c = idx & 31;
-                    LN[r * 33 + c] = xg_ldt<COH>(dinv + (cb + 32 + r) * 32 + c);
+                    LN[r * 33 + c] = dinv[(cb + 32 + r) * 32 + c];
                 }
             }
             __syncthreads();
@@ -625,7 +544,8 @@ __device__ __forceinline__ void xg_trsm_core(double *B, const double *L, int ld,
 #pragma unroll
             for (int p = 0; p < 8; ++p)
 #pragma unroll
-                for (int ni = 0; ni < 4; ++ni) bl[p][ni] = xg_ldro<COH>(L + (long long)(c0 + ni * 8 + g) * ld + cb + p * 4 + tq);
+                for (int ni = 0; ni < 4; ++ni)
+                    bl[p][ni] = __ldg(L + (long long)(c0 + ni * 8 + g) * ld + cb + p * 4 + tq);
             double acc[2][4][4];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
@@ -668,14 +588,13 @@ __device__ __forceinline__ void xg_trsm_core(double *B, const double *L, int ld,
     if (vk) {
         for (int r = warp; r < XG_TRSM_SR; r += nwarps) {
             double s = 0.0;
-            for (int c = lane; c < w; c += 32) s += S[r * LDS + c] * xg_ldt<COH>(vk + c);
+            for (int c = lane; c < w; c += 32) s += S[r * LDS + c] * vk[c];
             for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if (lane == 0) vi[r] = xg_ldt<COH>(vi + r) - s;
+            if (lane == 0) vi[r] -= s;
         }
     }
 }
 
-template <bool COH = false>
 __device__ __forceinline__ void xg_trsm_body(const XgTileArgs &T, int k, double *__restrict__ v, int with_rhs,
                                              const int *status, long long bid)
 {
@@ -686,7 +605,7 @@ __device__ __forceinline__ void xg_trsm_body(const XgTileArgs &T, int k, double 
     const int strip = (int)(bid % strips);
     double *B = T.data + xg_slot64(T, i, k) * (long long)ts * ts + (long long)strip * XG_TRSM_SR * ts;
     const double *L = T.data + xg_slot64(T, k, k) * (long long)ts * ts;
-    xg_trsm_core<COH>(B, L, ts, ts, T.dinv, with_rhs ? v + (long long)k * ts : nullptr,
+    xg_trsm_core(B, L, ts, ts, T.dinv, with_rhs ? v + (long long)k * ts : nullptr,
                       with_rhs ? v + (long long)i * ts + strip * XG_TRSM_SR : nullptr);
 }
 
@@ -717,7 +636,8 @@ __global__ void __launch_bounds__(XG_TRSM_THREADS, 1) xg_trsm_panel_kernel(XgTil
 /* One 128 x 128 block C -= A B^T on DMMA: A and B are 128-row boxes of the
  * TMA tensor `map` starting at rows rowA and rowB, K runs over KT 16-wide
  * slabs from column kx0 (a multiple of 16), C has leading dimension ldc.
- * Called by every CTA thread; the caller has done the status check. */
+ * Called by every CTA thread; the caller has done the status check.  COH: the
+ * CTA itself wrote A or C with ordinary stores in this launch, and calls again. */
 template <bool COH>
 __device__ __forceinline__ void xg_gemm_core(const CUtensorMap &map, int rowA, int rowB, int kx0, int KT,
                                              double *C, int ldc, int *status)
@@ -745,8 +665,7 @@ __device__ __forceinline__ void xg_gemm_core(const CUtensorMap &map, int rowA, i
         __syncthreads();
     }
     if (tid == 0) {
-        /* the operand tiles may have been written by other CTAs of this launch
-         * through ordinary stores: order them before the async-proxy reads */
+        /* order this CTA's own stores before the async-proxy reads */
         if (COH) asm volatile("fence.proxy.async.global;" ::: "memory");
         xg_prefetch_tensormap(&map);
         for (; issued < XG_G_STAGES && issued < KT; ++issued) {
@@ -769,7 +688,8 @@ __device__ __forceinline__ void xg_gemm_core(const CUtensorMap &map, int rowA, i
             for (int h = 0; h < 2; ++h) {
                 const int r = wm * 64 + mi * 16 + g + 8 * h;
                 const int c = wn * 32 + ni * 8 + 2 * tq;
-                const double2 cv = xg_ldt2<COH>(reinterpret_cast<const double2 *>(C + (long long)r * ldc + c));
+                const double2 *at = reinterpret_cast<const double2 *>(C + (long long)r * ldc + c);
+                const double2 cv = COH ? __ldcg(at) : *at;
                 acc[mi][ni][2 * h] = -cv.x;
                 acc[mi][ni][2 * h + 1] = -cv.y;
             }
@@ -862,7 +782,6 @@ __device__ __forceinline__ void xg_gemm_core(const CUtensorMap &map, int rowA, i
             }
 }
 
-template <bool COH = false>
 __device__ __forceinline__ void xg_gemm_body(const CUtensorMap &map, const XgTileArgs &T, int k, int j0,
                                              int single_col, int *status, long long bid)
 {
@@ -896,7 +815,7 @@ __device__ __forceinline__ void xg_gemm_body(const CUtensorMap &map, const XgTil
     const int rowB = T.band ? j * ts + bj * XG_G_BM
                             : (int)((T.tile_off + xg_tile_index(j, k, T.nt)) * ts + bj * XG_G_BM);
     double *C = T.data + xg_slot64(T, i, j) * (long long)ts * ts + (long long)(bi * XG_G_BM) * ts + bj * XG_G_BM;
-    xg_gemm_core<COH>(map, rowA, rowB, 0, ts / XG_G_BK, C, ts, status);
+    xg_gemm_core<false>(map, rowA, rowB, 0, ts / XG_G_BK, C, ts, status);
 }
 
 __global__ void __launch_bounds__(XG_G_THREADS, 1) xg_syrk_gemm_kernel(const __grid_constant__ CUtensorMap map,
@@ -924,7 +843,6 @@ __global__ void __launch_bounds__(XG_G_THREADS, 1) xg_syrk_gemm_kernel(const __g
  * strip TRSM up to the order of the sums: the solves use the same 32 x 32
  * inverses.  Fused: v_i -= L_ik v_k for the block's rows. */
 #define XG_TB 128                                           /* rows of A_ik per CTA, columns per block */
-#define XG_TB_S_BYTES ((size_t)XG_TB * XG_TB * sizeof(double)) /* the block, swizzled: fits the GEMM ring */
 
 /* element (r, c) of the 128 x 128 staged block: each group of four rows is
  * shifted by a different multiple of four columns, so a DMMA fragment read
@@ -935,12 +853,11 @@ __device__ __forceinline__ int xg_tb_idx(int r, int c) { return r * XG_TB + (c ^
  * L the 128 x 128 lower block (global, leading dimension ld), dinv its four
  * inverted 32 x 32 diagonal blocks ([(32 b + r) * 32 + c]); LDb: 2 x 32 x 33
  * doubles of shared memory.  256 threads. */
-template <bool COH>
 __device__ __forceinline__ void xg_block_trsm128(double *S, double *LDb, const double *L, int ld, const double *dinv)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    xg_stage_rows<COH, 4>(LDb, 33, dinv, 32, 32, 32);
+    xg_stage_rows<4>(LDb, 33, dinv, 32, 32, 32);
     for (int cb = 0; cb < XG_TB / 32; ++cb) {
         const double *LD = LDb + (cb & 1) * (32 * 33);
         /* the next block's inverse, loaded now and stored after the barrier */
@@ -950,7 +867,7 @@ __device__ __forceinline__ void xg_block_trsm128(double *S, double *LDb, const d
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int idx = tid + u * 256;
-                nd[u] = xg_ldt<COH>(dinv + (long long)(cb + 1) * 32 * 32 + idx);
+                nd[u] = dinv[(long long)(cb + 1) * 32 * 32 + idx];
             }
         __syncthreads(); /* S and LD[cb & 1] are complete */
         /* S[:, 32 cb : 32 cb + 32] <- that block D^T: warp w, rows 16 w .. + 15 */
@@ -995,7 +912,7 @@ __device__ __forceinline__ void xg_block_trsm128(double *S, double *LDb, const d
             for (int p = 0; p < 8; ++p)
 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni)
-                    bl[p][ni] = xg_ldro<COH>(L + (long long)(c0 + ni * 8 + g) * ld + 32 * cb + 4 * p + tq);
+                    bl[p][ni] = __ldg(L + (long long)(c0 + ni * 8 + g) * ld + 32 * cb + 4 * p + tq);
             double ac[2][4][4];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
@@ -1035,9 +952,7 @@ __device__ __forceinline__ void xg_block_trsm128(double *S, double *LDb, const d
 
 /* The TRSM of the 128-row block rb of panel tile (i, k); called by all 256
  * threads of a CTA after its status check.  Returns false (CTA-uniformly)
- * when a GEMM wait timed out.  Under the device scheduler (COH) the tiles and
- * inverses were written by other CTAs of the launch. */
-template <bool COH>
+ * when a GEMM wait timed out. */
 __device__ __forceinline__ bool xg_trsm_gemm_body(const CUtensorMap &map, const XgTileArgs &T, int k, int i, int rb,
                                                   double *v, int with_rhs, int *status)
 {
@@ -1081,7 +996,7 @@ __device__ __forceinline__ bool xg_trsm_gemm_body(const CUtensorMap &map, const 
                 }
             }
         }
-        xg_block_trsm128<COH>(S, LDb, Lkk + (long long)(c * XG_TB) * ts + c * XG_TB, ts,
+        xg_block_trsm128(S, LDb, Lkk + (long long)(c * XG_TB) * ts + c * XG_TB, ts,
                               T.dinv + (long long)(c * XG_TB) * 32);
         /* X_c back to the tile; v_i -= X_c v_k[c block] (row sums per warp) */
         for (int idx = tid; idx < XG_TB * XG_TB / 2; idx += 256) {
@@ -1101,7 +1016,7 @@ __device__ __forceinline__ bool xg_trsm_gemm_body(const CUtensorMap &map, const 
     }
     if (with_rhs) {
         double *vi = v + (long long)i * ts + rb * XG_TB;
-        for (int r = tid; r < XG_TB; r += blockDim.x) vi[r] = xg_ldt<COH>(vi + r) - vacc[r];
+        for (int r = tid; r < XG_TB; r += blockDim.x) vi[r] -= vacc[r];
     }
     return true;
 }
@@ -1112,7 +1027,7 @@ __global__ void __launch_bounds__(XG_G_THREADS, 1)
 {
     if (xg_cta_should_skip(status)) return;
     const int nb = T.ts / XG_TB;
-    xg_trsm_gemm_body<false>(map, T, k, k + 1 + (int)blockIdx.x / nb, (int)blockIdx.x % nb, v, with_rhs, status);
+    xg_trsm_gemm_body(map, T, k, k + 1 + (int)blockIdx.x / nb, (int)blockIdx.x % nb, v, with_rhs, status);
 }
 
 static size_t xg_trsm_gemm_smem_bytes()
@@ -1217,7 +1132,7 @@ __global__ void __launch_bounds__(XG_TRSM_THREADS, 1) xg_potrf_sub_trsm_kernel(X
     const int row = r0 + XG_SUB + (int)blockIdx.x * XG_TRSM_SR;
     double *A = T.data + xg_slot64(T, k, k) * (long long)ts * ts;
     double *vk = with_rhs ? v + (long long)k * ts : nullptr;
-    xg_trsm_core<false>(A + (long long)row * ts + r0, A + (long long)r0 * ts + r0, ts, XG_SUB,
+    xg_trsm_core(A + (long long)row * ts + r0, A + (long long)r0 * ts + r0, ts, XG_SUB,
                         T.dinv ? T.dinv + (long long)r0 * 32 : nullptr, vk ? vk + r0 : nullptr,
                         vk ? vk + row : nullptr);
 }

@@ -56,8 +56,7 @@
 #define XG_SL_BM 128 /* C rows per job (rows of the A operand, the MMA's N) */
 #define XG_SL_BN 128 /* C columns per job (rows of the B operand, the MMA's M) */
 #define XG_SL_BK 64  /* int8 per 64-byte swizzled row */
-#define XG_SL_SLICES 4
-#define XG_SL_LEVELS 4 /* level sums |L_t| <= (t + 1) 127^2 ts stay exact in S32 */
+#define XG_SL_SLICES 4 /* digits of the first pass; its level sums |L_t| <= (t + 1) 127^2 ts are exact in S32 */
 #define XG_SL_EPI_WARPS 8
 #define XG_SL_THREADS 384 /* warpgroup 0: TMA, MMA, 2 idle warps; warpgroups 1-2: epilogue */
 /* register split (setmaxnreg): launched at 168 per thread (64,512 in all);
