@@ -376,68 +376,216 @@ static int xg_factor_dag(XgTileMatrix &M, double *v, double *part, int *status, 
 static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits);
 static void xg_digits_free(XgDigits &D);
 
-/* X = L^-T tile column by tile column -- the update from the finished columns
- * (INT8, from the digit planes of X and L), the FP64 block solves with L_bb
- * (one dataflow launch), the slicing of column b -- then S = X X^T over the
- * factor in one launch.  (Overlapping the solve and slicing of column b with
- * the update of column b + 1 on two streams, as the factorisation does,
- * measured the same at N = 100 000: the update dominates each column.) */
-static void xg_inverse_product_sliced(XgTileMatrix &M, XgTileMatrix &X, XgSliced *sl, int *status, cudaStream_t st)
+/* SMs left free by the persistent trailing-update kernels (one CTA per SM,
+ * ~197 KB of shared memory each) while the lookahead panel of the next step
+ * (POTRF, TRSM, panel conversion) runs on the high-priority stream: resident
+ * CTAs are never preempted, so without free SMs the panel would wait for the
+ * whole update. */
+#define XG_PANEL_SMS 16
+
+/* Tile columns per group.  One column gives an update 16 (nt - j) jobs of 128
+ * x 128, whose last round leaves most of the persistent CTAs idle: counted
+ * over the columns 1.7 x the even distribution at 38 tile columns, 1.36 x at
+ * 79, 1.24 x at 137; groups of four bring that to 1.21, 1.09 and 1.05, but put
+ * three columns' panels between two updates, which the short matrices have
+ * nothing to run beside.  Log-likelihood in ms, tiles of 512, K = 4 below:
+ *   7 digits   N = 8200  10000  14000  20000  28000  40000
+ *     G = 1        6.00   8.80     -    46.6     -    316
+ *     G = 2        5.71   7.98   17.9   44.7   109    308
+ *     G = 3        6.13   8.17   16.6   42.2   107    305
+ *     G = 4        6.52   8.81   17.3   41.1   105    298
+ *   4 digits   N = 9000  20000  40000  70000
+ *     G = 1        5.00   20.2    117   560
+ *     G = 2        5.02   20.1    119   574
+ *     G = 3        5.20   21.4    118   573
+ * (28 pairs cost an update 2.8 times what ten do, the panels the same: the
+ * four-digit form has the panels to hide, not the last rounds.) */
+static int xg_sl_group(int nt, int digits)
+{
+    return digits == 4 ? 1 : nt < 24 ? 2 : nt < 36 ? 3 : 4;
+}
+
+static XgSlTask xg_sl_task(int mode, int col, int ncol, int k0, int k1)
+{
+    XgSlTask S;
+    S.mode = mode;
+    S.col = col;
+    S.ncol = ncol;
+    S.k0 = k0;
+    S.k1 = k1;
+    S.sign = mode == XG_SL_SYRK ? 1.0 : -1.0;
+    return S;
+}
+
+/* SMs left to the panels of the group that begins at tile column a while U1 of
+ * the next group runs on the others.  Per target tile the panels cost the DMMA
+ * flops of the TRSM and the group's own chunks, U1 a chunks: sms K / (K + a),
+ * clamped to [XG_PANEL_SMS, sms - XG_PANEL_SMS].  K = 4
+ * (EXAGEOSTAT_B200_PANEL_K overrides it): seven digits in groups of four at
+ * N = 10000 / 20000 / 40000 took 11.0 / 51.4 / 325 ms with K = 1, 9.9 / 46.5 /
+ * 317 with 2, 9.2 / 43.8 / 309 with 3, 8.9 / 41.6 / 308 with 4 and 8.6 / 43.6 /
+ * 311 with 6; four digits at 20000 / 70000 20.4 / 570 with 4 and 20.9 / 572
+ * with 7. */
+static int xg_panel_k()
+{
+    static int v = -1;
+    if (v < 0) {
+        const char *e = getenv("EXAGEOSTAT_B200_PANEL_K");
+        v = e ? atoi(e) : 0;
+        if (v < 1 || v > 64) v = 4;
+    }
+    return v;
+}
+
+static int xg_panel_share(int a, int sms)
+{
+    const int K = xg_panel_k();
+    int r = (int)((long long)sms * K / (K + a));
+    if (r < XG_PANEL_SMS) r = XG_PANEL_SMS;
+    if (r > sms - XG_PANEL_SMS) r = sms - XG_PANEL_SMS;
+    return r;
+}
+
+/* How the SMs are divided between the panel chain and the split update.
+ * "static" (default): the split update runs as a persistent launch on
+ * sms - xg_panel_share(a) CTAs, leaving the rest to the panel chain.
+ * "dynamic" (EXAGEOSTAT_B200_SL_SHARE=dynamic): both updates launch one CTA
+ * per job, so CTAs retire throughout the update and the hardware hands each
+ * freed SM to the pending panel kernels first (higher stream priority), the
+ * SMs the chain does not need staying with the update. */
+static bool xg_sl_dynamic_share()
+{
+    static int v = -1;
+    if (v < 0) {
+        const char *e = getenv("EXAGEOSTAT_B200_SL_SHARE");
+        v = (e && strcmp(e, "dynamic") == 0) ? 1 : 0;
+    }
+    return v == 1;
+}
+
+/* INT8 tile columns in groups of G = xg_sl_group [a, b), left-looking:
+ *   U1     chunks k < a0 (the group before begins at a0) to every target of the group (main stream,
+ *          on all but xg_panel_share SMs, beside the panels of the group before)
+ *   U2     chunks a0 <= k < a, when those panels are sliced: column a on the panel stream, the
+ *          others on the main stream
+ *   panel  per column c: chunks a <= k < c (for c > a), then panel(c)
+ * update(col, ncol, k0, k1, ctas, stream) and panel(c, stream) do the work.
+ * Profiling events (8 per column c, those of the main stream on a group's
+ * first column): panel stream before / after the column's updates, after its
+ * panel, after slicing (both panel's to record); main stream before / after U1. */
+template <class Update, class Panel>
+static void xg_sliced_groups(int nt, XgSliced *sl, const XgFactorStreams &fs, Update update, Panel panel)
+{
+    const bool la = fs.st_hi != nullptr;
+    cudaStream_t st = fs.st, sp = la ? fs.st_hi : fs.st;
+    auto rec = [&](int k, int e, cudaStream_t s) {
+        if (fs.pev) cudaEventRecord(fs.pev[8 * k + e], s);
+    };
+    const int sms = g_xg.sm_count;
+    const int G = xg_sl_group(nt, sl->L.digits);
+    const bool dyn = xg_sl_dynamic_share();
+    const int all = 1 << 30; /* one CTA per job */
+    if (la) {
+        cudaEventRecord(sl->ev_a, st); /* the matrix as it comes */
+        cudaStreamWaitEvent(sp, sl->ev_a, 0);
+    }
+    for (int a = 0; a < nt; a += G) {
+        const int b = a + G < nt ? a + G : nt, a0 = a - G;
+        const int share = dyn ? all : xg_panel_share(a, sms);
+        /* main stream: U1 of this group was issued with the group before; U2 of
+         * the columns after the first */
+        if (la && a > 0) {
+            cudaEventRecord(sl->ev_p[0], sp); /* the group before is sliced */
+            cudaEventRecord(sl->ev_a, st);    /* U1 of this group is done */
+            cudaStreamWaitEvent(st, sl->ev_p[0], 0);
+            cudaStreamWaitEvent(sp, sl->ev_a, 0);
+        }
+        if (a > 0) update(a + 1, b - a - 1, a0, a, sms, st);
+        if (la && a > 0) cudaEventRecord(sl->ev_p[1], st);
+        rec(a, 4, st);
+        const int b1 = b + G < nt ? b + G : nt; /* the next group: chunks k < a */
+        update(b, b1 - b, 0, a, !la ? sms : dyn ? all : sms - share, st);
+        rec(a, 5, st);
+        for (int c = a; c < b; ++c) {
+            rec(c, 0, sp);
+            if (c == a) {
+                /* alone in its group it runs beside U1 of the next column */
+                if (a > 0) update(a, 1, a0, a, la && G == 1 ? share : sms, sp);
+            } else {
+                if (la && a > 0 && c == a + 1) cudaStreamWaitEvent(sp, sl->ev_p[1], 0);
+                update(c, 1, a, c, la && b < nt ? share : sms, sp);
+            }
+            rec(c, 1, sp);
+            panel(c, sp);
+            rec(c, 3, sp);
+            if (c > a) {
+                rec(c, 4, st);
+                rec(c, 5, st);
+            }
+            rec(c, 6, st);
+            rec(c, 7, st);
+        }
+    }
+    if (la) {
+        cudaEventRecord(fs.ev_panel, sp);
+        cudaStreamWaitEvent(st, fs.ev_panel, 0);
+    }
+}
+
+/* X = L^-T by groups of tile columns: the updates from the finished columns
+ * (INT8, from the digit planes of X and L); a column's panel is the FP64 block
+ * solves with L_bb (one dataflow launch) and its slicing.  Then S = X X^T over
+ * the factor in one launch.  Gradients in ms, one column at a time on one
+ * stream / in groups beside the panels: seven digits N = 7000 11.1 / 9.7, 10000
+ * 22.4 / 20.0, 14000 49.3 / 46.3, 20000 132 / 131, 40000 941 / 942; four digits
+ * 9000 11.1 / 10.5, 40000 373 / 364, 70000 1814 / 1793. */
+static void xg_inverse_product_sliced(XgTileMatrix &M, XgTileMatrix &X, XgSliced *sl, int *status,
+                                      const XgFactorStreams &fs)
 {
     const int ts = M.ts, nt = M.nt, bpt = ts / XG_DAG_BLOCK;
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     XgTileArgs T{M.d, ts, nt}, TX{X.d, ts, nt};
     const long long plane = (long long)sl->X.plane_rows * ts;
     int *windows = X.dag + xg_dag_words(nb) - nb;
-    cudaMemsetAsync(X.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
-    xg_launch_zero_diag(X.d, nt, ts, st);
+    cudaMemsetAsync(X.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), fs.st);
+    xg_launch_zero_diag(X.d, nt, ts, fs.st);
     XgRowsMaps maps = {};
     maps.y[0] = X.map;
     maps.l[0] = M.map;
-    for (int b = 0; b < nt; ++b) {
-        if (b >= 1) {
-            XgSlTask S;
-            S.mode = XG_SL_INVERSE;
-            S.col = b;
-            S.k0 = 0;
-            S.k1 = b;
-            S.sign = -1.0;
-            S.overwrite = 1;
-            xg_launch_sliced(sl->X, sl->L, TX, S, g_xg.sm_count, status, st);
-        }
-        const int J0 = b * bpt, J1 = J0 + bpt < nb ? J0 + bpt : nb;
-        XgRows G = {};
-        G.y[0] = X.d;
-        G.dinv[0] = M.dinv;
-        G.s = M.d;
-        G.ts = ts;
-        G.nsys = 1;
-        G.J0 = J0;
-        G.one.nt = nt;
-        G.one.nb = nb;
-        G.ntasks = xg_num_lower_tiles(J1) - xg_num_lower_tiles(J0);
-        G.next = (unsigned *)(windows + b);
-        G.abort = X.dag + 1;
-        G.flags = X.dag + 2;
-        G.status = status;
-        xg_launch_rows(XG_ROWS_INVERSE, maps, G, g_xg.sm_count, st);
-        xg_launch_slice_panel(TX, b, 1, sl->X.digits, sl->X.dig, sl->X.scale, plane, status, st);
-    }
-    XgSlTask S;
-    S.mode = XG_SL_SYRK;
-    S.col = 0;
-    S.k0 = 0;
-    S.k1 = nt;
-    S.sign = 1.0;
-    S.overwrite = 1;
-    xg_launch_sliced(sl->X, sl->X, T, S, g_xg.sm_count, status, st);
+    xg_sliced_groups(
+        nt, sl, fs,
+        [&](int col, int ncol, int k0, int k1, int ctas, cudaStream_t s) {
+            if (ncol > 0 && k1 > k0)
+                xg_launch_sliced(sl->X, sl->L, TX, xg_sl_task(XG_SL_INVERSE, col, ncol, k0, k1), ctas, status, s);
+        },
+        [&](int b, cudaStream_t s) {
+            const int J0 = b * bpt, J1 = J0 + bpt < nb ? J0 + bpt : nb;
+            XgRows G = {};
+            G.y[0] = X.d;
+            G.dinv[0] = M.dinv;
+            G.s = M.d;
+            G.ts = ts;
+            G.nsys = 1;
+            G.J0 = J0;
+            G.one.nt = nt;
+            G.one.nb = nb;
+            G.ntasks = xg_num_lower_tiles(J1) - xg_num_lower_tiles(J0);
+            G.next = (unsigned *)(windows + b);
+            G.abort = X.dag + 1;
+            G.flags = X.dag + 2;
+            G.status = status;
+            xg_launch_rows(XG_ROWS_INVERSE, maps, G, g_xg.sm_count, s);
+            xg_launch_slice_panel(TX, b, 1, sl->X.digits, sl->X.dig, sl->X.scale, plane, status, s);
+        });
+    xg_launch_sliced(sl->X, sl->X, T, xg_sl_task(XG_SL_SYRK, 0, nt, 0, nt), g_xg.sm_count, status, fs.st);
 }
 
 /* X = L^-T, then Sigma^-1 = X X^T over the factor M (lower tiles) */
-void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st)
+void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, const XgFactorStreams &fs)
 {
+    cudaStream_t st = fs.st;
     if (M.i8_factor && M.i8 && (M.i8->X.dig || xg_i8_prepare_inverse(M))) {
-        xg_inverse_product_sliced(M, X, M.i8, status, st);
+        xg_inverse_product_sliced(M, X, M.i8, status, fs);
         return;
     }
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
@@ -887,7 +1035,12 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
     xg_solve_transposed(f->C, f->v, f->status, st);
-    xg_inverse_product(f->C, f->X, f->status, st);
+    XgFactorStreams fs;
+    fs.st = st;
+    fs.st_hi = g_xg.stream_hi;
+    fs.ev_panel = f->ev_panel;
+    fs.ev_upd = f->ev_upd;
+    xg_inverse_product(f->C, f->X, f->status, fs);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, f->C.nt, f->C.ts, f->x, f->y, f->v, f->N, p, f->kernel,
                             f->metric, dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));
@@ -917,13 +1070,6 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
 /* ------------------------------------------------------------------------- */
 /* banded mixed precision                                                    */
 /* ------------------------------------------------------------------------- */
-
-/* SMs left free by the persistent trailing-update kernels (one CTA per SM,
- * ~197 KB of shared memory each) while the lookahead panel of the next step
- * (POTRF, TRSM, panel conversion) runs on the high-priority stream: resident
- * CTAs are never preempted, so without free SMs the panel would wait for the
- * whole update. */
-#define XG_PANEL_SMS 16
 
 static int xg_encode(CUtensorMap *map, CUtensorMapDataType dt, size_t esize, void *base, cuuint64_t cols,
                      cuuint64_t rows, cuuint32_t box_cols, cuuint32_t box_rows,
@@ -1360,99 +1506,9 @@ int xg_field_set_sliced(XgField *f)
     return rc;
 }
 
-/* Left-looking factorisation with FP64 tiles and INT8-sliced updates, by
- * groups of G = xg_sl_group tile columns [a, b):
- *   U1     chunks k < a0 (the group before begins at a0) to every target of the group (main stream,
- *          on all but xg_panel_share SMs, beside the panels of the group before)
- *   U2     chunks a0 <= k < a, when those panels are sliced: column a on the panel stream, the
- *          others on the main stream
- *   panel  per column c: chunks a <= k < c (for c > a), POTRF and TRSM of the tile column (a window
- *          of the tile DAG, with log-det and z solve), slicing into digit planes
- * Profiling events (8 per column c, those of the main stream on a group's
- * first column): panel stream before / after the column's updates, after its
- * panel, after slicing; main stream before / after U1. */
-
-/* Tile columns per group.  One column gives an update 16 (nt - j) jobs of 128
- * x 128, whose last round leaves most of the persistent CTAs idle: counted
- * over the columns 1.7 x the even distribution at 38 tile columns, 1.36 x at
- * 79, 1.24 x at 137; groups of four bring that to 1.21, 1.09 and 1.05, but put
- * three columns' panels between two updates, which the short matrices have
- * nothing to run beside.  Log-likelihood in ms, tiles of 512, K = 4 below:
- *   7 digits   N = 8200  10000  14000  20000  28000  40000
- *     G = 1        6.00   8.80     -    46.6     -    316
- *     G = 2        5.71   7.98   17.9   44.7   109    308
- *     G = 3        6.13   8.17   16.6   42.2   107    305
- *     G = 4        6.52   8.81   17.3   41.1   105    298
- *   4 digits   N = 9000  20000  40000  70000
- *     G = 1        5.00   20.2    117   560
- *     G = 2        5.02   20.1    119   574
- *     G = 3        5.20   21.4    118   573
- * (28 pairs cost an update 2.8 times what ten do, the panels the same: the
- * four-digit form has the panels to hide, not the last rounds.) */
-static int xg_sl_group(int nt, int digits)
-{
-    return digits == 4 ? 1 : nt < 24 ? 2 : nt < 36 ? 3 : 4;
-}
-
-static XgSlTask factor_task(int col, int ncol, int k0, int k1)
-{
-    XgSlTask S;
-    S.mode = XG_SL_FACTOR;
-    S.col = col;
-    S.ncol = ncol;
-    S.k0 = k0;
-    S.k1 = k1;
-    S.sign = -1.0;
-    S.overwrite = 0;
-    return S;
-}
-
-/* SMs left to the panels of the group that begins at tile column a while U1 of
- * the next group runs on the others.  Per target tile the panels cost the DMMA
- * flops of the TRSM and the group's own chunks, U1 a chunks: sms K / (K + a),
- * clamped to [XG_PANEL_SMS, sms - XG_PANEL_SMS].  K = 4
- * (EXAGEOSTAT_B200_PANEL_K overrides it): seven digits in groups of four at
- * N = 10000 / 20000 / 40000 took 11.0 / 51.4 / 325 ms with K = 1, 9.9 / 46.5 /
- * 317 with 2, 9.2 / 43.8 / 309 with 3, 8.9 / 41.6 / 308 with 4 and 8.6 / 43.6 /
- * 311 with 6; four digits at 20000 / 70000 20.4 / 570 with 4 and 20.9 / 572
- * with 7. */
-static int xg_panel_k()
-{
-    static int v = -1;
-    if (v < 0) {
-        const char *e = getenv("EXAGEOSTAT_B200_PANEL_K");
-        v = e ? atoi(e) : 0;
-        if (v < 1 || v > 64) v = 4;
-    }
-    return v;
-}
-
-static int xg_panel_share(int a, int sms)
-{
-    const int K = xg_panel_k();
-    int r = (int)((long long)sms * K / (K + a));
-    if (r < XG_PANEL_SMS) r = XG_PANEL_SMS;
-    if (r > sms - XG_PANEL_SMS) r = sms - XG_PANEL_SMS;
-    return r;
-}
-
-/* How the SMs are divided between the panel chain and the split update.
- * "static" (default): the split update runs as a persistent launch on
- * sms - xg_panel_share(a) CTAs, leaving the rest to the panel chain.
- * "dynamic" (EXAGEOSTAT_B200_SL_SHARE=dynamic): both updates launch one CTA
- * per job, so CTAs retire throughout the update and the hardware hands each
- * freed SM to the pending panel kernels first (higher stream priority), the
- * SMs the chain does not need staying with the update. */
-static bool xg_sl_dynamic_share()
-{
-    static int v = -1;
-    if (v < 0) {
-        const char *e = getenv("EXAGEOSTAT_B200_SL_SHARE");
-        v = (e && strcmp(e, "dynamic") == 0) ? 1 : 0;
-    }
-    return v == 1;
-}
-
+/* Factorisation with FP64 tiles and INT8-sliced updates; a column's panel is
+ * POTRF and TRSM of the tile column (a window of the tile DAG, with log-det
+ * and z solve) and its slicing into digit planes. */
 static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *part, int *status,
                             const XgFactorStreams &fs)
 {
@@ -1461,68 +1517,18 @@ static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *pa
     const int nb = (M.N + XG_DAG_BLOCK - 1) / XG_DAG_BLOCK;
     const long long plane = (long long)sl->L.plane_rows * M.ts;
     int *windows = M.dag + xg_dag_words(nb) - nb;
-    const bool la = fs.st_hi != nullptr;
-    cudaStream_t st = fs.st, sp = la ? fs.st_hi : fs.st;
-    cudaEvent_t *pev = fs.pev;
-    auto rec = [&](int k, int e, cudaStream_t s) {
-        if (pev) cudaEventRecord(pev[8 * k + e], s);
-    };
-    const int sms = g_xg.sm_count;
-    const int G = xg_sl_group(nt, sl->L.digits);
-    const bool dyn = xg_sl_dynamic_share();
-    const int all = 1 << 30; /* one CTA per job */
-    auto update = [&](int col, int ncol, int k0, int k1, int ctas, cudaStream_t s) {
-        if (ncol > 0 && k1 > k0) xg_launch_sliced(sl->L, sl->L, T, factor_task(col, ncol, k0, k1), ctas, status, s);
-    };
-    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), st);
-    if (la) {
-        cudaEventRecord(sl->ev_a, st); /* the generated matrix */
-        cudaStreamWaitEvent(sp, sl->ev_a, 0);
-    }
-    for (int a = 0; a < nt; a += G) {
-        const int b = a + G < nt ? a + G : nt, a0 = a - G;
-        /* main stream: U1 of this group was issued with the group before; U2 of
-         * the columns after the first */
-        if (la && a > 0) {
-            cudaEventRecord(sl->ev_p[0], sp); /* the group before is sliced */
-            cudaEventRecord(sl->ev_a, st);    /* U1 of this group is done */
-            cudaStreamWaitEvent(st, sl->ev_p[0], 0);
-            cudaStreamWaitEvent(sp, sl->ev_a, 0);
-            update(a + 1, b - a - 1, a0, a, sms, st);
-            cudaEventRecord(sl->ev_p[1], st);
-        } else if (a > 0) {
-            update(a + 1, b - a - 1, a0, a, sms, st);
-        }
-        rec(a, 4, st);
-        const int b1 = b + G < nt ? b + G : nt; /* the next group: chunks k < a */
-        update(b, b1 - b, 0, a, !la ? sms : dyn ? all : sms - xg_panel_share(a, sms), st);
-        rec(a, 5, st);
-        for (int c = a; c < b; ++c) {
-            rec(c, 0, sp);
-            if (c == a) {
-                /* alone in its group it runs beside U1 of the next column */
-                if (a > 0) update(a, 1, a0, a, !la || G > 1 ? sms : dyn ? all : xg_panel_share(a, sms), sp);
-            } else {
-                if (la && a > 0 && c == a + 1) cudaStreamWaitEvent(sp, sl->ev_p[1], 0);
-                update(c, 1, a, c, la && b < nt ? (dyn ? all : xg_panel_share(a, sms)) : sms, sp);
-            }
-            rec(c, 1, sp);
-            xg_launch_dag_columns(M, c * bpt, (c + 1) * bpt, windows + c, v, part, status, sms, sp);
-            rec(c, 2, sp);
-            if (c + 1 < nt) xg_launch_slice_panel(T, c, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, sp);
-            rec(c, 3, sp);
-            if (c > a) {
-                rec(c, 4, st);
-                rec(c, 5, st);
-            }
-            rec(c, 6, st);
-            rec(c, 7, st);
-        }
-    }
-    if (la) {
-        cudaEventRecord(fs.ev_panel, sp);
-        cudaStreamWaitEvent(st, fs.ev_panel, 0);
-    }
+    cudaMemsetAsync(M.dag, 0, sizeof(int) * (size_t)xg_dag_words(nb), fs.st);
+    xg_sliced_groups(
+        nt, sl, fs,
+        [&](int col, int ncol, int k0, int k1, int ctas, cudaStream_t s) {
+            if (ncol > 0 && k1 > k0)
+                xg_launch_sliced(sl->L, sl->L, T, xg_sl_task(XG_SL_FACTOR, col, ncol, k0, k1), ctas, status, s);
+        },
+        [&](int c, cudaStream_t s) {
+            xg_launch_dag_columns(M, c * bpt, (c + 1) * bpt, windows + c, v, part, status, g_xg.sm_count, s);
+            if (fs.pev) cudaEventRecord(fs.pev[8 * c + 2], s);
+            if (c + 1 < nt) xg_launch_slice_panel(T, c, 0, sl->L.digits, sl->L.dig, sl->L.scale, plane, status, s);
+        });
     return nb;
 }
 
@@ -1651,8 +1657,8 @@ int xg_sliced_factor_dense(int n, const double *x, const double *y, const double
 
 /* Gradient with the sliced path: the forward factorisation as
  * xg_field_loglik_sliced, alpha = L^-T v in FP64, the inverse factor
- * X = L^-T column by column (INT8-sliced update from the digit planes of L and
- * of the already finished columns of X, then the FP64 triangular solve with
+ * X = L^-T by groups of columns (INT8-sliced updates from the digit planes of L
+ * and of the already finished columns of X, the FP64 triangular solve with
  * L_bb^T and the slicing of column b of X), S = X X^T by one sliced launch
  * written over the factor, and the FP64 contraction with dSigma/dtheta. */
 int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, double *grad, double *times)
@@ -1672,7 +1678,12 @@ int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, do
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
     xg_solve_transposed(f->C, f->v, f->status, st);
-    xg_inverse_product_sliced(f->C, f->X, sl, f->status, st);
+    XgFactorStreams fs;
+    fs.st = st;
+    fs.st_hi = g_xg.stream_hi;
+    fs.ev_panel = f->ev_panel;
+    fs.ev_upd = f->ev_upd;
+    xg_inverse_product_sliced(f->C, f->X, sl, f->status, fs);
     xg_launch_grad_contract(f->C.d, f->C.ij, f->C.ntiles, nt, ts, f->x, f->y, f->v, f->N, p, f->kernel, f->metric,
                             dlogcon, f->C.tab, f->gpart, f->gout, st);
     XG_CU(cudaEventRecord(f->ev[3], st));

@@ -194,6 +194,7 @@ struct XgSlJob {
     int ta, tb;       /* tile rows (A) and columns (B) index the operand slots */
     int bm, bn, k0, k1;
     long long c_slot;
+    bool fresh; /* C = sign sum (C is not read) */
 };
 
 /* job -> (output tile, block, chunk range) per mode (see XgSlTask); false
@@ -207,6 +208,7 @@ __device__ __forceinline__ bool xg_sl_job(const XgSlTask &S, long long job, int 
     const int blk = (int)(job % per);
     J.bm = blk / bpt;
     J.bn = blk % bpt;
+    J.fresh = S.mode == XG_SL_SYRK;
     bool diag = false;
     if (S.mode == XG_SL_FACTOR) { /* targets (i, j), i >= j, of columns col .. col + ncol - 1 */
         int c = S.col;
@@ -218,11 +220,12 @@ __device__ __forceinline__ bool xg_sl_job(const XgSlTask &S, long long job, int 
         J.k1 = S.k1;
         J.c_slot = xg_tile_index(J.ta, J.tb, nt);
         diag = J.ta == J.tb;
-    } else if (S.mode == XG_SL_INVERSE) { /* X(a, b), a < b = col, from chunks a <= c < b (within [k0, k1)) */
-        J.ta = (int)unit;
-        J.tb = S.col;
+    } else if (S.mode == XG_SL_INVERSE) { /* X(a, b), a < k1 <= b, from chunks max(a, k0) <= c < k1; the longest first */
+        J.ta = (int)(unit / S.ncol);
+        J.tb = S.col + (int)(unit % S.ncol);
         J.k0 = J.ta > S.k0 ? J.ta : S.k0;
-        J.k1 = S.col < S.k1 ? S.col : S.k1;
+        J.k1 = S.k1;
+        J.fresh = S.k0 <= J.ta;
         J.c_slot = xg_tile_index(J.tb, J.ta, nt);
     } else { /* SYRK: S(a, b), a >= b, from chunks a <= c < nt */
         int ii, jj;
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(XG_SL_THREADS, 1)
             for (int u0 = 0; u0 < 64; u0 += 16) {
                 double cv[16];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) cv[u] = S.overwrite ? 0.0 : __ldcg(Cc + (long long)u * ts);
+                for (int u = 0; u < 16; ++u) cv[u] = J.fresh ? 0.0 : __ldcg(Cc + (long long)u * ts);
 #pragma unroll
                 for (int u = 0; u < 16; ++u) __stcg(Cc + (long long)u * ts, cv[u] + res[u0 + u]);
                 Cc += 16LL * ts;
@@ -645,9 +648,11 @@ void xg_launch_sliced(const XgDigits &A, const XgDigits &B, const XgTileArgs &T,
     if (S.mode == XG_SL_FACTOR) {
         const int end = S.col + S.ncol < T.nt ? S.col + S.ncol : T.nt;
         units = xg_num_lower_tiles(T.nt - S.col) - xg_num_lower_tiles(T.nt - end);
+    } else if (S.mode == XG_SL_INVERSE) {
+        units = (long long)S.ncol * S.k1;
+    } else {
+        units = (long long)T.nt * (T.nt + 1) / 2;
     }
-    else if (S.mode == XG_SL_INVERSE) units = S.col;
-    else units = (long long)T.nt * (T.nt + 1) / 2;
     const long long njobs = units * per;
     if (njobs <= 0) return;
     const unsigned grid = (unsigned)(njobs < max_ctas ? njobs : max_ctas);

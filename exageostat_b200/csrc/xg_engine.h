@@ -141,7 +141,7 @@ void xg_factor_two(XgTileMatrix &A, XgTileMatrix &B, double *part_a, double *par
                    const XgFactorStreams &fs);
 int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits);
 bool xg_i8_release(XgTileMatrix &M);
-void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, cudaStream_t st);
+void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, const XgFactorStreams &fs);
 void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st);
 double xg_trailing_flops(int nt, int ts, int k);
 int xg_field_set_data(XgField *f, const double *x, const double *y, const double *z);

@@ -277,18 +277,18 @@ void xg_launch_offband_gemm(const XgMixedMaps &maps, const XgTileArgs &T, int k,
  * over panel chunks k, with A_k, B_k read from digit stores:
  *   XG_SL_FACTOR : ncol columns of the Cholesky factor from col on, chunks k0 <= k < k1:
  *                  L(i,j) -= sum L(i,k) L(j,k)^T
- *   XG_SL_INVERSE: column col of X = L^-T (X(a,b) at slot (b,a)): X(a,col) -= sum_{a<=c<col} X(a,c) L(col,c)^T
+ *   XG_SL_INVERSE: ncol columns of X = L^-T from col on (X(a,b) at slot (b,a)), chunks k0 <= c < k1:
+ *                  X(a,b) -= sum_{a<=c} X(a,c) L(b,c)^T, a < k1; the window that holds chunk a is
+ *                  X(a,b)'s first and overwrites it
  *   XG_SL_SYRK   : S = X X^T into the lower tiles: S(a,b) = sum_{c>=a} X(a,c) X(b,c)^T */
 #define XG_SL_FACTOR 0
 #define XG_SL_INVERSE 1
 #define XG_SL_SYRK 2
 struct XgSlTask {
     int mode;
-    int col;       /* target column (factor, inverse) */
-    int ncol;      /* factor: that many target columns from col on */
+    int col, ncol; /* target columns (factor, inverse) */
     int k0, k1;    /* chunk window */
     double sign;   /* -1: C -= sum; +1: C += sum */
-    int overwrite; /* C = sign sum (C is not read) */
 };
 cudaError_t xg_sliced_kernels_configure();
 /* a digit store: `digits` planes of plane_rows rows (ts bytes each), one scale per row */
