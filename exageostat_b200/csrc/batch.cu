@@ -126,10 +126,10 @@ static void xg_table_fill(XgBTable &t, const std::vector<long long> &cnt)
 }
 
 /* ------------------------------------------------------------------------- */
-/* task order of the device scheduler                                        */
+/* the tile-task planner (exageostat_b200_batch_plan)                        */
 /* ------------------------------------------------------------------------- */
 
-/* Relative durations of the scheduler's task bodies on one SM (units of a
+/* Relative durations of the tile tasks on one SM (units of a
  * tile update, 2 ts^3 DMMA flops): a TRSM task solves the tile's ts / 32 row
  * strips one after the other; a POTRF task is latency-bound. */
 #define XG_PLAN_GEMM 1.0
@@ -138,7 +138,7 @@ static void xg_table_fill(XgBTable &t, const std::vector<long long> &cnt)
 
 /* Bottom levels (longest path to the end of the field's DAG, the task's own
  * duration included) of every task of a tile Cholesky with nt tiles per side,
- * under the scheduler's dependencies: POTRF(k) <- the k updates of (k, k);
+ * under the dependencies: POTRF(k) <- the k updates of (k, k);
  * TRSM(i, k) <- POTRF(k) and the k updates of (i, k); update (i, j) <- k <-
  * TRSM(i, k), TRSM(j, k) and the update (i, j) <- k - 1. */
 struct XgPlanLevels {
@@ -177,7 +177,7 @@ static void xg_plan_levels(int nt, XgPlanLevels &L)
  * the ready task of largest bottom level (critical path first), with the
  * durations above; the list is the order in which tasks start.  A task
  * starts only after every task it waits on has finished, so the list is a
- * topological order and the device scheduler cannot deadlock on it. */
+ * topological order and workers that wait for their inputs cannot deadlock. */
 static void xg_batch_plan(const std::vector<int> &nts, int workers, std::vector<int4> &tl)
 {
     struct Task {

@@ -357,11 +357,15 @@ static void xg_launch_dag_columns(XgTileMatrix &M, int J0, int J1, int *next, do
 /* Smallest dimension whose FP64 factorisation runs its updates on the INT8
  * tensor cores (seven digits, sliced.cu) instead of DMMA, by tile size: a
  * panel is one chunk of the product, and each chunk's sums are brought back
- * and scaled once, so small tiles pay that more often.  Milliseconds per
- * evaluation, INT8 against DMMA: ts = 512 N = 5000 2.88 / 2.55, 7000 4.44 /
- * 5.03, 20000 46.5 / 90.3, 40000 313 / 681; ts = 384 N = 9000 7.60 / 9.60; ts =
- * 256 N = 9000 10.0 / 9.6, 14000 25.2 / 32.5; ts = 128 N = 20000 106 / 91.7. */
-static int xg_i8_min(int ts) { return ts >= 512 ? 6500 : ts >= 384 ? 8000 : ts >= 256 ? 11000 : 1 << 30; }
+ * and scaled once, so small tiles pay that more often.  Milliseconds, DMMA
+ * dataflow / INT8, of a log-likelihood and of a gradient: ts = 512 N = 6000
+ * 3.43 / 3.52 and 8.6 / 7.6, 20000 90 / 40 and - / 133; ts = 384 N = 6000 3.44 /
+ * 3.51 and 8.6 / 7.7, 7000 5.00 / 4.37 and 12.9 / 10.2; ts = 256 N = 6000 3.43 /
+ * 3.78 and 8.6 / 8.2, 7000 4.98 / 4.68 and 12.9 / 10.8, 8100 7.45 / 5.67 and
+ * 19.5 / 13.7, 10000 13.3 / 9.0 and 35.2 / 23.0.  At ts = 128
+ * the line would be 8500 (12000 21.8 / 16.8), but nothing chooses 128 there
+ * (512 takes 11.6), and it is the path that the digits are tested against. */
+static int xg_i8_min(int ts) { return ts >= 256 ? 6500 : 1 << 30; }
 
 /* The factorisation of M as one launch of the tile DAG (tile_dag.cu); returns
  * the number of partial sums of either kind. */
