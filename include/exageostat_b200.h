@@ -544,7 +544,7 @@ int exageostat_b200_mloe_mmom_host(int nmiss, const double *xmiss, const double 
  * the other (sum n[f] doubles each).  kernel / metric as for
  * exageostat_b200_dmle_host, ts = tile size (0 = 256).  The fields share one
  * device tile store and each evaluation of all of them is one CUDA-graph
- * launch (one launch per tile step covering every field). */
+ * launch (the factorisation of every field is one kernel). */
 int exageostat_b200_batch_create(int nfields, const int *n, const double *x, const double *y, const double *z,
                                  int kernel, int metric, int ts, void **handle);
 /* theta: nfields rows of 3 (4 with the nugget) parameters; loglik receives
@@ -568,12 +568,12 @@ int exageostat_b200_batch_autotune(int nfields, const int *n, const double *x, c
                                    int kernel, int metric, const double *theta, int *ts, double *report,
                                    void **handle);
 
-/* The device scheduler's task list for fields of nt[f] tiles per side and
- * `workers` persistent CTAs (host only, no GPU needed): writes 4 ints per
+/* A critical-path-first task list for fields of nt[f] tiles per side and
+ * `workers` workers (host only, no GPU needed): writes 4 ints per
  * task -- type | field << 2 (type 0 POTRF(k), 1 TRSM(i, k), 2 the update
  * (i, j) <- k), i, j, k -- to out when out is not NULL, and returns the
- * number of tasks.  exageostat_b200_batch_create builds its list this way;
- * exposed so the order can be checked (complete, topological). */
+ * number of tasks.  The order is complete and topological; the batches
+ * themselves are factored by 128 x 128 blocks and do not use it. */
 long long exageostat_b200_batch_plan(int nfields, const int *nt, int workers, int *out);
 
 /* ---- diagnostics used by the parity tests (no counterpart in the reference; all run on the GPU) ---- */
