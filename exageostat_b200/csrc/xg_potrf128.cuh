@@ -324,12 +324,15 @@ __device__ __forceinline__ void xg_potrf_inverse32(const double *S, const double
 __device__ __forceinline__ int xg_potrf128(double *S, double *W, double *T, double *vs, int rhs, double *Lg, int ldl,
                                            double *dinv, double *sums)
 {
-    __shared__ int s_fail;
+    /* warp 0 runs ahead into panel p + 1 while the others may still be about to
+     * read panel p's word: two words in turn, so that a word is written again
+     * only behind the barrier of the panel between */
+    __shared__ int s_fail[2];
     __shared__ __align__(16) double s_buf[4 * XG_P_NB];
     constexpr int NP = XG_SUB / XG_P_NB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    if (tid == 32) s_fail = 0;
+    if (tid < 2) s_fail[tid] = 0;
     for (int idx = tid; idx < NP * XG_P_NB * XG_P_NB; idx += XG_POTRF_SUB_THREADS) {
         const int r = (idx >> 4) & 15, c = idx & 15;
         W[(idx >> 8) * XG_P_WSZ + r * XG_P_LDW + c] = r == c ? 1.0 : 0.0;
@@ -342,10 +345,11 @@ __device__ __forceinline__ int xg_potrf128(double *S, double *W, double *T, doub
         const double *Wp = W + p * XG_P_WSZ;
         if (warp == 0) {
             const int f = xg_chol16_warp(S + c0 * XG_P_LDS + c0, W + p * XG_P_WSZ, s_buf, lane);
-            if (f && lane == 0) s_fail = c0 + f;
+            if (f && lane == 0) s_fail[p & 1] = c0 + f;
         }
         __syncthreads();
-        if (s_fail) return s_fail;
+        const int failed = s_fail[p & 1];
+        if (failed) return failed;
         if (warp == 0) {
             if (p + 1 < NP)
                 xg_potrf_next_diag(S, Wp, p, g, tq, [] {

@@ -81,3 +81,31 @@ def test_gradient_at_block_edges(gpu, ora, n, ts):
         _, gb = b.loglik([THETA] * 3, grad=True)
     for f in (0, 2):
         assert np.abs(gb[f] - ref).max() <= 1e-9 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("ts", [128, 256])
+def test_failing_pivot_of_every_panel(gpu, ora, ts):
+    """A NaN location in each 16-wide panel of the first and of a later block:
+    the pivot that fails, from the tile DAG, the per-step launches and a
+    batch; all three evaluate again afterwards."""
+    n = 301
+    x, y = ora.generate_xy_loc(n, 4)
+    z = ora.dzvg(x, y, THETA, ora.dlarnv(5, n))
+    with gpu.Session(x, y, dts=ts) as s:
+        s.set_data(z=z)
+        ref = s.loglik(THETA)
+        for bad in [16 * p + (3 * p) % 16 for p in range(8)] + [128 + 16 * p + 15 for p in range(8)]:
+            xb = x.copy()
+            xb[bad] = np.nan
+            s.set_data(x=xb)
+            for profiled in (False, True):
+                s.set_profiling(profiled)
+                with pytest.raises(gpu.XgError) as err:
+                    s.loglik(THETA)
+                assert err.value.code == gpu.XG_ERR_NOT_SPD and "pivot %d)" % (bad + 1) in str(err.value)
+            s.set_profiling(False)
+            with gpu.Batch([x, xb, x], [y, y, y], [z, z, z], ts=ts) as b:
+                ll = b.loglik([THETA] * 3)
+                assert ll[1] == -np.inf and ll[0] == ll[2] == pytest.approx(ref, rel=1e-12)
+        s.set_data(x=x)
+        assert s.loglik(THETA) == ref
