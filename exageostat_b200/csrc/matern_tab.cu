@@ -84,15 +84,20 @@ __device__ __forceinline__ bool xg_tab_wanted(const XgMaternParams &p, int n)
     return p.half_integer < 0 && n >= XG_TAB_MIN_N && p.nu <= XG_TAB_NU;
 }
 
-/* the tables of every field of a batch (blockIdx.y); fields that need none skip */
-__global__ void __launch_bounds__(64) xg_tab_build_batch_kernel(double *tab, const XgBField *__restrict__ F)
+/* the tables of every field of a batch (blockIdx.y and on by gridDim.y, which
+ * the hardware limits to 65535); fields that need none are passed over */
+__global__ void __launch_bounds__(64)
+    xg_tab_build_batch_kernel(double *tab, const XgBField *__restrict__ F, int nfields)
 {
     __shared__ double f[2][3][3][XG_TAB_NC];
-    const XgMaternParams &p = F[blockIdx.y].p;
-    if (!xg_tab_wanted(p, F[blockIdx.y].N)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    xg_tab_build_warp<false>(tab + (long long)blockIdx.y * XG_TAB_SIZE, ((int)blockIdx.x * 2 + warp) * 3, p.nu, p.con,
-                             p.tm, 0.0, 0.0, 0.0, f[warp], lane);
+    for (int field = (int)blockIdx.y; field < nfields; field += (int)gridDim.y) {
+        const XgMaternParams &p = F[field].p;
+        if (!xg_tab_wanted(p, F[field].N)) continue;
+        __syncwarp(); /* the last field's node values are read */
+        xg_tab_build_warp<false>(tab + (long long)field * XG_TAB_SIZE, ((int)blockIdx.x * 2 + warp) * 3, p.nu, p.con,
+                                 p.tm, 0.0, 0.0, 0.0, f[warp], lane);
+    }
 }
 #define XG_TAB_BUILD_BLOCKS ((XG_TAB_NINT + 5) / 6)
 
@@ -418,7 +423,8 @@ void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, int nfields,
                          const double *x, const double *y, int metric, double *tab, cudaStream_t st)
 {
     if (blocks <= 0) return;
-    xg_tab_build_batch_kernel<<<dim3(XG_TAB_BUILD_BLOCKS, nfields), 64, 0, st>>>(tab, F);
+    xg_tab_build_batch_kernel<<<dim3(XG_TAB_BUILD_BLOCKS, nfields < 65535 ? nfields : 65535), 64, 0, st>>>(tab, F,
+                                                                                                         nfields);
     xg_gen_tab_batch_kernel<<<xg_tab_grid(blocks, 6), XG_GT_THREADS, XG_TAB_SIZE * sizeof(double), st>>>(
         base, F, S, blocks, x, y, metric, tab);
 }

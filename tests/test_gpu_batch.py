@@ -127,3 +127,20 @@ def test_batch_gradients_match_the_single_field_adjoint(gpu, ora):
         fl = lambda u: ora.dmle(xs[f], ys[f], zs[f], u)[0]
         fd[k] = (8 * (fl(t + e) - fl(t - e)) - (fl(t + 2 * e) - fl(t - 2 * e))) / (12 * h)
     assert np.abs(g[f] - fd).max() / max(np.abs(fd).max(), 1.0) < 1e-6, (g[f], fd)
+
+
+def test_more_fields_than_a_grid_dimension(gpu, ora):
+    """A grid's y extent ends at 65535: the fields beyond it are evaluated
+    like the first ones, bit for bit (general order, so from their tables)."""
+    n, nfields, distinct = 64, 65600, 37
+    rng = np.random.default_rng(12)
+    x, y, z = rng.random((distinct, n)), rng.random((distinct, n)), rng.standard_normal((distinct, n))
+    th = np.stack([rng.uniform(0.5, 2.0, distinct), rng.uniform(0.02, 0.1, distinct), rng.uniform(0.55, 0.95, distinct)], 1)
+    with gpu.Batch(list(x), list(y), list(z), ts=128) as b:
+        few = b.loglik(th)
+    f = np.arange(nfields) % distinct
+    with gpu.Batch(list(x[f]), list(y[f]), list(z[f]), ts=128) as b:
+        many = b.loglik(th[f])
+    assert np.array_equal(many, few[f])
+    ref, scale = _oracle_ll(ora, x, y, z, th)
+    _assert_close(few, ref, scale)
