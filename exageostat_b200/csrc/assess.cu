@@ -462,10 +462,9 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
     double *Y = nullptr, *part = nullptr;
     int *w = nullptr;
     const XgPart parts[] = {{&Y, nsys * full}, {&part, 10 * (size_t)nctas}, {&w, words}};
-    while (xg_alloc_parts(parts, 3) != cudaSuccess) {
-        if (xg_i8_release(f->C)) continue;
+    if (xg_alloc_parts(parts, 3) != cudaSuccess)
         return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", nsys * full * sizeof(double) / 1e9);
-    }
+    XgI8Use use(f->C);
     std::vector<double> hp(10 * (size_t)nctas);
     int sv[2] = {0, 0};
     XgRowsMaps maps = {};
@@ -611,6 +610,7 @@ int xg_assess_run(XgAssess *q, const double *truth, const double *est, int kerne
     int rc = xg_check_theta(truth, kernel);
     if (!rc) rc = xg_check_theta(est, kernel);
     if (rc) return rc;
+    XgI8Use use_a(q->Ca), use_t(q->Ct);
     cudaStream_t st = g_xg.stream;
     const int nmiss = q->nmiss, nobs = q->nobs, nt = q->nt, mt = q->mt, ts = q->ts;
     const XgMaternParams pt = xg_params(truth, kernel), pa = xg_params(est, kernel);

@@ -360,15 +360,15 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
         if (fd.nt > b->maxnt) b->maxnt = fd.nt;
     }
     const size_t tile = (size_t)b->ts * b->ts;
-    cudaError_t e = cudaMalloc(&b->tiles, (size_t)b->total_tiles * tile * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->x, b->total_vec * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->y, b->total_vec * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->z, b->total_vec * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->v, b->total_vec * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->part, b->total_part * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->out, 2 * (size_t)nfields * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&b->status, 2 * (size_t)nfields * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&b->F_dev, nfields * sizeof(XgBField));
+    cudaError_t e = xg_malloc(&b->tiles, (size_t)b->total_tiles * tile * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->x, b->total_vec * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->y, b->total_vec * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->z, b->total_vec * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->v, b->total_vec * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->part, b->total_part * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->out, 2 * (size_t)nfields * sizeof(double));
+    if (e == cudaSuccess) e = xg_malloc(&b->status, 2 * (size_t)nfields * sizeof(int));
+    if (e == cudaSuccess) e = xg_malloc(&b->F_dev, nfields * sizeof(XgBField));
     if (e == cudaSuccess) e = cudaMallocHost(&b->F_pinned, nfields * sizeof(XgBField));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_out, 2 * (size_t)nfields * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_status, 2 * (size_t)nfields * sizeof(int));
@@ -401,16 +401,16 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
         xg_batch_order(D, tl, tt);
         b->ntasks = (long long)tl.size();
         b->nttasks = (long long)tt.size();
-        e = cudaMalloc(&b->tasks, tl.size() * sizeof(int4));
+        e = xg_malloc(&b->tasks, tl.size() * sizeof(int4));
         if (e == cudaSuccess) e = cudaMemcpy(b->tasks, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&b->ttasks, tt.size() * sizeof(int2));
+        if (e == cudaSuccess) e = xg_malloc(&b->ttasks, tt.size() * sizeof(int2));
         if (e == cudaSuccess) e = cudaMemcpy(b->ttasks, tt.data(), tt.size() * sizeof(int2), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&b->D_dev, nfields * sizeof(XgDagField));
+        if (e == cudaSuccess) e = xg_malloc(&b->D_dev, nfields * sizeof(XgDagField));
         if (e == cudaSuccess) e = cudaMemcpy(b->D_dev, D.data(), nfields * sizeof(XgDagField), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&b->words, (size_t)(2 + b->total_flags) * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&b->twords, (size_t)(2 + b->total_tflags) * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&b->dinv, (size_t)b->total_vec * 32 * sizeof(double));
-        if (e == cudaSuccess) e = cudaMalloc(&b->tab, (size_t)nfields * xg_tab_doubles() / 3 * sizeof(double));
+        if (e == cudaSuccess) e = xg_malloc(&b->words, (size_t)(2 + b->total_flags) * sizeof(int));
+        if (e == cudaSuccess) e = xg_malloc(&b->twords, (size_t)(2 + b->total_tflags) * sizeof(int));
+        if (e == cudaSuccess) e = xg_malloc(&b->dinv, (size_t)b->total_vec * 32 * sizeof(double));
+        if (e == cudaSuccess) e = xg_malloc(&b->tab, (size_t)nfields * xg_tab_doubles() / 3 * sizeof(double));
         if (e != cudaSuccess) {
             xg_batch_free(b);
             return xg_fail(XG_ERR_NO_MEMORY, "batch task list (%lld tasks): %s", (long long)tl.size(),
@@ -423,7 +423,7 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
     size_t bytes = 0;
     for (XgBTable *t : all) bytes += t->start.size() * sizeof(long long) + ((t->fields.size() * sizeof(int) + 7) & ~7ULL);
     std::vector<unsigned char> hbuf(bytes);
-    e = cudaMalloc(&b->table_buf, bytes);
+    e = xg_malloc(&b->table_buf, bytes);
     if (e != cudaSuccess) {
         xg_batch_free(b);
         return xg_fail(XG_ERR_NO_MEMORY, "batch tables");
@@ -564,13 +564,13 @@ static int xg_batch_grad_workspace(XgBatch *b)
         std::vector<int2> h(ntl);
         for (int j = 0; j < nt; ++j)
             for (int i = j; i < nt; ++i) h[xg_tile_index(i, j, nt)] = make_int2(i, j);
-        XG_CU(cudaMalloc(&b->ij_by_nt[nt], sizeof(int2) * ntl));
+        XG_CU(xg_malloc(&b->ij_by_nt[nt], sizeof(int2) * ntl));
         XG_CU(cudaMemcpy(b->ij_by_nt[nt], h.data(), sizeof(int2) * ntl, cudaMemcpyHostToDevice));
         maxblocks = std::max(maxblocks, xg_grad_contract_blocks(ntl, ts));
     }
     for (int s = 0; s < XgBatch::GS; ++s) {
-        XG_CU(cudaMalloc(&b->gpart[s], 4 * (size_t)maxblocks * sizeof(double)));
-        XG_CU(cudaMalloc(&b->gtab[s], xg_tab_doubles() * sizeof(double)));
+        XG_CU(xg_malloc(&b->gpart[s], 4 * (size_t)maxblocks * sizeof(double)));
+        XG_CU(xg_malloc(&b->gtab[s], xg_tab_doubles() * sizeof(double)));
         XG_CU(cudaStreamCreateWithFlags(&b->gst[s], cudaStreamNonBlocking));
     }
     /* Groups of consecutive fields whose inverse factors fit XG_BATCH_X_BYTES
@@ -579,7 +579,7 @@ static int xg_batch_grad_workspace(XgBatch *b)
     const size_t tile_bytes = (size_t)ts * ts * sizeof(double);
     const long long largest = xg_num_lower_tiles(b->maxnt);
     long long cap = std::min(b->total_tiles, std::max(largest, (long long)(XG_BATCH_X_BYTES / tile_bytes)));
-    while (cudaMalloc(&b->xstore, (size_t)cap * tile_bytes) != cudaSuccess) {
+    while (xg_malloc(&b->xstore, (size_t)cap * tile_bytes) != cudaSuccess) {
         cudaGetLastError();
         b->xstore = nullptr;
         if (cap <= largest)
@@ -616,13 +616,13 @@ static int xg_batch_grad_workspace(XgBatch *b)
         b->groups.push_back(g);
         f = g.f1;
     }
-    XG_CU(cudaMalloc(&b->R_dev, b->nfields * sizeof(XgRowsField)));
+    XG_CU(xg_malloc(&b->R_dev, b->nfields * sizeof(XgRowsField)));
     XG_CU(cudaMemcpy(b->R_dev, R.data(), b->nfields * sizeof(XgRowsField), cudaMemcpyHostToDevice));
-    XG_CU(cudaMalloc(&b->rtasks, tl.size() * sizeof(int4)));
+    XG_CU(xg_malloc(&b->rtasks, tl.size() * sizeof(int4)));
     XG_CU(cudaMemcpy(b->rtasks, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    XG_CU(cudaMalloc(&b->rwords, (size_t)(2 + maxflags) * sizeof(int)));
+    XG_CU(xg_malloc(&b->rwords, (size_t)(2 + maxflags) * sizeof(int)));
     XG_CU(cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming));
-    XG_CU(cudaMalloc(&b->gout, 4 * (size_t)b->nfields * sizeof(double)));
+    XG_CU(xg_malloc(&b->gout, 4 * (size_t)b->nfields * sizeof(double)));
     XG_CU(cudaMallocHost(&b->h_gout, 4 * (size_t)b->nfields * sizeof(double)));
     return XG_OK;
 }

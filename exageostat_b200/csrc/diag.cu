@@ -40,7 +40,7 @@ extern "C" int exageostat_b200_diag_wait_timeout(double limit_us, double *waited
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
     void *buf = nullptr;
-    cudaError_t e = cudaMalloc(&buf, 16);
+    cudaError_t e = xg_malloc(&buf, 16);
     if (e != cudaSuccess) return xg_fail(XG_ERR_CUDA, "bounded-wait diagnostic: %s", cudaGetErrorString(e));
     int *status = (int *)buf;
     unsigned long long *waited = (unsigned long long *)((char *)buf + 8);

@@ -102,6 +102,7 @@ int xg_context_start(int dts)
     if (e != cudaSuccess) return xg_cuda_fail(e, "kernel attribute setup");
     g_xg.device = dev;
     g_xg.sm_count = prop.multiProcessorCount;
+    g_xg.memory = prop.totalGlobalMem;
     g_xg.dts = dts;
     g_xg.initialized = true;
     return XG_OK;
@@ -129,13 +130,33 @@ int xg_choose_ts(int N, int dts)
     return ts;
 }
 
-cudaError_t xg_alloc_parts(const XgPart *parts, int n)
+static bool xg_i8_take_back();
+static void xg_i8_free(XgTileMatrix &M);
+
+cudaError_t xg_malloc_bytes(void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && xg_i8_take_back()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+    }
+    return e;
+}
+
+cudaError_t xg_alloc_parts(const XgPart *parts, int n, bool take_back)
 {
     size_t total = 0;
     for (int i = 0; i < n; ++i) total += (parts[i].bytes + 255) / 256 * 256;
     char *base = nullptr;
-    const cudaError_t e = cudaMalloc(&base, total);
-    if (e != cudaSuccess) cudaGetLastError();
+    const cudaError_t e = take_back ? xg_malloc(&base, total) : cudaMalloc(&base, total);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        base = nullptr;
+    }
     for (int i = 0; i < n; ++i) {
         *parts[i].p = base;
         if (base) base += (parts[i].bytes + 255) / 256 * 256;
@@ -191,8 +212,7 @@ int xg_encode_tiles(CUtensorMap *map, double *base, long long ntiles, int ts)
 void xg_tm_free(XgTileMatrix &M)
 {
     if (M.d) cudaFree(M.d);
-    xg_i8_release(M);
-    M.no_i8 = M.i8_factor = false; /* of the matrix that was freed */
+    xg_i8_free(M);
     M.tab = nullptr;
     M.dag = nullptr;
     M.d = nullptr;
@@ -326,8 +346,8 @@ int xg_check_theta(const double *theta, int kernel)
 
 static int xg_factor_sliced(XgTileMatrix &M, XgSliced *sl, double *v, double *part, int *status,
                             const XgFactorStreams &fs);
-static bool xg_i8_prepare(XgTileMatrix &M);
-static bool xg_i8_prepare_inverse(XgTileMatrix &M);
+static bool xg_i8_acquire(XgTileMatrix &M);
+static bool xg_i8_acquire_inverse(XgTileMatrix &M);
 
 /* Block columns J0 .. J1 - 1 of M by the tile DAG: the whole factorisation
  * (0, nb), or one window of it (words: its next-task word; the flags of the
@@ -588,7 +608,7 @@ static void xg_inverse_product_sliced(XgTileMatrix &M, XgTileMatrix &X, XgSliced
 void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, const XgFactorStreams &fs)
 {
     cudaStream_t st = fs.st;
-    if (M.i8_factor && M.i8 && (M.i8->X.dig || xg_i8_prepare_inverse(M))) {
+    if (M.i8_factor && M.i8 && xg_i8_acquire_inverse(M)) {
         xg_inverse_product_sliced(M, X, M.i8, status, fs);
         return;
     }
@@ -650,7 +670,7 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
     /* profiled evaluations keep the per-step launches, whose kernels the profile tells apart */
     M.i8_factor = false;
     if (M.dag && !fs.pev) {
-        if (M.N >= xg_i8_min(M.ts) && xg_i8_prepare(M)) {
+        if (M.N >= xg_i8_min(M.ts) && xg_i8_acquire(M)) {
             M.i8_factor = true;
             return xg_factor_sliced(M, M.i8, v, part, status, fs);
         }
@@ -795,7 +815,7 @@ int xg_field_set_data(XgField *f, const double *x, const double *y, const double
 
 static int xg_dev_alloc(double **p, size_t n)
 {
-    cudaError_t e = cudaMalloc(p, n * sizeof(double));
+    cudaError_t e = xg_malloc(p, n * sizeof(double));
     if (e != cudaSuccess) return xg_fail(XG_ERR_NO_MEMORY, "cudaMalloc(%zu doubles): %s", n, cudaGetErrorString(e));
     return cudaMemset(*p, 0, n * sizeof(double)) == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }
@@ -850,7 +870,7 @@ int xg_field_create(XgField **out, int N, int ts, const double *x, const double 
     if (!rc) rc = xg_dev_alloc(&f->e, Np);
     if (!rc) rc = xg_dev_alloc(&f->part, 2 * Np / XG_DAG_BLOCK);
     if (!rc) rc = xg_dev_alloc(&f->out, 8);
-    if (!rc && cudaMalloc(&f->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status word");
+    if (!rc && xg_malloc(&f->status, 2 * sizeof(int)) != cudaSuccess) rc = xg_fail(XG_ERR_NO_MEMORY, "status word");
     if (!rc && cudaMallocHost(&f->h_out, 8 * sizeof(double)) != cudaSuccess)
         rc = xg_fail(XG_ERR_NO_MEMORY, "pinned result buffer");
     for (int i = 0; i < 4 && !rc; ++i)
@@ -897,6 +917,7 @@ int xg_field_loglik(XgField *f, const double *theta, double *res, double *times)
     int rc = xg_check_theta(theta, f->kernel);
     if (rc) return rc;
     if (!f->have_z) return xg_fail(XG_ERR_BAD_ARGUMENT, "no observations: call MLE_zvg or set z first");
+    XgI8Use use(f->C);
     cudaStream_t st = g_xg.stream;
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, f->kernel);
@@ -939,6 +960,7 @@ int xg_field_zvg(XgField *f, const double *theta, const double *nrand, double *t
 {
     int rc = xg_check_theta(theta, f->kernel);
     if (rc) return rc;
+    XgI8Use use(f->C);
     cudaStream_t st = g_xg.stream;
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, f->kernel);
@@ -1003,23 +1025,19 @@ static void xg_exact_sigma2_grad(const XgField *f, const double *theta, const do
 }
 
 /* The gradient's inverse-factor store and contraction partials, each
- * allocated on first use (the Fisher path allocates only the store). */
+ * allocated on first use. */
 static int xg_grad_workspace(XgField *f)
 {
     if (!f->X.d) {
-        int rc = xg_tm_alloc(f->X, f->N, f->C.ts);
-        if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) {
-            xg_tm_free(f->X);
-            rc = xg_tm_alloc(f->X, f->N, f->C.ts);
-        }
+        const int rc = xg_tm_alloc(f->X, f->N, f->C.ts);
         if (rc) return rc;
     }
     const long long blocks = xg_grad_contract_blocks(f->C.ntiles, f->C.ts);
-    if (!f->gpart && cudaMalloc(&f->gpart, 4 * (size_t)blocks * sizeof(double)) != cudaSuccess) {
+    if (!f->gpart && xg_malloc(&f->gpart, 4 * (size_t)blocks * sizeof(double)) != cudaSuccess) {
         f->gpart = nullptr;
         return xg_fail(XG_ERR_NO_MEMORY, "gradient workspace");
     }
-    if (!f->gout && cudaMalloc(&f->gout, 4 * sizeof(double)) != cudaSuccess) {
+    if (!f->gout && xg_malloc(&f->gout, 4 * sizeof(double)) != cudaSuccess) {
         f->gout = nullptr;
         return xg_fail(XG_ERR_NO_MEMORY, "gradient workspace");
     }
@@ -1032,6 +1050,7 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
 {
     int rc = xg_grad_workspace(f);
     if (rc) return rc;
+    XgI8Use use(f->C); /* the factor's planes serve its inverse */
     rc = xg_field_loglik(f, theta, res, times);
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
@@ -1122,16 +1141,16 @@ static int xg_mixed_create(XgMixed **out, int N, int ts, int band, int passes)
     double *d64 = nullptr;
     float *d32 = nullptr;
     const long long noff = xg_num_offband_tiles(nt, band);
-    if (cudaMalloc(&d64, (size_t)nt * band * tile * sizeof(double)) != cudaSuccess)
+    if (xg_malloc(&d64, (size_t)nt * band * tile * sizeof(double)) != cudaSuccess)
         rc = xg_fail(XG_ERR_NO_MEMORY, "mixed band tiles");
-    if (!rc && noff > 0 && cudaMalloc(&d32, (size_t)noff * tile * sizeof(float)) != cudaSuccess)
+    if (!rc && noff > 0 && xg_malloc(&d32, (size_t)noff * tile * sizeof(float)) != cudaSuccess)
         rc = xg_fail(XG_ERR_NO_MEMORY, "mixed off-band tiles (%.2f GB)", noff * tile * 4.0 / 1e9);
     m->T.data = d64;
     m->T.data32 = d32;
     for (int b = 0; b < 2 && !rc; ++b) {
-        if (cudaMalloc(&m->p64[b], np * ts * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&m->phi[b], np * ts * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&m->plo[b], np * ts * sizeof(float)) != cudaSuccess) {
+        if (xg_malloc(&m->p64[b], np * ts * sizeof(double)) != cudaSuccess ||
+            xg_malloc(&m->phi[b], np * ts * sizeof(float)) != cudaSuccess ||
+            xg_malloc(&m->plo[b], np * ts * sizeof(float)) != cudaSuccess) {
             rc = xg_fail(XG_ERR_NO_MEMORY, "mixed panel buffers");
             break;
         }
@@ -1269,9 +1288,7 @@ int xg_field_set_mixed(XgField *f, int band, int passes)
         xg_mixed_destroy(f->mx);
         f->mx = nullptr;
     }
-    int rc = xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
-    if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) rc = xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
-    return rc;
+    return xg_mixed_create(&f->mx, f->N, f->C.ts, band, passes);
 }
 
 int xg_field_loglik_mixed(XgField *f, const double *theta, double *res, double *times)
@@ -1422,7 +1439,9 @@ static void xg_digits_free(XgDigits &D)
     D.scale = nullptr;
 }
 
-/* digit planes for every tile of M's packed store */
+/* digit planes for every tile of M's packed store; the four-digit ones are a
+ * workspace that the caller asked for, the seven-digit ones a cache, which
+ * takes nobody else's memory */
 static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits)
 {
     const long long rows = M.ntiles * M.ts;
@@ -1432,7 +1451,7 @@ static int xg_digits_alloc(XgDigits &D, const XgTileMatrix &M, int digits)
     D.digits = digits;
     D.plane_rows = (int)rows;
     const XgPart parts[] = {{&D.dig, digits * plane}, {&D.scale, (size_t)rows}};
-    if (xg_alloc_parts(parts, 2) != cudaSuccess)
+    if (xg_alloc_parts(parts, 2, digits == 4) != cudaSuccess)
         return xg_fail(XG_ERR_NO_MEMORY, "digit planes (%.2f GB)", digits * (double)plane / 1e9);
     /* both operands are staged in boxes of 128 rows x 64 bytes */
     int rc = xg_encode(&D.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, D.dig, M.ts, digits * rows, 64, 128,
@@ -1468,46 +1487,104 @@ int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits)
     return XG_OK;
 }
 
-/* Gives the seven-digit planes of M back (other allocations come first) */
-bool xg_i8_release(XgTileMatrix &M)
+/* The matrices that hold seven-digit planes.  Handles may be used from several
+ * threads, so the list, i8 and i8_users change under its mutex only; the
+ * planes of a matrix in use (XgI8Use) stay. */
+static std::mutex g_i8_mutex;
+static std::vector<XgTileMatrix *> &xg_i8_list()
 {
-    M.no_i8 = true;
-    if (!M.i8) return false;
+    static std::vector<XgTileMatrix *> *list = new std::vector<XgTileMatrix *>(); /* outlives handles closed at exit */
+    return *list;
+}
+
+XgI8Use::XgI8Use(XgTileMatrix &m) : M(m)
+{
+    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    ++M.i8_users;
+}
+
+XgI8Use::~XgI8Use()
+{
+    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    --M.i8_users;
+}
+
+/* with the mutex held */
+static void xg_i8_drop(XgTileMatrix &M)
+{
+    std::vector<XgTileMatrix *> &list = xg_i8_list();
+    list.erase(std::remove(list.begin(), list.end(), &M), list.end());
     xg_sliced_destroy(M.i8);
     M.i8 = nullptr;
     M.i8_factor = false;
+}
+
+static void xg_i8_free(XgTileMatrix &M)
+{
+    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    if (M.i8) xg_i8_drop(M);
+    M.i8_factor = false;
+}
+
+/* Gives the planes of every idle matrix back to the device; whether there were any */
+static bool xg_i8_take_back()
+{
+    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    const std::vector<XgTileMatrix *> held = xg_i8_list();
+    bool any = false;
+    for (XgTileMatrix *M : held)
+        if (M->i8_users == 0) {
+            xg_i8_drop(*M);
+            any = true;
+        }
+    return any;
+}
+
+/* Whether the planes of the factor (inverse: of its inverse too) belong to the
+ * plan of M: by its size and the device's memory alone, so that the path, and
+ * with it the last digits of a result, depend neither on the order of a
+ * program's calls nor on what else was allocated when the first was made.  A
+ * quarter of what the device has beside the matrix (its planes and the store
+ * of the inverse): on 180 GB up to N = 100000, gradients up to 86000. */
+static bool xg_i8_planned(const XgTileMatrix &M, bool inverse)
+{
+    const double e = (double)M.ntiles * M.ts * M.ts;
+    return 4.0 * 7.0 * e <= (double)g_xg.memory - (inverse ? 23.0 : 8.0) * e;
+}
+
+/* Whether the device has room for them now with three times as much, or a
+ * sixteenth of its memory, left for others.  Where it has not, the call runs on
+ * DMMA and the next one asks again. */
+static bool xg_i8_room(const XgTileMatrix &M)
+{
+    const size_t bytes = 7 * (size_t)M.ntiles * M.ts * M.ts;
+    size_t fr = 0, total = 0;
+    return cudaMemGetInfo(&fr, &total) == cudaSuccess && fr >= bytes + std::min(3 * bytes, g_xg.memory / 16);
+}
+
+/* The planes of M for a factorisation, allocated where they are wanted and
+ * missing; the caller holds an XgI8Use */
+static bool xg_i8_acquire(XgTileMatrix &M)
+{
+    if (M.i8) return true;
+    XgSliced *s = nullptr;
+    if (!xg_i8_planned(M, false) || !xg_i8_room(M) || xg_sliced_create(&s, M, 7) != XG_OK) return false;
+    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    M.i8 = s;
+    xg_i8_list().push_back(&M);
     return true;
 }
 
-/* whether the device has `bytes` and three times as much for others */
-static bool xg_i8_memory(size_t bytes)
+static bool xg_i8_acquire_inverse(XgTileMatrix &M)
 {
-    size_t fr = 0, total = 0;
-    return cudaMemGetInfo(&fr, &total) == cudaSuccess && bytes <= fr / 4;
-}
-
-static bool xg_i8_prepare(XgTileMatrix &M)
-{
-    if (M.i8) return true;
-    if (M.no_i8) return false;
-    const size_t bytes = 7 * (size_t)M.ntiles * M.ts * M.ts;
-    if (!xg_i8_memory(bytes) || xg_sliced_create(&M.i8, M, 7) != XG_OK) M.no_i8 = true;
-    return M.i8 != nullptr;
-}
-
-static bool xg_i8_prepare_inverse(XgTileMatrix &M)
-{
-    const size_t bytes = 7 * (size_t)M.ntiles * M.ts * M.ts;
-    return xg_i8_memory(bytes) && xg_digits_alloc(M.i8->X, M, 7) == XG_OK;
+    return M.i8->X.dig || (xg_i8_planned(M, true) && xg_i8_room(M) && xg_digits_alloc(M.i8->X, M, 7) == XG_OK);
 }
 
 int xg_field_set_sliced(XgField *f)
 {
     if (f->sl) return XG_OK;
     if (f->C.ts % 128 != 0) return xg_fail(XG_ERR_BAD_ARGUMENT, "the sliced path needs a tile size multiple of 128");
-    int rc = xg_sliced_create(&f->sl, f->C, 4);
-    if (rc == XG_ERR_NO_MEMORY && xg_i8_release(f->C)) rc = xg_sliced_create(&f->sl, f->C, 4);
-    return rc;
+    return xg_sliced_create(&f->sl, f->C, 4);
 }
 
 /* Factorisation with FP64 tiles and INT8-sliced updates; a column's panel is
@@ -1672,9 +1749,7 @@ int xg_field_loglik_grad_sliced(XgField *f, const double *theta, double *res, do
     XgSliced *sl = f->sl;
     if ((rc = xg_grad_workspace(f))) return rc;
     const int ts = f->C.ts, nt = f->C.nt;
-    if (!sl->X.dig && (rc = xg_digits_alloc(sl->X, f->C, 4))) {
-        if (rc != XG_ERR_NO_MEMORY || !xg_i8_release(f->C) || (rc = xg_digits_alloc(sl->X, f->C, 4))) return rc;
-    }
+    if (!sl->X.dig && (rc = xg_digits_alloc(sl->X, f->C, 4))) return rc;
     rc = xg_field_loglik_sliced(f, theta, res, times);
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
@@ -1889,6 +1964,7 @@ int xg_predict_run(XgPredict *q, const double *theta, int kernel, int metric, co
     const int nmiss = q->nmiss, nobs = q->nobs;
     /* bivariate: nmiss and nobs count matrix rows, two per location */
     const int lmiss = xg_bivariate(kernel) ? nmiss / 2 : nmiss, lobs = xg_bivariate(kernel) ? nobs / 2 : nobs;
+    XgI8Use use(q->C22);
     XgTileArgs T{q->C22.d, q->C22.ts, q->C22.nt};
     const XgMaternParams p = xg_params(theta, kernel);
     const size_t Np = (size_t)q->C22.nt * q->C22.ts;
@@ -1946,8 +2022,11 @@ int xg_covariance_dense(int n, const double *x, const double *y, const double *t
     const XgMaternParams p = xg_params(theta, kernel);
     cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
     xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, p, metric, 1, f->C.tab, st);
-    if (factor) xg_factor(f->C, nullptr, f->part, f->status, f->info, st);
-    rc = xg_tiles_to_dense(f, n, out);
+    {
+        XgI8Use use(f->C);
+        if (factor) xg_factor(f->C, nullptr, f->part, f->status, f->info, st);
+        rc = xg_tiles_to_dense(f, n, out);
+    }
     xg_field_destroy(f);
     return rc;
 }
@@ -1958,7 +2037,7 @@ int xg_bessel_knu_host(int n, const double *nu, const double *x, double *out)
     if (rc) return rc;
     if (n <= 0) return XG_OK;
     double *d = nullptr;
-    XG_CU(cudaMalloc(&d, 3 * (size_t)n * sizeof(double)));
+    XG_CU(xg_malloc(&d, 3 * (size_t)n * sizeof(double)));
     cudaStream_t st = g_xg.stream;
     cudaMemcpyAsync(d, nu, n * sizeof(double), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d + n, x, n * sizeof(double), cudaMemcpyHostToDevice, st);
@@ -1979,7 +2058,7 @@ int xg_matern_pairs_host(int n, const double *x1, const double *y1, const double
     if (rc) return rc;
     if (n <= 0) return XG_OK;
     double *d = nullptr;
-    XG_CU(cudaMalloc(&d, 5 * (size_t)n * sizeof(double)));
+    XG_CU(xg_malloc(&d, 5 * (size_t)n * sizeof(double)));
     cudaStream_t st = g_xg.stream;
     const double *src[4] = {x1, y1, x2, y2};
     for (int i = 0; i < 4; ++i)

@@ -16,6 +16,7 @@ struct XgContext {
     int device = 0;
     int sm_count = 0;
     int dts = 0;
+    size_t memory = 0; /* of the device, in bytes */
     cudaStream_t stream = nullptr;    /* trailing updates, generation, solves */
     cudaStream_t stream_hi = nullptr; /* high priority: the lookahead panel (POTRF + TRSM) */
     std::mutex mu;
@@ -50,7 +51,13 @@ struct XgPart {
     size_t bytes;
     template <class T> XgPart(T **q, size_t n) : p((void **)q), bytes(n * sizeof(T)) {}
 };
-cudaError_t xg_alloc_parts(const XgPart *parts, int n);
+cudaError_t xg_alloc_parts(const XgPart *parts, int n, bool take_back = true);
+
+/* cudaMalloc that gives the digit planes of idle matrices back to the device
+ * (XgTileMatrix::i8, a cache) before it reports that there is no memory; *p is
+ * null then and no error is left behind */
+cudaError_t xg_malloc_bytes(void **p, size_t bytes);
+template <class T> cudaError_t xg_malloc(T **p, size_t bytes) { return xg_malloc_bytes((void **)p, bytes); }
 
 struct XgTileMatrix {
     int N = 0, ts = 0, nt = 0;
@@ -63,10 +70,22 @@ struct XgTileMatrix {
     /* tile DAG and backward solve: next task, abort flag and block flags of each;
      * null where the matrix is factored by the per-step launches only */
     int *dag = nullptr;
-    XgSliced *i8 = nullptr; /* seven-digit planes: large FP64 factorisations on the INT8 tensor cores */
-    bool no_i8 = false;     /* their memory was refused or given back */
+    /* seven-digit planes: large FP64 factorisations on the INT8 tensor cores.
+     * Kept between calls; any allocation of the library that finds no memory takes
+     * them, unless a call is using them (XgI8Use), and the next call asks again. */
+    XgSliced *i8 = nullptr;
+    int i8_users = 0;
     bool i8_factor = false; /* the last factorisation went through them (they hold L) */
     double *tab = nullptr; /* element tables of the current parameters (xg_matern_tab.cuh) */
+};
+
+/* For as long as a call may use M's digit planes: nothing takes them back */
+struct XgI8Use {
+    XgTileMatrix &M;
+    explicit XgI8Use(XgTileMatrix &m);
+    ~XgI8Use();
+    XgI8Use(const XgI8Use &) = delete;
+    XgI8Use &operator=(const XgI8Use &) = delete;
 };
 
 /* Banded mixed-precision workspace (mixed.cu): compact FP64 band tiles,
@@ -140,7 +159,6 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
 void xg_factor_two(XgTileMatrix &A, XgTileMatrix &B, double *part_a, double *part_b, int *status, int *info,
                    const XgFactorStreams &fs);
 int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits);
-bool xg_i8_release(XgTileMatrix &M);
 void xg_inverse_product(XgTileMatrix &M, XgTileMatrix &X, int *status, const XgFactorStreams &fs);
 void xg_solve_transposed(XgTileMatrix &M, double *v, int *status, cudaStream_t st);
 double xg_trailing_flops(int nt, int ts, int k);

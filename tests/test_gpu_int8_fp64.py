@@ -87,3 +87,89 @@ def test_the_digit_planes_are_given_back(gpu, ora):
         torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[2] < 64 << 20, free
+
+
+class _Full:
+    """The device's memory but for `leave` bytes, held by another library."""
+
+    def __init__(self, leave):
+        import torch
+
+        torch.cuda.empty_cache()
+        self.t = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        import torch
+
+        del self.t
+        torch.cuda.empty_cache()
+
+
+def test_the_path_does_not_depend_on_the_order_of_calls(gpu, ora):
+    """Objective, gradient, objective, or the gradient first: the same values;
+    and a session that found no memory for the planes takes them, with the
+    same values again, once there is some."""
+    import torch
+
+    n, theta = 6657, [1.3, 0.07, 0.73]
+    x, y = ora.generate_xy_loc(n, 3)
+    z = np.random.default_rng(1).standard_normal(n)
+    with gpu.Session(x, y, dts=512) as s:
+        s.set_data(z=z)
+        ref = s.loglik(theta)
+        ll, gref = s.loglik(theta, grad=True)
+        assert ll == ref == s.loglik(theta)
+    with gpu.Session(x, y, dts=512) as s:
+        s.set_data(z=z)
+        ll, g = s.loglik(theta, grad=True)
+        assert ll == ref and np.array_equal(g, gref) and s.loglik(theta) == ref
+    with _Full(600 << 20):  # 0.22 GB of tiles, 0.19 of planes
+        s = gpu.Session(x, y, dts=512)
+        s.set_data(z=z)
+        free = torch.cuda.mem_get_info()[0]
+        assert s.loglik(theta) == pytest.approx(ref, rel=2e-12)
+        assert free - torch.cuda.mem_get_info()[0] < 16 << 20
+    ll, g = s.loglik(theta, grad=True)
+    s.close()
+    assert ll == ref and np.array_equal(g, gref)
+
+
+@pytest.mark.parametrize("what", ["session", "batch", "kriging", "assessment", "mixed"])
+def test_idle_planes_make_room_for_others(gpu, ora, what):
+    """An allocation that the device refuses while an idle session holds its
+    planes (0.31 GB) gets their memory; the session evaluates without them,
+    and with them again when there is room."""
+    n, m, theta = 9000, 50, [1.0, 0.1, 0.5]
+    x, y = ora.generate_xy_loc(n + m, 3)
+    z = np.random.default_rng(1).standard_normal(n + m)
+    k = 6000
+
+    def other(s):
+        if what == "session":
+            with gpu.Session(x[:k], y[:k], dts=256) as t:
+                t.set_data(z=z[:k])
+                return t.loglik(theta)
+        if what == "batch":
+            with gpu.Batch([x[:4000], x[4000:8000]], [y[:4000], y[4000:8000]], [z[:4000], z[4000:8000]]) as b:
+                return b.loglik([theta] * 2)
+        if what == "kriging":
+            return s.predict(theta, x[n:], y[n:], x[:k], y[:k], z[:k])[1]
+        if what == "mixed":
+            with gpu.Session(x[:4096], y[:4096], dts=256) as t:
+                t.set_data(z=z[:4096])
+                t.set_mixed(band=12)
+                return t.loglik(theta)
+        return gpu.mloe_mmom_host(x[n:], y[n:], x[:4000], y[:4000], theta, [1.1, 0.09, 0.52])[2]
+
+    with gpu.Session(x[:n], y[:n], dts=512) as s:
+        s.set_data(z=z[:n])
+        ref = s.loglik(theta)
+        want = other(s)
+        assert s.loglik(theta) == ref
+        with _Full(100 << 20):
+            assert np.array_equal(other(s), want)
+            assert s.loglik(theta) == pytest.approx(ref, rel=2e-12)
+        assert s.loglik(theta) == ref
