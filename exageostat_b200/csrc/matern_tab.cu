@@ -81,7 +81,8 @@ template <bool GRAD> __global__ void __launch_bounds__(64) xg_tab_build_kernel(d
  * elements are the same */
 __device__ __forceinline__ bool xg_tab_wanted(const XgMaternParams &p, int n)
 {
-    return p.half_integer < 0 && n >= XG_TAB_MIN_N && p.nu <= XG_TAB_NU;
+    return p.half_integer < 0 && n >= XG_TAB_MIN_N && p.nu <= XG_TAB_NU && xg_tab_scale_ok(p.con) &&
+           xg_tab_scale_ok(p.con / p.beta);
 }
 
 /* the tables of every field of a batch (blockIdx.y and on by gridDim.y, which
@@ -389,8 +390,10 @@ static unsigned xg_tab_grid(long long units, int per_sm)
 
 bool xg_tab_covers(const XgMaternParams &p, int n)
 {
-    if (n < XG_TAB_MIN_N || !(p.nu <= XG_TAB_NU)) return false;
-    return !p.bivariate || (p.nu2 <= XG_TAB_NU && p.nu12 <= XG_TAB_NU);
+    if (n < XG_TAB_MIN_N || !(p.nu <= XG_TAB_NU) || !xg_tab_scale_ok(p.con)) return false;
+    if (p.bivariate)
+        return p.nu2 <= XG_TAB_NU && p.nu12 <= XG_TAB_NU && xg_tab_scale_ok(p.con2) && xg_tab_scale_ok(p.con12);
+    return xg_tab_scale_ok(p.con / p.beta); /* of the derivatives; the covariance follows the same rule */
 }
 
 void xg_launch_gen_tab(const XgTileArgs &T, const int2 *tile_ij, long long ntiles, const double *xr, const double *yr,

@@ -33,6 +33,16 @@
 #define XG_TAB_BASE ((1023 - 16) << 4) /* leading bits of 2^-16 */
 #define XG_TAB_NU 5.0
 
+/* Whether tables of functions with the constant c hold them to full precision:
+ * the power-8 coefficients are up to 2^168 times the function on the smallest
+ * intervals and 2^-80 of it on the largest, so constants near the ends of the
+ * double range would overflow or lose bits there. */
+XG_HD inline bool xg_tab_scale_ok(double c)
+{
+    c = fabs(c);
+    return c == 0.0 || (c > 1.4996968138956309e-241 && c < 6.668014432879854e+240); /* 2^-800, 2^800 */
+}
+
 XG_HD inline uint64_t xg_tab_bits(double r)
 {
 #ifdef __CUDA_ARCH__

@@ -30,3 +30,33 @@ def test_table_elements_match_the_direct_form(gpu, nu, beta):
     assert np.all(err <= tol[big]), (err.max(), r[big][np.argmax(err / tol[big])])
     assert np.all(np.abs(C[i, j][~big]) <= 1.1e-290)
     assert np.array_equal(np.diag(C), np.full(n, 1.3))
+
+
+@pytest.mark.parametrize("e", [-960, -900, -700, 700, 900, 1000])
+def test_variances_at_the_ends_of_the_double_range(gpu, e):
+    """Powers of two as variances scale the covariance exactly: elements as
+    the direct form gives them, near neighbours included, and the gradient of
+    sigma^2 = 1 with the observations scaled, to 1e-9 of its largest entry."""
+    rng = np.random.default_rng(13)
+    n, s2 = 300, 2.0 ** e
+    x, y, z = rng.uniform(size=n), rng.uniform(size=n), rng.standard_normal(n)
+    x[1:100] = x[0] + 10.0 ** rng.uniform(-7, -3, 99)
+    y[1:100] = y[0]
+    i, j = np.tril_indices(n, -1)
+    r = np.hypot(x[i] - x[j], y[i] - y[j]) / 0.1
+    for nu in (0.3, 1.0, 2.2):
+        C = gpu.covariance_dense(x, y, [s2, 0.1, nu], ts=256)[i, j]
+        direct = gpu.matern_pairs(x[i], y[i], x[j], y[j], [s2, 0.1, nu])
+        tol = 2e-14 + 2.3e-16 * (r + (nu + 0.5) * np.abs(np.log(np.maximum(r, 1e-300))))
+        big = direct > 1e-290
+        assert np.all(np.isfinite(C)) and np.all(np.abs(C - direct)[big] <= (tol * direct)[big])
+        g = []
+        for s in (1.0, s2):
+            theta = [s, 0.1, nu, 0.25 * s]
+            with gpu.Session(x, y, kernel=1) as h:
+                h.set_data(z=z * np.sqrt(s))
+                g.append(h.loglik(theta, grad=True)[1] * [s, 1.0, 1.0, s])
+            with gpu.Batch([x], [y], [z * np.sqrt(s)], kernel=1) as b:
+                g.append(b.loglik([theta], grad=True)[1][0] * [s, 1.0, 1.0, s])
+        for v in g[1:]:
+            assert np.abs(v - g[0]).max() <= 1e-9 * np.abs(g[0]).max(), (nu, g)
