@@ -464,7 +464,7 @@ int xg_field_fisher(XgField *f, const double *theta, int kernel, double *F, doub
     const XgPart parts[] = {{&Y, nsys * full}, {&part, 10 * (size_t)nctas}, {&w, words}};
     if (xg_alloc_parts(parts, 3) != cudaSuccess)
         return xg_fail(XG_ERR_NO_MEMORY, "Fisher workspace: %.2f GB", nsys * full * sizeof(double) / 1e9);
-    XgI8Use use(f->C);
+    XgI8Use use(f->C, xg_params(theta, kernel));
     std::vector<double> hp(10 * (size_t)nctas);
     int sv[2] = {0, 0};
     XgRowsMaps maps = {};
@@ -610,10 +610,10 @@ int xg_assess_run(XgAssess *q, const double *truth, const double *est, int kerne
     int rc = xg_check_theta(truth, kernel);
     if (!rc) rc = xg_check_theta(est, kernel);
     if (rc) return rc;
-    XgI8Use use_a(q->Ca), use_t(q->Ct);
     cudaStream_t st = g_xg.stream;
     const int nmiss = q->nmiss, nobs = q->nobs, nt = q->nt, mt = q->mt, ts = q->ts;
     const XgMaternParams pt = xg_params(truth, kernel), pa = xg_params(est, kernel);
+    XgI8Use use_a(q->Ca, pa), use_t(q->Ct, pt);
     double *RA = q->R[0], *RU = q->R[1], *RT = q->R[2], *RW = q->R[3], *RV = q->R[4];
     const size_t rbytes = (size_t)mt * nt * ts * ts * sizeof(double);
     XG_ACU(cudaMemsetAsync(q->status, 0, 2 * sizeof(int), st));

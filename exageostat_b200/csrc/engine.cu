@@ -670,7 +670,7 @@ int xg_factor_lookahead(XgTileMatrix &M, double *v, double *part, int *status, i
     /* profiled evaluations keep the per-step launches, whose kernels the profile tells apart */
     M.i8_factor = false;
     if (M.dag && !fs.pev) {
-        if (M.N >= xg_i8_min(M.ts) && xg_i8_acquire(M)) {
+        if (M.N >= xg_i8_min(M.ts) && M.i8_scale && xg_i8_acquire(M)) {
             M.i8_factor = true;
             return xg_factor_sliced(M, M.i8, v, part, status, fs);
         }
@@ -917,10 +917,10 @@ int xg_field_loglik(XgField *f, const double *theta, double *res, double *times)
     int rc = xg_check_theta(theta, f->kernel);
     if (rc) return rc;
     if (!f->have_z) return xg_fail(XG_ERR_BAD_ARGUMENT, "no observations: call MLE_zvg or set z first");
-    XgI8Use use(f->C);
     cudaStream_t st = g_xg.stream;
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, f->kernel);
+    XgI8Use use(f->C, p);
     const size_t Np = (size_t)f->C.nt * f->C.ts;
     XG_CU(cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemcpyAsync(f->v, f->z, Np * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -960,10 +960,10 @@ int xg_field_zvg(XgField *f, const double *theta, const double *nrand, double *t
 {
     int rc = xg_check_theta(theta, f->kernel);
     if (rc) return rc;
-    XgI8Use use(f->C);
     cudaStream_t st = g_xg.stream;
     XgTileArgs T{f->C.d, f->C.ts, f->C.nt};
     const XgMaternParams p = xg_params(theta, f->kernel);
+    XgI8Use use(f->C, p);
     XG_CU(cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemcpyAsync(f->e, nrand, f->N * sizeof(double), cudaMemcpyHostToDevice, st));
     XG_CU(cudaEventRecord(f->ev[0], st));
@@ -1050,11 +1050,12 @@ int xg_field_loglik_grad(XgField *f, const double *theta, double *res, double *g
 {
     int rc = xg_grad_workspace(f);
     if (rc) return rc;
-    XgI8Use use(f->C); /* the factor's planes serve its inverse */
+    if ((rc = xg_check_theta(theta, f->kernel))) return rc;
+    const XgMaternParams p = xg_params(theta, f->kernel);
+    XgI8Use use(f->C, p); /* the factor's planes serve its inverse */
     rc = xg_field_loglik(f, theta, res, times);
     if (rc) return rc;
     cudaStream_t st = g_xg.stream;
-    const XgMaternParams p = xg_params(theta, f->kernel);
     const double dlogcon = -(log(2.0) + xg_digamma(theta[2]));
     XG_CU(cudaEventRecord(f->ev[0], st));
     xg_solve_transposed(f->C, f->v, f->status, st);
@@ -1497,8 +1498,15 @@ static std::vector<XgTileMatrix *> &xg_i8_list()
     return *list;
 }
 
-XgI8Use::XgI8Use(XgTileMatrix &m) : M(m)
+/* The epilogue weights a product with s_row s_column 254^-6: a subnormal number
+ * where the factor (or, for the largest variances, its inverse) is near the low
+ * end of the double range.  At sigma^2 = 2^-1000, N = 6700, order 0.5 l was
+ * wrong by 1.1e-10 of itself, on DMMA by 9e-15. */
+static bool xg_i8_scale_ok(double v) { return v > ldexp(1.0, -800) && v < ldexp(1.0, 800); }
+
+XgI8Use::XgI8Use(XgTileMatrix &m, const XgMaternParams &p) : M(m)
 {
+    M.i8_scale = xg_i8_scale_ok(p.sigma2 + p.nugget) && (!p.bivariate || xg_i8_scale_ok(p.sigma2b));
     std::lock_guard<std::mutex> lk(g_i8_mutex);
     ++M.i8_users;
 }
@@ -1964,9 +1972,9 @@ int xg_predict_run(XgPredict *q, const double *theta, int kernel, int metric, co
     const int nmiss = q->nmiss, nobs = q->nobs;
     /* bivariate: nmiss and nobs count matrix rows, two per location */
     const int lmiss = xg_bivariate(kernel) ? nmiss / 2 : nmiss, lobs = xg_bivariate(kernel) ? nobs / 2 : nobs;
-    XgI8Use use(q->C22);
     XgTileArgs T{q->C22.d, q->C22.ts, q->C22.nt};
     const XgMaternParams p = xg_params(theta, kernel);
+    XgI8Use use(q->C22, p);
     const size_t Np = (size_t)q->C22.nt * q->C22.ts;
     XG_CU(cudaMemsetAsync(q->status, 0, 2 * sizeof(int), st));
     XG_CU(cudaMemsetAsync(q->v, 0, Np * sizeof(double), st));
@@ -2023,7 +2031,7 @@ int xg_covariance_dense(int n, const double *x, const double *y, const double *t
     cudaMemsetAsync(f->status, 0, 2 * sizeof(int), st);
     xg_launch_gen(T, f->C.ij, f->C.ntiles, f->x, f->y, f->x, f->y, n, n, p, metric, 1, f->C.tab, st);
     {
-        XgI8Use use(f->C);
+        XgI8Use use(f->C, p);
         if (factor) xg_factor(f->C, nullptr, f->part, f->status, f->info, st);
         rc = xg_tiles_to_dense(f, n, out);
     }

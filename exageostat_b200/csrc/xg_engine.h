@@ -75,14 +75,16 @@ struct XgTileMatrix {
      * them, unless a call is using them (XgI8Use), and the next call asks again. */
     XgSliced *i8 = nullptr;
     int i8_users = 0;
+    bool i8_scale = false; /* this call's variances suit them */
     bool i8_factor = false; /* the last factorisation went through them (they hold L) */
     double *tab = nullptr; /* element tables of the current parameters (xg_matern_tab.cuh) */
 };
 
-/* For as long as a call may use M's digit planes: nothing takes them back */
+/* For as long as a call with the parameters p may use M's digit planes:
+ * nothing takes them back */
 struct XgI8Use {
     XgTileMatrix &M;
-    explicit XgI8Use(XgTileMatrix &m);
+    XgI8Use(XgTileMatrix &m, const XgMaternParams &p);
     ~XgI8Use();
     XgI8Use(const XgI8Use &) = delete;
     XgI8Use &operator=(const XgI8Use &) = delete;

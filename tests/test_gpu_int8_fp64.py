@@ -173,3 +173,20 @@ def test_idle_planes_make_room_for_others(gpu, ora, what):
             assert np.array_equal(other(s), want)
             assert s.loglik(theta) == pytest.approx(ref, rel=2e-12)
         assert s.loglik(theta) == ref
+
+
+@pytest.mark.parametrize("e", [-1000, -700, 700, 1000])
+def test_variances_at_the_ends_of_the_double_range(gpu, ora, e):
+    """Powers of two as variances: l and the gradient of sigma^2 = 1 with the
+    observations scaled, within the file's bars."""
+    n, s2 = 6657, 2.0 ** e
+    x, y = ora.generate_xy_loc(n, 3)
+    z = np.random.default_rng(1).standard_normal(n)
+    got = []
+    for s in (1.0, s2):
+        with gpu.Session(x, y, dts=512) as h:
+            h.set_data(z=z * np.sqrt(s))
+            ll, g = h.loglik([s, 0.1, 0.5], grad=True)
+        got.append((ll + 0.5 * n * np.log(s), g * [s, 1.0, 1.0]))
+    assert got[1][0] == pytest.approx(got[0][0], rel=2e-12)
+    assert np.abs(got[1][1] - got[0][1]).max() <= 1e-9 * np.abs(got[0][1]).max()
