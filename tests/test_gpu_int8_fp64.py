@@ -190,3 +190,39 @@ def test_variances_at_the_ends_of_the_double_range(gpu, ora, e):
         got.append((ll + 0.5 * n * np.log(s), g * [s, 1.0, 1.0]))
     assert got[1][0] == pytest.approx(got[0][0], rel=2e-12)
     assert np.abs(got[1][1] - got[0][1]).max() <= 1e-9 * np.abs(got[0][1]).max()
+
+
+@pytest.mark.parametrize("kernel,theta,ts", [
+    (2, [1.0, 2.0, 0.03, 0.5, 1.1, 0.4], 512),
+    (2, [1e-6, 3.0, 0.03, 0.5, 0.7, -0.3], 256),
+    (3, [0.08, 0.12, 1.0, 0.2, 0.5, 1.0, 0.2, 0.8, 1.24479, 4.41137, -0.4], 512),
+])
+def test_bivariate_fields(gpu, ora, kernel, theta, ts):
+    """Interleaved rows of two variances and orders, against the DMMA path
+    (kernel 3, whose ranges are three times longer, to the 1e-10 of its own
+    test)."""
+    n = 6658
+    x, y = ora.generate_xy_loc(n // 2, 3)
+    z = np.random.default_rng(1).standard_normal(n)
+    z[0::2] *= np.sqrt(theta[0]) if kernel == 2 else 1.0
+    got = []
+    for t in (ts, 128):
+        with gpu.Session(x, y, kernel=kernel, dts=t) as s:
+            s.set_data(z=z)
+            got.append(s.loglik(theta))
+    assert got[0] == pytest.approx(got[1], rel=2e-12 if kernel == 2 else 1e-10)
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_assessment(gpu, ora, kernel):
+    """Fisher matrix and MLOE / MMOM from seven-digit factors against tiles of
+    128, the bars of their own tests."""
+    n, m = 6657, 130
+    x, y = ora.generate_xy_loc(n + m, 3)
+    truth, est = [1.3, 0.07, 0.73] + [0.05] * kernel, [1.1, 0.08, 0.7] + [0.04] * kernel
+    F = [gpu.fisher_host(x[m:], y[m:], truth, kernel=kernel, ts=t) for t in (512, 128)]
+    scale = np.sqrt(np.outer(np.diag(F[1]), np.diag(F[1])))
+    assert (np.abs(F[0] - F[1]) / scale).max() < 1e-8
+    a, b = [gpu.mloe_mmom_host(x[:m], y[:m], x[m:], y[m:], truth, est, kernel=kernel, ts=t) for t in (512, 128)]
+    assert np.abs(a[2][:, :4] - b[2][:, :4]).max() < 1e-9 * truth[0]
+    assert abs(a[0] - b[0]) < 1e-8 and abs(a[1] - b[1]) < 1e-8

@@ -109,3 +109,42 @@ def test_failing_pivot_of_every_panel(gpu, ora, ts):
                 assert ll[1] == -np.inf and ll[0] == ll[2] == pytest.approx(ref, rel=1e-12)
         s.set_data(x=x)
         assert s.loglik(THETA) == ref
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("n,ts", [(1, 128), (127, 128), (129, 128), (385, 128), (257, 256), (513, 256), (700, 384),
+                                  (1153, 384), (513, 512), (1300, 512)])
+def test_per_step_factorisation(gpu, ora, n, ts, kernel):
+    """The per-step launches (a profiled evaluation runs them at any size) and
+    what reads their factor and inverted diagonal blocks afterwards: l against
+    the oracle to 1e-10, l and the gradient against the one-launch
+    factorisation to 1e-10 and 1e-9 of its largest entry."""
+    theta = [1.0, 0.1, 0.73] + [0.05] * kernel
+    x, y = ora.generate_xy_loc(n, 8)
+    z = ora.dzvg(x, y, theta, ora.dlarnv(9, n), kernel)
+    ref = ora.dmle(x, y, z, theta, kernel)[0]
+    with gpu.Session(x, y, kernel=kernel, dts=ts) as s:
+        s.set_data(z=z)
+        l0, g0 = s.loglik(theta, grad=True)
+        s.set_profiling(True)
+        assert s.loglik(theta) == pytest.approx(ref, rel=1e-10)
+        l1, g1 = s.loglik(theta, grad=True)
+        s.set_profiling(False)
+        assert l1 == pytest.approx(l0, rel=1e-10)
+        assert np.abs(g1 - g0).max() <= 1e-9 * np.abs(g0).max()
+        assert s.loglik(theta) == l0
+
+
+def test_per_step_factorisation_past_the_dataflow_sizes(gpu, ora):
+    """N = 22145 at tiles of 128 takes the per-step launches without a profile:
+    l and gradient against the seven-digit path, the bars of its own test."""
+    n, theta = 22145, [1.0, 0.1, 0.5]
+    x, y = ora.generate_xy_loc(n, 3)
+    z = np.random.default_rng(1).standard_normal(n)
+    got = []
+    for ts in (512, 128):
+        with gpu.Session(x, y, dts=ts) as s:
+            s.set_data(z=z)
+            got.append(s.loglik(theta, grad=True))
+    assert got[1][0] == pytest.approx(got[0][0], rel=2e-12)
+    assert np.abs(got[1][1] - got[0][1]).max() <= 1e-9 * np.abs(got[0][1]).max()
