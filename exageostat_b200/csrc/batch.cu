@@ -88,22 +88,39 @@ struct XgBatch {
     std::vector<int2 *> ij_by_nt;
 };
 
-static void xg_batch_free(XgBatch *b)
+/* the gradient workspace, whole or as far as it was made */
+static void xg_batch_grad_free(XgBatch *b)
 {
-    if (!b) return;
-    if (b->graph) cudaGraphExecDestroy(b->graph);
     for (int s = 0; s < XgBatch::GS; ++s) {
         if (b->gpart[s]) cudaFree(b->gpart[s]);
         if (b->gtab[s]) cudaFree(b->gtab[s]);
         if (b->gst[s]) cudaStreamDestroy(b->gst[s]);
+        b->gpart[s] = b->gtab[s] = nullptr;
+        b->gst[s] = nullptr;
     }
     if (b->ev) cudaEventDestroy(b->ev);
+    b->ev = nullptr;
     for (int2 *p : b->ij_by_nt)
         if (p) cudaFree(p);
-    if (b->gout) cudaFree(b->gout);
+    b->ij_by_nt.clear();
+    void *dev[] = {b->xstore, b->R_dev, b->rtasks, b->rwords, b->gout};
+    for (void *p : dev)
+        if (p) cudaFree(p);
+    b->xstore = b->gout = nullptr;
+    b->R_dev = nullptr;
+    b->rtasks = nullptr;
+    b->rwords = nullptr;
     if (b->h_gout) cudaFreeHost(b->h_gout);
+    b->h_gout = nullptr;
+}
+
+static void xg_batch_free(XgBatch *b)
+{
+    if (!b) return;
+    if (b->graph) cudaGraphExecDestroy(b->graph);
+    xg_batch_grad_free(b);
     void *dev[] = {b->F_dev, b->tiles, b->x, b->y, b->z, b->v, b->part, b->out, b->status, b->table_buf,
-                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv, b->tab, b->xstore, b->R_dev, b->rtasks, b->rwords};
+                   b->tasks, b->ttasks, b->D_dev, b->words, b->twords, b->dinv, b->tab};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (b->F_pinned) cudaFreeHost(b->F_pinned);
@@ -552,10 +569,8 @@ static void xg_group_order(const std::vector<XgRowsField> &R, int f0, int f1, st
         for (int J = 0; J <= c.J; ++J) tl.push_back(make_int4(c.f, c.J, J, 1));
 }
 
-/* gradient workspace of a batch (first gradient request) */
-static int xg_batch_grad_workspace(XgBatch *b)
+static int xg_batch_grad_create(XgBatch *b)
 {
-    if (b->gout) return XG_OK;
     const int ts = b->ts;
     long long maxblocks = 0;
     b->ij_by_nt.assign(b->maxnt + 1, nullptr);
@@ -625,6 +640,16 @@ static int xg_batch_grad_workspace(XgBatch *b)
     XG_CU(xg_malloc(&b->gout, 4 * (size_t)b->nfields * sizeof(double)));
     XG_CU(cudaMallocHost(&b->h_gout, 4 * (size_t)b->nfields * sizeof(double)));
     return XG_OK;
+}
+
+/* gradient workspace of a batch (first gradient request); a request that
+ * fails leaves nothing behind */
+static int xg_batch_grad_workspace(XgBatch *b)
+{
+    if (b->h_gout) return XG_OK;
+    const int rc = xg_batch_grad_create(b);
+    if (rc) xg_batch_grad_free(b);
+    return rc;
 }
 
 /* Log-likelihoods and their gradients of every field: the batched

@@ -144,3 +144,30 @@ def test_more_fields_than_a_grid_dimension(gpu, ora):
     assert np.array_equal(many, few[f])
     ref, scale = _oracle_ll(ora, x, y, z, th)
     _assert_close(few, ref, scale)
+
+
+def test_a_refused_gradient_leaves_nothing_behind(gpu, ora):
+    """Gradients of a batch whose inverse factors (71 MB for the larger field)
+    the device cannot hold: refused each time, no memory lost, and computed
+    once there is room."""
+    import torch
+
+    x, y = ora.generate_xy_loc(4000, 3)
+    z = np.random.default_rng(1).standard_normal(4000)
+    th = [[1.0, 0.05, 0.7]] * 2
+    with gpu.Batch([x, x[:900]], [y, y[:900]], [z, z[:900]]) as b:
+        ll = b.loglik(th)
+        torch.cuda.empty_cache()
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (60 << 20), dtype=torch.uint8, device="cuda")
+        free = []
+        for _ in range(12):
+            with pytest.raises(gpu.XgError) as err:
+                b.loglik(th, grad=True)
+            assert err.value.code == gpu.XG_ERR_NO_MEMORY
+            free.append(torch.cuda.mem_get_info()[0])
+        assert free[0] - free[-1] <= 4 << 20, free
+        assert np.array_equal(b.loglik(th), ll)
+        del hold
+        torch.cuda.empty_cache()
+        ll2, g = b.loglik(th, grad=True)
+        assert np.array_equal(ll2, ll) and np.all(np.isfinite(g))
