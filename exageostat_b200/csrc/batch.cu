@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/exageostat_b200.h"
+#include "xg_batch_order.h"
 #include "xg_common.cuh"
 #include "xg_engine.h"
 #include "xg_kernels.h"
@@ -308,30 +309,6 @@ extern "C" long long exageostat_b200_batch_plan(int nfields, const int *nt, int 
     return (long long)tl.size();
 }
 
-/* Block tasks of every field for the tile DAG and block columns of the
- * backward solves.  The fields advance together, each by the same share of
- * its columns (J / nb): neighbouring columns of one field then lie far apart
- * in the list, so a task rarely waits for the one before it, and the fields
- * end together, so the last columns of the largest one do not run alone. */
-static void xg_batch_order(const std::vector<XgDagField> &D, std::vector<int4> &tl, std::vector<int2> &tt)
-{
-    struct Col {
-        double key;
-        int f, J;
-    };
-    std::vector<Col> cols;
-    for (int f = 0; f < (int)D.size(); ++f)
-        for (int J = 0; J < D[f].nb; ++J) cols.push_back(Col{(double)J / D[f].nb, f, J});
-    std::sort(cols.begin(), cols.end(), [](const Col &a, const Col &b) {
-        return a.key != b.key ? a.key < b.key : a.f != b.f ? a.f < b.f : a.J < b.J;
-    });
-    tl.clear();
-    tt.clear();
-    for (const Col &c : cols)
-        for (int I = c.J; I < D[c.f].nb; ++I) tl.push_back(make_int4(c.f, I, c.J, 0));
-    for (size_t q = cols.size(); q-- > 0;) tt.push_back(make_int2(cols[q].f, cols[q].J));
-}
-
 extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const double *x, const double *y,
                                             const double *z, int kernel, int metric, int ts, void **handle)
 {
@@ -415,7 +392,11 @@ extern "C" int exageostat_b200_batch_create(int nfields, const int *n, const dou
     {
         std::vector<int4> tl;
         std::vector<int2> tt;
-        xg_batch_order(D, tl, tt);
+        const std::vector<XgBatchColumn> cols = xg_batch_columns(0, nfields, [&](int f) { return D[f].nb; });
+        xg_batch_factor_order(cols, [&](int f) { return D[f].nb; }, [&](int f, int I, int J) {
+            tl.push_back(make_int4(f, I, J, 0));
+        });
+        xg_batch_backward_order(cols, [&](int f, int J) { tt.push_back(make_int2(f, J)); });
         b->ntasks = (long long)tl.size();
         b->nttasks = (long long)tt.size();
         e = xg_malloc(&b->tasks, tl.size() * sizeof(int4));
@@ -544,31 +525,6 @@ extern "C" int exageostat_b200_batch_loglik(void *handle, const double *theta, d
 /* device memory for the inverse factors of one group of fields */
 #define XG_BATCH_X_BYTES (8ull << 30)
 
-/* The inverse tasks of fields f0 .. f1 - 1: the solves, the fields advancing
- * together by the same share of their columns as in xg_batch_order, then the
- * products, the longest sums first. */
-static void xg_group_order(const std::vector<XgRowsField> &R, int f0, int f1, std::vector<int4> &tl)
-{
-    struct Col {
-        double key;
-        int f, J;
-    };
-    std::vector<Col> cols;
-    for (int f = f0; f < f1; ++f)
-        for (int J = 0; J < R[f].nb; ++J) cols.push_back(Col{(double)J / R[f].nb, f, J});
-    std::sort(cols.begin(), cols.end(), [](const Col &a, const Col &b) {
-        return a.key != b.key ? a.key < b.key : a.f != b.f ? a.f < b.f : a.J < b.J;
-    });
-    for (const Col &c : cols)
-        for (int I = 0; I <= c.J; ++I) tl.push_back(make_int4(c.f, I, c.J, 0));
-    std::sort(cols.begin(), cols.end(), [&](const Col &a, const Col &b) {
-        const int la = R[a.f].nb - a.J, lb = R[b.f].nb - b.J;
-        return la != lb ? la > lb : a.f < b.f;
-    });
-    for (const Col &c : cols)
-        for (int J = 0; J <= c.J; ++J) tl.push_back(make_int4(c.f, c.J, J, 1));
-}
-
 static int xg_batch_grad_create(XgBatch *b)
 {
     const int ts = b->ts;
@@ -625,7 +581,10 @@ static int xg_batch_grad_create(XgBatch *b)
             tiles += n;
             g.flags += xg_num_lower_tiles(fd.nb);
         }
-        xg_group_order(R, g.f0, g.f1, tl);
+        const auto nb = [&](int q) { return R[q].nb; };
+        xg_batch_inverse_order(xg_batch_columns(g.f0, g.f1, nb), nb, [&](int q, int I, int J, int product) {
+            tl.push_back(make_int4(q, I, J, product));
+        });
         g.ntasks = (long long)tl.size() - g.task0;
         maxflags = std::max(maxflags, g.flags);
         b->groups.push_back(g);
