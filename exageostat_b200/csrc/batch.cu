@@ -7,13 +7,14 @@
  * Generation is one launch over every tile of every field; the whole
  * factorisation (with the fused log-det and z solve) of all fields is ONE
  * persistent launch of the tile DAG (tile_dag.cu): the task list -- every
- * 128 x 128 block of every field, in one topological order built here -- is
+ * 128 x 128 block of every field, in one topological order (xg_batch_order.h) -- is
  * taken by persistent CTAs, each task waiting (bounded) for the blocks it
  * reads, so the fields' columns interleave freely instead of proceeding in
  * lock-step.  The reduction to log-likelihoods is a third launch.  The
- * memsets and the three launches are captured once into a CUDA graph; each evaluation uploads the fields'
- * parameters (computed on the host exactly as for a single field) and replays
- * the graph.  Every field has its own status word, so a field whose
+ * memsets and the launches are captured once into a CUDA graph; each
+ * evaluation uploads the fields' parameters (computed on the host exactly as
+ * for a single field) and replays the graph.  Every field has its own status
+ * word, so a field whose
  * covariance is not positive definite reports -inf without stopping the
  * others.
  */

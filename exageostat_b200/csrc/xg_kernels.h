@@ -119,17 +119,6 @@ __device__ inline int xg_batch_resolve(const XgBStep &S, long long bid, long lon
 }
 
 /* (i, j) of packed lower tile t of an nt x nt tile grid */
-__host__ __device__ inline int2 xg_tile_decode(long long t, int nt)
-{
-    int j = 0;
-    while (t >= nt - j) {
-        t -= nt - j;
-        ++j;
-    }
-    return make_int2(j + (int)t, j);
-}
-
-/* the same in a constant number of steps (for the long lists of the tile DAG) */
 __device__ inline int2 xg_tile_decode_fast(long long t, int nt)
 {
     /* column j starts at j nt - j (j - 1) / 2 */
@@ -166,7 +155,7 @@ struct XgDag {
     const XgDagField *F;  /* several fields */
     const int4 *tasks;    /* (field, I, J, -) in an order that never puts a block before its operands */
     long long ntasks;
-    unsigned *next;       /* zero on launch: tasks taken beyond each CTA's first */
+    unsigned *next;       /* zero on launch: tasks taken so far */
     int *abort;           /* zero on launch; set by a wait that timed out */
     int *flags;           /* zero on launch */
     double *dinv, *v, *part; /* v may be null */
@@ -306,7 +295,7 @@ void xg_launch_sliced(const XgDigits &A, const XgDigits &B, const XgTileArgs &T,
 void xg_launch_finalize(const double *part_logdet, const double *part_dot, int nt, int N, double *out,
                         const int *status, const int *info, cudaStream_t st);
 
-/* batched fields (one launch per tile step covering every active field) */
+/* batched fields (every field's strips in one launch) */
 void xg_launch_batch_gen(const XgTileArgs &base, const XgBField *F, int nfields, const XgBStep &S, long long blocks,
                          const double *x, const double *y, int metric, double *tab, cudaStream_t st);
 void xg_launch_batch_finalize(const XgBField *F, int nfields, const double *part, double *out, cudaStream_t st);
