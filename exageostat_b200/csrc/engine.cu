@@ -19,6 +19,7 @@
 #include <sys/time.h>
 
 #include <algorithm>
+#include <condition_variable>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -130,16 +131,17 @@ int xg_choose_ts(int N, int dts)
     return ts;
 }
 
-static bool xg_i8_take_back();
+static bool xg_i8_take_back(bool in_use);
 static void xg_i8_free(XgTileMatrix &M);
 
 cudaError_t xg_malloc_bytes(void **p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && xg_i8_take_back()) {
-        cudaGetLastError();
-        e = cudaMalloc(p, bytes);
-    }
+    for (int in_use = 0; in_use < 2 && e == cudaErrorMemoryAllocation; ++in_use)
+        if (xg_i8_take_back(in_use != 0)) {
+            cudaGetLastError();
+            e = cudaMalloc(p, bytes);
+        }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
@@ -1489,13 +1491,25 @@ int xg_sliced_create(XgSliced **out, const XgTileMatrix &M, int digits)
 }
 
 /* The matrices that hold seven-digit planes.  Handles may be used from several
- * threads, so the list, i8 and i8_users change under its mutex only; the
- * planes of a matrix in use (XgI8Use) stay. */
+ * threads, so the list, i8, i8_users and i8_wanted change under its mutex only;
+ * the planes of a matrix in use (XgI8Use) stay until its call ends, which gives
+ * them back itself where an allocation waits for them. */
 static std::mutex g_i8_mutex;
+static std::condition_variable &g_i8_given = *new std::condition_variable(); /* these two outlive handles closed at exit */
 static std::vector<XgTileMatrix *> &xg_i8_list()
 {
-    static std::vector<XgTileMatrix *> *list = new std::vector<XgTileMatrix *>(); /* outlives handles closed at exit */
+    static std::vector<XgTileMatrix *> *list = new std::vector<XgTileMatrix *>();
     return *list;
+}
+
+/* with the mutex held */
+static void xg_i8_drop(XgTileMatrix &M)
+{
+    std::vector<XgTileMatrix *> &list = xg_i8_list();
+    list.erase(std::remove(list.begin(), list.end(), &M), list.end());
+    xg_sliced_destroy(M.i8);
+    M.i8 = nullptr;
+    M.i8_factor = false;
 }
 
 /* The epilogue weights a product with s_row s_column 254^-6: a subnormal number
@@ -1514,38 +1528,40 @@ XgI8Use::XgI8Use(XgTileMatrix &m, const XgMaternParams &p) : M(m)
 XgI8Use::~XgI8Use()
 {
     std::lock_guard<std::mutex> lk(g_i8_mutex);
-    --M.i8_users;
-}
-
-/* with the mutex held */
-static void xg_i8_drop(XgTileMatrix &M)
-{
-    std::vector<XgTileMatrix *> &list = xg_i8_list();
-    list.erase(std::remove(list.begin(), list.end(), &M), list.end());
-    xg_sliced_destroy(M.i8);
-    M.i8 = nullptr;
-    M.i8_factor = false;
+    if (--M.i8_users == 0 && M.i8_wanted) {
+        if (M.i8) xg_i8_drop(M);
+        M.i8_wanted = false;
+        g_i8_given.notify_all();
+    }
 }
 
 static void xg_i8_free(XgTileMatrix &M)
 {
     std::lock_guard<std::mutex> lk(g_i8_mutex);
     if (M.i8) xg_i8_drop(M);
-    M.i8_factor = false;
+    M.i8_factor = M.i8_wanted = false;
+    g_i8_given.notify_all();
 }
 
-/* Gives the planes of every idle matrix back to the device; whether there were any */
-static bool xg_i8_take_back()
+/* Gives the planes of every idle matrix back to the device, or (in_use) waits
+ * for those of the matrices in a call; whether there were any */
+static bool xg_i8_take_back(bool in_use)
 {
-    std::lock_guard<std::mutex> lk(g_i8_mutex);
+    std::unique_lock<std::mutex> lk(g_i8_mutex);
     const std::vector<XgTileMatrix *> held = xg_i8_list();
-    bool any = false;
-    for (XgTileMatrix *M : held)
-        if (M->i8_users == 0) {
+    for (XgTileMatrix *M : held) {
+        if (M->i8_users == 0)
             xg_i8_drop(*M);
-            any = true;
-        }
-    return any;
+        else if (in_use)
+            M->i8_wanted = true;
+    }
+    if (in_use)
+        g_i8_given.wait(lk, [] {
+            for (XgTileMatrix *M : xg_i8_list())
+                if (M->i8_wanted) return false;
+            return true;
+        });
+    return !held.empty();
 }
 
 /* Whether the planes of the factor (inverse: of its inverse too) belong to the

@@ -53,9 +53,10 @@ struct XgPart {
 };
 cudaError_t xg_alloc_parts(const XgPart *parts, int n, bool take_back = true);
 
-/* cudaMalloc that gives the digit planes of idle matrices back to the device
- * (XgTileMatrix::i8, a cache) before it reports that there is no memory; *p is
- * null then and no error is left behind */
+/* cudaMalloc that gives the digit planes (XgTileMatrix::i8, a cache) back to the
+ * device before it reports that there is no memory: those of idle matrices, then
+ * those of matrices in a call of another thread, when it ends.  *p is null on
+ * failure and no error is left behind.  Not for a thread that holds an XgI8Use. */
 cudaError_t xg_malloc_bytes(void **p, size_t bytes);
 template <class T> cudaError_t xg_malloc(T **p, size_t bytes) { return xg_malloc_bytes((void **)p, bytes); }
 
@@ -72,16 +73,18 @@ struct XgTileMatrix {
     int *dag = nullptr;
     /* seven-digit planes: large FP64 factorisations on the INT8 tensor cores.
      * Kept between calls; any allocation of the library that finds no memory takes
-     * them, unless a call is using them (XgI8Use), and the next call asks again. */
+     * them, from a matrix in a call (XgI8Use) when that ends, and the next call
+     * asks again. */
     XgSliced *i8 = nullptr;
     int i8_users = 0;
+    bool i8_wanted = false; /* by an allocation that waits for them */
     bool i8_scale = false; /* this call's variances suit them */
     bool i8_factor = false; /* the last factorisation went through them (they hold L) */
     double *tab = nullptr; /* element tables of the current parameters (xg_matern_tab.cuh) */
 };
 
 /* For as long as a call with the parameters p may use M's digit planes:
- * nothing takes them back */
+ * they stay, and no xg_malloc in this thread */
 struct XgI8Use {
     XgTileMatrix &M;
     XgI8Use(XgTileMatrix &m, const XgMaternParams &p);

@@ -226,3 +226,47 @@ def test_assessment(gpu, ora, kernel):
     a, b = [gpu.mloe_mmom_host(x[:m], y[:m], x[m:], y[m:], truth, est, kernel=kernel, ts=t) for t in (512, 128)]
     assert np.abs(a[2][:, :4] - b[2][:, :4]).max() < 1e-9 * truth[0]
     assert abs(a[0] - b[0]) < 1e-8 and abs(a[1] - b[1]) < 1e-8
+
+
+def test_planes_in_use_by_other_threads_make_room_too(gpu, ora):
+    """Two threads evaluate without a pause while a third opens sessions that
+    the device has no memory for: it gets the planes when a call ends, and the
+    evaluations stay right throughout (the file's bars: some run without)."""
+    import threading
+
+    theta, k = [1.0, 0.1, 0.5], 6000
+    x, y = ora.generate_xy_loc(9000, 3)
+    z = np.random.default_rng(1).standard_normal(9000)
+    sessions, ref = [], []
+    for n in (9000, 8000):
+        s = gpu.Session(x[:n], y[:n], dts=512)
+        s.set_data(z=z[:n])
+        sessions.append(s)
+        ref.append(s.loglik(theta))
+    with gpu.Session(x[:k], y[:k], dts=256) as t:
+        t.set_data(z=z[:k])
+        want = t.loglik(theta)
+    got, stop = [[], []], threading.Event()
+
+    def evaluate(i):
+        while not stop.is_set():
+            got[i].append(sessions[i].loglik(theta))
+
+    with _Full(100 << 20):
+        threads = [threading.Thread(target=evaluate, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        try:
+            for _ in range(5):
+                with gpu.Session(x[:k], y[:k], dts=256) as t:
+                    t.set_data(z=z[:k])
+                    assert t.loglik(theta) == want
+        finally:
+            stop.set()
+            for t in threads:
+                t.join()
+    for i in range(2):
+        assert len(got[i]) > 0
+        assert np.abs(np.array(got[i]) / ref[i] - 1).max() < 2e-12
+        assert sessions[i].loglik(theta) == ref[i]
+        sessions[i].close()
